@@ -86,6 +86,55 @@ gr_status get_jump_polys(int dev, int64_t J, int delta, int need, const uint64_t
   return GR_OK;
 }
 
+// Scratch that calls take and give back in stream order, from a pool of the
+// library's own per device: the default pool returns its memory to the driver
+// at every synchronisation, and a call that follows one then pays for mapping
+// it again (rejection call of 10^6 doubles: 0.69 ms back to back, 0.81 ms when
+// each was waited for).  This pool keeps at most kScratchKeep bytes across
+// synchronisations and gives all of it back with the device's last engine.
+constexpr uint64_t kScratchKeep = (uint64_t)1 << 30;
+struct ScratchPools {
+  std::mutex mu;
+  std::map<int, std::pair<cudaMemPool_t, int>> tab;  // device -> pool, engines alive
+};
+ScratchPools& scratch_pools() {
+  static ScratchPools p;
+  return p;
+}
+void scratch_engine(int dev, int delta) {
+  ScratchPools& sp = scratch_pools();
+  std::lock_guard<std::mutex> lk(sp.mu);
+  auto& e = sp.tab[dev];
+  e.second += delta;
+  if (e.second <= 0 && e.first) cudaMemPoolTrimTo(e.first, 0);
+}
+cudaError_t scratch_alloc(void** p, size_t bytes, int dev, cudaStream_t s) {
+  cudaMemPool_t pool = nullptr;
+  {
+    ScratchPools& sp = scratch_pools();
+    std::lock_guard<std::mutex> lk(sp.mu);
+    auto& e = sp.tab[dev];
+    if (!e.first) {
+      cudaMemPoolProps props{};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      cudaMemPool_t made = nullptr;
+      cudaError_t err = cudaMemPoolCreate(&made, &props);
+      if (err != cudaSuccess) return err;
+      uint64_t keep = kScratchKeep;
+      err = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
+      if (err != cudaSuccess) {
+        cudaMemPoolDestroy(made);
+        return err;
+      }
+      e.first = made;
+    }
+    pool = e.first;
+  }
+  return cudaMallocFromPoolAsync(p, bytes, pool, s);
+}
+
 }  // namespace
 
 struct gr_engine {
@@ -171,6 +220,7 @@ gr_status gr_engine_create(gr_engine** out, uint64_t seed, int32_t lanes, int32_
     delete e;
     return cuda_fail(err, "seed kernel");
   }
+  scratch_engine(e->device, 1);
   *out = e;
   return GR_OK;
 }
@@ -183,6 +233,7 @@ gr_status gr_engine_destroy(gr_engine* e) {
   cudaFree(e->snap);
   cudaFree(e->scratch_gen);
   cudaFree(e->tailw);
+  scratch_engine(e->device, -1);
   delete e;
   return GR_OK;
 }
@@ -550,15 +601,10 @@ Family family_of(const DistParams& dp) {
   return Family::Unsupported;
 }
 
-// Sets up prefix / jump windows for an S-segment call; exponents s*J - delta.
-gr_status prepare_segments(gr_engine* e, Plan& p, int S, int64_t J, int delta, cudaStream_t stream) {
-  p.S = S;
-  p.J = J;
-  if (S <= 1) return GR_OK;
-  if (!e->prefix) {
-    GR_CUDA(cudaMalloc(&e->prefix, sizeof(uint64_t) * (size_t)kPrefixLen * kLanes * (size_t)e->K));
-    GR_CUDA(cudaMalloc(&e->snap, sizeof(CallSnap) * (size_t)e->K));
-  }
+// Room for the prefix and for the windows of an S-segment call.
+gr_status reserve_windows(gr_engine* e, int S) {
+  if (!e->prefix) GR_CUDA(cudaMalloc(&e->prefix, sizeof(uint64_t) * (size_t)kPrefixLen * kLanes * (size_t)e->K));
+  if (!e->snap) GR_CUDA(cudaMalloc(&e->snap, sizeof(CallSnap) * (size_t)e->K));
   const size_t need = (size_t)e->K * (S - 1) * kLanes * kN;
   if (e->segwin_words < need) {
     cudaFree(e->segwin);
@@ -566,13 +612,150 @@ gr_status prepare_segments(gr_engine* e, Plan& p, int S, int64_t J, int delta, c
     GR_CUDA(cudaMalloc(&e->segwin, sizeof(uint64_t) * need));
     e->segwin_words = need;
   }
+  return GR_OK;
+}
+
+// Sets up prefix / jump windows for an S-segment call; exponents s*J - delta.
+gr_status prepare_segments(gr_engine* e, Plan& p, int S, int64_t J, int delta, cudaStream_t stream) {
+  p.S = S;
+  p.J = J;
+  if (S <= 1) return GR_OK;
+  gr_status st = reserve_windows(e, S);
+  if (st != GR_OK) return st;
   const uint64_t* polys = nullptr;
-  gr_status st = get_jump_polys(e->device, J, delta, S - 1, &polys);
+  st = get_jump_polys(e->device, J, delta, S - 1, &polys);
   if (st != GR_OK) return st;
   GR_CUDA(launch_prefix(e->st, p.gen, e->K, e->prefix, e->snap, stream));
   GR_CUDA(launch_jump(e->prefix, polys, e->K, S, e->segwin, stream));
   p.segwin = e->segwin;
   p.prefix = e->prefix;
+  return GR_OK;
+}
+
+// Calls on few engines: the raw words of every engine are made in memory
+// first (launch_words, S jump-ahead segments per engine when that is shorter
+// than making them in a row), and the transforms then read them on the whole
+// GPU.  A scratch buffer holds at most kWordsCap packets per engine set.
+constexpr int64_t kWordsCap = (int64_t)1 << 22;  // packets of all engines (128 MB: about one L2)
+
+// Segments for n packets per engine.  In a row a lane makes 156 words in
+// about 16 ns; a segment more costs the jump kernel about 0.25 us of the whole
+// GPU per engine, and the prefix and its launches about 10 us once.
+void plan_words(int K, int64_t n, int& S, int64_t& J) {
+  S = 1;
+  J = n + (n & 1);
+  double best = (double)n * 0.1;  // ns
+  for (int m = 12; m <= 24; ++m) {
+    const int64_t j = (int64_t)1 << m;
+    const int64_t segs = (n + j - 1) / j;
+    if (segs < 2) break;
+    if (segs > 128 || segs * K > 1024) continue;
+    const double cost = (double)j * 0.1 + (double)(segs - 1) * K * 250.0 + 10000.0;
+    if (cost < best) {
+      best = cost;
+      S = (int)segs;
+      J = j;
+    }
+  }
+}
+
+// Makes n packets of raw words per engine in new scratch (freed by the caller
+// in stream order) and fills the plan's words fields; the engine's state is
+// left as it is.  first: also snapshot the caches.  *got = false: no scratch
+// memory, nothing was launched, and the caller takes the path that needs none.
+gr_status make_words(gr_engine* e, Plan& p, int64_t n, bool first, void** buf, bool* got, cudaStream_t stream) {
+  n += n & 1;
+  const int64_t stride = kN + n;
+  *got = false;
+  if (!e->snap) GR_CUDA(cudaMalloc(&e->snap, sizeof(CallSnap) * (size_t)e->K));
+  WordsArgs a{};
+  plan_words(e->K, n, a.S, a.J);
+  if (a.S > 1) {
+    gr_status st = reserve_windows(e, a.S);
+    if (st != GR_OK) return st;
+    const uint64_t* polys = nullptr;
+    st = get_jump_polys(e->device, a.J, 0, a.S - 1, &polys);
+    if (st != GR_OK) return st;
+    p.segwin = polys;  // until the launch below
+  }
+  const cudaError_t err = scratch_alloc(buf, sizeof(uint64_t) * (size_t)e->K * kLanes * (size_t)stride, e->device, stream);
+  if (err == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return GR_OK;
+  }
+  if (err != cudaSuccess) return cuda_fail(err, "scratch memory");
+  a.words = static_cast<uint64_t*>(*buf);
+  a.stride = stride;
+  a.n = n;
+  a.snap = first ? e->snap : nullptr;
+  cudaError_t le = cudaSuccess;
+  if (a.S > 1) {
+    le = launch_prefix(e->st, p.gen, e->K, e->prefix, first ? e->snap : nullptr, stream);
+    if (le == cudaSuccess) le = launch_jump(e->prefix, p.segwin, e->K, a.S, e->segwin, stream);
+    a.segwin = e->segwin;
+    a.snap = nullptr;
+  }
+  if (le == cudaSuccess) le = launch_words(e->st, p.gen, e->K, a, stream);
+  p.segwin = nullptr;
+  if (le != cudaSuccess) {
+    cudaFreeAsync(*buf, stream);
+    return cuda_fail(le, "raw word kernels");
+  }
+  p.words = a.words;
+  p.wstride = stride;
+  p.wcount = n;
+  *got = true;
+  return GR_OK;
+}
+
+// Packets per engine above which a fixed-draw call on few engines goes through
+// words in memory.  One CTA per engine spends 0.9 us (bit conversions), 3 us
+// (float log, sincos) or 25 us (their double forms) per 312 packets; the
+// second launch and the scratch take about 6 us.  One engine, 2 048 packets:
+// float uniform 11.8 us fused and 13.6 us through memory, float normal 21.4
+// and 14.7, double normal (4 096 packets) 152 and 21; 131 072 values: 43 and
+// 17, 118 and 18, 1146 and 28.
+int64_t words_from(const DistParams& dp) {
+  const int k = dp.kind >= kVecBase ? dp.kind - kVecBase : dp.kind;
+  const bool light = k == kRawKind || k == kRawLane0Kind || k == GR_UNIFORM_REAL || k == GR_UNIFORM_REAL2 ||
+                     k == GR_BALANCED || k == GR_BALANCED2 || k == GR_BERNOULLI || k == kBernoulliVKind ||
+                     k == GR_RANDBITS || k == GR_UNIFORM_INT;
+  if (light) return 2560;
+  return dp.dtype == GR_F64 ? 156 : 624;
+}
+
+// A fixed-draw kind (launch_direct) over `packets` packets per engine at
+// most, whole units of ppu packets.
+gr_status run_fixed(gr_engine* e, Plan p, const DistParams& dp, int64_t packets, int ppu, cudaStream_t stream,
+                    const char* what) {
+  if (e->K < 128 && packets > words_from(dp) && p.out) {
+    const int64_t chunk = std::max<int64_t>(kWordsCap / e->K & ~(int64_t)1, 2);
+    bool done = true;
+    for (int64_t at = 0; at < packets; at += chunk) {
+      void* buf = nullptr;
+      bool got = false;
+      gr_status st = make_words(e, p, std::min(chunk, packets - at), at == 0, &buf, &got, stream);
+      if (st != GR_OK) return st;
+      if (!got && at == 0) {
+        done = false;
+        break;
+      }
+      if (!got) return fail(GR_ERR_CUDA, "out of memory for the call's scratch");
+      p.wbase = at;
+      const cudaError_t err = launch_direct(p, dp, e->snap, stream);
+      cudaFreeAsync(buf, stream);
+      if (err != cudaSuccess) return cuda_fail(err, what);
+    }
+    if (done) return GR_OK;
+    p.words = nullptr;
+  }
+  int S;
+  int64_t J;
+  plan_segments(e, packets, ppu, S, J);
+  gr_status st = prepare_segments(e, p, S, J, 0, stream);
+  if (st != GR_OK) return st;
+  const cudaError_t err = launch_direct(p, dp, e->snap, stream);
+  if (err != cudaSuccess) return cuda_fail(err, what);
   return GR_OK;
 }
 
@@ -739,14 +922,7 @@ gr_status run_two_lane(gr_engine* e, const DistParams& dp0, void* out, size_t n,
   p.gran_rem = granules % e->K;
   p.out = out;
   const int64_t packets_max = p.gran_per_k + (p.gran_rem ? 1 : 0);
-  int S;
-  int64_t J;
-  plan_segments(e, packets_max, 1, S, J);
-  gr_status st = prepare_segments(e, p, S, J, 0, stream);
-  if (st != GR_OK) return st;
-  cudaError_t err = launch_direct(p, dp, e->snap, stream);
-  if (err != cudaSuccess) return cuda_fail(err, "2-lane sampling kernel");
-  return GR_OK;
+  return run_fixed(e, p, dp, packets_max, 1, stream, "2-lane sampling kernel");
 }
 
 gr_status run_call(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, size_t n, cudaStream_t stream) {
@@ -807,14 +983,7 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
     const int ppu = kind_packets_per_unit(dp.kind, dp.dtype);
     int64_t packets_max = (nk_max + opp - 1) / opp;
     if (ppu == 2) packets_max += packets_max & 1;
-    int S;
-    int64_t J;
-    plan_segments(e, packets_max, ppu, S, J);
-    gr_status st = prepare_segments(e, p, S, J, 0, stream);
-    if (st != GR_OK) return st;
-    cudaError_t err = launch_direct(p, dp, e->snap, stream);
-    if (err != cudaSuccess) return cuda_fail(err, "sampling kernel");
-    return GR_OK;
+    return run_fixed(e, p, dp, packets_max, ppu, stream, "sampling kernel");
   }
 
   if (fam == Family::Reject) {
@@ -1649,17 +1818,8 @@ namespace gr {
 // windows for up to max_segments segments, the temporary-generator caches), so
 // that later calls on this engine allocate nothing.
 gr_status engine_reserve(gr_engine* e, int max_segments) {
-  if (!e->prefix) {
-    GR_CUDA(cudaMalloc(&e->prefix, sizeof(uint64_t) * (size_t)kPrefixLen * kLanes * (size_t)e->K));
-    GR_CUDA(cudaMalloc(&e->snap, sizeof(CallSnap) * (size_t)e->K));
-  }
-  const size_t need = (size_t)e->K * (size_t)std::max(max_segments - 1, 1) * kLanes * kN;
-  if (e->segwin_words < need) {
-    cudaFree(e->segwin);
-    e->segwin = nullptr;
-    GR_CUDA(cudaMalloc(&e->segwin, sizeof(uint64_t) * need));
-    e->segwin_words = need;
-  }
+  gr_status st = reserve_windows(e, std::max(max_segments, 2));
+  if (st != GR_OK) return st;
   if (!e->scratch_gen) GR_CUDA(cudaMalloc(&e->scratch_gen, sizeof(GenState) * (size_t)e->K));
   return GR_OK;
 }
@@ -1682,14 +1842,7 @@ gr_status draw_first_words(gr_engine* e, uint64_t* out, int64_t per_sample, int6
   p.gran_rem = samples % e->K;
   p.out = out;
   const int64_t packets_max = (p.gran_per_k + (p.gran_rem ? 1 : 0)) * per_sample;
-  int S;
-  int64_t J;
-  plan_segments(e, packets_max, 1, S, J);
-  gr_status st = prepare_segments(e, p, S, J, 0, s);
-  if (st != GR_OK) return st;
-  const cudaError_t err = launch_direct(p, dp, e->snap, s);
-  if (err != cudaSuccess) return cuda_fail(err, "scalar draws");
-  return GR_OK;
+  return run_fixed(e, p, dp, packets_max, 1, s, "scalar draws");
 }
 
 }  // namespace gr

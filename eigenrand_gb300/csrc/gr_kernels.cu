@@ -64,103 +64,263 @@ cudaError_t launch_seed(EngState* st, int K, uint64_t seed, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// ---------------------------------------------------------------- prefix
-// prefix[k][l][0..312) = current window, then the raw recurrence
-// x[i+312] = twist(x[i], x[i+1], x[i+156]) in chunks of 156 independent words.
-// Also snapshots the caches the call starts from (block lane 0).
-__global__ void __launch_bounds__(160) k_prefix(const EngState* st, uint64_t* prefix, CallSnap* snap,
-                                                const GenState* gen) {
-  __shared__ uint64_t ring[2 * kN];
-  const int k = blockIdx.x / kLanes, l = blockIdx.x % kLanes;
-  const int tid = threadIdx.x;
-  uint64_t* out = prefix + ((size_t)k * kLanes + l) * kPrefixLen;
-  for (int i = tid; i < kN; i += blockDim.x) {
-    uint64_t v = st[k].win[l][i];
-    ring[i] = v;
-    out[i] = v;
-  }
-  if (l == 0 && tid == 0) {
-    snap[k].half_valid = st[k].half_valid;
-    for (int q = 0; q < kLanes; ++q) snap[k].half_cache[q] = st[k].half_cache[q];
-    snap[k].gen_valid = gen ? gen[k].s[0].valid : 0;
-    for (int q = 0; q < 16; ++q) snap[k].gen_cache[q] = gen ? gen[k].s[0].cache[q] : 0u;
-  }
-  __syncthreads();
-  for (int base = 0; base + kN < kPrefixLen; base += kM) {
-    if (tid < kM) {
-      int i = base + tid;  // computes x[i+312]
-      uint64_t a = ring[i % (2 * kN)], b = ring[(i + 1) % (2 * kN)], c = ring[(i + kM) % (2 * kN)];
-      uint64_t v = twist1(a, b, c);
-      ring[(i + kN) % (2 * kN)] = v;
-      out[i + kN] = v;
+// ---------------------------------------------------------------- word streams
+// The recurrence x[i+312] = twist(x[i], x[i+1], x[i+156]) gives 156 words at a
+// time (a phase).  A word's own two predecessors x[i], x[i+156] are the words
+// the same thread made two phases and one phase before, so they stay in
+// registers and only x[i+1], two phases old, comes from the next lane by a
+// shuffle: no shared memory and no barrier between phases.
+__device__ __forceinline__ uint64_t shfl64(uint64_t v, int src) {
+  return ((uint64_t)__shfl_sync(0xffffffffu, (uint32_t)(v >> 32), src) << 32) |
+         (uint64_t)__shfl_sync(0xffffffffu, (uint32_t)v, src);
+}
+
+// One MT19937-64 lane on four warps of a CTA, for calls with too few lanes to
+// fill the GPU: warp w holds the phase's words [40 w, 40 w + 64), two per
+// thread, of which the first 40 (36) are its own and the rest a halo that
+// repeats the next warp's work.  The halo loses one word every two phases (its
+// last word misses its neighbour), so the warps exchange words only every 48
+// phases.  Bound by issue: 24 instructions per warp and phase.  Measured
+// against the one-barrier-per-phase form (156 threads, three shared-memory
+// reads per word): 20 280 words in 4.5 us against 17 us.
+// win: the CTA's 312-word window in shared memory (loaded, all threads past
+// a barrier); put(i, v0, v1) stores words i, i + 1 (i even) after the window.
+constexpr int kWideThreads = 128;
+template <class Put>
+__device__ __forceinline__ void lane_words_wide(uint64_t* win, int64_t n, Put&& put) {
+  const int w = threadIdx.x >> 5, q = threadIdx.x & 31;
+  const int i0 = 40 * w + 2 * q;
+  const bool own = q < 20 && i0 < kM;
+  const int src = q < 31 ? q + 1 : 31;
+  for (int64_t base = 0; base < n;) {
+    uint64_t a[2], c[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int i = i0 + j;
+      a[j] = win[i];
+      // words past the window (the last warp's halo) are made here
+      c[j] = i < kM ? win[kM + i] : twist1(win[i - kM], win[i - kM + 1], win[i]);
+    }
+    const int phases = (int)min((int64_t)48, (n - base + kM - 1) / kM);
+    for (int ph = 0; ph < phases; ++ph) {
+      const uint64_t nb = shfl64(a[0], src);
+      const uint64_t v0 = twist1(a[0], a[1], c[0]), v1 = twist1(a[1], nb, c[1]);
+      const int64_t i = base + i0;
+      if (own && i < n) put(i, v0, v1);
+      a[0] = c[0];
+      a[1] = c[1];
+      c[0] = v0;
+      c[1] = v1;
+      base += kM;
+    }
+    if (base >= n) break;
+    __syncthreads();
+    if (own) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        win[i0 + j] = a[j];
+        win[kM + i0 + j] = c[j];
+      }
     }
     __syncthreads();
   }
 }
 
-// ---------------------------------------------------------------- jump
-// One CTA per (engine k, segment s >= 1, lane l).  16 warps; warp g covers
-// polynomial terms i in [1248 g, 1248 g + 1248), lane q of the warp covers
-// output words j in [10 q, 10 q + 10).  Per 8 terms a thread loads 8 new
-// prefix words into a sliding register window and XORs them into its 10
-// accumulators under the (warp-uniform) coefficient bits.
-constexpr int kJumpThreads = 512;
-constexpr int kJumpPer = 1248;  // terms per warp (16 * 1248 = 19968 >= 19937)
+// prefix[k][l][0..312) = current window, then the lane's next 20 280 raw words.
+// Also snapshots the caches the call starts from (lane 0's CTA).
+__device__ __forceinline__ void snap_caches(const EngState& st, const GenState* gen, CallSnap& snap) {
+  snap.half_valid = st.half_valid;
+  for (int q = 0; q < kLanes; ++q) snap.half_cache[q] = st.half_cache[q];
+  snap.gen_valid = gen ? gen->s[0].valid : 0;
+  for (int q = 0; q < 16; ++q) snap.gen_cache[q] = gen ? gen->s[0].cache[q] : 0u;
+}
 
-__global__ void __launch_bounds__(kJumpThreads, 1)
-    k_jump(const uint64_t* prefix, const uint64_t* polys, int S, uint64_t* segwin) {
-  extern __shared__ uint64_t sm[];
-  uint64_t* px = sm;                  // kPrefixLen words
-  uint64_t* cf = sm + kPrefixLen;     // 312 coefficient words
+__global__ void __launch_bounds__(kWideThreads) k_prefix(const EngState* st, uint64_t* prefix, CallSnap* snap,
+                                                         const GenState* gen) {
+  __shared__ uint64_t win[kN];
+  const int k = blockIdx.x / kLanes, l = blockIdx.x % kLanes;
+  uint64_t* out = prefix + ((size_t)k * kLanes + l) * kPrefixLen;
+  for (int i = threadIdx.x; i < kN; i += kWideThreads) out[i] = win[i] = st[k].win[l][i];
+  if (snap && l == 0 && threadIdx.x == 0) snap_caches(st[k], gen ? gen + k : nullptr, snap[k]);
+  __syncthreads();
+  lane_words_wide(win, kPrefixLen - kN, [&](int64_t i, uint64_t v0, uint64_t v1) {
+    *reinterpret_cast<ulonglong2*>(out + kN + i) = make_ulonglong2(v0, v1);
+  });
+}
+
+// Raw words of a call into memory: words[(k * 4 + l) * stride + 312 + i] =
+// raw word i of lane l of engine k (the window before them at [0, 312)), i <
+// n, segment s of an engine making words [s J, (s + 1) J) from its jump
+// window.  The transforms then run over the whole GPU whatever the number of
+// engines (k_xform below, gr_chain.cu).  k_words_wide: one CTA per lane and
+// segment; k_words_warp: one warp per lane and segment (26 threads of 6
+// consecutive words per phase), 28% fewer instructions per word, where there
+// are enough lanes to fill the GPU.
+__global__ void __launch_bounds__(kWideThreads) k_words_wide(const EngState* st, const GenState* gen, WordsArgs a) {
+  __shared__ uint64_t win[kN];
+  const int l = blockIdx.x % kLanes, s = (blockIdx.x / kLanes) % a.S, k = blockIdx.x / (kLanes * a.S);
+  uint64_t* out = a.words + ((size_t)k * kLanes + l) * a.stride;
+  const uint64_t* src = s == 0 ? st[k].win[l] : a.segwin + (((size_t)k * (a.S - 1) + (s - 1)) * kLanes + l) * kN;
+  for (int i = threadIdx.x; i < kN; i += kWideThreads) {
+    win[i] = src[i];
+    if (s == 0) out[i] = src[i];
+  }
+  if (a.snap && s == 0 && l == 0 && threadIdx.x == 0) snap_caches(st[k], gen ? gen + k : nullptr, a.snap[k]);
+  __syncthreads();
+  const int64_t i0 = (int64_t)s * a.J;
+  uint64_t* o = out + kN + i0;
+  lane_words_wide(win, min(a.J, a.n - i0), [&](int64_t i, uint64_t v0, uint64_t v1) {
+    *reinterpret_cast<ulonglong2*>(o + i) = make_ulonglong2(v0, v1);
+  });
+}
+
+__global__ void __launch_bounds__(32 * kLanes) k_words_warp(const EngState* st, const GenState* gen, WordsArgs a) {
+  const int l = threadIdx.x >> 5, q = threadIdx.x & 31;
+  const int s = blockIdx.x % a.S, k = blockIdx.x / a.S;
+  uint64_t* out = a.words + ((size_t)k * kLanes + l) * a.stride;
+  const uint64_t* src = s == 0 ? st[k].win[l] : a.segwin + (((size_t)k * (a.S - 1) + (s - 1)) * kLanes + l) * kN;
+  if (s == 0)
+    for (int i = q; i < kN; i += 32) out[i] = src[i];
+  if (a.snap && s == 0 && threadIdx.x == 0) snap_caches(st[k], gen ? gen + k : nullptr, a.snap[k]);
+  const int qq = min(q, 25);
+  uint64_t x[6], c[6];
+#pragma unroll
+  for (int j = 0; j < 6; ++j) {
+    x[j] = src[6 * qq + j];
+    c[j] = src[kM + 6 * qq + j];
+  }
+  const int64_t i0 = (int64_t)s * a.J, n = min(a.J, a.n - i0);
+  uint64_t* o = out + kN + i0;
+  const int nsrc = q == 25 ? 0 : min(q + 1, 31);
+  for (int64_t base = 0; base < n; base += kM) {
+    // the last thread's neighbour is the first word of the next phase, one phase old
+    const uint64_t nb = shfl64(q == 0 ? c[0] : x[0], nsrc);
+    uint64_t v[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) v[j] = twist1(x[j], j < 5 ? x[j + 1] : nb, c[j]);
+    const int64_t i = base + 6 * q;
+    if (q < 26) {
+#pragma unroll
+      for (int j = 0; j < 6; j += 2)
+        if (i + j < n) *reinterpret_cast<ulonglong2*>(o + i + j) = make_ulonglong2(v[j], v[j + 1]);
+    }
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+      x[j] = c[j];
+      c[j] = v[j];
+    }
+  }
+}
+
+cudaError_t launch_words(const EngState* st, const GenState* gen, int K, const WordsArgs& a, cudaStream_t s) {
+  // four lanes of one warp each per CTA: the narrow form fills the SMs'
+  // schedulers from about one CTA per SM on
+  if ((int64_t)K * a.S >= 256) k_words_warp<<<K * a.S, 32 * kLanes, 0, s>>>(st, gen, a);
+  else k_words_wide<<<K * a.S * kLanes, kWideThreads, 0, s>>>(st, gen, a);
+  return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------- jump
+// segwin[k][s1][l][j] = XOR over the polynomial's set coefficients i of
+// prefix word i + j.  One CTA per (engine, segment s >= 1, lane, quarter of the
+// terms); its warps split the quarter, lane q of a warp covers output words
+// [11 q, 11 q + 11) (an odd stride: the 8-byte shared-memory reads are free of
+// bank conflicts).  A thread slides a register window over the prefix words;
+// four coefficients at a time, the same for the whole warp, pick one of 16
+// unrolled cases, in which three-input XORs take 1.25 operations per 32-bit
+// word on average where one conditional XOR per term takes 2.  Quarters meet
+// by atomic XOR (segwin zeroed beforehand).  Bound by issue.
+constexpr int kJumpThreads = 256;
+constexpr int kJumpParts = 4;
+constexpr int kJumpPer = 19968 / (kJumpParts * (kJumpThreads / 32));  // 624 terms per warp
+constexpr int kJumpOut = 11;
+constexpr int kJumpSpan = kJumpPer * (kJumpThreads / 32);             // terms per CTA
+constexpr int kJumpLoad = kJumpSpan + 32 * kJumpOut + 8;              // prefix words a CTA reads
+
+template <int N>
+__device__ __forceinline__ void xor_nibble(uint64_t (&acc)[kJumpOut], const uint64_t* w) {
+#pragma unroll
+  for (int j = 0; j < kJumpOut; ++j) {
+    uint64_t v = acc[j];
+    if (N & 1) v ^= w[j];
+    if (N & 2) v ^= w[j + 1];
+    if (N & 4) v ^= w[j + 2];
+    if (N & 8) v ^= w[j + 3];
+    acc[j] = v;
+  }
+}
+
+__device__ __forceinline__ void xor_terms4(uint64_t (&acc)[kJumpOut], const uint64_t* w, uint32_t c) {
+  switch (c) {
+    case 1: xor_nibble<1>(acc, w); break;
+    case 2: xor_nibble<2>(acc, w); break;
+    case 3: xor_nibble<3>(acc, w); break;
+    case 4: xor_nibble<4>(acc, w); break;
+    case 5: xor_nibble<5>(acc, w); break;
+    case 6: xor_nibble<6>(acc, w); break;
+    case 7: xor_nibble<7>(acc, w); break;
+    case 8: xor_nibble<8>(acc, w); break;
+    case 9: xor_nibble<9>(acc, w); break;
+    case 10: xor_nibble<10>(acc, w); break;
+    case 11: xor_nibble<11>(acc, w); break;
+    case 12: xor_nibble<12>(acc, w); break;
+    case 13: xor_nibble<13>(acc, w); break;
+    case 14: xor_nibble<14>(acc, w); break;
+    case 15: xor_nibble<15>(acc, w); break;
+    default: break;
+  }
+}
+
+__global__ void __launch_bounds__(kJumpThreads, 4)
+    k_jump(const uint64_t* prefix, const uint64_t* polys, int S, unsigned long long* segwin) {
+  __shared__ uint64_t px[kJumpLoad];
+  __shared__ uint64_t cf[kJumpSpan / 64];
   const int nseg = S - 1;
-  const int l = blockIdx.x % kLanes;
-  const int s1 = (blockIdx.x / kLanes) % nseg;  // segment - 1
-  const int k = blockIdx.x / (kLanes * nseg);
+  const int part = blockIdx.x % kJumpParts;
+  const int l = (blockIdx.x / kJumpParts) % kLanes;
+  const int s1 = (blockIdx.x / (kJumpParts * kLanes)) % nseg;  // segment - 1
+  const int k = blockIdx.x / (kJumpParts * kLanes * nseg);
   const int tid = threadIdx.x;
-  const uint64_t* src = prefix + ((size_t)k * kLanes + l) * kPrefixLen;
-  for (int i = tid; i < kPrefixLen / 2; i += kJumpThreads)
-    reinterpret_cast<uint4*>(px)[i] = reinterpret_cast<const uint4*>(src)[i];
-  for (int i = tid; i < kN; i += kJumpThreads) cf[i] = polys[(size_t)s1 * kN + i];
+  const int t0 = part * kJumpSpan;
+  const uint64_t* src = prefix + ((size_t)k * kLanes + l) * kPrefixLen + t0;
+  for (int i = tid; i < kJumpLoad; i += kJumpThreads) px[i] = t0 + i < kPrefixLen ? src[i] : 0;
+  for (int i = tid; i < kJumpSpan / 64; i += kJumpThreads) cf[i] = polys[(size_t)s1 * kN + t0 / 64 + i];
   __syncthreads();
 
   const int g = tid >> 5, q = tid & 31;
-  const int j0 = 10 * q;
-  uint64_t acc[10];
-#pragma unroll
-  for (int jj = 0; jj < 10; ++jj) acc[jj] = 0;
-  uint64_t w[17];
   const int ibeg = g * kJumpPer;
+  const uint64_t* p = px + ibeg + kJumpOut * q;
+  uint64_t acc[kJumpOut];
 #pragma unroll
-  for (int m = 0; m < 9; ++m) w[m] = px[ibeg + j0 + m];
-  for (int i0 = ibeg; i0 < ibeg + kJumpPer; i0 += 8) {
+  for (int j = 0; j < kJumpOut; ++j) acc[j] = 0;
+  uint64_t w[kJumpOut + 7];
 #pragma unroll
-    for (int m = 0; m < 8; ++m) w[9 + m] = px[i0 + j0 + 9 + m];
-    const uint32_t cb = (uint32_t)(cf[i0 >> 6] >> (i0 & 63)) & 0xffu;
-    if (cb) {
+  for (int m = 0; m < kJumpOut - 1; ++m) w[m] = p[m];
+#pragma unroll 1
+  for (int i0 = 0; i0 < kJumpPer; i0 += 8) {
 #pragma unroll
-      for (int ii = 0; ii < 8; ++ii) {
-        if (cb & (1u << ii)) {
+    for (int m = 0; m < 8; ++m) w[kJumpOut - 1 + m] = p[i0 + kJumpOut - 1 + m];
+    const uint32_t cb = (uint32_t)(cf[(ibeg + i0) >> 6] >> ((ibeg + i0) & 63)) & 0xffu;
+    xor_terms4(acc, w, cb & 15u);
+    xor_terms4(acc, w + 4, cb >> 4);
 #pragma unroll
-          for (int jj = 0; jj < 10; ++jj) acc[jj] ^= w[ii + jj];
-        }
-      }
-    }
-#pragma unroll
-    for (int m = 0; m < 9; ++m) w[m] = w[m + 8];
+    for (int m = 0; m < kJumpOut - 1; ++m) w[m] = w[m + 8];
   }
   __syncthreads();
-  uint64_t* red = sm;  // reuse: [16][320]
+  uint64_t* red = px;  // reuse: [8][352]
 #pragma unroll
-  for (int jj = 0; jj < 10; ++jj) red[g * 320 + j0 + jj] = acc[jj];
+  for (int j = 0; j < kJumpOut; ++j) red[g * (32 * kJumpOut) + kJumpOut * q + j] = acc[j];
   __syncthreads();
-  uint64_t* dst = segwin + (((size_t)k * nseg + s1) * kLanes + l) * kN;
+  unsigned long long* dst = segwin + (((size_t)k * nseg + s1) * kLanes + l) * kN;
   for (int j = tid; j < kN; j += kJumpThreads) {
     uint64_t v = 0;
 #pragma unroll
-    for (int gg = 0; gg < 16; ++gg) v ^= red[gg * 320 + j];
-    dst[j] = v;
+    for (int gg = 0; gg < kJumpThreads / 32; ++gg) v ^= red[gg * (32 * kJumpOut) + j];
+    atomicXor(dst + j, (unsigned long long)v);
   }
 }
+static_assert(kJumpSpan % 64 == 0 && kJumpPer % 8 == 0, "coefficient bytes stay within one word");
+static_assert((kJumpThreads / 32) * 32 * kJumpOut <= kJumpLoad, "the reduction reuses the prefix buffer");
 
 // ---------------------------------------------------------------- transforms
 __device__ __forceinline__ float ur_f(uint32_t x) { return u2f((x & 0x7fffffu) | (127u << 23)) - 1.0f; }
@@ -389,6 +549,214 @@ __device__ __forceinline__ void st16(void* p, uint32_t a, uint32_t b, uint32_t c
   *reinterpret_cast<uint4*>(p) = make_uint4(a, b, c, d);
 }
 
+// int32 kinds whose packets are rng.half() words leave raw words in the
+// engine's half cache; DiscreteGen caches its own computed results
+template <int MODE, int KIND>
+struct CacheUse {
+  static constexpr bool half_kind =
+      KIND == GR_RANDBITS || KIND == GR_BERNOULLI || KIND == GR_GEOMETRIC || KIND == GR_UNIFORM_INT;
+  static constexpr bool half = (MODE == M_W64) || (MODE == M_W32 && half_kind);
+  static constexpr bool gen = (MODE == M_N32) || (MODE == M_N64) || (MODE == M_W32 && KIND == GR_DISCRETE);
+};
+
+// The samples of packet pidx of a call (pk: its four tempered words), output
+// element obase + pidx * OPP on; oend: end of the engine's slice (the half of
+// a packet or unit past it goes to the cache).  Called by whole warps whose
+// lanes hold consecutive packets from an even one on: the Box-Muller kinds
+// exchange words within packet pairs.
+template <int MODE, int KIND>
+__device__ __forceinline__ void emit_packet(const uint64_t (&pk)[kLanes], const int64_t pidx, const bool valid,
+                                            const Plan& p, const DistParams& d, const int64_t obase,
+                                            const int64_t oend, EngState* st, GenState* gs) {
+  constexpr bool kHalfKind = CacheUse<MODE, KIND>::half_kind;
+  if (MODE == M_RAW) {
+    if (valid && p.out) {  // p.out == nullptr: discard
+      uint64_t* o = reinterpret_cast<uint64_t*>(p.out) + obase + pidx * 4;
+      reinterpret_cast<ulonglong2*>(o)[0] = make_ulonglong2(pk[0], pk[1]);
+      reinterpret_cast<ulonglong2*>(o)[1] = make_ulonglong2(pk[2], pk[3]);
+    }
+  } else if (MODE == M_RAW2) {
+    if (valid && p.out)
+      reinterpret_cast<ulonglong2*>(reinterpret_cast<uint64_t*>(p.out) + obase + pidx * 2)[0] =
+          make_ulonglong2(pk[0], pk[1]);
+  } else if (MODE == M_F32H) {
+    if (valid) {
+      float* o = reinterpret_cast<float*>(p.out) + obase + pidx * 4;
+      const int64_t ib = obase + pidx * 4;
+      reinterpret_cast<float4*>(o)[0] =
+          make_float4(tf32i<KIND>((uint32_t)pk[0], d, ib), tf32i<KIND>((uint32_t)(pk[0] >> 32), d, ib + 1),
+                      tf32i<KIND>((uint32_t)pk[1], d, ib + 2), tf32i<KIND>((uint32_t)(pk[1] >> 32), d, ib + 3));
+    }
+  } else if (MODE == M_F64H) {
+    if (valid) {
+      double* o = reinterpret_cast<double*>(p.out) + obase + pidx * 2;
+      const int64_t ib = obase + pidx * 2;
+      reinterpret_cast<double2*>(o)[0] = make_double2(tf64i<KIND>(pk[0], d, ib), tf64i<KIND>(pk[1], d, ib + 1));
+    }
+  } else if (MODE == M_RAW0) {
+    // a scalar draw takes the engine's whole packet and keeps its first
+    // element (StdUniformRealGen::operator(), Dists/Basic.h:533-540)
+    if (valid) reinterpret_cast<uint64_t*>(p.out)[obase / 4 + pidx] = pk[0];
+  } else if (MODE == M_F32) {
+    if (valid) {
+      float* o = reinterpret_cast<float*>(p.out) + obase + pidx * 8;
+      float v[8];
+      if (KIND == kBernoulliVKind) {
+        // BernoulliVGen<float>: p = cvttps(a * 2^31), compared signed with
+        // the masked word (Basic.h:735-745)
+        const float4* pv = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(d.vparam) + obase + pidx * 8);
+        const float4 q0 = pv[0], q1 = pv[1];
+        const float pa[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const uint32_t w = (q & 1) ? (uint32_t)(pk[q >> 1] >> 32) : (uint32_t)pk[q >> 1];
+          v[q] = ((int32_t)(w & 0x7fffffffu) < cvtt_f32(pa[q] * 2147483648.0f)) ? 1.0f : 0.0f;
+        }
+      } else {
+#pragma unroll
+        for (int l = 0; l < kLanes; ++l) {
+          v[2 * l] = tf32i<KIND>((uint32_t)pk[l], d, obase + pidx * 8 + 2 * l);
+          v[2 * l + 1] = tf32i<KIND>((uint32_t)(pk[l] >> 32), d, obase + pidx * 8 + 2 * l + 1);
+        }
+      }
+      reinterpret_cast<float4*>(o)[0] = make_float4(v[0], v[1], v[2], v[3]);
+      reinterpret_cast<float4*>(o)[1] = make_float4(v[4], v[5], v[6], v[7]);
+    }
+  } else if (MODE == M_F64) {
+    if (valid) {
+      double* o = reinterpret_cast<double*>(p.out) + obase + pidx * 4;
+      double v[4];
+#pragma unroll
+      for (int l = 0; l < kLanes; ++l) v[l] = tf64i<KIND>(pk[l], d, obase + pidx * 4 + l);
+      reinterpret_cast<double2*>(o)[0] = make_double2(v[0], v[1]);
+      reinterpret_cast<double2*>(o)[1] = make_double2(v[2], v[3]);
+    }
+  } else if (MODE == M_W32 || MODE == M_W64) {
+    if (valid) {
+      const int64_t ob = obase + pidx * 8;
+      uint32_t wd[8];
+#pragma unroll
+      for (int l = 0; l < kLanes; ++l) {
+        wd[2 * l] = (uint32_t)pk[l];
+        wd[2 * l + 1] = (uint32_t)(pk[l] >> 32);
+      }
+      const bool full = ob + 8 <= oend;
+      if (MODE == M_W32) {
+        int32_t v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = tw32<KIND>(wd[q], d);
+        int32_t* o = reinterpret_cast<int32_t*>(p.out) + ob;
+        st16(o, v[0], v[1], v[2], v[3]);
+        if (full) st16(o + 4, v[4], v[5], v[6], v[7]);
+        else if (gs || kHalfKind) {
+          // leftover half: rng.half() kinds leave raw words in the engine's
+          // half() cache; DiscreteGen caches its computed upper 4 results
+          uint32_t* cdst = kHalfKind ? st->half_cache : gs->s[0].cache;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) cdst[q] = kHalfKind ? wd[4 + q] : (uint32_t)v[4 + q];
+        }
+      } else {
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = tw64i<KIND>(wd[q], d, ob + q);
+        double* o = reinterpret_cast<double*>(p.out) + ob;
+        reinterpret_cast<double2*>(o)[0] = make_double2(v[0], v[1]);
+        reinterpret_cast<double2*>(o)[1] = make_double2(v[2], v[3]);
+        if (full) {
+#pragma unroll
+          for (int q = 4; q < 8; ++q) v[q] = tw64i<KIND>(wd[q], d, ob + q);
+          reinterpret_cast<double2*>(o)[2] = make_double2(v[4], v[5]);
+          reinterpret_cast<double2*>(o)[3] = make_double2(v[6], v[7]);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) st->half_cache[q] = wd[4 + q];
+        }
+      }
+    }
+  } else if (MODE == M_N32) {
+    // unit = packets (2j, 2j+1): u1 words in the even thread, u2 in the odd.
+    // Even thread handles lanes i = 0..3 of the unit, odd handles 4..7.
+    const bool odd = (pidx & 1);
+    uint32_t wd[8];
+#pragma unroll
+    for (int l = 0; l < kLanes; ++l) {
+      wd[2 * l] = (uint32_t)pk[l];
+      wd[2 * l + 1] = (uint32_t)(pk[l] >> 32);
+    }
+    uint32_t other[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) other[q] = __shfl_xor_sync(0xffffffffu, odd ? wd[q] : wd[4 + q], 1);
+    if (valid) {
+      const int64_t unit = pidx >> 1;
+      const int i0 = odd ? 4 : 0;
+      float sv[4], cv[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float u1 = ur_f(odd ? other[q] : wd[q]);
+        const float u2 = ur_f(odd ? wd[4 + q] : other[q]);
+        const float radius = sqrtf((float)-2 * logf_(1.0f - u1));
+        const float theta = (float)(2 * 3.1415926535897932) * u2;
+        float sn, cs;
+        sincosf_(theta, sn, cs);
+        sv[q] = radius * sn;
+        cv[q] = radius * cs;
+      }
+      const int64_t ob = obase + unit * 16;
+      float* o = reinterpret_cast<float*>(p.out) + ob;
+      reinterpret_cast<float4*>(o + i0)[0] =
+          make_float4(nscale32i<KIND>(sv[0], d, ob + i0), nscale32i<KIND>(sv[1], d, ob + i0 + 1),
+                      nscale32i<KIND>(sv[2], d, ob + i0 + 2), nscale32i<KIND>(sv[3], d, ob + i0 + 3));
+      if (ob + 16 <= oend) {
+        reinterpret_cast<float4*>(o + 8 + i0)[0] =
+            make_float4(nscale32i<KIND>(cv[0], d, ob + 8 + i0), nscale32i<KIND>(cv[1], d, ob + 9 + i0),
+                        nscale32i<KIND>(cv[2], d, ob + 10 + i0), nscale32i<KIND>(cv[3], d, ob + 11 + i0));
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) gs->s[0].cache[i0 + q] = f2u(cv[q]);
+      }
+    }
+  } else if (MODE == M_N64) {
+    const bool odd = (pidx & 1);
+    uint64_t other[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      uint64_t sendv = odd ? pk[q] : pk[2 + q];
+      other[q] = ((uint64_t)__shfl_xor_sync(0xffffffffu, (uint32_t)(sendv >> 32), 1) << 32) |
+                 (uint64_t)__shfl_xor_sync(0xffffffffu, (uint32_t)sendv, 1);
+    }
+    if (valid) {
+      const int64_t unit = pidx >> 1;
+      const int i0 = odd ? 2 : 0;
+      double sv[2], cv[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const double u2 = ur_d(odd ? pk[2 + q] : other[q]);
+        const double radius = sqrt(-2.0 * log_(one_minus_ur_d(odd ? other[q] : pk[q])));
+        const double theta = (2 * 3.1415926535897932) * u2;
+        double sn, cs;
+        sincos_(theta, sn, cs);
+        sv[q] = radius * sn;
+        cv[q] = radius * cs;
+      }
+      const int64_t ob = obase + unit * 8;
+      double* o = reinterpret_cast<double*>(p.out) + ob;
+      reinterpret_cast<double2*>(o + i0)[0] =
+          make_double2(nscale64i<KIND>(sv[0], d, ob + i0), nscale64i<KIND>(sv[1], d, ob + i0 + 1));
+      if (ob + 8 <= oend) {
+        reinterpret_cast<double2*>(o + 4 + i0)[0] =
+            make_double2(nscale64i<KIND>(cv[0], d, ob + 4 + i0), nscale64i<KIND>(cv[1], d, ob + 5 + i0));
+      } else {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          uint64_t b = d2u(cv[q]);
+          gs->s[0].cache[2 * (i0 + q)] = (uint32_t)b;
+          gs->s[0].cache[2 * (i0 + q) + 1] = (uint32_t)(b >> 32);
+        }
+      }
+    }
+  }
+}
+
 template <int MODE, int KIND>
 __global__ void __maxnreg__(64) k_direct(Plan p, DistParams d, const CallSnap* snap) {
   __shared__ uint64_t raw[2][kLanes][kN];
@@ -403,12 +771,9 @@ __global__ void __maxnreg__(64) k_direct(Plan p, DistParams d, const CallSnap* s
   if (n == 0) return;
 
   // --- caches the call starts from
-  // int32 kinds whose packets are rng.half() words leave raw words in the
-  // engine's half cache; DiscreteGen caches its own computed results
-  constexpr bool kHalfKind =
-      KIND == GR_RANDBITS || KIND == GR_BERNOULLI || KIND == GR_GEOMETRIC || KIND == GR_UNIFORM_INT;
-  constexpr bool kUsesHalf = (MODE == M_W64) || (MODE == M_W32 && kHalfKind);
-  constexpr bool kUsesGen = (MODE == M_N32) || (MODE == M_N64) || (MODE == M_W32 && KIND == GR_DISCRETE);
+  constexpr bool kHalfKind = CacheUse<MODE, KIND>::half_kind;
+  constexpr bool kUsesHalf = CacheUse<MODE, KIND>::half;
+  constexpr bool kUsesGen = CacheUse<MODE, KIND>::gen;
   int cvalid = 0;
   const uint32_t* cwords = nullptr;
   if (kUsesHalf) {
@@ -479,193 +844,7 @@ __global__ void __maxnreg__(64) k_direct(Plan p, DistParams d, const CallSnap* s
       }
       const int64_t pidx = base + i;
       const bool valid = act && pidx < pend;
-      // ---- emit
-      if (MODE == M_RAW) {
-        if (valid && p.out) {  // p.out == nullptr: discard
-          uint64_t* o = reinterpret_cast<uint64_t*>(p.out) + obase + pidx * 4;
-          reinterpret_cast<ulonglong2*>(o)[0] = make_ulonglong2(pk[0], pk[1]);
-          reinterpret_cast<ulonglong2*>(o)[1] = make_ulonglong2(pk[2], pk[3]);
-        }
-      } else if (MODE == M_RAW2) {
-        if (valid && p.out)
-          reinterpret_cast<ulonglong2*>(reinterpret_cast<uint64_t*>(p.out) + obase + pidx * 2)[0] =
-              make_ulonglong2(pk[0], pk[1]);
-      } else if (MODE == M_F32H) {
-        if (valid) {
-          float* o = reinterpret_cast<float*>(p.out) + obase + pidx * 4;
-          const int64_t ib = obase + pidx * 4;
-          reinterpret_cast<float4*>(o)[0] =
-              make_float4(tf32i<KIND>((uint32_t)pk[0], d, ib), tf32i<KIND>((uint32_t)(pk[0] >> 32), d, ib + 1),
-                          tf32i<KIND>((uint32_t)pk[1], d, ib + 2), tf32i<KIND>((uint32_t)(pk[1] >> 32), d, ib + 3));
-        }
-      } else if (MODE == M_F64H) {
-        if (valid) {
-          double* o = reinterpret_cast<double*>(p.out) + obase + pidx * 2;
-          const int64_t ib = obase + pidx * 2;
-          reinterpret_cast<double2*>(o)[0] = make_double2(tf64i<KIND>(pk[0], d, ib), tf64i<KIND>(pk[1], d, ib + 1));
-        }
-      } else if (MODE == M_RAW0) {
-        // a scalar draw takes the engine's whole packet and keeps its first
-        // element (StdUniformRealGen::operator(), Dists/Basic.h:533-540)
-        if (valid) reinterpret_cast<uint64_t*>(p.out)[obase / 4 + pidx] = pk[0];
-      } else if (MODE == M_F32) {
-        if (valid) {
-          float* o = reinterpret_cast<float*>(p.out) + obase + pidx * 8;
-          float v[8];
-          if (KIND == kBernoulliVKind) {
-            // BernoulliVGen<float>: p = cvttps(a * 2^31), compared signed with
-            // the masked word (Basic.h:735-745)
-            const float4* pv = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(d.vparam) + obase + pidx * 8);
-            const float4 q0 = pv[0], q1 = pv[1];
-            const float pa[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              const uint32_t w = (q & 1) ? (uint32_t)(pk[q >> 1] >> 32) : (uint32_t)pk[q >> 1];
-              v[q] = ((int32_t)(w & 0x7fffffffu) < cvtt_f32(pa[q] * 2147483648.0f)) ? 1.0f : 0.0f;
-            }
-          } else {
-#pragma unroll
-            for (int l = 0; l < kLanes; ++l) {
-              v[2 * l] = tf32i<KIND>((uint32_t)pk[l], d, obase + pidx * 8 + 2 * l);
-              v[2 * l + 1] = tf32i<KIND>((uint32_t)(pk[l] >> 32), d, obase + pidx * 8 + 2 * l + 1);
-            }
-          }
-          reinterpret_cast<float4*>(o)[0] = make_float4(v[0], v[1], v[2], v[3]);
-          reinterpret_cast<float4*>(o)[1] = make_float4(v[4], v[5], v[6], v[7]);
-        }
-      } else if (MODE == M_F64) {
-        if (valid) {
-          double* o = reinterpret_cast<double*>(p.out) + obase + pidx * 4;
-          double v[4];
-#pragma unroll
-          for (int l = 0; l < kLanes; ++l) v[l] = tf64i<KIND>(pk[l], d, obase + pidx * 4 + l);
-          reinterpret_cast<double2*>(o)[0] = make_double2(v[0], v[1]);
-          reinterpret_cast<double2*>(o)[1] = make_double2(v[2], v[3]);
-        }
-      } else if (MODE == M_W32 || MODE == M_W64) {
-        if (valid) {
-          const int64_t ob = obase + pidx * 8;
-          uint32_t wd[8];
-#pragma unroll
-          for (int l = 0; l < kLanes; ++l) {
-            wd[2 * l] = (uint32_t)pk[l];
-            wd[2 * l + 1] = (uint32_t)(pk[l] >> 32);
-          }
-          const bool full = ob + 8 <= oend;
-          if (MODE == M_W32) {
-            int32_t v[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) v[q] = tw32<KIND>(wd[q], d);
-            int32_t* o = reinterpret_cast<int32_t*>(p.out) + ob;
-            st16(o, v[0], v[1], v[2], v[3]);
-            if (full) st16(o + 4, v[4], v[5], v[6], v[7]);
-            else if (gs || kHalfKind) {
-              // leftover half: rng.half() kinds leave raw words in the engine's
-              // half() cache; DiscreteGen caches its computed upper 4 results
-              uint32_t* cdst = kHalfKind ? st->half_cache : gs->s[0].cache;
-#pragma unroll
-              for (int q = 0; q < 4; ++q) cdst[q] = kHalfKind ? wd[4 + q] : (uint32_t)v[4 + q];
-            }
-          } else {
-            double v[8];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) v[q] = tw64i<KIND>(wd[q], d, ob + q);
-            double* o = reinterpret_cast<double*>(p.out) + ob;
-            reinterpret_cast<double2*>(o)[0] = make_double2(v[0], v[1]);
-            reinterpret_cast<double2*>(o)[1] = make_double2(v[2], v[3]);
-            if (full) {
-#pragma unroll
-              for (int q = 4; q < 8; ++q) v[q] = tw64i<KIND>(wd[q], d, ob + q);
-              reinterpret_cast<double2*>(o)[2] = make_double2(v[4], v[5]);
-              reinterpret_cast<double2*>(o)[3] = make_double2(v[6], v[7]);
-            } else {
-#pragma unroll
-              for (int q = 0; q < 4; ++q) st->half_cache[q] = wd[4 + q];
-            }
-          }
-        }
-      } else if (MODE == M_N32) {
-        // unit = packets (2j, 2j+1): u1 words in the even thread, u2 in the odd.
-        // Even thread handles lanes i = 0..3 of the unit, odd handles 4..7.
-        const bool odd = (tid & 1);
-        uint32_t wd[8];
-#pragma unroll
-        for (int l = 0; l < kLanes; ++l) {
-          wd[2 * l] = (uint32_t)pk[l];
-          wd[2 * l + 1] = (uint32_t)(pk[l] >> 32);
-        }
-        uint32_t other[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) other[q] = __shfl_xor_sync(0xffffffffu, odd ? wd[q] : wd[4 + q], 1);
-        if (valid) {
-          const int64_t unit = pidx >> 1;
-          const int i0 = odd ? 4 : 0;
-          float sv[4], cv[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float u1 = ur_f(odd ? other[q] : wd[q]);
-            const float u2 = ur_f(odd ? wd[4 + q] : other[q]);
-            const float radius = sqrtf((float)-2 * logf_(1.0f - u1));
-            const float theta = (float)(2 * 3.1415926535897932) * u2;
-            float sn, cs;
-            sincosf_(theta, sn, cs);
-            sv[q] = radius * sn;
-            cv[q] = radius * cs;
-          }
-          const int64_t ob = obase + unit * 16;
-          float* o = reinterpret_cast<float*>(p.out) + ob;
-          reinterpret_cast<float4*>(o + i0)[0] =
-              make_float4(nscale32i<KIND>(sv[0], d, ob + i0), nscale32i<KIND>(sv[1], d, ob + i0 + 1),
-                          nscale32i<KIND>(sv[2], d, ob + i0 + 2), nscale32i<KIND>(sv[3], d, ob + i0 + 3));
-          if (ob + 16 <= oend) {
-            reinterpret_cast<float4*>(o + 8 + i0)[0] =
-                make_float4(nscale32i<KIND>(cv[0], d, ob + 8 + i0), nscale32i<KIND>(cv[1], d, ob + 9 + i0),
-                            nscale32i<KIND>(cv[2], d, ob + 10 + i0), nscale32i<KIND>(cv[3], d, ob + 11 + i0));
-          } else {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) gs->s[0].cache[i0 + q] = f2u(cv[q]);
-          }
-        }
-      } else if (MODE == M_N64) {
-        const bool odd = (tid & 1);
-        uint64_t other[2];
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          uint64_t sendv = odd ? pk[q] : pk[2 + q];
-          other[q] = ((uint64_t)__shfl_xor_sync(0xffffffffu, (uint32_t)(sendv >> 32), 1) << 32) |
-                     (uint64_t)__shfl_xor_sync(0xffffffffu, (uint32_t)sendv, 1);
-        }
-        if (valid) {
-          const int64_t unit = pidx >> 1;
-          const int i0 = odd ? 2 : 0;
-          double sv[2], cv[2];
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const double u2 = ur_d(odd ? pk[2 + q] : other[q]);
-            const double radius = sqrt(-2.0 * log_(one_minus_ur_d(odd ? other[q] : pk[q])));
-            const double theta = (2 * 3.1415926535897932) * u2;
-            double sn, cs;
-            sincos_(theta, sn, cs);
-            sv[q] = radius * sn;
-            cv[q] = radius * cs;
-          }
-          const int64_t ob = obase + unit * 8;
-          double* o = reinterpret_cast<double*>(p.out) + ob;
-          reinterpret_cast<double2*>(o + i0)[0] =
-              make_double2(nscale64i<KIND>(sv[0], d, ob + i0), nscale64i<KIND>(sv[1], d, ob + i0 + 1));
-          if (ob + 8 <= oend) {
-            reinterpret_cast<double2*>(o + 4 + i0)[0] =
-                make_double2(nscale64i<KIND>(cv[0], d, ob + 4 + i0), nscale64i<KIND>(cv[1], d, ob + 5 + i0));
-          } else {
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              uint64_t b = d2u(cv[q]);
-              gs->s[0].cache[2 * (i0 + q)] = (uint32_t)b;
-              gs->s[0].cache[2 * (i0 + q) + 1] = (uint32_t)(b >> 32);
-            }
-          }
-        }
-      }
+      emit_packet<MODE, KIND>(pk, pidx, valid, p, d, obase, oend, st, gs);
       __syncthreads();
     }
     cur ^= 1;
@@ -695,40 +874,91 @@ __global__ void __maxnreg__(64) k_direct(Plan p, DistParams d, const CallSnap* s
   }
 }
 
+// The same transforms over words that k_words_* left in memory: one thread per
+// packet, grid (packets, engines).  Packets [wbase, wbase + wcount) of every
+// engine's call are in memory; block 0 of an engine leaves the engine state.
+constexpr int kXfThreads = 256;
+template <int MODE, int KIND>
+__global__ void __launch_bounds__(kXfThreads) k_xform(Plan p, DistParams d, const CallSnap* snap) {
+  const int k = blockIdx.y, tid = threadIdx.x;
+  EngState* st = p.eng + k;
+  GenState* gs = p.gen ? p.gen + k : nullptr;
+  const int64_t g0 = (int64_t)k * p.gran_per_k + min((int64_t)k, p.gran_rem);
+  const int64_t ng = p.gran_per_k + ((int64_t)k < p.gran_rem ? 1 : 0);
+  const int64_t off = g0 * p.gran, n = ng * p.gran;
+  if (n == 0) return;
+  constexpr bool kHalfKind = CacheUse<MODE, KIND>::half_kind;
+  constexpr bool kUsesHalf = CacheUse<MODE, KIND>::half;
+  constexpr bool kUsesGen = CacheUse<MODE, KIND>::gen;
+  const int cvalid = kUsesHalf ? snap[k].half_valid : (kUsesGen ? snap[k].gen_valid : 0);
+  const uint32_t* cwords = kUsesHalf ? snap[k].half_cache : snap[k].gen_cache;
+  constexpr int CO = ModeInfo<MODE>::kCacheOut;
+  constexpr int OPP = ModeInfo<MODE>::OPP;
+  const int64_t Q0 = (cvalid && CO) ? min((int64_t)CO, n) : 0;
+  const int64_t r = n - Q0;
+  const int64_t Np = (MODE == M_N32 || MODE == M_N64) ? 2 * ((r + 2 * OPP - 1) / (2 * OPP)) : (r + OPP - 1) / OPP;
+  const int64_t obase = off + Q0, oend = off + n;
+  const int64_t pend = min(p.wbase + p.wcount, Np);
+  const int64_t pidx = p.wbase + (int64_t)blockIdx.x * kXfThreads + tid;
+  const uint64_t* w = p.words + (size_t)k * kLanes * p.wstride;
+  const bool valid = pidx < pend;
+  uint64_t pk[kLanes];
+#pragma unroll
+  for (int l = 0; l < kLanes; ++l) pk[l] = valid ? temper(w[(size_t)l * p.wstride + kN + (pidx - p.wbase)]) : 0;
+  emit_packet<MODE, KIND>(pk, pidx, valid, p, d, obase, oend, st, gs);
+  if (blockIdx.x != 0) return;
+  if (p.wbase == 0 && tid < Q0) {  // outputs served from the cache
+    const int i = tid;
+    if (MODE == M_W64) reinterpret_cast<double*>(p.out)[off + i] = tw64i<KIND>(cwords[i], d, off + i);
+    if (MODE == M_W32)
+      reinterpret_cast<int32_t*>(p.out)[off + i] = kHalfKind ? tw32<KIND>(cwords[i], d) : (int32_t)cwords[i];
+    if (MODE == M_N32) reinterpret_cast<float*>(p.out)[off + i] = nscale32i<KIND>(u2f(cwords[i]), d, off + i);
+    if (MODE == M_N64) {
+      const uint64_t b = (uint64_t)cwords[2 * i] | ((uint64_t)cwords[2 * i + 1] << 32);
+      reinterpret_cast<double*>(p.out)[off + i] = nscale64i<KIND>(u2d(b), d, off + i);
+    }
+  }
+  const int64_t used = max(pend - p.wbase, (int64_t)0);  // packets of this run
+  if (used > 0)
+    for (int t = tid; t < kLanes * kN; t += kXfThreads)
+      st->win[t / kN][t % kN] = w[(size_t)(t / kN) * p.wstride + used + t % kN];
+  if (tid == 0) {
+    if (Np <= p.wbase + p.wcount && (p.wbase < Np || p.wbase == 0)) {  // the call ends here
+      int64_t left = 0;  // leftover outputs cached for the next call
+      if (MODE == M_W32 || MODE == M_W64) left = (r % 8) ? 4 : 0;
+      if (MODE == M_N32) left = (r % 16) ? 8 : 0;
+      if (MODE == M_N64) left = (r % 8) ? 4 : 0;
+      if (kUsesHalf) st->half_valid = left ? 1 : (Q0 ? 0 : cvalid);
+      if (kUsesGen) gs->s[0].valid = left ? 1 : 0;
+    }
+    st->consumed += (uint64_t)used;
+  }
+}
+
 template <int MODE, int KIND>
 static cudaError_t run_direct(const Plan& p, const DistParams& d, const CallSnap* snap, cudaStream_t s) {
-  k_direct<MODE, KIND><<<p.K * p.S, 160, 0, s>>>(p, d, snap);
+  if (p.words) {
+    const dim3 grid((unsigned)((p.wcount + kXfThreads - 1) / kXfThreads), (unsigned)p.K);
+    k_xform<MODE, KIND><<<grid, kXfThreads, 0, s>>>(p, d, snap);
+  } else {
+    k_direct<MODE, KIND><<<p.K * p.S, 160, 0, s>>>(p, d, snap);
+  }
   return cudaGetLastError();
 }
 
 cudaError_t launch_prefix(const EngState* st, const GenState* gen, int K, uint64_t* prefix, CallSnap* snap,
                           cudaStream_t s) {
-  k_prefix<<<K * kLanes, 160, 0, s>>>(st, prefix, snap, gen);
+  k_prefix<<<K * kLanes, kWideThreads, 0, s>>>(st, prefix, snap, gen);
   return cudaGetLastError();
-}
-
-static constexpr size_t kJumpSmem = (size_t)(kPrefixLen + kN) * sizeof(uint64_t);
-
-// k_jump's dynamic shared-memory limit, set once per device.
-static cudaError_t jump_attr() {
-  static bool attr[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  if (!attr[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(k_jump, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJumpSmem);
-    if (e != cudaSuccess) return e;
-    attr[dev] = true;
-  }
-  return cudaSuccess;
 }
 
 cudaError_t launch_jump(const uint64_t* prefix, const uint64_t* polys, int K, int S, uint64_t* segwin,
                         cudaStream_t s) {
   if (S <= 1) return cudaSuccess;
-  cudaError_t e = jump_attr();
+  const int ctas = K * (S - 1) * kLanes;
+  cudaError_t e = cudaMemsetAsync(segwin, 0, (size_t)ctas * kN * sizeof(uint64_t), s);
   if (e != cudaSuccess) return e;
-  k_jump<<<K * (S - 1) * kLanes, kJumpThreads, kJumpSmem, s>>>(prefix, polys, S, segwin);
+  k_jump<<<ctas * kJumpParts, kJumpThreads, 0, s>>>(prefix, polys, S, reinterpret_cast<unsigned long long*>(segwin));
   return cudaGetLastError();
 }
 
@@ -737,7 +967,6 @@ cudaError_t preload_raw_stream_kernels() {
   cudaError_t e = cudaFuncGetAttributes(&a, k_prefix);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_jump);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_direct<M_RAW, kRawKind>);
-  if (e == cudaSuccess) e = jump_attr();
   return e;
 }
 

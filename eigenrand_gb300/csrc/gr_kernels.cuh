@@ -67,6 +67,23 @@ struct Plan {
   int64_t gran_rem;       // ... plus one for the first gran_rem engines
   int32_t gran;           // outputs per granule
   void* out;
+  // raw words of the call in memory (launch_words; null: the kernels generate
+  // their own): packets [wbase, wbase + wcount) of every engine
+  const uint64_t* words;
+  int64_t wstride, wbase, wcount;
+};
+
+// launch_words: n raw words per lane (even) of every engine, in S segments of
+// J (even), into words[(k * 4 + l) * stride + 312 ...] behind the current
+// window; snap (may be null) receives the caches as they are at call start.
+struct WordsArgs {
+  uint64_t* words;
+  int64_t stride;  // even
+  int64_t n;
+  const uint64_t* segwin;
+  int32_t S;
+  int64_t J;
+  CallSnap* snap;
 };
 
 // kernels (gr_kernels.cu)
@@ -75,9 +92,9 @@ cudaError_t launch_prefix(const EngState* st, const GenState* gen, int K, uint64
                           cudaStream_t s);
 cudaError_t launch_jump(const uint64_t* prefix, const uint64_t* polys, int K, int S, uint64_t* segwin,
                         cudaStream_t s);
+cudaError_t launch_words(const EngState* st, const GenState* gen, int K, const WordsArgs& a, cudaStream_t s);
 // Loads the code of k_prefix, k_jump and the raw-stream k_direct on the
-// current device and sets k_jump's shared-memory limit, so that later
-// launches of them load nothing.
+// current device, so that later launches of them load nothing.
 cudaError_t preload_raw_stream_kernels();
 // Fused engine + transform for kinds whose draws per output are fixed and
 // packet aligned.  Returns cudaErrorNotSupported for other kinds.
