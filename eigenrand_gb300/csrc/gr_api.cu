@@ -868,6 +868,76 @@ double poisson_step_halves(float fe) {
   return m;
 }
 
+// Probability that a lane of a GammaGen rejection trial is accepted: GS
+// (Ahrens and Dieter 1974) e G(a + 1) / (e + a), the tan proposal
+// G(a) e^(a-1) / (pi sqrt(2a - 1) (a - 1)^(a-1)).
+double gamma_yield(int branch, double a) {
+  const double e1 = 2.718281828459045;
+  if ((branch >> 8) == 2) return e1 * std::tgamma(a + 1) / (e1 + a);
+  const double b = a - 1;
+  return std::exp(std::lgamma(a) + b - b * std::log(b)) / (3.141592653589793 * std::sqrt(2 * a - 1));
+}
+
+// BetaGen's general branch through words in memory (gr_chain.cu), then the
+// one-CTA-per-engine walk for whatever the planned packets did not hold
+// (usually nothing).  The expected packets per output only size the plan.
+constexpr int64_t kChainMin = 192;              // output packets per engine
+constexpr int kChainMaxK = 256;                 // engines
+constexpr int64_t kChainCap = (int64_t)1 << 23;  // packets of words at a time, all engines
+gr_status run_chain_call(gr_engine* e, const Plan& p0, const DistParams& wd, int64_t npk, int64_t max_blocks,
+                         cudaStream_t stream) {
+  const int br[2] = {wd.ia, wd.ib};
+  const double al[2] = {wd.da, wd.db};
+  double per = 0;
+  for (int c = 0; c < 2; ++c) per += (br[c] & 255) / ((br[c] >> 8) >= 2 ? gamma_yield(br[c], al[c]) : 1.0);
+  const char* sc = std::getenv("GR_WALK_PLAN_SCALE");  // tests: see run_packets
+  const double scale = sc ? std::max(0.0, std::atof(sc)) : 1.0;
+  const bool closed = (br[0] >> 8) < 2 && (br[1] >> 8) < 2;
+  int64_t left = (int64_t)std::ceil(per * ((double)npk + (closed ? 0.0 : 8.0 * std::sqrt((double)npk))) * scale) + 64;
+  const bool both = (br[0] >> 8) >= 2 && (br[1] >> 8) >= 2;
+  Plan p = p0;
+  int64_t* done = nullptr;
+  cudaError_t err = scratch_alloc(reinterpret_cast<void**>(&done), sizeof(int64_t) * (size_t)e->K, e->device, stream);
+  if (err != cudaSuccess) return cuda_fail(err, "scratch memory");
+  err = cudaMemsetAsync(done, 0, sizeof(int64_t) * (size_t)e->K, stream);
+  gr_status st = err == cudaSuccess ? GR_OK : cuda_fail(err, "beta chain");
+  const int64_t chunk = std::max<int64_t>(kChainCap / e->K, 1024);
+  while (st == GR_OK && left > 0) {
+    // what a chunk leaves over (less than one output's packets) is made again
+    const int64_t n = std::min(chunk, left + 64);
+    left -= n - 64;
+    const bool seg = n > 8192 && (both ? e->K < 64 : (e->K < 256 || n > 65536));
+    const ChainLayout L = chain_layout(wd, e->K, n, seg ? 1024 : 0);
+    void *words = nullptr, *scratch = nullptr;
+    bool got = false;
+    if (L.bytes) {
+      err = scratch_alloc(&scratch, L.bytes, e->device, stream);
+      if (err != cudaSuccess) {
+        cudaGetLastError();
+        break;
+      }
+    }
+    st = make_words(e, p, n, false, &words, &got, stream);
+    if (st == GR_OK && got) {
+      err = launch_chain(p, wd, L, static_cast<char*>(scratch), done, stream);
+      if (err != cudaSuccess) st = cuda_fail(err, "beta chain kernels");
+      cudaFreeAsync(words, stream);
+    }
+    if (scratch) cudaFreeAsync(scratch, stream);
+    p.words = nullptr;
+    if (!got) break;
+  }
+  if (st == GR_OK) {
+    p.words = nullptr;
+    p.done = done;
+    p.S = 1;
+    err = launch_walk(p, wd, max_blocks, stream);
+    if (err != cudaSuccess) st = cuda_fail(err, "walk sampling kernel");
+  }
+  cudaFreeAsync(done, stream);
+  return st;
+}
+
 gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, size_t n, cudaStream_t stream);
 
 // The n % P elements after the last whole packet of a call: the scalar
@@ -1092,6 +1162,7 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
       wd.fa = (float)dp.da;
       wd.fb = (float)dp.db;
       max_blocks = (npk * 64) / kN + 64;
+      if (npk >= kChainMin && e->K <= kChainMaxK) return run_chain_call(e, p, wd, npk, block_cap(max_blocks), stream);
     }
     max_blocks = block_cap(max_blocks);
     cudaError_t err = launch_walk(p, wd, max_blocks, stream);

@@ -231,43 +231,24 @@ cudaError_t launch_words(const EngState* st, const GenState* gen, int K, const W
 // word on average where one conditional XOR per term takes 2.  Quarters meet
 // by atomic XOR (segwin zeroed beforehand).  Bound by issue.
 constexpr int kJumpThreads = 256;
-constexpr int kJumpParts = 4;
-constexpr int kJumpPer = 19968 / (kJumpParts * (kJumpThreads / 32));  // 624 terms per warp
+constexpr int kJumpParts = 8;
+constexpr int kJumpPer = 19968 / (kJumpParts * (kJumpThreads / 32));  // 312 terms per warp
 constexpr int kJumpOut = 11;
 constexpr int kJumpSpan = kJumpPer * (kJumpThreads / 32);             // terms per CTA
 constexpr int kJumpLoad = kJumpSpan + 32 * kJumpOut + 8;              // prefix words a CTA reads
 
-template <int N>
-__device__ __forceinline__ void xor_nibble(uint64_t (&acc)[kJumpOut], const uint64_t* w) {
+// acc[j] ^= the words of terms 0 / 1 (at w[j], w[j + 1]) whose coefficient
+// bits are set; c is the same in every thread of the warp
+__device__ __forceinline__ void xor_terms2(uint64_t (&acc)[kJumpOut], const uint64_t* w, uint32_t c) {
+  if (c == 3) {
 #pragma unroll
-  for (int j = 0; j < kJumpOut; ++j) {
-    uint64_t v = acc[j];
-    if (N & 1) v ^= w[j];
-    if (N & 2) v ^= w[j + 1];
-    if (N & 4) v ^= w[j + 2];
-    if (N & 8) v ^= w[j + 3];
-    acc[j] = v;
-  }
-}
-
-__device__ __forceinline__ void xor_terms4(uint64_t (&acc)[kJumpOut], const uint64_t* w, uint32_t c) {
-  switch (c) {
-    case 1: xor_nibble<1>(acc, w); break;
-    case 2: xor_nibble<2>(acc, w); break;
-    case 3: xor_nibble<3>(acc, w); break;
-    case 4: xor_nibble<4>(acc, w); break;
-    case 5: xor_nibble<5>(acc, w); break;
-    case 6: xor_nibble<6>(acc, w); break;
-    case 7: xor_nibble<7>(acc, w); break;
-    case 8: xor_nibble<8>(acc, w); break;
-    case 9: xor_nibble<9>(acc, w); break;
-    case 10: xor_nibble<10>(acc, w); break;
-    case 11: xor_nibble<11>(acc, w); break;
-    case 12: xor_nibble<12>(acc, w); break;
-    case 13: xor_nibble<13>(acc, w); break;
-    case 14: xor_nibble<14>(acc, w); break;
-    case 15: xor_nibble<15>(acc, w); break;
-    default: break;
+    for (int j = 0; j < kJumpOut; ++j) acc[j] ^= w[j] ^ w[j + 1];
+  } else if (c == 1) {
+#pragma unroll
+    for (int j = 0; j < kJumpOut; ++j) acc[j] ^= w[j];
+  } else if (c == 2) {
+#pragma unroll
+    for (int j = 0; j < kJumpOut; ++j) acc[j] ^= w[j + 1];
   }
 }
 
@@ -301,8 +282,8 @@ __global__ void __launch_bounds__(kJumpThreads, 4)
 #pragma unroll
     for (int m = 0; m < 8; ++m) w[kJumpOut - 1 + m] = p[i0 + kJumpOut - 1 + m];
     const uint32_t cb = (uint32_t)(cf[(ibeg + i0) >> 6] >> ((ibeg + i0) & 63)) & 0xffu;
-    xor_terms4(acc, w, cb & 15u);
-    xor_terms4(acc, w + 4, cb >> 4);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) xor_terms2(acc, w + 2 * t, (cb >> (2 * t)) & 3u);
 #pragma unroll
     for (int m = 0; m < kJumpOut - 1; ++m) w[m] = w[m + 8];
   }

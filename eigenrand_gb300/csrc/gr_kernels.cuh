@@ -71,7 +71,23 @@ struct Plan {
   // their own): packets [wbase, wbase + wcount) of every engine
   const uint64_t* words;
   int64_t wstride, wbase, wcount;
+  // granules of every engine's slice that earlier kernels of the call have
+  // made (null: none); the walk and rejection kernels make the rest
+  const int64_t* done;
 };
+
+// Engine k's slice of the output without what is done: first element, count.
+__device__ __forceinline__ void slice_left(const Plan& p, int k, int64_t& off, int64_t& n) {
+  int64_t g0 = (int64_t)k * p.gran_per_k + min((int64_t)k, p.gran_rem);
+  int64_t ng = p.gran_per_k + ((int64_t)k < p.gran_rem ? 1 : 0);
+  if (p.done) {
+    const int64_t d = min(p.done[k], ng);
+    g0 += d;
+    ng -= d;
+  }
+  off = g0 * p.gran;
+  n = ng * p.gran;
+}
 
 // launch_words: n raw words per lane (even) of every engine, in S segments of
 // J (even), into words[(k * 4 + l) * stride + 312 ...] behind the current
@@ -150,6 +166,23 @@ cudaError_t launch_poisson_segmented(const Plan& p, const DistParams& d, const P
 // BetaGen with a or b >= 1 (f32/f64; d.ia / d.ib hold (gamma branch << 8) |
 // packets for the two GammaGens).
 cudaError_t launch_walk(const Plan& p, const DistParams& d, int64_t max_blocks, cudaStream_t s);
+
+// BetaGen / FisherFGen's general branch over words in memory (gr_chain.cu):
+// as many output packets per engine as p.wcount packets hold, added to
+// done[k]; the engine and generator state follow.  scratch: chain_layout's
+// bytes.  Sg > 1: the chain runs in Sg segments of J positions per engine.
+struct ChainLayout {
+  int64_t n;           // packets per engine in memory
+  int32_t Sg, J;       // segments per engine, positions per segment
+  int32_t ns;          // entry states per segment (0: one segment)
+  int32_t rcap;        // output packets per segment
+  int32_t groups, gsz; // segment groups of the composition, segments per group
+  int64_t mstride;     // positions of a mask array
+  size_t o_mask, o_vis, o_tab, o_gtab, o_entry, o_seg, o_ebase, o_rec, bytes;
+};
+ChainLayout chain_layout(const DistParams& d, int K, int64_t n, int32_t J);
+cudaError_t launch_chain(const Plan& p, const DistParams& d, const ChainLayout& L, char* scratch, int64_t* done,
+                         cudaStream_t s);
 
 // Samples drawn with a scalar engine as the Urng (gr_kernels.cu): npk output
 // packets from the engine's 64-bit words w (scalar_words_per_packet(kind,

@@ -20,10 +20,9 @@
 #include "gr_kernels.cuh"
 #include "gr_math.cuh"
 #include "gr_mt.cuh"
+#include "gr_samplers.cuh"
 
 namespace gr {
-
-enum StagedDT { SD_F32 = 0, SD_F64 = 1, SD_I32H = 2 };
 
 template <int KIND, int DT>
 __global__ void __launch_bounds__(160)
@@ -304,8 +303,6 @@ namespace gr {
 // ===========================================================================
 namespace {
 
-enum RejKind { RK_GAMMA_GS = 0, RK_GAMMA_TAN = 1, RK_BETA_SMALL = 2, RK_POISSON = 3, RK_BINOMIAL = 4 };
-
 constexpr int kRejThreads = 160;
 constexpr int kMaxTrials = 320;  // trials resolved per block of packets (<= 2496 / 8 + 1)
 constexpr int kMaxCand = 1280;   // candidate lanes per block: <= 2496 words / Wt * P + P
@@ -334,166 +331,6 @@ __device__ __forceinline__ uint32_t block_incl_scan(uint32_t v, uint32_t* warp_t
 }
 
 }  // namespace
-
-// Accept test of a double GS trial (GammaGen, alpha < 1, NormalExp.h:535-556)
-// decided in float arithmetic where the float result lies clearly on one side
-// of both comparisons: 1 accept, 0 reject, -1 undecided (evaluate in double).
-// Bounds: vx converts with relative error < 2^-19 (vx >= 2^-12 here), ux2
-// with absolute error < 2^-24, float log / exp are within 1 ulp and
-// |log vx| <= 8.4, so the float qx is within 1e-5 (1 + 1/alpha) of the double
-// qx, relatively (qx >= 0.027); the band used is 2^-18 (1 + 40/alpha), over
-// 14 times wider.  The branch test ux < px is trusted outside
-// |ux - px| <= 2^-21 (float ux is within 2^-24 of ux).
-__device__ __forceinline__ int gs_filter_f64(uint64_t bux, uint64_t bvx, uint64_t bux2, float pxf, float inv_a,
-                                             float am1, float band) {
-  constexpr uint64_t M = 0xfffffffffffffull;
-  // top 32 of the 52 fraction bits (absolute error < 2^-32); vx below 2^-12
-  // is left to the double test, so vx keeps a relative error below 2^-19
-  const float ux = __uint2float_rn((uint32_t)((bux & M) >> 20)) * 0x1p-32f;
-  if (fabsf(ux - pxf) <= 0x1p-21f) return -1;
-  const uint64_t mv = bvx & M;
-  if ((mv >> 40) == 0) return -1;
-  const float vx = __uint2float_rn((uint32_t)(mv >> 20)) * 0x1p-32f;
-  const float ux2 = __uint2float_rn((uint32_t)((bux2 & M) >> 20)) * 0x1p-32f;
-  const float lv = logf_(vx);
-  const bool c = ux < pxf;
-  const float e1 = expf_(c ? inv_a * lv : logf_(1.0f - lv) * am1);  // one exp for both branches
-  const float qx = c ? expf_(-e1) : e1;
-  if (ux2 < qx * (1.0f - band)) return 1;
-  if (ux2 > qx * (1.0f + band)) return 0;
-  return -1;
-}
-
-// Candidate of a double GS trial already known to be accepted: xx only
-// (no acceptance bound); ux < px is decided on the integer fraction against
-// tpx = ceil(px * 2^52).
-__device__ __forceinline__ double gs_value_f64(uint64_t bux, uint64_t bvx, uint64_t tpx, double inv_a) {
-  const double vx = ur_d(bvx) + 2.220446049250313e-16 / 8;
-  const double lv = log_(vx);
-  return ((bux & 0xfffffffffffffull) < tpx) ? exp_(inv_a * lv) : 1.0 - lv;
-}
-
-// One rejection trial, lane j: candidate bits and accept flag.  Trial t
-// reads words [t * Wt, (t + 1) * Wt) of the cache-inclusive word stream
-// (word(w)); full-packet double kinds read u64 lane values (rval(r)).
-template <int RK, int DT, class WF, class RF>
-__device__ __forceinline__ bool rej_trial(const DistParams& d, int64_t t, int j, WF&& word, RF&& rval,
-                                          uint64_t& cbits) {
-  constexpr int Wt = (RK == RK_GAMMA_GS) ? 3 * 8 : (RK == RK_POISSON || RK == RK_BINOMIAL) ? 8 : 2 * 8;
-  bool acc = false;
-  cbits = 0;
-
-  const int64_t w0 = t * Wt;
-  if (DT == SD_F32) {
-    if (RK == RK_GAMMA_GS) {
-      const float ux = ur_f(word(w0 + j));
-      const float vx = ur_f(word(w0 + 8 + j)) + 1.1920928955078125e-07f / 8;
-      const float ux2 = ur_f(word(w0 + 16 + j));
-      // the reference evaluates both branches and blends (NormalExp.h:543-553);
-      // evaluating only the selected one gives the same bits
-      // branch c: xx = exp(lv / alpha), bound exp(-xx); else xx = 1 - lv,
-      // bound exp(log(xx) (alpha - 1)).  One exp serves both branches, so a
-      // warp with lanes in both runs three transcendentals after lv, not four
-      const float lv = logf_(vx);
-      const bool c = ux < d.fe;  // px
-      const float e1 = expf_(c ? d.fc * lv : logf_(1.0f - lv) * d.fd);  // 1/alpha, alpha - 1
-      const float xx = c ? e1 : 1.0f - lv;
-      const float qx = c ? expf_(-e1) : e1;
-      cbits = f2u(d.fb * xx);
-      acc = ux2 < qx;
-    } else if (RK == RK_GAMMA_TAN) {
-      const float u = ur_f(word(w0 + j));
-      const float ux = ur_f(word(w0 + 8 + j));
-      float ys, yc;
-      sincosf_((float)3.1415926535897932 * u, ys, yc);
-      const float yx = ys / yc;
-      const float xx = d.ff * yx + d.fd;  // sqrt * yx + (alpha - 1)
-      const bool c = 0.0f < xx;
-      const float ub = (yx * yx + 1.0f) * expf_(d.fd * logf_(xx / d.fd) - yx * d.ff);
-      acc = c && (ux <= ub);
-      cbits = f2u(d.fb * xx);
-    } else if (RK == RK_BETA_SMALL) {
-      const float u1 = ur_f(word(w0 + j));
-      const float u2 = ur_f(word(w0 + 8 + j));
-      const float p1 = expf_(logf_(u1) * d.fc);  // 1/a
-      const float p2 = expf_(logf_(u2) * d.fd);  // 1/b
-      const float x = p1 + p2;
-      cbits = f2u(p1 / x);
-      acc = x <= 1.0f;
-    }
-  } else if (DT == SD_F64) {
-    const int64_t r0 = (t * Wt / 8) * 4 + j;  // u64 lane index of the trial's first packet
-    if (RK == RK_GAMMA_GS) {
-      // float filter first: rejected lanes need nothing more, accepted ones
-      // only the candidate (the exact branch is known)
-      const int f = gs_filter_f64(rval(r0), rval(r0 + 4), rval(r0 + 8), d.fe, d.fc, d.fd, d.fh);
-      if (f == 0) {
-        acc = false;
-      } else if (f == 1) {
-        cbits = d2u(d.db * gs_value_f64(rval(r0), rval(r0 + 4), d2u(d.dg), d.dc));  // dg holds tpx as bits
-        acc = true;
-      } else {
-        const double ux = ur_d(rval(r0));
-        const double vx = ur_d(rval(r0 + 4)) + 2.220446049250313e-16 / 8;
-        const double ux2 = ur_d(rval(r0 + 8));
-        const double lv = log_(vx);
-        const bool c = ux < d.de;
-        double xx, qx;
-        if (c) {
-          xx = exp_(d.dc * lv);
-          qx = exp_(-xx);
-        } else {
-          xx = 1.0 - lv;
-          qx = exp_(log_(xx) * d.dd);
-        }
-        cbits = d2u(d.db * xx);
-        acc = ux2 < qx;
-      }
-    } else if (RK == RK_GAMMA_TAN) {
-      const double u = ur_d(rval(r0));
-      const double ux = ur_d(rval(r0 + 4));
-      double ys, yc;
-      sincos_(3.1415926535897932 * u, ys, yc);
-      const double yx = ys / yc;
-      const double xx = d.df * yx + d.dd;
-      const bool c = 0.0 < xx;
-      const double ub = (yx * yx + 1.0) * exp_(d.dd * log_(xx / d.dd) - yx * d.df);
-      acc = c && (ux <= ub);
-      cbits = d2u(d.db * xx);
-    } else if (RK == RK_BETA_SMALL) {
-      const double u1 = ur_d(rval(r0));
-      const double u2 = ur_d(rval(r0 + 4));
-      const double p1 = exp_(log_(u1) * d.dc);
-      const double p2 = exp_(log_(u2) * d.dd);
-      const double x = p1 + p2;
-      cbits = d2u(p1 / x);
-      acc = x <= 1.0;
-    }
-  } else {  // int32 kinds with Packet4f internals over half packets
-    const float u = ur_f(word(w0 + j));
-    const float u2 = ur_f(word(w0 + 4 + j));
-    float s, c;
-    sincosf_((float)3.1415926535897932 * u, s, c);
-    const float yx = s / c;
-    if (RK == RK_POISSON) {
-      const float fres = truncf(d.fa * yx + d.fb);  // sqrt(2 mean) * yx + mean
-      const float p1 = (yx * yx + 1.0f) * 0.9f;
-      const float p2 = expf_((fres * d.fc - lgamma_approxf_(fres + 1.0f)) - d.fd);
-      acc = (0.0f <= fres) && (u2 <= p1 * p2);
-      cbits = f2u(fres);
-    } else {  // binomial, BinomialGen::packetOp tan branch (Discrete.h:1014-1046)
-      const float fres = truncf(d.fa * yx + d.fb);  // sqrt_v * ys + mean
-      const float p1 = ((float)1.2 * d.fa) * (1.0f + yx * yx);
-      float tt = (d.fg - lgamma_approxf_(fres + 1.0f)) - lgamma_approxf_((d.fh + 1.0f) - fres);
-      tt = tt + fres * d.fc;
-      tt = tt + (d.fh - fres) * d.fd;
-      const float p2 = expf_(tt);
-      acc = (0.0f <= fres) && (fres <= d.fh) && (u2 <= p1 * p2);
-      cbits = f2u(fres);
-    }
-  }
-        return acc;
-}
 
 // GammaGen's rejection trials drawn with a scalar engine (std::mt19937_64,
 // P8_mt19937_64) as the Urng: trial t's candidate lanes from pre-drawn 64-bit
@@ -1991,117 +1828,6 @@ namespace {
 
 constexpr int kBetaRing = 1024;  // positions whose accept masks are kept (a power of two)
 
-template <int DT>
-__host__ __device__ constexpr int beta_lanes() {
-  return DT == SD_F64 ? 4 : 8;
-}
-
-// Constants of one GammaGen component of a BetaGen, computed on the host
-// with the same IEEE expressions the generator uses (so with the same bits),
-// and passed as a kernel parameter: in the sampling loops they cost a
-// constant-bank load, never a division.
-struct BetaComp {
-  int type, U;                      // gamma_branch: type << 8 | packets
-  float af, f_px, f_inv, f_am1, f_sq;
-  float f_band;                     // band of the float pre-test of a double GS trial
-  double ad, d_px, d_inv, d_am1, d_sq;
-  uint64_t tpx;                     // ceil(px * 2^52): double GS branch on the integer fraction
-};
-struct BetaConsts {
-  BetaComp c[2];
-  int post;              // FisherFGen: write (b/a) x / (1 - x)
-  float fpost;           // b/a in the scalar type
-  double dpost;
-};
-
-BetaComp beta_component(int branch, float af, double ad) {
-  BetaComp b;
-  b.type = branch >> 8;
-  b.U = branch & 0xff;
-  b.af = af;
-  b.f_px = (float)(2.7182818284590452 / ((double)af + 2.7182818284590452));
-  b.f_inv = 1 / af;
-  b.f_am1 = af - 1;
-  b.f_sq = std::sqrt(2 * af - 1);
-  b.f_band = (float)(0x1p-18 * (1.0 + 40.0 / ad));
-  b.ad = ad;
-  b.d_px = 2.7182818284590452 / (ad + 2.7182818284590452);
-  b.d_inv = 1 / ad;
-  b.d_am1 = ad - 1;
-  b.d_sq = std::sqrt(2 * ad - 1);
-  b.tpx = (uint64_t)std::ceil(b.d_px * 0x1p52);
-  return b;
-}
-
-// Value (closed form) or candidate (rejection trial) of one GammaGen
-// component of sampler type `type` at one lane: Uf(q) / Ud(q) give the
-// lane's uniform in the q-th packet of the draw.  ACC: also decide
-// acceptance (the rejection types); without it only the candidate is
-// computed, for lanes already known to be accepted (the same expressions,
-// so the same bits).
-template <int DT, bool ACC, class UFF, class UDF>
-__device__ __forceinline__ uint64_t beta_comp_u(const BetaComp g, const int type, UFF&& Uf, UDF&& Ud, bool& acc) {
-  acc = true;
-  const int U = g.U;
-  if (DT == SD_F32) {
-    if (type == 0) return f2u(1.0f * (-(logf_(1.0f - Uf(0)) / 1.0f)));
-    if (type == 1) {
-      float y = Uf(0) + 1.1920928955078125e-07f / 8;
-      for (int t = 1; t < U; ++t) y = y * (Uf(t) + 1.1920928955078125e-07f / 8);
-      return f2u(-(1.0f * logf_(y)));
-    }
-    if (type == 2) {
-      const float ux = Uf(0), vx = Uf(1) + 1.1920928955078125e-07f / 8;
-      const float lv = logf_(vx);
-      const bool c = ux < g.f_px;
-      if (!ACC) return f2u(1.0f * (c ? expf_(g.f_inv * lv) : 1.0f - lv));
-      const float e1 = expf_(c ? g.f_inv * lv : logf_(1.0f - lv) * g.f_am1);  // one exp for both branches
-      acc = Uf(2) < (c ? expf_(-e1) : e1);
-      return f2u(1.0f * (c ? e1 : 1.0f - lv));
-    }
-    const float a1 = g.f_am1, sq = g.f_sq;
-    float ys, yc;
-    sincosf_((float)3.1415926535897932 * Uf(0), ys, yc);
-    const float yx = ys / yc;
-    const float xx = sq * yx + a1;
-    if (ACC) {
-      const float ub = (yx * yx + 1.0f) * expf_(a1 * logf_(xx / a1) - yx * sq);
-      acc = (0.0f < xx) && (Uf(1) <= ub);
-    }
-    return f2u(1.0f * xx);
-  } else {
-    if (type == 0) return d2u(1.0 * (-(log_(1.0 - Ud(0)) / 1.0)));
-    if (type == 1) {
-      double y = Ud(0) + 2.220446049250313e-16 / 8;
-      for (int t = 1; t < U; ++t) y = y * (Ud(t) + 2.220446049250313e-16 / 8);
-      return d2u(-(1.0 * log_(y)));
-    }
-    if (type == 2) {
-      const double ux = Ud(0), vx = Ud(1) + 2.220446049250313e-16 / 8;
-      const double lv = log_(vx);
-      double xx;
-      if (ux < g.d_px) {
-        xx = exp_(g.d_inv * lv);
-        if (ACC) acc = Ud(2) < exp_(-xx);
-      } else {
-        xx = 1.0 - lv;
-        if (ACC) acc = Ud(2) < exp_(log_(xx) * g.d_am1);
-      }
-      return d2u(1.0 * xx);
-    }
-    const double a1 = g.d_am1, sq = g.d_sq;
-    double ys, yc;
-    sincos_(3.1415926535897932 * Ud(0), ys, yc);
-    const double yx = ys / yc;
-    const double xx = sq * yx + a1;
-    if (ACC) {
-      const double ub = (yx * yx + 1.0) * exp_(a1 * log_(xx / a1) - yx * sq);
-      acc = (0.0 < xx) && (Ud(1) <= ub);
-    }
-    return d2u(1.0 * xx);
-  }
-}
-
 }  // namespace
 
 // ===========================================================================
@@ -2132,8 +1858,6 @@ __device__ __forceinline__ uint64_t beta_comp_u(const BetaComp g, const int type
 namespace {
 
 constexpr int kBcThreads = 192;       // four CTAs per SM
-constexpr int kBcThreadsAlone = 512;  // one CTA per SM (no more engines than SMs): fifteen worker warps
-constexpr uint16_t kBcTabNone = 0xffffu;  // visit-table entry not known yet
 constexpr int kBcRec = 160;         // output packets per step (a block holds at most 156)
 constexpr int kBcFifo = 112;        // FIFO outputs per component per step (at most 104 per block)
 constexpr int kBcFull = 112;        // full-trial outputs of the buffered component per step
@@ -2149,10 +1873,9 @@ struct BcStep {
   int nrec, nf, fs[2], A[2], f[2];
 };
 
-template <int DT, bool TAB>
+template <int DT>
 __host__ __device__ constexpr size_t bc_smem_bytes() {
-  return (TAB ? (size_t)kBetaRing * beta_lanes<DT>() * 2 + (size_t)2 * kBcRec * 6 : 0) +  // visit table, record starts
-         (size_t)3 * kLanes * kN * 8 +                                                   // raw windows
+  return (size_t)3 * kLanes * kN * 8 +                                                   // raw windows
          ((size_t)2 * bc_lb<DT>() + (size_t)(kBcFull + kBcRec) * beta_lanes<DT>()) *     // lane buffers, full-
              (DT == SD_F64 ? 8 : 4) +                                                    //   trial and positional values
          (size_t)2 * kBcRec * 2 * 2 +                                                    // records
@@ -2163,17 +1886,10 @@ __host__ __device__ constexpr size_t bc_smem_bytes() {
 
 }  // namespace
 
-// ALONE: one CTA per SM.  For the GS + integral-alpha pairs it also keeps a
-// visit table: for every position and carry, where the GS visit starting
-// there ends, whether on a full trial, and the lanes its partial trials
-// accept.  The chase then reads one entry per record, and the workers
-// expand each record's partial trials into FIFO slots themselves.
-template <int DT, int TY0, int TY1, bool ALONE>  // DT: SD_F32 or SD_F64
+template <int DT, int TY0, int TY1>  // DT: SD_F32 or SD_F64
 __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks) {
-  constexpr int NT = ALONE ? kBcThreadsAlone : kBcThreads;
+  constexpr int NT = kBcThreads;
   constexpr int kBcWork = NT - 32;
-  constexpr bool kFusedPair = (TY0 == 2 && TY1 == 1) || (TY0 == 1 && TY1 == 2);
-  constexpr bool TAB = ALONE && kFusedPair;
   constexpr int P = beta_lanes<DT>();
   constexpr int LB = bc_lb<DT>();
   constexpr unsigned FULL = 0xffffffffu;
@@ -2187,22 +1903,16 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
   int16_t* fpos = rec + 2 * kBcRec * 2;                                  // [2][kBcFull]
   uint16_t* ptask = reinterpret_cast<uint16_t*>(fpos + 2 * kBcFull);     // [2][2][LB]
   uint8_t* pmask = reinterpret_cast<uint8_t*>(ptask + 2 * 2 * LB);       // [2][kBetaRing]
-  uint16_t* vtab = reinterpret_cast<uint16_t*>(pmask + 2 * kBetaRing);    // [kBetaRing][P] (TAB)
-  int16_t* rxs = reinterpret_cast<int16_t*>(vtab + (TAB ? kBetaRing * P : 0));  // [2][kBcRec] visit starts (TAB)
-  uint16_t* ras = reinterpret_cast<uint16_t*>(rxs + (TAB ? 2 * kBcRec : 0));    // [2][kBcRec] FIFO tail at the start
-  uint16_t* rfs = ras + (TAB ? 2 * kBcRec : 0);                                 // [2][kBcRec] carry at the start
   __shared__ BcStep s_step[2];
   __shared__ int s_done, s_err, s_fc[2];
   __shared__ int64_t s_end;
-  __shared__ unsigned long long s_inv[2];  // TAB: first position whose table entry is still unknown
 
   const int k = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   EngState* st = p.eng + k;
   GenState* gs = p.gen + k;
-  const int64_t g0 = (int64_t)k * p.gran_per_k + min((int64_t)k, p.gran_rem);
-  const int64_t ng = p.gran_per_k + ((int64_t)k < p.gran_rem ? 1 : 0);
-  const int64_t off = g0 * p.gran, n = ng * p.gran;
+  int64_t off, n;
+  slice_left(p, k, off, n);
   if (n == 0) return;
   const int64_t Npk = n / P;
 
@@ -2338,7 +2048,13 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
         bool acc = false;
         if (valid) {
           int f = -1;
-          if (DT == SD_F64 && ty == 2)  // float pre-test of a double GS trial
+          if (DT == SD_F32 && ty == 2) {  // special-function pre-test of a GS trial
+            const BetaComp& g = c == 0 ? bk.c[0] : bk.c[1];
+            const int sh = (j & 1) * 32;
+            f = gs_filter(ur_f((uint32_t)(w0 >> sh)), ur_f((uint32_t)(w1 >> sh)) + 1.1920928955078125e-07f / 8,
+                          ur_f((uint32_t)(w2 >> sh)), g.f_px, g.f_inv, g.f_am1, g.f_band);
+          }
+          if (DT == SD_F64 && ty == 2)
             f = c == 0 ? gs_filter_f64(w0, w1, w2, bk.c[0].f_px, bk.c[0].f_inv, bk.c[0].f_am1, bk.c[0].f_band)
                        : gs_filter_f64(w0, w1, w2, bk.c[1].f_px, bk.c[1].f_inv, bk.c[1].f_am1, bk.c[1].f_band);
           if (f >= 0) {
@@ -2360,47 +2076,10 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
       }
     }
   };
-  // TAB: visit-table entries of positions [from, to) (masks known below
-  // `to`), by threads t = 0 .. T-1; an entry whose visit runs past `to` stays
-  // unknown and its position is noted in *inv
-  constexpr int gcomp = TY0 == 2 ? 0 : 1;  // the GS component of a fused pair
-  auto build_table = [&](int64_t from, int64_t to, int t, int T, unsigned long long* inv) {
-    if (!TAB || to <= from) return;
-    const int U = gcomp == 0 ? U0 : U1;
-    const int cnt = (int)(to - from) * P;
-    for (int u = t; u < cnt; u += T) {
-      const int64_t x = from + u / P;
-      const int f = u % P;
-      uint16_t e = kBcTabNone;
-      int acc = 0;
-      for (int d = 0; d < 1024 - U; d += U) {
-        const int64_t xr = x + d;
-        if (xr >= to) break;
-        const uint32_t m = pmask[gcomp * kBetaRing + (int)(xr & (kBetaRing - 1))];
-        const int cn = __popc(m);
-        if (cn == P) {
-          e = (uint16_t)(d | (1 << 10) | (acc << 11));
-          break;
-        }
-        acc += cn;
-        if (f + acc >= P) {
-          e = (uint16_t)(d | (acc << 11));
-          break;
-        }
-      }
-      vtab[(int)(x & (kBetaRing - 1)) * P + f] = e;
-      if (e == kBcTabNone) atomicMin(inv, (unsigned long long)x);
-    }
-  };
   // block 0 and its masks (all threads)
   mt_block(raw[2], raw[0], [&](int, const uint64_t*) {});
   set_ring(0);
   masks(0, kN - umax + 1, tid, NT);
-  if (TAB) {
-    if (tid == 0) s_inv[0] = (unsigned long long)(kN - umax + 1);
-    __syncthreads();
-    build_table(0, kN - umax + 1, tid, NT, &s_inv[0]);
-  }
   __syncthreads();
 
   // chase state (warp 0, the same in every lane)
@@ -2423,9 +2102,6 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
         int16_t* rq = rec + q * kBcRec * 2;
         int16_t* fq = fpos + q * kBcFull;
         uint16_t* tq = ptask + q * 2 * LB;
-        int16_t* xq = rxs + q * kBcRec;
-        uint16_t* aq = ras + q * kBcRec;
-        uint16_t* fsq = rfs + q * kBcRec;
         const int64_t base = cx, e0 = cE;
         const int fs0 = cf[0], fs1 = cf[1];
         int nrec = 0, nf = 0, A[2] = {cf[0], cf[1]};
@@ -2449,40 +2125,6 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
               const int fsc = c == 0 ? fs0 : fs1;
               int acc = 0;
               int xr = (int)(cx - base);  // trial position relative to the step
-              if (TAB) {
-                // one table entry: the visit's end, its kind and the lanes its
-                // partial trials accept; the workers place those lanes
-                if (xr >= Mr) return 2;
-                const uint32_t e = vtab[((bm + xr) & (kBetaRing - 1)) * P + cf[c]];
-                if (e == kBcTabNone) return 2;
-                acc = (int)(e >> 11);
-                if (A[c] + acc > LB) return 1;
-                const int xe = xr + (int)(e & 1023u);
-                if (lane == 0) {
-                  xq[nrec] = (int16_t)xr;
-                  aq[nrec] = (uint16_t)A[c];
-                  fsq[nrec] = (uint16_t)cf[c];
-                }
-                if (e & (1u << 10)) {
-                  if (c == bc) {
-                    if (nf >= kBcFull) return 1;
-                    if (lane == 0) {
-                      fq[nf] = (int16_t)xe;
-                      rq[nrec * 2 + c] = (int16_t)(kBcFullTag + nf);
-                    }
-                    ++nf;
-                  } else if (lane == 0) {
-                    rq[nrec * 2 + c] = (int16_t)xe;
-                  }
-                  cf[c] += acc;
-                } else {
-                  if (lane == 0) rq[nrec * 2 + c] = (int16_t)(-(1 + (A[c] - cf[c])));
-                  cf[c] += acc - P;
-                }
-                A[c] += acc;
-                cx = base + xe + U;
-                return 0;
-              }
               for (;;) {
                 if (xr >= Mr) return 2;
                 const uint32_t m = pmask[c * kBetaRing + ((bm + xr) & (kBetaRing - 1))];
@@ -2563,29 +2205,6 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
         const int16_t* rq = rec + q * kBcRec * 2;
         uint16_t* tq = ptask + q * 2 * LB;
         set_ring(t);
-        if (TAB) {
-          // the accepted lanes of each record's partial trials at their FIFO
-          // slots (the visit walked again from its start)
-          const int U = gcomp == 0 ? U0 : U1;
-          const int bmq = (int)(base & (kBetaRing - 1));
-          const int fsg = gcomp == 0 ? fs0 : fs1;
-          for (int i = tt; i < nrec; i += kBcWork) {
-            int xr = rxs[q * kBcRec + i], run = 0;
-            const int a0 = ras[q * kBcRec + i] - fsg, f0 = rfs[q * kBcRec + i];
-            for (int d = 0; d < 1024; d += U, xr += U) {
-              const uint32_t m = pmask[gcomp * kBetaRing + ((bmq + xr) & (kBetaRing - 1))];
-              const int cn = __popc(m);
-              if (cn == P) break;
-              for (uint32_t mm = m; mm; mm &= mm - 1) {
-                const int j = __ffs(mm) - 1;
-                tq[gcomp * LB + a0 + run + __popc(m & ((1u << j) - 1u))] = (uint16_t)((xr << 3) | j);
-              }
-              run += cn;
-              if (f0 + run >= P) break;
-            }
-          }
-          asm volatile("bar.sync 1, %0;" ::"r"(kBcWork) : "memory");
-        }
         // one task list, one lane per thread: full trials of the buffered
         // component, the accepted partial-trial lanes, positional values of
         // the other component
@@ -2668,17 +2287,6 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
         asm volatile("bar.sync 1, %0;" ::"r"(kBcWork) : "memory");
         set_ring(t + 1);
         masks(M, M + kN, tt, kBcWork);
-        if (TAB) {
-          // entries still unknown from the last build and the new positions;
-          // positions below (t - 1) * kN are behind any chase that has not
-          // failed, so their entries are never read again
-          const int q1 = (int)((t + 1) & 1);
-          if (tt == 0) s_inv[q1] = (unsigned long long)(M + kN);
-          asm volatile("bar.sync 1, %0;" ::"r"(kBcWork) : "memory");
-          int64_t from = (int64_t)min(s_inv[t & 1], (unsigned long long)M);
-          from = max(from, (t - 1) * (int64_t)kN);
-          build_table(from, M + kN, tt, kBcWork, &s_inv[q1]);
-        }
       }
     }
     __syncthreads();
@@ -2746,40 +2354,25 @@ static cudaError_t run_beta(const Plan& p, const DistParams& d, int64_t max_bloc
   bk.fpost = d.fh;
   bk.dpost = d.dh;
   static bool attr[64] = {};
-  static int sms[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  constexpr size_t smem = bc_smem_bytes<DT, false>(), smem_t = bc_smem_bytes<DT, true>();
+  constexpr size_t smem = bc_smem_bytes<DT>();
   if (!attr[dev]) {
-    cudaError_t e = cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
+    cudaError_t e = cudaFuncSetAttribute(k_beta<DT, -1, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_beta<DT, -1, -1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      e = cudaFuncSetAttribute(k_beta<DT, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_beta<DT, 2, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_beta<DT, 1, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_beta<DT, 2, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_beta<DT, 1, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t);
+      e = cudaFuncSetAttribute(k_beta<DT, 1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     attr[dev] = true;
   }
   // the GS + integral-alpha pairs (beta(a < 1, integer b) and the mirror)
-  // have kernels of their own; with no more engines than SMs each engine's
-  // CTA has an SM to itself and runs the visit-table form
+  // have kernels of their own
   const int t0 = bk.c[0].type, t1 = bk.c[1].type;
-  const bool alone = p.K <= sms[dev];
-  if (t0 == 2 && t1 == 1) {
-    if (alone) k_beta<DT, 2, 1, true><<<p.K, kBcThreadsAlone, smem_t, s>>>(p, bk, max_blocks);
-    else k_beta<DT, 2, 1, false><<<p.K, kBcThreads, smem, s>>>(p, bk, max_blocks);
-  } else if (t0 == 1 && t1 == 2) {
-    if (alone) k_beta<DT, 1, 2, true><<<p.K, kBcThreadsAlone, smem_t, s>>>(p, bk, max_blocks);
-    else k_beta<DT, 1, 2, false><<<p.K, kBcThreads, smem, s>>>(p, bk, max_blocks);
-  } else {
-    k_beta<DT, -1, -1, false><<<p.K, kBcThreads, smem, s>>>(p, bk, max_blocks);
-  }
+  if (t0 == 2 && t1 == 1) k_beta<DT, 2, 1><<<p.K, kBcThreads, smem, s>>>(p, bk, max_blocks);
+  else if (t0 == 1 && t1 == 2) k_beta<DT, 1, 2><<<p.K, kBcThreads, smem, s>>>(p, bk, max_blocks);
+  else k_beta<DT, -1, -1><<<p.K, kBcThreads, smem, s>>>(p, bk, max_blocks);
   return cudaGetLastError();
 }
 
