@@ -639,18 +639,19 @@ gr_status prepare_segments(gr_engine* e, Plan& p, int S, int64_t J, int delta, c
 constexpr int64_t kWordsCap = (int64_t)1 << 22;  // packets of all engines (128 MB: about one L2)
 
 // Segments for n packets per engine.  In a row a lane makes 156 words in
-// about 16 ns; a segment more costs the jump kernel about 0.25 us of the whole
-// GPU per engine, and the prefix and its launches about 10 us once.
+// about 16 ns; a segment more costs the jump kernel about 1.9 us of the whole
+// GPU per engine, and the prefix, the jump kernel's shortest run and their
+// launches about 25 us once.
 void plan_words(int K, int64_t n, int& S, int64_t& J) {
   S = 1;
   J = n + (n & 1);
   double best = (double)n * 0.1;  // ns
-  for (int m = 12; m <= 24; ++m) {
+  for (int m = 14; m <= 24; ++m) {
     const int64_t j = (int64_t)1 << m;
     const int64_t segs = (n + j - 1) / j;
     if (segs < 2) break;
     if (segs > 128 || segs * K > 1024) continue;
-    const double cost = (double)j * 0.1 + (double)(segs - 1) * K * 250.0 + 10000.0;
+    const double cost = (double)j * 0.1 + (double)(segs - 1) * K * 1900.0 + 25000.0;
     if (cost < best) {
       best = cost;
       S = (int)segs;
@@ -878,6 +879,69 @@ double gamma_yield(int branch, double a) {
   return std::exp(std::lgamma(a) + b - b * std::log(b)) / (3.141592653589793 * std::sqrt(2 * a - 1));
 }
 
+// Expected share of accepted candidate lanes of a rejection family, and how far
+// off it may be, relatively.
+double expected_yield(int rk, const DistParams& d, double& slack) {
+  slack = 0;
+  if (rk <= 1) return gamma_yield(rk == 0 ? 2 << 8 : 3 << 8, d.dtype == GR_F64 ? d.da : (double)d.fa);
+  slack = 0.04;
+  return reject_yield(rk, d);
+}
+
+// Rejection samplers through words in memory (gr_rejw.cu), then the
+// one-CTA-per-engine kernel for whatever the planned trials did not make
+// (usually nothing).
+constexpr int64_t kRejectMin = 512;              // output packets per engine
+constexpr int kRejectMaxK = 256;                 // engines
+constexpr int64_t kRejectCap = (int64_t)1 << 23;  // packets of words at a time, all engines
+gr_status run_reject_call(gr_engine* e, const Plan& p0, const DistParams& dp, int rk, int64_t npk, int64_t max_blocks,
+                          cudaStream_t stream) {
+  double slack = 0;
+  const double q = expected_yield(rk, dp, slack);
+  // GR_REJECT_PLAN_SCALE (tests) scales the planned trials; below 1 the
+  // one-CTA kernel makes the rest, which must give the same result
+  const char* sc = std::getenv("GR_REJECT_PLAN_SCALE");
+  const double scale = sc ? std::max(0.0, std::atof(sc)) : 1.0;
+  int64_t left = (int64_t)std::ceil(((double)npk + 8.0 * std::sqrt((double)npk)) / q * (1.0 + slack) * scale) + 16;
+  const int64_t U = rk == 0 ? 3 : (rk >= 3 ? 1 : 2);  // packets per trial
+  Plan p = p0;
+  int64_t* done = nullptr;
+  cudaError_t err = scratch_alloc(reinterpret_cast<void**>(&done), sizeof(int64_t) * (size_t)e->K, e->device, stream);
+  if (err != cudaSuccess) return cuda_fail(err, "scratch memory");
+  err = cudaMemsetAsync(done, 0, sizeof(int64_t) * (size_t)e->K, stream);
+  gr_status st = err == cudaSuccess ? GR_OK : cuda_fail(err, "rejection sampler");
+  const int64_t chunk = std::max<int64_t>(kRejectCap / e->K / U, 64);
+  while (st == GR_OK && left > 0) {
+    const int64_t T = std::min(chunk, left);
+    left -= T;
+    const RwLayout L = reject_words_layout(e->K, T);
+    void *words = nullptr, *scratch = nullptr;
+    bool got = false;
+    err = scratch_alloc(&scratch, L.bytes, e->device, stream);
+    if (err != cudaSuccess) {
+      cudaGetLastError();
+      break;
+    }
+    st = make_words(e, p, T * U, true, &words, &got, stream);
+    if (st == GR_OK && got) {
+      err = launch_reject_words(p, dp, rk, e->snap, L, static_cast<char*>(scratch), done, stream);
+      if (err != cudaSuccess) st = cuda_fail(err, "rejection sampling kernels");
+      cudaFreeAsync(words, stream);
+    }
+    cudaFreeAsync(scratch, stream);
+    p.words = nullptr;
+    if (!got) break;
+  }
+  if (st == GR_OK) {
+    p.done = done;
+    p.S = 1;
+    err = launch_reject(p, dp, rk, max_blocks, stream);
+    if (err != cudaSuccess) st = cuda_fail(err, "rejection sampling kernel");
+  }
+  cudaFreeAsync(done, stream);
+  return st;
+}
+
 // BetaGen's general branch through words in memory (gr_chain.cu), then the
 // one-CTA-per-engine walk for whatever the planned packets did not hold
 // (usually nothing).  The expected packets per output only size the plan.
@@ -1063,43 +1127,8 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
     const int64_t wt = rk == 0 ? 24 : (rk >= 3 ? 8 : 16);  // words per trial
     const int64_t npk = nk_max / P;
     const int64_t max_blocks = block_cap(((16 * npk + 4096) * wt) / (kN * 8) + 64);
-    if (e->K < 16 && npk >= ((int64_t)1 << 12)) {
-      // long call on few engines: jump-ahead segments over the trial stream
-      const double q = reject_yield(rk, dp);
-      // GR_REJECT_PLAN_SCALE (tests) scales the planned trials; below 1 the
-      // last segment runs on past its plan, which must give the same result
-      const char* sc = std::getenv("GR_REJECT_PLAN_SCALE");
-      const double scale = sc ? std::max(0.0, std::atof(sc)) : 1.0;
-      const int64_t t_need = (int64_t)std::ceil((double)npk / q * 1.04 * scale) + 256;
-      const int64_t smax = std::max(2, 128 / e->K);
-      const int64_t Ts = std::max<int64_t>((t_need + smax - 1) / smax, 2048);
-      const int S = (int)((t_need + Ts - 1) / Ts);
-      if (S >= 2) {
-        const int64_t J = Ts * (wt / 8);
-        gr_status st = prepare_segments(e, p, S, J, dp.dtype == GR_I32 ? 1 : 0, stream);
-        if (st != GR_OK) return st;
-        RsArgs a{};
-        a.Ts = Ts;
-        a.lane_cap = P * (npk + 2) + 16;
-        a.pos_cap = npk + 2;
-        a.max_blocks = max_blocks;
-        const size_t K = (size_t)e->K;
-        // lane buffer: K * lane_cap lanes of 8 (double) or 4 bytes
-        const size_t lane_words = dp.dtype == GR_F64 ? K * (size_t)a.lane_cap : (K * (size_t)a.lane_cap + 1) / 2;
-        const size_t words = K * S * 4 + K * 4 + lane_words + K * (size_t)a.pos_cap;
-        int64_t* buf = nullptr;
-        GR_CUDA(cudaMallocAsync(&buf, sizeof(int64_t) * words, stream));
-        a.cnt = buf;
-        a.start = buf + K * S * 2;
-        a.fin = buf + K * S * 4;
-        a.lanes = reinterpret_cast<uint64_t*>(buf + K * S * 4 + K * 4);
-        a.pos = buf + K * S * 4 + K * 4 + lane_words;
-        cudaError_t err = launch_reject_segmented(p, dp, rk, e->snap, a, a.lane_cap, stream);
-        cudaFreeAsync(buf, stream);
-        if (err != cudaSuccess) return cuda_fail(err, "segmented rejection kernels");
-        return GR_OK;
-      }
-    }
+    if (e->K <= kRejectMaxK && npk >= kRejectMin)
+      return run_reject_call(e, p, dp, rk, npk, max_blocks, stream);
     cudaError_t err = launch_reject(p, dp, rk, max_blocks, stream);
     if (err != cudaSuccess) return cuda_fail(err, "rejection sampling kernel");
     return GR_OK;

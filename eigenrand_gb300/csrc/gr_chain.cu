@@ -651,32 +651,42 @@ __global__ void __launch_bounds__(kEmitThreads) k_chain_emit(ChainArgs a, int pa
   const uint64_t* w = a.p.words + (size_t)k * kLanes * a.p.wstride;
   const int64_t g0 = (int64_t)k * a.p.gran_per_k + min((int64_t)k, a.p.gran_rem) + a.done[k];
   const uint32_t* rec = a.rec + ((size_t)k * Sg + s) * a.L.rcap;
-  for (int64_t u = i0 * P + threadIdx.x; u < i1 * P; u += kEmitThreads) {
-    const int64_t i = u / P;
+  for (int64_t u0 = i0 * P; u0 < i1 * P; u0 += kEmitThreads) {
+    const int64_t u = u0 + threadIdx.x, i = u / P;
+    const bool valid = u < i1 * P;
     const int j = (int)(u % P);
-    const uint32_t r = CLOSED ? 0 : __ldg(rec + i);
+    const uint32_t r = (CLOSED || !valid) ? 0 : __ldg(rec + i);
     int x = CLOSED ? (int)(i * (U0 + U1)) : (int)(r & 0xffffffu);
-    uint64_t v[2];
+    uint32_t pos[2];
+    int lane[2];
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-      uint32_t pos = (uint32_t)x;
-      int lane = j;
+      pos[c] = (uint32_t)x;
+      lane[c] = j;
       if (c ? R1 : R0) {
-        const int f = (int)((r >> (c ? 27 : 24)) & 7u);
-        const Visits vis = visits_of<DT>(a, k, c, R0, R1);
-        int last, pushed;
-        if (vis.scan(x, f, j - f, last, pushed, pos, lane)) {
-          pos = (uint32_t)last;
-          lane = j;
-        } else if (j < f) {
-          carried_lane<DT>(a, k, c, R0, R1, s, i, f - j, pos, lane);
+        if (valid) {
+          const int f = (int)((r >> (c ? 27 : 24)) & 7u);
+          const Visits vis = visits_of<DT>(a, k, c, R0, R1);
+          int last, pushed;
+          if (vis.scan(x, f, j - f, last, pushed, pos[c], lane[c])) {
+            pos[c] = (uint32_t)last;
+            lane[c] = j;
+          } else if (j < f) {
+            carried_lane<DT>(a, k, c, R0, R1, s, i, f - j, pos[c], lane[c]);
+          }
+          x = last + vis.U;
         }
-        x = last + vis.U;
       } else {
         x += c ? U1 : U0;
       }
-      v[c] = chain_value<DT, T0, T1>(a, w, k, c, pos, lane);
     }
+    // the searches take different times: the warp meets again before the
+    // values, which are most of the work
+    __syncwarp();
+    if (!valid) continue;
+    uint64_t v[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) v[c] = chain_value<DT, T0, T1>(a, w, k, c, pos[c], lane[c]);
     const int64_t at = (g0 + eb + i) * P + j;
     if (DT == SD_F32) {
       const float p1 = u2f((uint32_t)v[0]), p2 = u2f((uint32_t)v[1]);

@@ -127,22 +127,18 @@ cudaError_t launch_staged(const Plan& p, const DistParams& d, const CallSnap* sn
 // 2 beta with a,b < 1, 3 poisson mean >= 12, 4 binomial tan proposal.
 cudaError_t launch_reject(const Plan& p, const DistParams& d, int rk, int64_t max_blocks, cudaStream_t s);
 
-// Segmented form of launch_reject for long calls on few engines (see
-// gr_samplers.cu): p.S segments of a.Ts trials per engine, windows from
-// prepare_segments with J = Ts * packets per trial (one packet earlier for the
-// int32 kinds).  gather_n bounds the FIFO lanes of one engine.
-struct RsArgs {
-  int64_t Ts;
-  int64_t* cnt;    // [K * S][2]
-  int64_t* start;  // [K * S][2]
-  int64_t* fin;    // [K][4]
-  uint64_t* lanes; // [K][lane_cap] lanes of 8 bytes (double) or 4 bytes (float / int32)
-  int64_t* pos;    // [K][pos_cap]
-  int64_t lane_cap, pos_cap;
-  int64_t max_blocks;
+// The same over words in memory (gr_rejw.cu): T trials per engine, whose
+// packets p.words holds; output packets made are added to done[k] and the
+// engine and generator state follow.
+struct RwLayout {
+  int64_t T;
+  int32_t tiles;
+  int64_t mstride;
+  size_t o_mask, o_cnt, o_start, o_end, bytes;
 };
-cudaError_t launch_reject_segmented(const Plan& p, const DistParams& d, int rk, const CallSnap* snap, const RsArgs& a,
-                                    int64_t gather_n, cudaStream_t s);
+RwLayout reject_words_layout(int K, int64_t T);
+cudaError_t launch_reject_words(const Plan& p, const DistParams& d, int rk, const CallSnap* snap, const RwLayout& L,
+                                char* scratch, int64_t* done, cudaStream_t s);
 
 // PoissonGen (mean < 12) / BinomialGen (mean < 1) on few engines over S
 // jump-ahead segments of J packets per engine (gr_samplers.cu): a scan per

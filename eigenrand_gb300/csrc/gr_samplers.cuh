@@ -202,6 +202,43 @@ __device__ __forceinline__ bool rej_trial(const DistParams& d, int64_t t, int j,
         return acc;
 }
 
+// The candidate of a trial's lane that is known to be accepted: rej_trial's
+// expressions for it alone.
+template <int RK, int DT, class WF, class RF>
+__device__ __forceinline__ uint64_t rej_value(const DistParams& d, int64_t t, int j, WF&& word, RF&& rval) {
+  constexpr int Wt = (RK == RK_GAMMA_GS) ? 3 * 8 : (RK == RK_POISSON || RK == RK_BINOMIAL) ? 8 : 2 * 8;
+  const int64_t w0 = t * Wt;
+  if (DT == SD_F32) {
+    if (RK == RK_GAMMA_GS) {
+      const float lv = logf_(ur_f(word(w0 + 8 + j)) + 1.1920928955078125e-07f / 8);
+      return f2u(d.fb * (ur_f(word(w0 + j)) < d.fe ? expf_(d.fc * lv) : 1.0f - lv));
+    }
+    if (RK == RK_GAMMA_TAN) {
+      float ys, yc;
+      sincosf_((float)3.1415926535897932 * ur_f(word(w0 + j)), ys, yc);
+      return f2u(d.fb * (d.ff * (ys / yc) + d.fd));
+    }
+    const float p1 = expf_(logf_(ur_f(word(w0 + j))) * d.fc);
+    const float p2 = expf_(logf_(ur_f(word(w0 + 8 + j))) * d.fd);
+    return f2u(p1 / (p1 + p2));
+  }
+  if (DT == SD_F64) {
+    const int64_t r0 = (t * Wt / 8) * 4 + j;
+    if (RK == RK_GAMMA_GS) return d2u(d.db * gs_value_f64(rval(r0), rval(r0 + 4), d2u(d.dg), d.dc));
+    if (RK == RK_GAMMA_TAN) {
+      double ys, yc;
+      sincos_(3.1415926535897932 * ur_d(rval(r0)), ys, yc);
+      return d2u(d.db * (d.df * (ys / yc) + d.dd));
+    }
+    const double p1 = exp_(log_(ur_d(rval(r0))) * d.dc);
+    const double p2 = exp_(log_(ur_d(rval(r0 + 4))) * d.dd);
+    return d2u(p1 / (p1 + p2));
+  }
+  float ys, yc;
+  sincosf_((float)3.1415926535897932 * ur_f(word(w0 + j)), ys, yc);
+  return f2u(truncf(d.fa * (ys / yc) + d.fb));
+}
+
 template <int DT>
 __host__ __device__ constexpr int beta_lanes() {
   return DT == SD_F64 ? 4 : 8;
