@@ -879,6 +879,61 @@ double gamma_yield(int branch, double a) {
   return std::exp(std::lgamma(a) + b - b * std::log(b)) / (3.141592653589793 * std::sqrt(2 * a - 1));
 }
 
+// Fixed units over words in memory.
+constexpr int64_t kStagedMin = 624;               // packets per engine
+constexpr int kStagedMaxK = 128;                  // engines
+constexpr int64_t kStagedCap = (int64_t)1 << 22;  // packets of words at a time, all engines
+
+// PoissonGen's walk through words in memory (gr_chain.cu), then the one-CTA
+// walk for whatever the planned packets did not hold.
+constexpr int64_t kPoisMin = 512;               // output packets per engine
+constexpr int64_t kPoisCap = (int64_t)1 << 22;  // packets of words at a time, all engines
+gr_status run_poisson_call(gr_engine* e, const Plan& p0, const DistParams& wd, int64_t npk, int64_t max_blocks,
+                           cudaStream_t stream) {
+  const char* sc = std::getenv("GR_WALK_PLAN_SCALE");  // tests: see run_chain_call
+  const double scale = sc ? std::max(0.0, std::atof(sc)) : 1.0;
+  const double hl = poisson_step_halves(wd.fe);
+  int64_t left = (int64_t)std::ceil(((double)npk + 4.0 * std::sqrt((double)npk)) * hl * 0.5 * 1.03 * scale) + 64;
+  Plan p = p0;
+  int64_t* done = nullptr;
+  cudaError_t err = scratch_alloc(reinterpret_cast<void**>(&done), sizeof(int64_t) * (size_t)e->K, e->device, stream);
+  if (err != cudaSuccess) return cuda_fail(err, "scratch memory");
+  err = cudaMemsetAsync(done, 0, sizeof(int64_t) * (size_t)e->K, stream);
+  gr_status st = err == cudaSuccess ? GR_OK : cuda_fail(err, "Poisson chain");
+  const int64_t chunk = std::max<int64_t>(kPoisCap / e->K & ~(int64_t)1, 512);
+  while (st == GR_OK && left > 0) {
+    // what a chunk leaves over (less than one step's packets) is made again
+    const int64_t n = std::min(chunk, left + 32 + (left & 1));
+    left -= n - 32;
+    const ChainLayout L = poisson_layout(e->K, n, n > 4096 ? 1024 : 0);
+    void *words = nullptr, *scratch = nullptr;
+    bool got = false;
+    err = scratch_alloc(&scratch, L.bytes, e->device, stream);
+    if (err != cudaSuccess) {
+      cudaGetLastError();
+      break;
+    }
+    st = make_words(e, p, n, true, &words, &got, stream);
+    if (st == GR_OK && got) {
+      err = launch_poisson_words(p, wd, e->snap, L, static_cast<char*>(scratch), done, stream);
+      if (err != cudaSuccess) st = cuda_fail(err, "Poisson chain kernels");
+      cudaFreeAsync(words, stream);
+    }
+    cudaFreeAsync(scratch, stream);
+    p.words = nullptr;
+    if (!got) break;
+  }
+  if (st == GR_OK) {
+    p.words = nullptr;
+    p.done = done;
+    p.S = 1;
+    err = launch_walk(p, wd, max_blocks, stream);
+    if (err != cudaSuccess) st = cuda_fail(err, "walk sampling kernel");
+  }
+  cudaFreeAsync(done, stream);
+  return st;
+}
+
 // Expected share of accepted candidate lanes of a rejection family, and how far
 // off it may be, relatively.
 double expected_yield(int rk, const DistParams& d, double& slack) {
@@ -1153,37 +1208,7 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
       wd.ia = dp.kind == GR_BINOMIAL ? dp.ia : 0;
       wd.ic = dp.kind == GR_BINOMIAL ? dp.ib : 0;
       max_blocks = block_cap((npk * 64) / (2 * kN) + 64);
-      if (e->K < 16 && npk >= ((int64_t)1 << 14)) {
-        // long call on few engines: the step chain over jump-ahead segments
-        const int64_t J = (int64_t)1 << 15;
-        const double hl = poisson_step_halves(wd.fe);
-        // GR_WALK_PLAN_SCALE (tests) scales the planned packets: below 1 the
-        // last segment runs on past its plan, above 1 the call ends in an
-        // earlier segment; the result is the same
-        const char* sc = std::getenv("GR_WALK_PLAN_SCALE");
-        const double scale = sc ? std::max(0.0, std::atof(sc)) : 1.0;
-        const int64_t need = (int64_t)std::ceil((double)npk * hl * 0.5 * 1.03 * scale) + 64;
-        const int S = (int)std::max<int64_t>(2, (need + J - 1) / J);
-        gr_status st = prepare_segments(e, p, S, J, 0, stream);
-        if (st != GR_OK) return st;
-        PwArgs a{};
-        a.J = J;
-        a.snap = e->snap;
-        a.words_per_seg = (2 * J + 1) / 32 + 2;
-        a.max_blocks = max_blocks;
-        const size_t KS = (size_t)e->K * S;
-        const size_t bytes = KS * (4 * 4 + kPwEntries * 2 * 4 + 3 * 8 + (size_t)a.words_per_seg * 4);
-        char* buf = nullptr;
-        GR_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&buf), bytes, stream));
-        a.plan = reinterpret_cast<int64_t*>(buf);
-        a.info = reinterpret_cast<int32_t*>(buf + KS * 3 * 8);
-        a.ent = a.info + KS * 4;
-        a.bits = reinterpret_cast<uint32_t*>(a.ent + KS * kPwEntries * 2);
-        cudaError_t err = launch_poisson_segmented(p, wd, a, stream);
-        cudaFreeAsync(buf, stream);
-        if (err != cudaSuccess) return cuda_fail(err, "segmented Poisson kernels");
-        return GR_OK;
-      }
+      if (e->K <= kChainMaxK && npk >= kPoisMin) return run_poisson_call(e, p, wd, npk, max_blocks, stream);
     } else {
       const bool f32 = dp.dtype == GR_F32;
       wd.ia = gamma_branch(dp.da, f32);
@@ -1207,21 +1232,31 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
   if (dp.kind == GR_STUDENT_T) U = 2;
   if (dp.kind == GR_BINOMIAL) U = dp.ia;
   const int64_t units = nk_max / P;
-  const int64_t packets_max = half ? (units * U + 1) / 2 + 1 : units * U;
-  int S = 1;
-  int64_t Us = std::max<int64_t>(units, 1), J = packets_max;
-  if (e->K < 16 && packets_max >= ((int64_t)1 << 17)) {
-    const int64_t target = std::max<int64_t>(1, 128 / e->K);
-    int64_t us = 2;
-    while (us * target < units || (half ? us * U / 2 : us * U) < ((int64_t)1 << 14)) us <<= 1;
-    Us = us;
-    J = half ? us * U / 2 : us * U;
-    S = (int)((units + us - 1) / us);
+  // few engines: words in memory.  A unit is U words and one value, so the
+  // threshold is a few blocks' worth of packets
+  const int64_t per_u = half ? (U + 1) / 2 : U;
+  if (e->K <= kStagedMaxK && units * per_u > kStagedMin) {
+    const int64_t chunk = std::max<int64_t>(kStagedCap / e->K / per_u, 1);
+    bool started = false;
+    for (int64_t u0 = 0; u0 < units; u0 += chunk) {
+      const int64_t cnt = std::min(chunk, units - u0);
+      void* buf = nullptr;
+      bool got = false;
+      gr_status st = make_words(e, p, half ? (cnt * U + 1) / 2 : cnt * U, true, &buf, &got, stream);
+      if (st != GR_OK) return st;
+      if (!got) {
+        if (started) return fail(GR_ERR_CUDA, "out of memory for the call's scratch");
+        break;
+      }
+      started = true;
+      const cudaError_t err = launch_staged(p, dp, e->snap, U, u0, cnt, stream);
+      cudaFreeAsync(buf, stream);
+      if (err != cudaSuccess) return cuda_fail(err, "staged sampling kernel");
+    }
+    if (started) return GR_OK;
   }
-  const int delta = half ? 1 : 0;
-  gr_status st = prepare_segments(e, p, S, J, delta, stream);
-  if (st != GR_OK) return st;
-  cudaError_t err = launch_staged(p, dp, e->snap, U, Us, delta, stream);
+  p.words = nullptr;
+  const cudaError_t err = launch_staged(p, dp, nullptr, U, 0, units, stream);
   if (err != cudaSuccess) return cuda_fail(err, "staged sampling kernel");
   return GR_OK;
 }

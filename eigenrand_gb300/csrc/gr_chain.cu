@@ -72,7 +72,15 @@ struct ChainArgs {
   int64_t* done;
   int32_t M;       // positions with masks
 };
-constexpr int kNoVisit = 31;  // trials - 1 of a draw that the masks in memory do not finish
+// A visit entry: trials - 1 << 3 | lanes left; with nothing carried (P = 1,
+// PoissonGen's chain) the step's half packets - 1.  kNoVisit: a draw that the
+// positions in memory do not finish.
+template <int P>
+constexpr int kNoVisit = P == 1 ? 255 : 31;
+template <int P>
+__device__ __forceinline__ int visit_trials(uint32_t e) {
+  return P == 1 ? (int)e : (int)(e >> 3);
+}
 
 __device__ __forceinline__ int64_t limit_of(const ChainArgs& a, int k) {
   const int64_t ng = a.p.gran_per_k + ((int64_t)k < a.p.gran_rem ? 1 : 0);
@@ -167,7 +175,7 @@ __global__ void __launch_bounds__(kVisThreads) k_chain_visits(ChainArgs a) {
   const uint8_t* mk = a.mask + ((size_t)k * NR + r) * a.L.mstride;
   uint64_t out = ~0ull;  // every f: no visit
   int cum = 0;
-  for (int t = 0, y = x; t < kNoVisit && y < a.M; ++t, y += U) {
+  for (int t = 0, y = x; t < kNoVisit<P> && y < a.M; ++t, y += U) {
     const int cn = __popc((uint32_t)__ldg(mk + y));
     const bool full = cn == P;
     const int top = P - cum;  // f below this are open
@@ -186,20 +194,20 @@ __global__ void __launch_bounds__(kVisThreads) k_chain_visits(ChainArgs a) {
 // ---------------------------------------------------------------- the chain
 // One output packet from state (x, f0, f1); v0 / v1: the components' visit
 // entries.  False: a draw the masks do not finish.
-template <bool R0, bool R1, class V0, class V1>
+template <int P, bool R0, bool R1, class V0, class V1>
 __device__ __forceinline__ bool chain_step(int& x, int& f0, int& f1, int U0, int U1, V0&& v0, V1&& v1) {
   int y = x + U0, g0 = f0;
   if (R0) {
     const uint32_t e = v0(x, f0);
-    const int t = (int)(e >> 3);
-    if (t == kNoVisit) return false;
+    const int t = visit_trials<P>(e);
+    if (t == kNoVisit<P>) return false;
     y = x + (t + 1) * U0;
-    g0 = (int)(e & 7u);
+    g0 = P == 1 ? 0 : (int)(e & 7u);
   }
   if (R1) {
     const uint32_t e = v1(y, f1);
-    const int t = (int)(e >> 3);
-    if (t == kNoVisit) return false;
+    const int t = visit_trials<P>(e);
+    if (t == kNoVisit<P>) return false;
     y += (t + 1) * U1;
     f1 = (int)(e & 7u);
   } else {
@@ -307,7 +315,7 @@ __global__ void __launch_bounds__(32 * table_warps<P, R0, R1>()) k_chain_table(C
       const uint32_t v = st[i];
       int sx = (int)(v & 0xffffu), c0 = (int)((v >> 16) & 255), c1 = (int)(v >> 24);
       bool ok = v != 0xffffffffu;
-      while (ok && sx < be) ok = chain_step<R0, R1>(sx, c0, c1, U0, U1, v0, v1);
+      while (ok && sx < be) ok = chain_step<P, R0, R1>(sx, c0, c1, U0, U1, v0, v1);
       const int code = ok ? state_code<P, R0, R1>(sx - be, c0, c1) : kEsc;
       st[i] = code == kEsc ? 0xffffffffu : ((uint32_t)sx | (uint32_t)c0 << 16 | (uint32_t)c1 << 24);
       if (code != kEsc) claim[code] = (uint16_t)i;
@@ -393,7 +401,7 @@ __global__ void __launch_bounds__(512) k_chain_compose(ChainArgs a, int up) {
   }
   if (tid == 0) {
     const GenState& gs = a.p.gen[k];
-    int c = state_code<P, R0, R1>(0, R0 ? gs.s[1].rest_cnt : 0, R1 ? gs.s[2].rest_cnt : 0);
+    int c = state_code<P, R0, R1>(0, R0 && P > 1 ? gs.s[1].rest_cnt : 0, R1 ? gs.s[2].rest_cnt : 0);
     for (int q = 0; q < g && c != kEsc; ++q) c = a.gtab[((size_t)k * ng + q) * NS + c];
     s_entry = c;
   }
@@ -427,7 +435,7 @@ __global__ void __launch_bounds__(32) k_chain_walk(ChainArgs a) {
   const int hi = s == Sg - 1 ? INT32_MAX : lo + a.L.J;
   int o = 0, f0 = 0, f1 = 0;
   if (s == 0) {
-    f0 = R0 ? a.p.gen[k].s[1].rest_cnt : 0;
+    f0 = R0 && P > 1 ? a.p.gen[k].s[1].rest_cnt : 0;
     f1 = R1 ? a.p.gen[k].s[2].rest_cnt : 0;
   } else {
     const int code = a.entry[sg];
@@ -467,7 +475,7 @@ __global__ void __launch_bounds__(32) k_chain_walk(ChainArgs a) {
       while (x < stop && nrec < want) {
         const uint32_t r = (uint32_t)x | (uint32_t)f0 << 24 | (uint32_t)f1 << 27;
         int y = x;
-        if (!chain_step<R0, R1>(y, f0, f1, U0, U1, v0, v1) || (R0 && !R1 && y > (int)a.L.n)) {
+        if (!chain_step<P, R0, R1>(y, f0, f1, U0, U1, v0, v1) || (R0 && !R1 && P > 1 && y > (int)a.L.n)) {
           bad = 1;
           break;
         }
@@ -774,7 +782,157 @@ __global__ void __launch_bounds__(256) k_chain_finish(ChainArgs a) {
   }
 }
 
+// ---------------------------------------------------------------- Poisson
+// PoissonGen with mean < 12 (Discrete.h:870-882), also BinomialGen with trials
+// min(p, 1 - p) < 1: one packetOp multiplies half packets of uniforms until
+// every lane's product is <= exp(-mean) and returns, per lane, how many
+// products stayed above it.  A step from half packet x takes L(x) half
+// packets and the next output starts at x + L(x): a chain with nothing
+// carried.  Position 0 is the engine's cached half packet when there is one.
+struct PoisArgs {
+  ChainArgs c;
+  const CallSnap* snap;
+  uint32_t* pos;  // [K][c.L.mstride] the four counts, 6 bits each
+  float thr;      // exp(-mean)
+  int trials, flip;
+};
+constexpr int kPoisLook = 64;  // half packets one step may read (so 6 bits hold a count)
+
+constexpr int kStepThreads = 256;
+__global__ void __launch_bounds__(kStepThreads) k_pois_steps(PoisArgs a) {
+  __shared__ float4 su[kStepThreads + kPoisLook];
+  const int k = blockIdx.y, tid = threadIdx.x;
+  const int x0 = blockIdx.x * kStepThreads;
+  const int cached = a.snap[k].half_valid ? 1 : 0;
+  const uint64_t* w = a.c.p.words + (size_t)k * kLanes * a.c.p.wstride;
+  const int nh = 2 * (int)a.c.p.wcount + cached;  // half packets that exist
+  for (int i = tid; i < kStepThreads + kPoisLook; i += kStepThreads) {
+    const int x = x0 + i;
+    float4 u = make_float4(0, 0, 0, 0);
+    if (x < cached) {
+      const uint32_t* h = a.snap[k].half_cache;
+      u = make_float4(ur_f(h[0]), ur_f(h[1]), ur_f(h[2]), ur_f(h[3]));
+    } else if (x < nh) {
+      const int h = x - cached, l = 2 * (h & 1);
+      const uint64_t p = tw(w, a.c.p.wstride, h >> 1, l), q = tw(w, a.c.p.wstride, h >> 1, l + 1);
+      u = make_float4(ur_f((uint32_t)p), ur_f((uint32_t)(p >> 32)), ur_f((uint32_t)q), ur_f((uint32_t)(q >> 32)));
+    }
+    su[i] = u;
+  }
+  __syncthreads();
+  const int x = x0 + tid;
+  if (x >= a.c.M) return;
+  float v[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+  uint32_t n[4] = {0, 0, 0, 0};
+  bool any = true;
+  int L = 0;
+  while (any && L < kPoisLook) {
+    const float4 u = su[tid + L];
+    v[0] *= u.x;
+    v[1] *= u.y;
+    v[2] *= u.z;
+    v[3] *= u.w;
+    any = false;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const bool c = a.thr < v[j];
+      n[j] += c ? 1u : 0u;
+      any |= c;
+    }
+    ++L;
+  }
+  const size_t at = (size_t)k * a.c.L.mstride + x;
+  // a step longer than the look-ahead, or past what exists, ends the chain
+  a.c.vis[at] = (any || x + L > nh) ? (uint8_t)255 : (uint8_t)(L - 1);
+  a.pos[at] = n[0] | n[1] << 6 | n[2] << 12 | n[3] << 18;
+}
+
+__global__ void __launch_bounds__(256) k_pois_emit(PoisArgs a) {
+  const ChainArgs& c = a.c;
+  const int k = blockIdx.y, s = blockIdx.x, Sg = c.L.Sg;
+  const int64_t limit = limit_of(c, k);
+  const int64_t eb = c.ebase[(size_t)k * (Sg + 1) + s];
+  const int64_t all = min(limit, c.ebase[(size_t)k * (Sg + 1) + s + 1]) - eb;
+  const int64_t g0 = (int64_t)k * c.p.gran_per_k + min((int64_t)k, c.p.gran_rem) + c.done[k] + eb;
+  const uint32_t* rec = c.rec + ((size_t)k * Sg + s) * c.L.rcap;
+  const uint32_t* pos = a.pos + (size_t)k * c.L.mstride;
+  for (int64_t i = threadIdx.x; i < all; i += blockDim.x) {
+    const uint32_t q = __ldg(pos + (rec[i] & 0xffffffu));
+    int v[4] = {(int)(q & 63), (int)((q >> 6) & 63), (int)((q >> 12) & 63), (int)((q >> 18) & 63)};
+    if (a.flip) {  // BinomialGen: trials - res when p > 1/2
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = a.trials - v[j];
+    }
+    reinterpret_cast<int4*>(c.p.out)[g0 + i] = make_int4(v[0], v[1], v[2], v[3]);
+  }
+}
+
+__global__ void __launch_bounds__(256) k_pois_finish(PoisArgs a) {
+  const ChainArgs& c = a.c;
+  const int k = blockIdx.x, tid = threadIdx.x, Sg = c.L.Sg;
+  const int64_t* eb = c.ebase + (size_t)k * (Sg + 1);
+  const int64_t tot = min(limit_of(c, k), eb[Sg]);
+  if (tot <= 0) return;
+  int lo = 0, hi = Sg;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) / 2;
+    if (eb[mid] <= tot - 1) lo = mid;
+    else hi = mid;
+  }
+  const int x = (int)(c.rec[((size_t)k * Sg + lo) * c.L.rcap + (tot - 1 - eb[lo])] & 0xffffffu);
+  const int cached = a.snap[k].half_valid ? 1 : 0;
+  const int fresh = x + c.vis[(size_t)k * c.L.mstride + x] + 1 - cached;  // half packets drawn
+  const int np = (fresh + 1) / 2;
+  EngState* st = c.p.eng + k;
+  const uint64_t* w = c.p.words + (size_t)k * kLanes * c.p.wstride;
+  for (int t = tid; t < kLanes * kN; t += blockDim.x)
+    st->win[t / kN][t % kN] = w[(size_t)(t / kN) * c.p.wstride + np + t % kN];
+  if (tid == 0) {
+    if (fresh & 1) {  // the last packet's upper half stays cached
+      const uint64_t p = tw(w, c.p.wstride, np - 1, 2), q = tw(w, c.p.wstride, np - 1, 3);
+      st->half_cache[0] = (uint32_t)p;
+      st->half_cache[1] = (uint32_t)(p >> 32);
+      st->half_cache[2] = (uint32_t)q;
+      st->half_cache[3] = (uint32_t)(q >> 32);
+    }
+    st->half_valid = fresh & 1;
+    st->consumed += (uint64_t)np;
+    c.done[k] += tot;
+  }
+}
+
 constexpr size_t al(size_t x) { return (x + 255) / 256 * 256; }
+
+// From the visit entries to the recorded chain and the outputs before each
+// segment.
+template <int P, bool R0, bool R1>
+cudaError_t run_core(const ChainArgs& a, cudaStream_t s) {
+  constexpr int NR = (R0 ? 1 : 0) + (R1 ? 1 : 0);
+  const int K = a.p.K, Sg = a.L.Sg;
+  if (Sg > 1) {
+    const size_t tsm = table_smem<P, R0, R1>(a.L.J);
+    const size_t csm = (size_t)a.L.gsz * entry_states<P, R0, R1>() * 2;
+    static bool attr[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (!attr[dev]) {
+      cudaError_t e = cudaFuncSetAttribute(k_chain_table<P, R0, R1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 98304);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_chain_compose<P, R0, R1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 98304);
+      if (e != cudaSuccess) return e;
+      attr[dev] = true;
+    }
+    constexpr int W = table_warps<P, R0, R1>();
+    const int64_t segs = (int64_t)K * Sg;
+    k_chain_table<P, R0, R1><<<(unsigned)((segs + W - 1) / W), 32 * W, tsm, s>>>(a);
+    if (a.L.groups > 1) k_chain_compose<P, R0, R1><<<dim3(a.L.groups, K), 512, csm, s>>>(a, 1);
+    k_chain_compose<P, R0, R1><<<dim3(a.L.groups, K), 512, csm, s>>>(a, 0);
+  }
+  k_chain_walk<P, R0, R1><<<(unsigned)(K * Sg), 32, (size_t)2 * NR * (kTile + kPad) * P, s>>>(a);
+  k_chain_scan<<<K, Sg > 256 ? 1024 : 256, 0, s>>>(a);
+  return cudaGetLastError();
+}
 
 template <int DT, bool R0, bool R1, int T0, int T1>
 cudaError_t run_chain(const ChainArgs& a0, cudaStream_t s) {
@@ -786,28 +944,8 @@ cudaError_t run_chain(const ChainArgs& a0, cudaStream_t s) {
     constexpr int NR = (R0 ? 1 : 0) + (R1 ? 1 : 0);
     k_chain_masks<DT, T0, T1><<<dim3((unsigned)((a.M + kMaskThreads - 1) / kMaskThreads), K), kMaskThreads, 0, s>>>(a);
     k_chain_visits<P, R0, R1><<<dim3((unsigned)((a.M + kVisThreads - 1) / kVisThreads), K * NR), kVisThreads, 0, s>>>(a);
-    if (Sg > 1) {
-      const size_t tsm = table_smem<P, R0, R1>(a.L.J);
-      const size_t csm = (size_t)a.L.gsz * entry_states<P, R0, R1>() * 2;
-      static bool attr[64] = {};
-      int dev = 0;
-      cudaGetDevice(&dev);
-      if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-      if (!attr[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(k_chain_table<P, R0, R1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 98304);
-        if (e == cudaSuccess)
-          e = cudaFuncSetAttribute(k_chain_compose<P, R0, R1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 98304);
-        if (e != cudaSuccess) return e;
-        attr[dev] = true;
-      }
-      constexpr int W = table_warps<P, R0, R1>();
-      const int64_t segs = (int64_t)K * Sg;
-      k_chain_table<P, R0, R1><<<(unsigned)((segs + W - 1) / W), 32 * W, tsm, s>>>(a);
-      if (a.L.groups > 1) k_chain_compose<P, R0, R1><<<dim3(a.L.groups, K), 512, csm, s>>>(a, 1);
-      k_chain_compose<P, R0, R1><<<dim3(a.L.groups, K), 512, csm, s>>>(a, 0);
-    }
-    k_chain_walk<P, R0, R1><<<(unsigned)(K * Sg), 32, (size_t)2 * NR * (kTile + kPad) * P, s>>>(a);
-    k_chain_scan<<<K, Sg > 256 ? 1024 : 256, 0, s>>>(a);
+    const cudaError_t e = run_core<P, R0, R1>(a, s);
+    if (e != cudaSuccess) return e;
   }
   // about 400 output lanes per CTA
   const int64_t lanes = a.L.rcap * (int64_t)P;
@@ -831,22 +969,17 @@ cudaError_t run_chain_types(const ChainArgs& a, cudaStream_t s) {
 
 }  // namespace
 
-ChainLayout chain_layout(const DistParams& d, int K, int64_t n, int32_t J) {
+namespace {
+// M positions of visits, P entries each; NR rejection components, ns entry
+// states per segment; minu: fewest positions of an output.
+ChainLayout layout_of(int K, int64_t n, int64_t M, int32_t J, int P, int NR, int ns, int minu, int pos_bytes) {
   ChainLayout L{};
-  const bool f32 = d.dtype == GR_F32;
-  const int P = f32 ? 8 : 4;
-  const int t0 = d.ia >> 8, t1 = d.ib >> 8, U0 = d.ia & 255, U1 = d.ib & 255;
-  const bool R0 = t0 >= 2, R1 = t1 >= 2, RR = R0 && R1;
   L.n = n;
-  const int64_t M = n - std::max({U0, U1, 3}) + 1;
-  L.Sg = (J > 0 && (R0 || R1) && M > J) ? (int32_t)((M + J - 1) / J) : 1;
-  L.J = L.Sg > 1 ? J : (int32_t)n;
-  L.rcap = (int32_t)(L.J / (U0 + U1) + 2);
-  if (!R0 && !R1) {
-    L.bytes = 0;
-    return L;
-  }
-  L.ns = L.Sg > 1 ? (RR ? 32 * P * P : 64 * P) : 0;
+  L.Sg = (J > 0 && NR && M > J) ? (int32_t)((M + J - 1) / J) : 1;
+  L.J = L.Sg > 1 ? J : (int32_t)std::max<int64_t>(n, M);
+  L.rcap = (int32_t)(L.J / minu + 2);
+  if (!NR) return L;
+  L.ns = L.Sg > 1 ? ns : 0;
   L.gsz = L.ns ? std::max(1, 65536 / (L.ns * 2)) : 0;
   L.groups = L.ns ? (L.Sg + L.gsz - 1) / L.gsz : 0;
   L.mstride = (int64_t)al((size_t)std::max<int64_t>(M, 1) + 256);
@@ -857,8 +990,8 @@ ChainLayout chain_layout(const DistParams& d, int K, int64_t n, int32_t J) {
     o += al(b);
     return at;
   };
-  L.o_mask = take((size_t)K * (RR ? 2 : 1) * L.mstride);
-  L.o_vis = take((size_t)K * (RR ? 2 : 1) * L.mstride * P);
+  L.o_mask = take(pos_bytes ? (size_t)K * L.mstride * pos_bytes : (size_t)K * NR * L.mstride);
+  L.o_vis = take((size_t)K * NR * L.mstride * P);
   L.o_tab = take(segs * L.ns * 2);
   L.o_gtab = take((size_t)K * L.groups * L.ns * 2);
   L.o_entry = take(segs * 4);
@@ -867,6 +1000,48 @@ ChainLayout chain_layout(const DistParams& d, int K, int64_t n, int32_t J) {
   L.o_rec = take(segs * L.rcap * 4);
   L.bytes = o;
   return L;
+}
+}  // namespace
+
+ChainLayout chain_layout(const DistParams& d, int K, int64_t n, int32_t J) {
+  const int P = d.dtype == GR_F32 ? 8 : 4;
+  const int U0 = d.ia & 255, U1 = d.ib & 255;
+  const bool R0 = (d.ia >> 8) >= 2, R1 = (d.ib >> 8) >= 2, RR = R0 && R1;
+  return layout_of(K, n, n - std::max({U0, U1, 3}) + 1, J, P, (R0 ? 1 : 0) + (R1 ? 1 : 0), RR ? 32 * P * P : 64 * P,
+                   U0 + U1, 0);
+}
+
+ChainLayout poisson_layout(int K, int64_t n, int32_t J) {
+  return layout_of(K, n, 2 * n, J, 1, 1, entry_states<1, true, false>(), 1, 4);
+}
+
+cudaError_t launch_poisson_words(const Plan& p, const DistParams& d, const CallSnap* snap, const ChainLayout& L,
+                                 char* scratch, int64_t* done, cudaStream_t s) {
+  PoisArgs a{};
+  a.c.p = p;
+  a.c.bk.c[0].U = 1;
+  a.c.bk.c[1].U = 0;
+  a.c.L = L;
+  a.c.vis = reinterpret_cast<uint8_t*>(scratch + L.o_vis);
+  a.c.tab = reinterpret_cast<uint16_t*>(scratch + L.o_tab);
+  a.c.gtab = reinterpret_cast<uint16_t*>(scratch + L.o_gtab);
+  a.c.entry = reinterpret_cast<int32_t*>(scratch + L.o_entry);
+  a.c.seg = reinterpret_cast<ChainSeg*>(scratch + L.o_seg);
+  a.c.ebase = reinterpret_cast<int64_t*>(scratch + L.o_ebase);
+  a.c.rec = reinterpret_cast<uint32_t*>(scratch + L.o_rec);
+  a.c.done = done;
+  a.c.M = (int32_t)(2 * L.n);
+  a.pos = reinterpret_cast<uint32_t*>(scratch + L.o_mask);
+  a.snap = snap;
+  a.thr = d.fe;
+  a.trials = d.ia;
+  a.flip = d.ic;
+  k_pois_steps<<<dim3((unsigned)((a.c.M + kStepThreads - 1) / kStepThreads), p.K), kStepThreads, 0, s>>>(a);
+  cudaError_t e = run_core<1, true, false>(a.c, s);
+  if (e != cudaSuccess) return e;
+  k_pois_emit<<<dim3((unsigned)L.Sg, p.K), 256, 0, s>>>(a);
+  k_pois_finish<<<p.K, 256, 0, s>>>(a);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_chain(const Plan& p, const DistParams& d, const ChainLayout& L, char* scratch, int64_t* done,

@@ -117,9 +117,9 @@ cudaError_t preload_raw_stream_kernels();
 cudaError_t launch_direct(const Plan& p, const DistParams& d, const CallSnap* snap, cudaStream_t s);
 
 // Multi-packet fixed units (gr_samplers.cu): U packets (or half packets) per
-// unit of P outputs, Us units per jump segment; segment s starts at packet
-// s*J - delta.
-cudaError_t launch_staged(const Plan& p, const DistParams& d, const CallSnap* snap, int U, int64_t Us, int delta,
+// unit of P outputs.  With words in memory (p.words): units [u0, u0 + cnt) of
+// every engine; without, the whole call, one CTA per engine.
+cudaError_t launch_staged(const Plan& p, const DistParams& d, const CallSnap* snap, int U, int64_t u0, int64_t cnt,
                           cudaStream_t s);
 
 // Rejection samplers resolved with CompressMask semantics (gr_samplers.cu);
@@ -139,23 +139,6 @@ struct RwLayout {
 RwLayout reject_words_layout(int K, int64_t T);
 cudaError_t launch_reject_words(const Plan& p, const DistParams& d, int rk, const CallSnap* snap, const RwLayout& L,
                                 char* scratch, int64_t* done, cudaStream_t s);
-
-// PoissonGen (mean < 12) / BinomialGen (mean < 1) on few engines over S
-// jump-ahead segments of J packets per engine (gr_samplers.cu): a scan per
-// segment, a plan per engine, a write per segment.  Scratch per engine and
-// segment; bits: words_per_seg bitmap words per segment.
-constexpr int kPwEntries = 64;  // entry offsets into a segment (the step look-ahead)
-struct PwArgs {
-  int64_t J;                // packets per segment
-  const CallSnap* snap;     // caches at call start, per engine
-  int32_t* info;            // [K*S][4]: exit offset, steps, every entry merged, unused
-  int32_t* ent;             // [K*S][kPwEntries][2]: steps, exit offset
-  int64_t* plan;            // [K*S][3]: entry offset, first output packet, steps
-  uint32_t* bits;           // [K*S][words_per_seg]
-  int64_t words_per_seg;
-  int64_t max_blocks;       // blocks the last segment of an engine may run to
-};
-cudaError_t launch_poisson_segmented(const Plan& p, const DistParams& d, const PwArgs& a, cudaStream_t s);
 
 // Data-dependent consumption (gr_samplers.cu), one CTA per stream: k_poisson
 // for PoissonGen mean < 12 and BinomialGen mean < 1 (int32), k_beta for
@@ -179,6 +162,13 @@ struct ChainLayout {
 ChainLayout chain_layout(const DistParams& d, int K, int64_t n, int32_t J);
 cudaError_t launch_chain(const Plan& p, const DistParams& d, const ChainLayout& L, char* scratch, int64_t* done,
                          cudaStream_t s);
+
+// PoissonGen (mean < 12) / BinomialGen (mean < 1) over words in memory
+// (gr_chain.cu): n packets per engine hold 2 n half packets; d.fe = exp(-mean),
+// d.ia / d.ic: trials - res.  snap: the caches at the start.
+ChainLayout poisson_layout(int K, int64_t n, int32_t J);
+cudaError_t launch_poisson_words(const Plan& p, const DistParams& d, const CallSnap* snap, const ChainLayout& L,
+                                 char* scratch, int64_t* done, cudaStream_t s);
 
 // Samples drawn with a scalar engine as the Urng (gr_kernels.cu): npk output
 // packets from the engine's 64-bit words w (scalar_words_per_packet(kind,

@@ -24,12 +24,61 @@
 
 namespace gr {
 
+// Lane j of unit u (the call's words: word / rword) to output element o.
+template <int KIND, int DT, class WF, class RF>
+__device__ __forceinline__ void staged_value(const Plan& p, const DistParams& d, int U, int64_t u, int j, int64_t o,
+                                             WF&& word, RF&& rword) {
+  const int64_t wpu = (DT == SD_I32H) ? 4 * (int64_t)U : 8 * (int64_t)U;  // u32 words per unit
+  if (DT == SD_F32) {
+    const int64_t w0 = u * wpu + j;  // full kinds: c0w == 0
+    if (KIND == GR_GAMMA || KIND == GR_CHI_SQUARED) {
+      float y = ur_f(word(w0)) + 1.1920928955078125e-07f / 8;
+      for (int t = 1; t < U; ++t) y = y * (ur_f(word(w0 + 8 * t)) + 1.1920928955078125e-07f / 8);
+      reinterpret_cast<float*>(p.out)[o] = -(d.fb * logf_(y));
+    } else if (KIND == GR_STUDENT_T) {
+      const float u1 = 1.0f - ur_f(word(w0));
+      const float u2 = ur_f(word(w0 + 8));
+      // StudentTVGen (NormalExp.h:327-342): n of the element, -2 / n per lane
+      const float nn = (d.flags & kParamVecA) ? __ldg(static_cast<const float*>(d.vparam) + o) : d.fa;
+      const float ex = (d.flags & kParamVecA) ? -2.0f / nn : d.fc;
+      const float radius = sqrtf(nn * (expf_(logf_(u1) * ex) - 1.0f));
+      float sn, cs;
+      sincosf_((float)(2 * 3.1415926535897932) * u2, sn, cs);
+      reinterpret_cast<float*>(p.out)[o] = radius * sn;
+    }
+  } else if (DT == SD_F64) {
+    const int64_t r0 = u * (int64_t)U * 4 + j;
+    if (KIND == GR_GAMMA || KIND == GR_CHI_SQUARED) {
+      double y = ur_d(rword(r0)) + 2.220446049250313e-16 / 8;
+      for (int t = 1; t < U; ++t) y = y * (ur_d(rword(r0 + 4 * t)) + 2.220446049250313e-16 / 8);
+      const double l = log_(y);
+      reinterpret_cast<double*>(p.out)[o] = (d.flags & kParamUnitScale) ? -l : -(d.db * l);
+    } else if (KIND == GR_STUDENT_T) {
+      const double u1 = one_minus_ur_d(rword(r0));
+      const double u2 = ur_d(rword(r0 + 4));
+      const double nn = (d.flags & kParamVecA) ? __ldg(static_cast<const double*>(d.vparam) + o) : d.da;
+      const double ex = (d.flags & kParamVecA) ? -2.0 / nn : d.dc;
+      const double radius = sqrt(nn * (exp_(log_(u1) * ex) - 1.0));
+      double sn, cs;
+      sincos_((2 * 3.1415926535897932) * u2, sn, cs);
+      reinterpret_cast<double*>(p.out)[o] = radius * sn;
+    }
+  } else {  // int32 over half packets
+    const int64_t w0 = u * wpu + j;
+    if (KIND == GR_BINOMIAL) {
+      int32_t res = d.ia;  // trials
+      for (int t = 0; t < U; ++t) res += (d.fa <= ur_f(word(w0 + 4 * t))) ? -1 : 0;
+      reinterpret_cast<int32_t*>(p.out)[o] = res;
+    }
+  }
+}
+
 template <int KIND, int DT>
 __global__ void __launch_bounds__(160)
-    k_staged(Plan p, DistParams d, const CallSnap* snap, int U, int64_t Us, int delta) {
+    k_staged(Plan p, DistParams d, int U) {
   __shared__ uint64_t raw[2][kLanes][kN];
   __shared__ uint64_t tp[2][kN][kLanes];
-  const int k = blockIdx.x / p.S, s = blockIdx.x % p.S;
+  const int k = blockIdx.x;
   const int tid = threadIdx.x;
   EngState* st = p.eng + k;
   constexpr int P = DT == SD_F32 ? 8 : 4;
@@ -43,29 +92,19 @@ __global__ void __launch_bounds__(160)
   int c0w = 0;
   uint32_t cw[4] = {0, 0, 0, 0};
   if (DT == SD_I32H) {
-    const int hv = p.S > 1 ? snap[k].half_valid : st->half_valid;
-    if (hv) {
+    if (st->half_valid) {
       c0w = 4;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) cw[q] = p.S > 1 ? snap[k].half_cache[q] : st->half_cache[q];
+      for (int q = 0; q < 4; ++q) cw[q] = st->half_cache[q];
     }
   }
   const int64_t wpu = (DT == SD_I32H) ? 4 * (int64_t)U : 8 * (int64_t)U;  // u32 words per unit
-  const int64_t Nu = n / P;
-  const int64_t u_beg = (int64_t)s * Us;
-  const int64_t u_end = min(u_beg + Us, Nu);
-  if (u_beg >= Nu) return;
-  const bool last = (u_end == Nu);
-  const int64_t seg_p0 = (s == 0) ? 0 : (int64_t)s * p.J - delta;
+  const int64_t u_end = n / P;
   // last packet holding a word of unit u_end-1
   const int64_t w_last = u_end * wpu - 1 - c0w;
   const int64_t p_last = w_last < 0 ? -1 : w_last / 8;
-  const int64_t np_seg = p_last + 1 - seg_p0;
-
-  // lane windows
-  if (s == 0 && p.S > 1) load_window(raw[0], p.prefix + (size_t)k * kLanes * kPrefixLen, kPrefixLen);
-  else if (s == 0) load_window(raw[0], &st->win[0][0], kN);
-  else load_window(raw[0], p.segwin + ((size_t)k * (p.S - 1) + (s - 1)) * kLanes * kN, kN);
+  const int64_t np_seg = p_last + 1;
+  load_window(raw[0], &st->win[0][0], kN);
   __syncthreads();
 
   int64_t ring_new = 0;  // newest ring block's first packet (ring_packet)
@@ -73,18 +112,14 @@ __global__ void __launch_bounds__(160)
   auto word = [&](int64_t wq) -> uint32_t {  // cache-inclusive u32 word
     if (wq < c0w) return cw[wq];
     const int64_t w = wq - c0w;
-    const int64_t pp = w >> 3;
-    const int64_t rel = pp - seg_p0;
-    const uint64_t v = ring_packet(tp, rel, ring_new, ring_slot)[(w & 7) >> 1];
+    const uint64_t v = ring_packet(tp, w >> 3, ring_new, ring_slot)[(w & 7) >> 1];
     return (w & 1) ? (uint32_t)(v >> 32) : (uint32_t)v;
   };
   auto rword = [&](int64_t r) -> uint64_t {  // u64 lane value r of the packet stream (full kinds)
-    const int64_t pp = r >> 2;
-    const int64_t rel = pp - seg_p0;
-    return ring_packet(tp, rel, ring_new, ring_slot)[r & 3];
+    return ring_packet(tp, r >> 2, ring_new, ring_slot)[r & 3];
   };
 
-  int64_t u_next = u_beg;
+  int64_t u_next = 0;
   int cur = 0;
   int64_t nb = 0;
   for (int64_t base = 0; base < np_seg || (np_seg <= 0 && base == 0); base += kN, ++nb) {
@@ -99,7 +134,7 @@ __global__ void __launch_bounds__(160)
       cur ^= 1; ring_new = nb * kN; ring_slot = slot;
     }
     // units whose last packet is now available
-    const int64_t avail = seg_p0 + base + kN;  // packets [.., avail) exist
+    const int64_t avail = base + kN;  // packets [.., avail) exist
     int64_t u_ready = u_end;
     {
       // largest u with ((u+1)*wpu - 1 - c0w)/8 < avail
@@ -112,80 +147,84 @@ __global__ void __launch_bounds__(160)
       const int64_t u = u_next + e / P;
       const int j = (int)(e % P);
       const int64_t o = off + u * P + j;
-      if (DT == SD_F32) {
-        const int64_t w0 = u * wpu + j;  // full kinds: c0w == 0
-        if (KIND == GR_GAMMA || KIND == GR_CHI_SQUARED) {
-          float y = ur_f(word(w0)) + 1.1920928955078125e-07f / 8;
-          for (int t = 1; t < U; ++t) y = y * (ur_f(word(w0 + 8 * t)) + 1.1920928955078125e-07f / 8);
-          reinterpret_cast<float*>(p.out)[o] = -(d.fb * logf_(y));
-        } else if (KIND == GR_STUDENT_T) {
-          const float u1 = 1.0f - ur_f(word(w0));
-          const float u2 = ur_f(word(w0 + 8));
-          // StudentTVGen (NormalExp.h:327-342): n of the element, -2 / n per lane
-          const float nn = (d.flags & kParamVecA) ? __ldg(static_cast<const float*>(d.vparam) + o) : d.fa;
-          const float ex = (d.flags & kParamVecA) ? -2.0f / nn : d.fc;
-          const float radius = sqrtf(nn * (expf_(logf_(u1) * ex) - 1.0f));
-          float sn, cs;
-          sincosf_((float)(2 * 3.1415926535897932) * u2, sn, cs);
-          reinterpret_cast<float*>(p.out)[o] = radius * sn;
-        }
-      } else if (DT == SD_F64) {
-        const int64_t r0 = u * (int64_t)U * 4 + j;
-        if (KIND == GR_GAMMA || KIND == GR_CHI_SQUARED) {
-          double y = ur_d(rword(r0)) + 2.220446049250313e-16 / 8;
-          for (int t = 1; t < U; ++t) y = y * (ur_d(rword(r0 + 4 * t)) + 2.220446049250313e-16 / 8);
-          const double l = log_(y);
-          reinterpret_cast<double*>(p.out)[o] = (d.flags & kParamUnitScale) ? -l : -(d.db * l);
-        } else if (KIND == GR_STUDENT_T) {
-          const double u1 = one_minus_ur_d(rword(r0));
-          const double u2 = ur_d(rword(r0 + 4));
-          const double nn = (d.flags & kParamVecA) ? __ldg(static_cast<const double*>(d.vparam) + o) : d.da;
-          const double ex = (d.flags & kParamVecA) ? -2.0 / nn : d.dc;
-          const double radius = sqrt(nn * (exp_(log_(u1) * ex) - 1.0));
-          double sn, cs;
-          sincos_((2 * 3.1415926535897932) * u2, sn, cs);
-          reinterpret_cast<double*>(p.out)[o] = radius * sn;
-        }
-      } else {  // int32 over half packets
-        const int64_t w0 = u * wpu + j;
-        if (KIND == GR_BINOMIAL) {
-          int32_t res = d.ia;  // trials
-          for (int t = 0; t < U; ++t) res += (d.fa <= ur_f(word(w0 + 4 * t))) ? -1 : 0;
-          reinterpret_cast<int32_t*>(p.out)[o] = res;
-        }
-      }
+      staged_value<KIND, DT>(p, d, U, u, j, o, word, rword);
     }
     u_next = u_ready;
     __syncthreads();
     if (u_next >= u_end) break;
   }
 
-  if (last) {
-    // the loop stops right after the block holding p_last: ceil(np_seg/312)
-    // blocks were generated and raw[cur] is the last of them
-    if (np_seg > 0) {
-      const int64_t nblk = (np_seg + kN - 1) / kN;
-      const int rr2 = (int)(np_seg - (nblk - 1) * kN);  // in [1, 312]
-      store_window(st, raw[cur], raw[cur ^ 1], rr2);
-    }
-    if (tid == 0) {
-      if (DT == SD_I32H) {
-        // the last unit ends mid-packet: its upper half stays cached
-        const bool half_left = (w_last >= 0) && ((w_last & 7) == 3);
-        if (half_left) {
-          const int64_t rel = p_last - seg_p0;
-          const int slot = (int)((rel / kN) & 1);
-          st->half_cache[0] = (uint32_t)tp[slot][rel % kN][2];
-          st->half_cache[1] = (uint32_t)(tp[slot][rel % kN][2] >> 32);
-          st->half_cache[2] = (uint32_t)tp[slot][rel % kN][3];
-          st->half_cache[3] = (uint32_t)(tp[slot][rel % kN][3] >> 32);
-          st->half_valid = 1;
-        } else {
-          st->half_valid = 0;
-        }
+  // the loop stops right after the block holding p_last: ceil(np_seg/312)
+  // blocks were generated and raw[cur] is the last of them
+  if (np_seg > 0) {
+    const int64_t nblk = (np_seg + kN - 1) / kN;
+    const int rr2 = (int)(np_seg - (nblk - 1) * kN);  // in [1, 312]
+    store_window(st, raw[cur], raw[cur ^ 1], rr2);
+  }
+  if (tid == 0) {
+    if (DT == SD_I32H) {
+      // the last unit ends mid-packet: its upper half stays cached
+      const bool half_left = (w_last >= 0) && ((w_last & 7) == 3);
+      if (half_left) {
+        const int64_t rel = p_last;
+        const int slot = (int)((rel / kN) & 1);
+        st->half_cache[0] = (uint32_t)tp[slot][rel % kN][2];
+        st->half_cache[1] = (uint32_t)(tp[slot][rel % kN][2] >> 32);
+        st->half_cache[2] = (uint32_t)tp[slot][rel % kN][3];
+        st->half_cache[3] = (uint32_t)(tp[slot][rel % kN][3] >> 32);
+        st->half_valid = 1;
+      } else {
+        st->half_valid = 0;
       }
-      st->consumed += (uint64_t)(p_last + 1);
     }
+    st->consumed += (uint64_t)(p_last + 1);
+  }
+}
+
+// Units [u0, u0 + cnt) of every engine over words in memory, one thread per
+// output lane; block 0 of an engine leaves its state.
+template <int KIND, int DT>
+__global__ void __launch_bounds__(256) k_staged_words(Plan p, DistParams d, const CallSnap* snap, int U, int64_t u0,
+                                                      int64_t cnt) {
+  constexpr int P = DT == SD_F32 ? 8 : 4;
+  const int k = blockIdx.y, tid = threadIdx.x;
+  int64_t off, n;
+  slice_left(p, k, off, n);
+  const int64_t m = min(cnt, n / P - u0);  // this engine's units
+  if (m <= 0) return;
+  const int c0w = (DT == SD_I32H && snap[k].half_valid) ? 4 : 0;
+  const uint64_t* w = p.words + (size_t)k * kLanes * p.wstride;
+  auto lane64 = [&](int64_t packet, int l) { return mt_temper(__ldg(w + (size_t)l * p.wstride + kN + packet)); };
+  auto word = [&](int64_t q) -> uint32_t {
+    if (q < c0w) return snap[k].half_cache[q];
+    q -= c0w;
+    const uint64_t v = lane64(q >> 3, (int)((q & 7) >> 1));
+    return (q & 1) ? (uint32_t)(v >> 32) : (uint32_t)v;
+  };
+  auto rword = [&](int64_t r) { return lane64(r >> 2, (int)(r & 3)); };
+  const int64_t e = (int64_t)blockIdx.x * 256 + tid;
+  if (e < m * P) staged_value<KIND, DT>(p, d, U, e / P, (int)(e % P), off + u0 * P + e, word, rword);
+  if (blockIdx.x != 0) return;
+  const int64_t wpu = (DT == SD_I32H) ? 4 * (int64_t)U : 8 * (int64_t)U;
+  const int64_t w_last = m * wpu - 1 - c0w;
+  const int64_t np = w_last < 0 ? 0 : w_last / 8 + 1;
+  EngState* st = p.eng + k;
+  if (np > 0)
+    for (int t = tid; t < kLanes * kN; t += 256) st->win[t / kN][t % kN] = w[(size_t)(t / kN) * p.wstride + np + t % kN];
+  if (tid == 0) {
+    if (DT == SD_I32H) {
+      // the last unit may end mid-packet: the packet's upper half stays cached
+      const bool half_left = w_last >= 0 && (w_last & 7) == 3;
+      if (half_left) {
+        const uint64_t lo = lane64(np - 1, 2), hi = lane64(np - 1, 3);
+        st->half_cache[0] = (uint32_t)lo;
+        st->half_cache[1] = (uint32_t)(lo >> 32);
+        st->half_cache[2] = (uint32_t)hi;
+        st->half_cache[3] = (uint32_t)(hi >> 32);
+      }
+      st->half_valid = half_left ? 1 : 0;
+    }
+    st->consumed += (uint64_t)np;
   }
 }
 
@@ -264,23 +303,29 @@ cudaError_t launch_sx_staged(const uint64_t* w, void* out, int64_t npk, const Di
 }
 
 template <int KIND, int DT>
-static cudaError_t run_staged(const Plan& p, const DistParams& d, const CallSnap* snap, int U, int64_t Us,
-                              int delta, cudaStream_t s) {
-  k_staged<KIND, DT><<<p.K * p.S, 160, 0, s>>>(p, d, snap, U, Us, delta);
+static cudaError_t run_staged(const Plan& p, const DistParams& d, const CallSnap* snap, int U, int64_t u0, int64_t cnt,
+                              cudaStream_t s) {
+  if (p.words) {
+    constexpr int P = DT == SD_F32 ? 8 : 4;
+    k_staged_words<KIND, DT>
+        <<<dim3((unsigned)((cnt * P + 255) / 256), (unsigned)p.K), 256, 0, s>>>(p, d, snap, U, u0, cnt);
+  } else {
+    k_staged<KIND, DT><<<p.K, 160, 0, s>>>(p, d, U);
+  }
   return cudaGetLastError();
 }
 
-cudaError_t launch_staged(const Plan& p, const DistParams& d, const CallSnap* snap, int U, int64_t Us, int delta,
+cudaError_t launch_staged(const Plan& p, const DistParams& d, const CallSnap* snap, int U, int64_t u0, int64_t cnt,
                           cudaStream_t s) {
   if (d.kind == GR_GAMMA || d.kind == GR_CHI_SQUARED) {
-    if (d.dtype == GR_F32) return run_staged<GR_GAMMA, SD_F32>(p, d, snap, U, Us, delta, s);
-    if (d.dtype == GR_F64) return run_staged<GR_GAMMA, SD_F64>(p, d, snap, U, Us, delta, s);
+    if (d.dtype == GR_F32) return run_staged<GR_GAMMA, SD_F32>(p, d, snap, U, u0, cnt, s);
+    if (d.dtype == GR_F64) return run_staged<GR_GAMMA, SD_F64>(p, d, snap, U, u0, cnt, s);
   }
   if (d.kind == GR_STUDENT_T) {
-    if (d.dtype == GR_F32) return run_staged<GR_STUDENT_T, SD_F32>(p, d, snap, U, Us, delta, s);
-    if (d.dtype == GR_F64) return run_staged<GR_STUDENT_T, SD_F64>(p, d, snap, U, Us, delta, s);
+    if (d.dtype == GR_F32) return run_staged<GR_STUDENT_T, SD_F32>(p, d, snap, U, u0, cnt, s);
+    if (d.dtype == GR_F64) return run_staged<GR_STUDENT_T, SD_F64>(p, d, snap, U, u0, cnt, s);
   }
-  if (d.kind == GR_BINOMIAL && d.dtype == GR_I32) return run_staged<GR_BINOMIAL, SD_I32H>(p, d, snap, U, Us, delta, s);
+  if (d.kind == GR_BINOMIAL && d.dtype == GR_I32) return run_staged<GR_BINOMIAL, SD_I32H>(p, d, snap, U, u0, cnt, s);
   return cudaErrorNotSupported;
 }
 
@@ -870,9 +915,8 @@ __global__ void __launch_bounds__(kPoisThreads) k_poisson(Plan p, DistParams d, 
   const int k = blockIdx.x;
   const int tid = threadIdx.x;
   EngState* st = p.eng + k;
-  const int64_t g0 = (int64_t)k * p.gran_per_k + min((int64_t)k, p.gran_rem);
-  const int64_t ng = p.gran_per_k + ((int64_t)k < p.gran_rem ? 1 : 0);
-  const int64_t off = g0 * p.gran, n = ng * p.gran;
+  int64_t off, n;
+  slice_left(p, k, off, n);
   if (n == 0) return;
   const int64_t Npk = n / 4;
   const int c0w = st->half_valid ? 4 : 0;  // the first half packet comes from the engine's cache
@@ -1014,356 +1058,6 @@ static cudaError_t run_poisson(const Plan& p, const DistParams& d, int64_t max_b
     attr[dev] = true;
   }
   k_poisson<<<p.K, kPoisThreads, kPoisSmem, s>>>(p, d, max_blocks);
-  return cudaGetLastError();
-}
-
-// ===========================================================================
-// PoissonGen (mean < 12) and BinomialGen (mean < 1) on few engines over
-// jump-ahead segments.  The steps x -> x + L(x) of one engine form a chain
-// that a single CTA would have to follow from start to end; here segment s of
-// engine k (fresh packets [sJ, (s+1)J)) runs on its own CTA, in three
-// launches:
-//   scan   follows a speculative chain from the segment's first position,
-//          marking its step starts in a bitmap, and the chains from each of
-//          the other kPwEntries - 1 positions where the true chain can enter
-//          the segment (the previous segment's last step overshoots its end
-//          by less than kPoisLook) until they meet the marked chain; records,
-//          per entry offset, the steps the chain takes in the segment and the
-//          offset at which it leaves it;
-//   plan   (one CTA per engine) chains the entry offsets from segment to
-//          segment and turns the step counts into output offsets;
-//   write  follows its segment's true chain and writes its steps at their
-//          offsets; the segment holding the call's last step leaves the
-//          engine state, and an engine's last segment runs on past its end
-//          when the planned segments hold too few steps.
-// A step depends only on its start position, so two chains that meet share
-// every later step: the outputs equal the single-CTA walk's, bit for bit.
-// ===========================================================================
-template <int MODE>  // 0 scan, 1 write
-__global__ void __launch_bounds__(kPoisThreads) k_pw(Plan p, DistParams d, PwArgs a) {
-  extern __shared__ __align__(16) uint64_t pois_dyn[];
-  uint64_t(*raw)[kLanes][kN] = reinterpret_cast<uint64_t(*)[kLanes][kN]>(pois_dyn);
-  float(*uf)[kN][8] = reinterpret_cast<float(*)[kN][8]>(pois_dyn + 3 * kLanes * kN);
-  uint32_t* pos = reinterpret_cast<uint32_t*>(pois_dyn + 3 * kLanes * kN + kN * 8);
-  uint16_t* rec = reinterpret_cast<uint16_t*>(pos + kPoisRing);
-  __shared__ int s_nrec, s_stop, s_err, s_walkers, s_cnt0;
-  __shared__ int64_t s_ebase, s_end, s_x0;
-  __shared__ float4 s_cache;
-  const int S = p.S;
-  const int k = blockIdx.x / S, sg = blockIdx.x % S;
-  const int tid = threadIdx.x;
-  EngState* st = p.eng + k;
-  const int64_t g0 = (int64_t)k * p.gran_per_k + min((int64_t)k, p.gran_rem);
-  const int64_t ng = p.gran_per_k + ((int64_t)k < p.gran_rem ? 1 : 0);
-  const int64_t off = g0 * p.gran, n = ng * p.gran;
-  if (n == 0) return;
-  const int64_t Npk = n / 4;
-  const int c = a.snap[k].half_valid ? 1 : 0;  // position 0 is the engine's cached half packet
-  const int c0w = 4 * c;
-  const int64_t pk0 = (int64_t)sg * a.J;  // first fresh packet of the segment
-  const int64_t seg_lo = sg == 0 ? 0 : 2 * pk0 + c;
-  const int64_t seg_hi = 2 * (pk0 + a.J) + c;
-  const bool lastseg = sg == S - 1;
-  const size_t sidx = (size_t)k * S + sg;
-  int64_t start = seg_lo, O = 0, nsteps = INT64_MAX;
-  if (MODE == 1) {
-    start = seg_lo + a.plan[sidx * 3 + 0];
-    O = a.plan[sidx * 3 + 1];
-    if (!lastseg) nsteps = a.plan[sidx * 3 + 2];
-    if (O >= Npk) return;  // the call ends in an earlier segment
-  }
-  // lane windows: segment 0 from the call-start copy, the others from the jumps
-  if (sg == 0) load_window(raw[0], p.prefix + (size_t)k * kLanes * kPrefixLen, kPrefixLen);
-  else load_window(raw[0], p.segwin + ((size_t)k * (S - 1) + (sg - 1)) * kLanes * kN, kN);
-  if (tid == 0) {
-    s_err = 0;
-    s_stop = 0;
-    s_walkers = (MODE == 0 && sg > 0) ? kPwEntries - 1 : 0;
-    const uint32_t* hc = a.snap[k].half_cache;
-    s_cache = make_float4(ur_f(hc[0]), ur_f(hc[1]), ur_f(hc[2]), ur_f(hc[3]));
-  }
-  __syncthreads();
-  uint32_t* bits = a.bits + sidx * (size_t)a.words_per_seg;
-  const int64_t max_blocks = lastseg ? a.max_blocks : (2 * a.J + 4 * kPoisLook) / (2 * kN) + 3;
-  // chain of thread 0 (the speculative chain, or the true one); scan-mode
-  // walkers: thread t in [1, kPwEntries) follows the chain entering at seg_lo + t
-  int64_t x0 = start, E = 0;
-  int32_t cnt0 = 0;
-  int64_t bw = -1;  // bitmap word held by thread 0
-  uint32_t bv = 0;
-  int64_t xt = seg_lo + tid, mt = 0;
-  int32_t nt = 0;
-  int wstate = (MODE == 0 && sg > 0 && tid >= 1 && tid < kPwEntries) ? 1 : 0;  // 1 active, 2 met, 3 left
-  int64_t done_pos = start;
-  int cur = 0;
-  int64_t nb = 0;
-  for (; nb < max_blocks; ++nb) {
-    const int slot = (int)(nb & 1);
-    const int nxt = cur == 2 ? 0 : cur + 1;
-    mt_block(raw[cur], raw[nxt], [&](int i, const uint64_t* pk) {
-#pragma unroll
-      for (int l = 0; l < kLanes; ++l) {
-        uf[slot][i][2 * l] = ur_f((uint32_t)pk[l]);
-        uf[slot][i][2 * l + 1] = ur_f((uint32_t)(pk[l] >> 32));
-      }
-    });
-    cur = nxt;
-    const int64_t lim = c + 2 * pk0 + 2 * (nb + 1) * kN - kPoisLook;
-    if (tid == 0 && lim - x0 > kPoisRing) s_err = 1;  // positions still needed would leave the ring
-    // ---- steps of the new start positions (as in k_poisson)
-    for (int64_t x = done_pos + tid; x < lim; x += kPoisThreads) {
-      const bool cached = 4 * x < c0w;
-      int w = (int)(4 * (x - c - 2 * pk0) - 8 * nb * (int64_t)kN);
-      float val[4] = {1.0f, 1.0f, 1.0f, 1.0f};
-      int kk[4] = {0, 0, 0, 0};
-      int L = 0;
-      bool any = true;
-      for (int it = 0; it < kPoisLook && any; ++it, w += 4) {
-        float4 u;
-        if (it == 0 && cached) {
-          u = s_cache;
-        } else {
-          int pkk = w >> 3, sl = slot;
-          if (pkk < 0) {
-            pkk += kN;
-            sl ^= 1;
-          }
-          u = *reinterpret_cast<const float4*>(&uf[sl][pkk][w & 7]);
-        }
-        const float uu[4] = {u.x, u.y, u.z, u.w};
-        any = false;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          val[j] = val[j] * uu[j];
-          const bool cc = d.fe < val[j];
-          kk[j] += cc ? 1 : 0;
-          any |= cc;
-        }
-        L = it + 1;
-      }
-      if (any) atomicOr(&s_err, 1);
-      pos[(int)(x & (kPoisRing - 1))] =
-          ((uint32_t)L << 24) | (uint32_t)kk[0] | ((uint32_t)kk[1] << 6) | ((uint32_t)kk[2] << 12) | ((uint32_t)kk[3] << 18);
-    }
-    done_pos = max(done_pos, lim);
-    __syncthreads();
-    if (MODE == 0) {
-      // ---- the speculative chain (thread 0), its step starts marked
-      if (tid == 0) {
-        while (x0 < done_pos && x0 < seg_hi) {
-          const int64_t r = x0 - seg_lo;
-          if ((r >> 5) != bw) {
-            if (bw >= 0) bits[bw] = bv;
-            for (int64_t q = bw + 1; q < (r >> 5); ++q) bits[q] = 0u;
-            bw = r >> 5;
-            bv = 0;
-          }
-          bv |= 1u << (r & 31);
-          ++cnt0;
-          x0 += pos[(int)(x0 & (kPoisRing - 1))] >> 24;
-        }
-        if (bw >= 0) bits[bw] = bv;
-        s_x0 = x0;
-        if (x0 >= seg_hi && s_walkers == 0) s_stop = 1;
-      }
-      __syncthreads();
-      // ---- walkers: until they meet the marked chain or leave the segment
-      if (wstate == 1) {
-        const int64_t xs = s_x0;
-        while (xt < done_pos) {
-          if (xt >= seg_hi) {
-            wstate = 3;
-            break;
-          }
-          const int64_t r = xt - seg_lo;
-          if (xt == xs || (xt < xs && ((bits[r >> 5] >> (r & 31)) & 1u))) {
-            wstate = 2;
-            mt = xt;
-            break;
-          }
-          ++nt;
-          xt += pos[(int)(xt & (kPoisRing - 1))] >> 24;
-        }
-        if (wstate != 1) atomicSub(&s_walkers, 1);
-      }
-      __syncthreads();
-      if (tid == 0 && s_x0 >= seg_hi && s_walkers == 0) s_stop = 1;
-      __syncthreads();
-    } else {
-      // ---- the true chain (thread 0), as k_poisson's walk
-      if (tid == 0) {
-        s_ebase = E;
-        int nrec = 0;
-        const int64_t want = min(nsteps, Npk - O);
-        while (x0 < done_pos && E < want && nrec < kPoisRec) {
-          const int ri = (int)(x0 & (kPoisRing - 1));
-          rec[nrec++] = (uint16_t)ri;
-          x0 += pos[ri] >> 24;
-          ++E;
-        }
-        s_nrec = nrec;
-        if (E >= want) {
-          s_stop = (O + E >= Npk) ? 1 : 2;  // 1: the call ends here
-          s_end = x0;
-        }
-      }
-      __syncthreads();
-      const int nrec = s_nrec;
-      const int64_t e_first = O + s_ebase;
-      for (int e = tid; e < nrec * 4; e += kPoisThreads) {
-        const int i = e >> 2, j = e & 3;
-        int32_t v = (int32_t)((pos[rec[i]] >> (6 * j)) & 63);
-        if (d.ic) v = d.ia - v;  // BinomialGen: trials - res when p > 1/2
-        reinterpret_cast<int32_t*>(p.out)[off + (e_first + i) * 4 + j] = v;
-      }
-      __syncthreads();
-    }
-    if (s_stop || s_err) break;
-  }
-  if (MODE == 0) {
-    if (tid == 0 && (!s_stop || s_err)) atomicOr(&st->status, (int)GR_DEV_REJECT_LIMIT);
-    const int64_t xs = s_x0;
-    if (tid == 0) {
-      s_cnt0 = cnt0;  // the chain's steps, for the walkers' counts below
-      int32_t* info = a.info + sidx * 4;
-      info[0] = (int32_t)(xs - seg_hi);
-      info[1] = cnt0;
-      info[2] = 1;  // every entry met the chain (cleared below otherwise)
-      int32_t* en = a.ent + sidx * kPwEntries * 2;
-      en[0] = cnt0;
-      en[1] = (int32_t)(xs - seg_hi);
-    }
-    __syncthreads();
-    if (wstate == 2) {
-      // steps of the marked chain before the meeting point
-      const int64_t r = mt - seg_lo;
-      int32_t rank = 0;
-      for (int64_t q = 0; q < (r >> 5); ++q) rank += __popc(bits[q]);
-      rank += __popc(bits[r >> 5] & ((1u << (r & 31)) - 1u));
-      int32_t* en = a.ent + (sidx * kPwEntries + tid) * 2;
-      en[0] = nt + s_cnt0 - rank;
-      en[1] = (int32_t)(xs - seg_hi);
-    } else if (wstate == 3 || wstate == 1) {
-      int32_t* en = a.ent + (sidx * kPwEntries + tid) * 2;
-      en[0] = nt;
-      en[1] = (int32_t)(xt - seg_hi);
-      a.info[sidx * 4 + 2] = 0;
-    }
-    return;
-  }
-  // ---- write mode: the engine state, from the segment that ends the call
-  if (tid == 0 && (s_stop == 0 || s_err)) {
-    // an engine's last segment ran out of blocks, or a step was too long
-    atomicOr(&st->status, (int)GR_DEV_REJECT_LIMIT);
-  }
-  __syncthreads();
-  if (s_stop != 1) return;
-  const int64_t fresh = s_end - c;    // half packets drawn fresh, from the call start
-  const int64_t np = (fresh + 1) / 2;  // packets consumed
-  const int64_t lp = np - pk0;          // ... of this segment's blocks
-  const int prv = cur == 0 ? 2 : cur - 1, prv2 = prv == 0 ? 2 : prv - 1;
-  const int64_t nblk = min(nb + 1, max_blocks);
-  if (lp > 0) {
-    const int64_t lastb = (lp - 1) / kN;
-    const int64_t rr = lp - lastb * kN;
-    if (lastb == nblk - 1) store_window(st, raw[cur], raw[prv], (int)rr);
-    else if (lastb == nblk - 2) store_window(st, raw[prv], raw[prv2], (int)rr);
-    else if (tid == 0) atomicOr(&st->status, (int)GR_DEV_BAD_INPUT);
-  } else if (tid == 0) {
-    atomicOr(&st->status, (int)GR_DEV_BAD_INPUT);
-  }
-  if (tid == 0) {
-    if (fresh & 1) {  // the last packet's upper half stays in the engine's half cache
-      const int64_t pl = lp - 1;
-      const int buf = (pl / kN == nblk - 1) ? cur : prv;
-      const uint64_t aa = mt_temper(raw[buf][2][pl % kN]), bb = mt_temper(raw[buf][3][pl % kN]);
-      st->half_cache[0] = (uint32_t)aa;
-      st->half_cache[1] = (uint32_t)(aa >> 32);
-      st->half_cache[2] = (uint32_t)bb;
-      st->half_cache[3] = (uint32_t)(bb >> 32);
-      st->half_valid = 1;
-    } else {
-      st->half_valid = 0;
-    }
-    st->consumed += (uint64_t)max(np, (int64_t)0);
-  }
-}
-
-// One CTA per engine: entry offsets chained from segment to segment, output
-// offsets from the step counts.
-__global__ void __launch_bounds__(1024) k_pw_plan(Plan p, PwArgs a) {
-  __shared__ int32_t s_tot[32];
-  __shared__ int64_t s_carry;
-  const int S = p.S, k = blockIdx.x, tid = threadIdx.x;
-  const size_t base = (size_t)k * S;
-  // entry offsets: known where the previous segment's entries all met
-  for (int sg = tid; sg < S; sg += blockDim.x) {
-    int64_t dv = -1;
-    if (sg == 0) dv = 0;
-    else if (a.info[(base + sg - 1) * 4 + 2]) dv = a.info[(base + sg - 1) * 4 + 0];
-    a.plan[(base + sg) * 3 + 0] = dv;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    for (int sg = 1; sg < S; ++sg) {
-      if (a.plan[(base + sg) * 3 + 0] >= 0) continue;
-      const int64_t dp = a.plan[(base + sg - 1) * 3 + 0];
-      a.plan[(base + sg) * 3 + 0] = a.ent[((base + sg - 1) * kPwEntries + dp) * 2 + 1];
-    }
-    s_carry = 0;
-  }
-  __syncthreads();
-  // steps per segment, then their exclusive prefix sums
-  for (int b0 = 0; b0 < S; b0 += blockDim.x) {
-    const int sg = b0 + tid;
-    int32_t v = 0;
-    if (sg < S) {
-      int64_t dv = a.plan[(base + sg) * 3 + 0];
-      if (dv < 0 || dv >= kPwEntries) dv = 0;  // unreachable: offsets stay below kPoisLook
-      v = a.ent[((base + sg) * kPwEntries + dv) * 2 + 0];
-    }
-    // block-wide inclusive scan of v
-    int32_t x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if ((tid & 31) >= o) x += y;
-    }
-    if ((tid & 31) == 31) s_tot[tid >> 5] = x;
-    __syncthreads();
-    if (tid < 32) {
-      int32_t t = s_tot[tid];
-      for (int o = 1; o < 32; o <<= 1) {
-        const int32_t y = __shfl_up_sync(0xffffffffu, t, o);
-        if (tid >= o) t += y;
-      }
-      s_tot[tid] = t;
-    }
-    __syncthreads();
-    const int64_t incl = s_carry + x + ((tid >> 5) ? s_tot[(tid >> 5) - 1] : 0);
-    if (sg < S) {
-      a.plan[(base + sg) * 3 + 1] = incl - v;
-      a.plan[(base + sg) * 3 + 2] = v;
-    }
-    __syncthreads();
-    if (tid == blockDim.x - 1) s_carry = incl;
-    __syncthreads();
-  }
-}
-
-cudaError_t launch_poisson_segmented(const Plan& p, const DistParams& d, const PwArgs& a, cudaStream_t s) {
-  static bool attr[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  if (!attr[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(k_pw<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPoisSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pw<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPoisSmem);
-    if (e != cudaSuccess) return e;
-    attr[dev] = true;
-  }
-  k_pw<0><<<p.K * p.S, kPoisThreads, kPoisSmem, s>>>(p, d, a);
-  k_pw_plan<<<p.K, 1024, 0, s>>>(p, a);
-  k_pw<1><<<p.K * p.S, kPoisThreads, kPoisSmem, s>>>(p, d, a);
   return cudaGetLastError();
 }
 

@@ -66,3 +66,39 @@ def test_short_plan(gpulib, oracle, monkeypatch, scale):
 
 def test_more_than_one_buffer(gpulib, oracle):
     check(gpulib, oracle, "BETA", torch.float32, 0.5, 2.0, 1, (1500000, 192))
+
+
+@pytest.mark.parametrize("kind,a,t", [("POISSON", 4.0, 0), ("POISSON", 11.9, 0), ("POISSON", 0.05, 0),
+                                      ("BINOMIAL", 0.004, 100), ("BINOMIAL", 0.996, 200)])
+@pytest.mark.parametrize("streams", [1, 3])
+def test_poisson_walk(gpulib, oracle, kind, a, t, streams):
+    """PoissonGen (mean < 12) and BinomialGen (mean < 1): the same chain over
+    half packets, with and without a cached half packet at the start."""
+    er = gpulib
+    u = er.Vmt19937_64(31, streams=streams)
+    g = er._Gen(torch.int32, a, 0.0, trials=t, kind=kind)
+    es = [oracle.Engine(31 + 4 * k) for k in range(streams)]
+    ogs = [oracle.Gen() for _ in range(streams)]
+    er.randBits(4 * streams, 1, u)
+    for e in es:
+        oracle.generate(e, oracle.Gen(), "RANDBITS", 4, np.int32)
+    for pk in (511, 512, 513, 1300, 3, 9001, 60000):
+        n = 4 * pk
+        out = g.generate(n * streams, 1, u).reshape(-1).cpu().numpy()
+        for k in range(streams):
+            ref = oracle.generate(es[k], ogs[k], kind, n, np.int32, a, 0.0, t)
+            assert np.array_equal(out[k * n:(k + 1) * n], ref), f"packets={pk} stream {k}"
+    u.sync()
+    raw = er.raw_u64(u, 64 * streams).cpu().numpy().view(np.uint64)
+    for k in range(streams):
+        assert np.array_equal(raw[64 * k:64 * (k + 1)], es[k].raw(16)), "engine after the calls"
+
+
+def test_poisson_more_than_one_buffer(gpulib, oracle):
+    er = gpulib
+    u = er.Vmt19937_64(8)
+    e, og = oracle.Engine(8), oracle.Gen()
+    for n in (4 * 1400000, 4 * 600):
+        out = er.poisson(n, 1, u, 4.0).reshape(-1).cpu().numpy()
+        assert np.array_equal(out, oracle.generate(e, og, "POISSON", n, np.int32, 4.0))
+    u.sync()

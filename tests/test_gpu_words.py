@@ -62,3 +62,31 @@ def test_more_than_one_buffer(gpulib, oracle):
     got = er.raw_u64(u, 4 * pk).cpu().numpy().view(np.uint64)
     assert np.array_equal(got, e.raw(pk))
     assert np.array_equal(er.raw_u64(u, 64).cpu().numpy().view(np.uint64), e.raw(16))
+
+
+@pytest.mark.parametrize("kind,tdt,a,t", [("GAMMA", torch.float32, 5.0, 0), ("GAMMA", torch.float64, 19.0, 0),
+                                          ("STUDENT_T", torch.float32, 4.0, 0), ("STUDENT_T", torch.float64, 2.5, 0),
+                                          ("BINOMIAL", torch.int32, 0.3, 20), ("BINOMIAL", torch.int32, 0.3, 1),
+                                          ("BINOMIAL", torch.int32, 0.9, 7)])
+@pytest.mark.parametrize("streams", [1, 3])
+def test_units_of_packets(gpulib, oracle, kind, tdt, a, t, streams):
+    """Kinds whose output takes a fixed run of packets (k_staged_words): around
+    the threshold, with half packets carried (binomial), and in several
+    scratch buffers."""
+    er = gpulib
+    npdt = {torch.float32: np.float32, torch.float64: np.float64, torch.int32: np.int32}[tdt]
+    P = 8 if tdt == torch.float32 else 4
+    u = er.Vmt19937_64(12, streams=streams)
+    g = er._Gen(tdt, a, 1.0 if kind == "GAMMA" else 0.0, trials=t, kind=kind)
+    es = [oracle.Engine(12 + 4 * k) for k in range(streams)]
+    og = oracle.Gen()
+    U = {"GAMMA": int(a), "STUDENT_T": 2, "BINOMIAL": max(1, (t + 1) // 2)}[kind]
+    for un in (624 // U, 624 // U + 1, 701, 3, 20001) + ((1 << 22) // U + 77,) * (streams == 1):
+        n = un * P
+        out = g.generate(n * streams, 1, u).reshape(-1).cpu().numpy()
+        for k in range(streams):
+            ref = oracle.generate(es[k], og, kind, n, npdt, a, 1.0 if kind == "GAMMA" else 0.0, t)
+            assert np.array_equal(bits(out[k * n:(k + 1) * n]), bits(ref)), f"{kind} units={un} stream {k}"
+    raw = er.raw_u64(u, 64 * streams).cpu().numpy().view(np.uint64)
+    for k in range(streams):
+        assert np.array_equal(raw[64 * k:64 * (k + 1)], es[k].raw(16)), "engine after the calls"
