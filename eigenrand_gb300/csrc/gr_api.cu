@@ -938,7 +938,12 @@ gr_status run_poisson_call(gr_engine* e, const Plan& p0, const DistParams& wd, i
 // off it may be, relatively.
 double expected_yield(int rk, const DistParams& d, double& slack) {
   slack = 0;
-  if (rk <= 1) return gamma_yield(rk == 0 ? 2 << 8 : 3 << 8, d.dtype == GR_F64 ? d.da : (double)d.fa);
+  const bool f64 = d.dtype == GR_F64;
+  if (rk <= 1) return gamma_yield(rk == 0 ? 2 << 8 : 3 << 8, f64 ? d.da : (double)d.fa);
+  if (rk == 2) {  // Johnk: G(a + 1) G(b + 1) / G(a + b + 1)
+    const double a = f64 ? d.da : (double)d.fa, b = f64 ? d.db : (double)d.fb;
+    return std::tgamma(a + 1) * std::tgamma(b + 1) / std::tgamma(a + b + 1);
+  }
   slack = 0.04;
   return reject_yield(rk, d);
 }
@@ -990,7 +995,7 @@ gr_status run_reject_call(gr_engine* e, const Plan& p0, const DistParams& dp, in
   if (st == GR_OK) {
     p.done = done;
     p.S = 1;
-    err = launch_reject(p, dp, rk, max_blocks, stream);
+    err = launch_reject(p, dp, rk, (float)(1.0 / q), max_blocks, stream);
     if (err != cudaSuccess) st = cuda_fail(err, "rejection sampling kernel");
   }
   cudaFreeAsync(done, stream);
@@ -1184,7 +1189,10 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
     const int64_t max_blocks = block_cap(((16 * npk + 4096) * wt) / (kN * 8) + 64);
     if (e->K <= kRejectMaxK && npk >= kRejectMin)
       return run_reject_call(e, p, dp, rk, npk, max_blocks, stream);
-    cudaError_t err = launch_reject(p, dp, rk, max_blocks, stream);
+    double slack = 0;
+    // the integer samplers accept about half of their candidates
+    const float per_packet = rk <= 2 ? (float)(1.0 / expected_yield(rk, dp, slack)) : 2.0f;
+    cudaError_t err = launch_reject(p, dp, rk, per_packet, max_blocks, stream);
     if (err != cudaSuccess) return cuda_fail(err, "rejection sampling kernel");
     return GR_OK;
   }

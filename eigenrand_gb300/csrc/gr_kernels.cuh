@@ -122,10 +122,25 @@ cudaError_t launch_direct(const Plan& p, const DistParams& d, const CallSnap* sn
 cudaError_t launch_staged(const Plan& p, const DistParams& d, const CallSnap* snap, int U, int64_t u0, int64_t cnt,
                           cudaStream_t s);
 
-// Rejection samplers resolved with CompressMask semantics (gr_samplers.cu);
-// one CTA per stream.  rk: 0 gamma alpha<1 (GS), 1 gamma tan proposal,
+// Rejection samplers resolved with CompressMask semantics (gr_trials.cu); one
+// CTA per stream.  rk: 0 gamma alpha<1 (GS), 1 gamma tan proposal,
 // 2 beta with a,b < 1, 3 poisson mean >= 12, 4 binomial tan proposal.
-cudaError_t launch_reject(const Plan& p, const DistParams& d, int rk, int64_t max_blocks, cudaStream_t s);
+// per_packet: expected trials per output packet (only sizes the last batch).
+cudaError_t launch_reject(const Plan& p, const DistParams& d, int rk, float per_packet, int64_t max_blocks,
+                          cudaStream_t s);
+// Several GammaGen rows, each p's outputs, drawn one after the other from each
+// stream: row i at p.out + i * row_stride elements.  rk: 0, 1 as above, or a
+// fixed run of packets (integral alpha, alpha = 1).
+constexpr int kRowInt = 5, kRowExp = 6;
+struct TrialRow {
+  DistParams d;
+  GenState* gen;  // [streams]
+  int32_t rk, packets;
+  float per_packet;
+  int32_t pad;
+};
+cudaError_t launch_gamma_rows(const Plan& p, int dtype, const TrialRow* rows, int nrows, int64_t row_stride,
+                              int64_t max_blocks, cudaStream_t s);
 
 // The same over words in memory (gr_rejw.cu): T trials per engine, whose
 // packets p.words holds; output packets made are added to done[k] and the

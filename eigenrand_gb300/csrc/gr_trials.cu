@@ -1,0 +1,351 @@
+// Samplers driven by CompressMask::compress_append (EigenRand/arch/AVX/
+// PacketFilter.h:147-184), one CTA per stream.
+//
+// Each trial consumes a fixed run of words and yields P candidates with an
+// accept mask.  The reference's packetOp loop is an automaton over trials: a
+// fully accepted trial is returned as is; otherwise its accepted lanes are
+// appended, in lane order, to a FIFO carried in the generator, and a packet is
+// returned once the FIFO holds P lanes.  With  NF_t = fully accepted trials
+// before t  and  A_t = carried lanes + lanes appended before t,  trial t's
+// emission (if any) is packet  E + NF_t + floor(A_t / P),  so a batch of
+// trials is resolved with one block-wide prefix sum.  The call stops at the
+// trial that completes its last output packet; later trials are not consumed.
+//
+// k_trials draws one row (one generator call) or several rows one after the
+// other from the same stream (Dirichlet's GammaGen rows, Wishart's chi-squared
+// rows), which stay in one launch with the stream's window and its unused
+// words in shared memory.  Rows may be fixed runs of packets (integral alpha,
+// alpha = 1): trials that are always fully accepted.
+//
+// Bound by instruction issue.  The tempered words of the two newest engine
+// blocks are a ring of 4 992 32-bit words, a trial's words follow each other
+// in it, and all indices are 32-bit: gamma(0.5) float at 4096 x 4096 on 608
+// engines took 20 warp-instructions per sample (348 us) with 64-bit stream
+// positions mapped to the ring per word.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+
+#include "../../include/gpurand.h"
+#include "gr_samplers.cuh"
+
+namespace gr {
+
+namespace {
+
+constexpr int kTrThreads = 320;     // ten warps; 312 of the threads make a block's words
+constexpr int kTrRing = 16 * kN;    // ring words: two blocks of 312 packets of 8
+constexpr int kTrBatch = kN + 1;    // most trials of a batch (one packet each, one straddling)
+constexpr int kTrCand = 8 * (kN + 1) + 8;
+
+struct TrialSmem {
+  uint64_t raw[2][kLanes][kN];
+  alignas(16) uint32_t w[kTrRing];
+  alignas(16) uint32_t cand[kTrCand];  // accepted candidates (double: kTrCand / 2 of them)
+  uint32_t scan[kTrBatch + 7];         // exclusive: (fulls << 16) | lanes appended
+  uint32_t emit[kTrBatch + 7];         // output packet (from the batch's first) of each FIFO packet
+  uint64_t fifo[2][16];                // carried lanes (ping-pong)
+  uint32_t warp_tot[kTrThreads / 32];
+  int tstar;
+  uint8_t mask[kTrBatch + 7];
+  TrialRow row;
+};
+
+// A row's candidate at the ring index a of its trial, lane j.
+template <int DT, int RK>
+__device__ __forceinline__ bool trial_eval(const TrialSmem& sm, const DistParams& d, const int rk, const int U, const int a,
+                                           const int j, uint64_t& c) {
+  auto word = [&](int q) -> uint32_t {
+    int i = a + q;
+    i -= i >= kTrRing ? kTrRing : 0;
+    return sm.w[i];
+  };
+  auto rval = [&](int r) -> uint64_t {
+    int i = a + 2 * r;
+    i -= i >= kTrRing ? kTrRing : 0;
+    return *reinterpret_cast<const uint64_t*>(&sm.w[i]);
+  };
+  auto rej = [&](auto k) { return rej_trial<decltype(k)::value, DT>(d, 0, j, word, rval, c); };
+  if (RK >= 0) return rej(std::integral_constant<int, RK < 0 ? 0 : RK>{});
+  if (rk == RK_GAMMA_GS) return rej(std::integral_constant<int, RK_GAMMA_GS>{});
+  if (rk == RK_GAMMA_TAN) return rej(std::integral_constant<int, RK_GAMMA_TAN>{});
+  // NormalExp.h:527-534 (alpha = 1), :577-587 (integral alpha)
+  if (DT == SD_F32) {
+    if (rk == kRowExp) {
+      c = f2u(d.fb * (-(logf_(1.0f - ur_f(word(j))) / 1.0f)));
+    } else {
+      constexpr float e = 1.1920928955078125e-07f / 8;
+      float y = ur_f(word(j)) + e;
+      for (int t = 1; t < U; ++t) y = y * (ur_f(word(8 * t + j)) + e);
+      c = f2u(-(d.fb * logf_(y)));
+    }
+  } else {
+    if (rk == kRowExp) {
+      const double l = -(log_(one_minus_ur_d(rval(j))) / 1.0);
+      c = d2u((d.flags & kParamUnitScale) ? l : d.db * l);
+    } else {
+      constexpr double e = 2.220446049250313e-16 / 8;
+      double y = ur_d(rval(j)) + e;
+      for (int t = 1; t < U; ++t) y = y * (ur_d(rval(4 * t + j)) + e);
+      const double l = log_(y);
+      c = d2u((d.flags & kParamUnitScale) ? -l : -(d.db * l));
+    }
+  }
+  return true;
+}
+
+// RK >= 0: one row (args) of that kind; RK < 0: `rows` rows from memory, row i
+// written at out + i * row_stride elements.
+template <int DT, int RK>
+__global__ void __launch_bounds__(kTrThreads, 4) k_trials(Plan p, TrialRow args, const TrialRow* rows, int nrows,
+                                                          int64_t row_stride, int64_t max_blocks) {
+  constexpr int P = DT == SD_F32 ? 8 : 4;
+  constexpr uint32_t kFull = (1u << P) - 1u;
+  constexpr bool kHalf = DT == SD_I32H;
+  using V = typename std::conditional<DT == SD_F64, uint64_t, uint32_t>::type;
+  extern __shared__ __align__(16) uint8_t tr_dyn[];
+  TrialSmem& sm = *reinterpret_cast<TrialSmem*>(tr_dyn);
+  V* cand = reinterpret_cast<V*>(sm.cand);
+  const int k = blockIdx.x, tid = threadIdx.x;
+  EngState* st = p.eng + k;
+  int64_t off, n;
+  slice_left(p, k, off, n);
+  if (n == 0) return;
+  const int64_t Npk = n / P;  // output packets of a row
+
+  const int c0w = (kHalf && st->half_valid) ? 4 : 0;
+  for (int i = tid; i < kLanes * kN; i += kTrThreads) (&sm.raw[0][0][0])[i] = (&st->win[0][0])[i];
+  // the engine's cached half packet goes before the first block's words
+  if (kHalf && tid < 4) sm.w[kTrRing - 4 + tid] = st->half_cache[tid];
+  int sp = c0w ? kTrRing - 4 : 0;  // ring index of the next trial's first word
+  int av = c0w;                    // words there
+  int cur = 0;
+  int64_t nb = 0;  // blocks made
+  bool over = false;
+
+  for (int r = 0; r < (RK < 0 ? nrows : 1) && !over; ++r) {
+    __syncthreads();  // the window is there; the last row's carried lanes are out
+    if (RK < 0) {
+      const uint32_t* src = reinterpret_cast<const uint32_t*>(rows + r);
+      for (int i = tid; i < (int)(sizeof(TrialRow) / 4); i += kTrThreads) reinterpret_cast<uint32_t*>(&sm.row)[i] = src[i];
+      __syncthreads();
+    }
+    const TrialRow& row = RK < 0 ? sm.row : args;
+    const DistParams& d = row.d;
+    const int U = row.packets, Wt = 8 * U, rk = row.rk;
+    GenSlot* gs = &row.gen[k].s[0];
+    V* out = reinterpret_cast<V*>(p.out) + (RK < 0 ? (int64_t)r * row_stride : 0) + off;
+    int rcnt = (RK >= 0 || rk <= RK_GAMMA_TAN) ? gs->rest_cnt : 0;
+    if (tid < 16)
+      sm.fifo[0][tid] = DT == SD_F64
+                            ? ((uint64_t)gs->rest[2 * (tid & 7)] | ((uint64_t)gs->rest[2 * (tid & 7) + 1] << 32))
+                            : (uint64_t)gs->rest[tid];
+    int fsl = 0;
+    int64_t left = Npk;
+    while (left > 0) {
+      if (av < Wt) {
+        if (nb >= max_blocks) {
+          over = true;
+          break;
+        }
+        // the next engine block: two lanes per thread (words 2 h and 2 h + 1 of
+        // a packet are neighbours in the ring), word i + 156 from word i made
+        // by the same thread, word 311 with the block's word 0 made again
+        uint64_t(*old)[kN] = sm.raw[cur];
+        uint64_t(*nw)[kN] = sm.raw[cur ^ 1];
+        uint32_t* ring = sm.w + (nb & 1) * (kTrRing / 2);
+        if (tid < 2 * kM) {
+          const int h = tid >= kM ? 1 : 0, i = tid - h * kM;
+          uint64_t lo[2], hi[2];
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const int l = 2 * h + q;
+            const uint64_t c = old[l][i + kM];
+            lo[q] = mt_twist(old[l][i], old[l][i + 1], c);
+            const uint64_t b = i == kM - 1 ? mt_twist(old[l][0], old[l][1], old[l][kM]) : old[l][i + kM + 1];
+            hi[q] = mt_twist(c, b, lo[q]);
+            nw[l][i] = lo[q];
+            nw[l][i + kM] = hi[q];
+          }
+          *reinterpret_cast<ulonglong2*>(ring + 8 * i + 4 * h) = make_ulonglong2(mt_temper(lo[0]), mt_temper(lo[1]));
+          *reinterpret_cast<ulonglong2*>(ring + 8 * (i + kM) + 4 * h) =
+              make_ulonglong2(mt_temper(hi[0]), mt_temper(hi[1]));
+        }
+        cur ^= 1;
+        ++nb;
+        av += 8 * kN;
+        __syncthreads();
+      }
+      // a batch: the trials whose words exist, and near the end of the row no
+      // more than it should still need
+      const int need = (int)min(left, (int64_t)1 << 20);
+      const int B = min(av / Wt, min(kTrBatch, (int)((float)need * row.per_packet) + 4));
+      // ---- candidates and accept masks
+      for (int e0 = 0; e0 < B * P; e0 += kTrThreads) {
+        const int e = e0 + tid, t = e / P, j = e % P;
+        bool acc = false;
+        uint64_t c = 0;
+        if (e < B * P) {
+          int a = sp + t * Wt;
+          a -= a >= kTrRing ? kTrRing : 0;
+          acc = trial_eval<DT, RK>(sm, d, rk, U, a, j, c);
+        }
+        const uint32_t bal = __ballot_sync(0xffffffffu, acc);
+        if (acc) cand[e] = (V)c;
+        if (j == 0 && e < B * P) sm.mask[t] = (uint8_t)((bal >> (tid & 31)) & kFull);
+      }
+      __syncthreads();
+      // ---- prefix sums over trials: (fulls << 16) | appended lanes
+      const uint32_t m0 = tid < B ? sm.mask[tid] : 0;
+      const uint32_t v0 = m0 == kFull ? 1u << 16 : (uint32_t)__popc(m0);
+      uint32_t v = v0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, v, o);
+        if ((tid & 31) >= o) v += x;
+      }
+      if ((tid & 31) == 31) sm.warp_tot[tid >> 5] = v;
+      if (tid == 0) sm.tstar = B;
+      __syncthreads();
+#pragma unroll
+      for (int w = 0; w < kTrThreads / 32; ++w) v += w < (tid >> 5) ? sm.warp_tot[w] : 0u;
+      // ---- this thread's trial: its emission, if any
+      const uint32_t ex = v - v0;
+      if (tid < B) {
+        const int at = rcnt + (int)(ex & 0xffffu), nf = (int)(ex >> 16);
+        const bool full = m0 == kFull;
+        const bool cross = !full && (at + (int)__popc(m0)) / P > at / P;
+        const int ei = nf + at / P;
+        sm.scan[tid] = ex;
+        if (cross) sm.emit[at / P] = (uint32_t)ei;
+        if ((full || cross) && ei == need - 1) sm.tstar = tid + 1;
+      }
+      __syncthreads();
+      // trials consumed, and the FIFO level and emissions after them
+      const int Bu = sm.tstar;
+      const uint32_t ml = sm.mask[Bu - 1], sl = sm.scan[Bu - 1];
+      const int a_end = rcnt + (int)(sl & 0xffffu) + (ml == kFull ? 0 : __popc(ml));
+      const int nf_end = (int)(sl >> 16) + (ml == kFull ? 1 : 0);
+      const int qe = a_end / P;  // FIFO packets emitted
+      auto put = [&](int at, uint64_t x) {
+        if (RK == RK_BETA_SMALL) x = beta_post<DT == SD_F64>(x, d);
+        if (DT == SD_I32H) {
+          // BinomialGen returns trials - res when p > 1/2 (Discrete.h:1051)
+          const int32_t q = (int32_t)u2f((uint32_t)x);
+          x = (uint32_t)((RK == RK_BINOMIAL && d.ib) ? (int32_t)d.fh - q : q);
+        }
+        out[at] = (V)x;
+      };
+      // ---- write outputs
+      for (int e = tid; e < Bu * P; e += kTrThreads) {
+        const int t = e / P, j = e % P;
+        const uint32_t m = sm.mask[t];
+        if (!((m >> j) & 1u)) continue;
+        const uint32_t s = sm.scan[t];
+        const int at = rcnt + (int)(s & 0xffffu);
+        if (m == kFull) {
+          put(((int)(s >> 16) + at / P) * P + j, cand[e]);
+        } else {
+          const int f = at + __popc(m & ((1u << j) - 1u)), q = f / P;
+          if (q < qe) put((int)sm.emit[q] * P + f % P, cand[e]);
+          else sm.fifo[fsl ^ 1][f - qe * P] = cand[e];  // the FIFO keeps the plain draws
+        }
+      }
+      // carried lanes: emitted with the batch's first FIFO packet, or still carried
+      if (tid < rcnt) {
+        if (qe > 0) put((int)sm.emit[0] * P + tid, sm.fifo[fsl][tid]);
+        else sm.fifo[fsl ^ 1][tid] = sm.fifo[fsl][tid];
+      }
+      out += (int64_t)(nf_end + qe) * P;
+      left -= nf_end + qe;
+      rcnt = a_end - qe * P;
+      fsl ^= 1;
+      sp += Bu * Wt;
+      sp -= sp >= kTrRing ? kTrRing : 0;
+      av -= Bu * Wt;
+      __syncthreads();
+    }
+    if (RK >= 0 || rk <= RK_GAMMA_TAN) {
+      if (tid == 0) gs->rest_cnt = rcnt;
+      if (DT == SD_F64) {
+        if (tid < 8) {
+          gs->rest[2 * tid] = (uint32_t)sm.fifo[fsl][tid];
+          gs->rest[2 * tid + 1] = (uint32_t)(sm.fifo[fsl][tid] >> 32);
+        }
+      } else if (tid < 16) {
+        gs->rest[tid] = (uint32_t)sm.fifo[fsl][tid];
+      }
+    }
+  }
+
+  // ---- engine state: the call ends inside the newest block (a trial is
+  // evaluated in the batch after the block that holds its last word)
+  if (tid == 0 && over) atomicOr(&st->status, (int)GR_DEV_REJECT_LIMIT);
+  if (nb > 0) {
+    const int rr = kN - av / 8;  // packets used of it; a half packet counts as used
+    for (int t = tid; t < kLanes * kN; t += kTrThreads) {
+      const int l = t / kN, i = t % kN;
+      st->win[l][i] = i < kN - rr ? sm.raw[cur ^ 1][l][rr + i] : sm.raw[cur][l][i - (kN - rr)];
+    }
+  }
+  if (tid == 0) {
+    if (kHalf && nb > 0) {
+      const bool half = (av & 7) == 4;  // ends mid-packet: the upper half stays cached
+      if (half)
+        for (int q = 0; q < 4; ++q) st->half_cache[q] = sm.w[sp + q];
+      st->half_valid = half ? 1 : 0;
+    }
+    st->consumed += (uint64_t)(nb * kN - av / 8);
+  }
+}
+
+template <int DT, int RK>
+cudaError_t run_trials(const Plan& p, const TrialRow& row, const TrialRow* rows, int nrows, int64_t row_stride,
+                       int64_t max_blocks, cudaStream_t s) {
+  static bool attr[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  constexpr size_t smem = sizeof(TrialSmem);
+  if (!attr[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(k_trials<DT, RK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    attr[dev] = true;
+  }
+  k_trials<DT, RK><<<p.K, kTrThreads, smem, s>>>(p, row, rows, nrows, row_stride, max_blocks);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_reject(const Plan& p, const DistParams& d, int rk, float per_packet, int64_t max_blocks,
+                          cudaStream_t s) {
+  const int dt = d.dtype == GR_F32 ? SD_F32 : d.dtype == GR_F64 ? SD_F64 : SD_I32H;
+  TrialRow row{};
+  row.d = d;
+  row.gen = p.gen;
+  row.rk = rk;
+  row.packets = rk == RK_GAMMA_GS ? 3 : (rk >= RK_POISSON ? 1 : 2);
+  row.per_packet = per_packet;
+#define GR_RJ(R)                                                                               \
+  if (rk == R) {                                                                               \
+    if (dt == SD_F32) return run_trials<SD_F32, R>(p, row, nullptr, 1, 0, max_blocks, s);      \
+    if (dt == SD_F64) return run_trials<SD_F64, R>(p, row, nullptr, 1, 0, max_blocks, s);      \
+  }
+  GR_RJ(RK_GAMMA_GS)
+  GR_RJ(RK_GAMMA_TAN)
+  GR_RJ(RK_BETA_SMALL)
+#undef GR_RJ
+  if (rk == RK_POISSON && dt == SD_I32H) return run_trials<SD_I32H, RK_POISSON>(p, row, nullptr, 1, 0, max_blocks, s);
+  if (rk == RK_BINOMIAL && dt == SD_I32H) return run_trials<SD_I32H, RK_BINOMIAL>(p, row, nullptr, 1, 0, max_blocks, s);
+  return cudaErrorNotSupported;
+}
+
+cudaError_t launch_gamma_rows(const Plan& p, int dtype, const TrialRow* rows, int nrows, int64_t row_stride,
+                              int64_t max_blocks, cudaStream_t s) {
+  if (dtype == GR_F64) return run_trials<SD_F64, -1>(p, TrialRow{}, rows, nrows, row_stride, max_blocks, s);
+  return run_trials<SD_F32, -1>(p, TrialRow{}, rows, nrows, row_stride, max_blocks, s);
+}
+
+}  // namespace gr
