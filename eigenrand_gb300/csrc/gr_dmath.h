@@ -21,6 +21,13 @@
 // 2^(j/64) in Q63 (j = n mod 64), scaled by 2^(n div 64) and rounded once,
 // subnormal results included.
 //
+// Both have a short form that computes the same rounded result from the same
+// tables with products only as wide as the rounding needs, and hands the rare
+// argument whose rounding those cannot decide to the long form (their error
+// bounds are at the functions); a CPU test compares the two.  Per argument the
+// short log takes about 120 instructions where the long one takes 370, exp 140
+// against 350.
+//
 // Tables and coefficients: derive_math_tables.py (mpmath), emitted to
 // gr_math_tables.h.  The header compiles for the host as well, so the same
 // code is checked on the CPU.
@@ -32,8 +39,10 @@
 
 #ifdef __CUDACC__
 #define GRD_HD __host__ __device__ __forceinline__
+#define GRD_SLOW static __host__ __device__ __noinline__
 #else
 #define GRD_HD static inline
+#define GRD_SLOW static
 #endif
 
 #ifdef __CUDA_ARCH__
@@ -165,7 +174,7 @@ GRD_HD double grd_round(grd_u128 A, int q, int neg) {
   return grd_double(sgn | sig);  // subnormal (a carry to 2^52 gives the smallest normal)
 }
 
-GRD_HD double grd_log(double x) {
+GRD_SLOW double grd_log_long(double x) {
   const uint64_t ux = grd_bits(x);
   if ((ux & 0x7fffffffffffffffull) > 0x7ff0000000000000ull) return x;  // NaN
   if (ux >> 63)
@@ -206,7 +215,7 @@ GRD_HD double grd_log(double x) {
   return grd_round_norm(h, l, 127 - lz - 116, neg);  // |log x| is within [2^-53, 745]: normal
 }
 
-GRD_HD double grd_exp(double x) {
+GRD_SLOW double grd_exp_long(double x) {
   const uint64_t ux = grd_bits(x);
   const uint64_t ax = ux & 0x7fffffffffffffffull;
   if (ax > 0x7ff0000000000000ull) return x;                   // NaN
@@ -243,6 +252,147 @@ GRD_HD double grd_exp(double x) {
   const uint64_t h = top ? (hi << 2) | (lo >> 62) : (hi << 3) | (lo >> 61);
   const uint64_t l = top ? lo << 2 : lo << 3;
   return grd_round_norm(h, l, E, 0);
+}
+
+GRD_HD uint64_t grd_wide(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
+
+// floor(a b / 2^64) or up to 2 less: the product of the low halves left out
+GRD_HD uint64_t grd_umulhi3(uint64_t a, uint64_t b) {
+  const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a, bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
+  return grd_wide(ah, bh) + (grd_wide(ah, bl) >> 32) + (grd_wide(al, bh) >> 32);
+}
+
+GRD_HD uint32_t grd_umulhi32(uint32_t a, uint32_t b) { return (uint32_t)(grd_wide(a, b) >> 32); }
+
+// c + p or c - p
+GRD_HD uint64_t grd_addsub(uint64_t c, uint64_t p, bool sub) { return sub ? c - p : c + p; }
+
+// log of a positive normal x.  The same v = e ln2 + L1 + L2 + r S(r) as the
+// long form in Q116, r S(r) = r - a (a/2 - s a^2/3 + a^3/4), a = |r|, s its
+// sign: r is exact, the bracket is in Q62 (squares from the top 29 bits of a:
+// error below 2^-59.6, times a 2^-74.6), its product with a in Q91, and the
+// r^5 / 5 term below 2^-77 is left out; the long form's own error is below
+// 2^-75.  So the two sums differ by less than 2^-73, and round alike unless
+// this one lies that close to the middle between two doubles.
+GRD_HD bool grd_log_short(uint64_t ux, double& y) {
+  const uint32_t hx = (uint32_t)(ux >> 32), Ml = (uint32_t)ux;
+  const uint32_t Mh = (hx & 0xfffffu) | 0x100000u;
+  const int i = (int)((Mh >> 13) & 127);
+  const uint32_t K1 = GRD_LD(GRT_ILOG_K1[i]);
+  const uint64_t y1 = grd_wide(Ml, K1) + ((uint64_t)(Mh * K1) << 32);  // (1 + r1) 2^60
+  const uint32_t y1h = (uint32_t)(y1 >> 32);
+  int j = ((int32_t)(y1h - (1u << 28) + (1u << 13)) >> 14) + GRT_ILOG_J0;
+  j = j < 0 ? 0 : (j > GRT_ILOG_JN - 1 ? GRT_ILOG_JN - 1 : j);
+  const uint32_t K2 = (uint32_t)GRD_LD(GRT_ILOG_K2[j]);
+  const uint64_t p0 = grd_wide((uint32_t)y1, K2), p1 = grd_wide(y1h, K2) + (p0 >> 32);  // (1 + r2) 2^80
+  const int64_t r = (int64_t)((p1 << 28) + ((uint32_t)p0 >> 4));                        // r2 2^76
+  const bool neg = r < 0;
+  const uint64_t a = (uint64_t)(neg ? -r : r);
+  const uint32_t ah = (uint32_t)(a >> 32);      // Q44
+  const uint64_t a2 = grd_wide(ah, ah);         // Q88
+  const uint32_t third = grd_umulhi32((uint32_t)(a2 >> 27), 0xaaaaaaabu);             // a^2 / 3, Q62
+  const uint32_t cube = (uint32_t)(grd_wide((uint32_t)(a2 >> 32), ah) >> 40);         // a^3 / 4, Q62
+  const uint64_t T = grd_addsub((a >> 15) + cube, third, !neg);
+  const uint64_t W = grd_umulhi3(a, T << 17);   // Q91
+  // k ln2 - 1023 ln2 with the biased exponent k, modulo 2^128
+  const uint32_t k = hx >> 20;
+  const uint64_t q0 = grd_wide(k, (uint32_t)GRT_ILOG_LN2_LO);
+  const uint64_t q1 = grd_wide(k, (uint32_t)(GRT_ILOG_LN2_LO >> 32)) + (q0 >> 32);
+  const uint64_t q2 = (uint64_t)k * GRT_ILOG_LN2_HI + (q1 >> 32);
+  grd_u128 v = grd_u128_of(q2, (q1 << 32) | (uint32_t)q0);
+  const grd_u128 bias = grd_u128_of(GRT_ILOG_LN2_HI, GRT_ILOG_LN2_LO) * 1023u;
+  v -= bias;
+  v += grd_u128_of(GRD_LD(GRT_ILOG_L1[2 * i]), GRD_LD(GRT_ILOG_L1[2 * i + 1]));
+  v += grd_u128_of(GRD_LD(GRT_ILOG_L2[2 * j]), GRD_LD(GRT_ILOG_L2[2 * j + 1]));
+  v += grd_u128_of((uint64_t)(r >> 24), (uint64_t)r << 40);
+  v -= grd_u128_of(W >> 39, W << 25);
+  uint64_t hi = (uint64_t)(v >> 64), lo = (uint64_t)v;
+  const uint64_t sgn = hi & 0x8000000000000000ull;
+  if (sgn) {
+    lo = 0 - lo;
+    hi = ~hi + (lo == 0 ? 1 : 0);
+  }
+  if (hi < (1ull << 34)) return false;  // |log x| < 2^-18: the error is too large a part of it
+  const int lz = grd_clz64(hi);          // 8 .. 29
+  const uint64_t h = (hi << lz) | (lo >> (64 - lz));
+  // the 32 bits below the rounding position; 2^-73 is 2^(43 + lz - 43) of them
+  const uint32_t f = ((uint32_t)h << 21) | (uint32_t)((lo << lz) >> 43);
+  const uint32_t t = (1u << lz) + 2u;
+  if (f - 0x80000000u + t <= 2u * t) return false;
+  // the significand's leading bit adds 1 to the exponent field
+  const uint64_t bits = ((uint64_t)(11 - lz + 1022) << 52) + (h >> 11) + (f >> 31);
+  y = grd_double(sgn | bits);
+  return true;
+}
+
+// exp of x with 2^-30 <= |x| < 708.  n and r as in the long form, bit for bit.
+// With c6 = 1 + r/2 + r^2/6 + ..., the long form's last step is c = 2^62 +
+// floor(c6 r) in Q62 and its result the rounded 2^(j/64) c.  Its c6 is within
+// 2 units (of 2^-62) of the one here, so c6 r (|r| < 2^-7.5) within 0.012
+// units, and the floors agree unless the fraction is within that of an
+// integer; then c is one unit off at most, which matters only next to the
+// middle between two doubles.
+GRD_HD bool grd_exp_short(uint64_t ux, double& y) {
+  const uint32_t hx = (uint32_t)(ux >> 32);
+  const bool xneg = (hx >> 31) != 0;
+  const int ex = (int)((hx >> 20) & 0x7ff) - 1023;
+  const uint64_t M = (ux & 0xfffffffffffffull) | 0x10000000000000ull;
+  const int sx = ex + 48;  // |x| 2^100 = M 2^sx, 18 <= sx <= 57
+  const int sq = 80 - sx;  // x in Q20, floor
+  const int64_t xq = xneg ? (int64_t)~((M - 1) >> sq) : (int64_t)(M >> sq);
+  const int64_t n = (xq * GRT_IEXP_INVL + (1ll << 39)) >> 40;
+  const uint32_t an = (uint32_t)(xneg ? -n : n);
+  const uint64_t q0 = grd_wide(an, (uint32_t)GRT_IEXP_LN2_64_LO);
+  const uint64_t q1 = grd_wide(an, (uint32_t)(GRT_IEXP_LN2_64_LO >> 32)) + (q0 >> 32);
+  const uint64_t q2 = grd_wide(an, (uint32_t)GRT_IEXP_LN2_64_HI) + (q1 >> 32);
+  const grd_u128 nl = grd_u128_of(q2, (q1 << 32) | (uint32_t)q0);
+  const grd_u128 X = grd_u128_of(M >> (64 - sx), M << sx);
+  const grd_u128 D = xneg ? nl - X : X - nl;  // Q100
+  const int64_t r = (int64_t)(uint64_t)(D >> 36);  // Q64
+  const bool neg = r < 0;
+  const uint64_t a = (uint64_t)(neg ? -r : r);
+  // q = 1/24 + r (1/120 + r/720 + r^2/5040), the bracket in Q38
+  const uint32_t ar = (uint32_t)(a >> 26);              // Q38
+  const uint32_t aa = grd_umulhi32(ar, ar);             // Q44
+  const uint32_t r720 = grd_umulhi32(ar, 5965232u);
+  const uint32_t t = (neg ? 2290649225u - r720 : 2290649225u + r720) + (grd_umulhi32(aa, 852176u) >> 6);
+  const uint64_t at = grd_wide((uint32_t)(a >> 32), t) + (grd_wide((uint32_t)a, t) >> 32);  // Q70
+  const uint64_t q = grd_addsub(0x0aaaaaaaaaaaaaabull, at >> 6, neg);                        // Q64
+  const uint64_t c4 = grd_addsub(0x2aaaaaaaaaaaaaabull, grd_umulhi3(a, q), neg);             // Q64
+  const uint64_t c5 = grd_addsub(0x8000000000000000ull, grd_umulhi3(a, c4), neg);            // Q64
+  const uint64_t c6 = grd_addsub(0x4000000000000000ull, grd_umulhi3(a, c5) >> 2, neg);       // Q62
+  const grd_u128 w = (grd_u128)c6 * a;
+  const uint64_t wh = (uint64_t)(w >> 64), wl = (uint64_t)w;
+  const uint64_t c = neg ? 0x4000000000000000ull - wh - (wl ? 1 : 0) : 0x4000000000000000ull + wh;  // exp(r), Q62
+  const int jj = (int)(n & 63), m = (int)(n >> 6);
+  const grd_u128 P = (grd_u128)GRD_LD(GRT_IEXP_T[jj]) * c;  // Q125, in [2^124, 2^126)
+  const uint64_t hi = (uint64_t)(P >> 64), lo = (uint64_t)P;
+  const int top = (int)(hi >> 61);  // leading bit at 125 or 124
+  const int sh = 3 - top;
+  const uint64_t h = (hi << sh) | (lo >> (64 - sh)), l = lo << sh;
+  const uint32_t f = ((uint32_t)h << 21) | (uint32_t)(l >> 43);
+  // a unit of c moves f by at most 2^24
+  if ((uint32_t)(wl >> 32) + 0x08000000u < 0x10000000u && f - 0x80000000u + 0x02000000u < 0x04000000u) return false;
+  uint64_t sig = h >> 11;
+  const bool up = f > 0x80000000u || (f == 0x80000000u && (((l << 21) != 0) || (sig & 1)));
+  sig += up ? 1 : 0;
+  y = grd_double(((uint64_t)(m + top - 1 + 1022) << 52) + sig);
+  return true;
+}
+
+GRD_HD double grd_log(double x) {
+  const uint64_t ux = grd_bits(x);
+  double y;
+  if ((uint32_t)(ux >> 32) - 0x00100000u < 0x7fe00000u && grd_log_short(ux, y)) return y;
+  return grd_log_long(x);
+}
+
+GRD_HD double grd_exp(double x) {
+  const uint64_t ux = grd_bits(x);
+  double y;
+  // 2^-30 <= |x| < 708
+  if (((uint32_t)(ux >> 32) & 0x7fffffffu) - 0x3e100000u < 0x40862000u - 0x3e100000u && grd_exp_short(ux, y)) return y;
+  return grd_exp_long(x);
 }
 
 }  // namespace gr

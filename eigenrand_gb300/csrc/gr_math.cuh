@@ -31,12 +31,12 @@ __device__ __forceinline__ double u2d(uint64_t u) { return __longlong_as_double(
 
 __device__ __forceinline__ float logf_(float x) {
   uint32_t ux = f2u(x);
-  if (x != x) return x;
-  if (x < 0.0f) return u2f(0x7fc00000u);
-  if (x == 0.0f) return -__int_as_float(0x7f800000);
-  if (ux == 0x7f800000u) return x;
   int e = 0;
-  if (ux < 0x00800000u) {
+  if (ux - 0x00800000u >= 0x7f000000u) {  // not a positive normal number
+    if (x != x) return x;
+    if (x < 0.0f) return u2f(0x7fc00000u);
+    if (x == 0.0f) return -__int_as_float(0x7f800000);
+    if (ux == 0x7f800000u) return x;
     x = x * 8388608.0f;
     ux = f2u(x);
     e = -23;
@@ -70,9 +70,12 @@ __device__ __forceinline__ float logf_(float x) {
 }
 
 __device__ __forceinline__ float expf_(float x) {
-  if (x != x) return x;
-  if (x > 88.72283935546875f) return __int_as_float(0x7f800000);
-  if (x < -103.972084045410156f) return 0.0f;
+  const bool wide = !(fabsf(x) <= 87.0f);  // beyond, 2^n leaves the normal range (or x is NaN)
+  if (wide) {
+    if (x != x) return x;
+    if (x > 88.72283935546875f) return __int_as_float(0x7f800000);
+    if (x < -103.972084045410156f) return 0.0f;
+  }
   float n = rintf(x * 1.442695022e+00f);
   float r = fmaf(-n, 6.933593750e-01f, x);
   r = fmaf(-n, -2.121944417e-04f, r);
@@ -85,13 +88,15 @@ __device__ __forceinline__ float expf_(float x) {
   float r2 = r * r;
   float y = fmaf(r2, p, r) + 1.0f;
   int ni = (int)n;
-  if (ni > 127) {
-    y = y * 2.0f;
-    ni -= 1;
-  }
-  if (ni < -126) {
-    y = y * u2f((uint32_t)(ni + 126 + 127) << 23);
-    return y * u2f(0x00800000u);
+  if (wide) {
+    if (ni > 127) {
+      y = y * 2.0f;
+      ni -= 1;
+    }
+    if (ni < -126) {
+      y = y * u2f((uint32_t)(ni + 126 + 127) << 23);
+      return y * u2f(0x00800000u);
+    }
   }
   return y * u2f((uint32_t)(ni + 127) << 23);
 }
