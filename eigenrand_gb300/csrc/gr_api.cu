@@ -1954,6 +1954,94 @@ gr_status run_multinomial(gr_engine* e, GenState* gst, const MnArgs& a0, int64_t
 
 }  // namespace gr
 
+// ---- rows of gamma draws (Dirichlet, Wishart) ---------------------------------
+namespace gr {
+
+// With many engines one launch draws every row (gr_trials.cu): a launch per
+// row reloads each engine's window, starts a new block and leaves most of the
+// last one unused (64 rows of 10^6 on 608 engines: 31-40 us each).  With few
+// engines a row is long enough for the words-in-memory path.
+constexpr int kRowsMinK = 128;
+
+gr_status generate_gamma_rows(gr_engine* e, const std::vector<gr_gen*>& gens, GammaRows& rows, void* out, int dtype,
+                              int64_t samples, cudaStream_t s) {
+  const size_t es = dtype == GR_F64 ? 8 : 4;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(s, &cap);
+  std::vector<TrialRow> tab(gens.size());
+  bool ok = e->K >= kRowsMinK && gens.size() > 1;
+  double blocks = 64;
+  const int P = dtype == GR_F64 ? 4 : 8;
+  const double npk = (double)(samples / P) / e->K + 1;
+  for (size_t i = 0; ok && i < gens.size(); ++i) {
+    const DistParams& d = gens[i]->dp;
+    if (gens[i]->trunc_base || d.kind != GR_GAMMA || d.dtype != dtype) {
+      ok = false;
+      break;
+    }
+    TrialRow& r = tab[i];
+    r.d = d;
+    if (d.ia) {
+      r.rk = kRowExp;
+      r.packets = 1;
+      r.per_packet = 1.0f;
+    } else if (d.ib >= 2) {
+      r.rk = kRowInt;
+      r.packets = d.ib;
+      r.per_packet = 1.0f;
+    } else {
+      r.rk = d.ic ? 0 : 1;
+      r.packets = d.ic ? 3 : 2;
+      double slack;
+      r.per_packet = (float)(1.0 / expected_yield(r.rk, d, slack));
+    }
+    blocks += (16 * npk + 4096) * 8 * r.packets / (kN * 8) + 1;
+  }
+  if (ok) {
+    bool same = rows.dev && rows.state.size() == gens.size();
+    std::vector<GenState*> state(gens.size());
+    for (size_t i = 0; i < gens.size(); ++i) {
+      gr_status st = ensure_gen_state(gens[i], e->K, s);
+      if (st != GR_OK) return st;
+      state[i] = tab[i].gen = gens[i]->gst;
+      same = same && rows.state[i] == state[i];
+    }
+    if (!same && cap != cudaStreamCaptureStatusNone) ok = false;  // the table's upload cannot be captured
+    if (ok && !same) {
+      if (!rows.dev) GR_CUDA(cudaMalloc(&rows.dev, sizeof(TrialRow) * gens.size()));
+      // pageable source: staged before the call returns
+      GR_CUDA(cudaMemcpyAsync(rows.dev, tab.data(), sizeof(TrialRow) * gens.size(), cudaMemcpyHostToDevice, s));
+      rows.state = state;
+    }
+  }
+  if (!ok) {
+    for (size_t i = 0; i < gens.size(); ++i) {
+      gr_status st = gr_generate(gens[i], e, static_cast<char*>(out) + i * (size_t)samples * es, (size_t)samples, s);
+      if (st != GR_OK) return st;
+    }
+    return GR_OK;
+  }
+  if (samples <= 0) return GR_OK;
+  Plan p{};
+  p.eng = e->st;
+  p.K = e->K;
+  p.S = 1;
+  p.gran = P;
+  p.gran_per_k = samples / P / e->K;
+  p.gran_rem = samples / P % e->K;
+  p.out = out;
+  const cudaError_t err = launch_gamma_rows(p, dtype, rows.dev, (int)gens.size(), samples, block_cap((int64_t)blocks), s);
+  if (err != cudaSuccess) return cuda_fail(err, "gamma rows kernel");
+  return GR_OK;
+}
+
+void gamma_rows_free(GammaRows& rows) {
+  cudaFree(rows.dev);
+  rows.dev = nullptr;
+}
+
+}  // namespace gr
+
 // ---- engine scratch reservation (serving loop) -------------------------------
 namespace gr {
 

@@ -116,11 +116,9 @@ __global__ void __launch_bounds__(kMaskThreads) k_chain_masks(ChainArgs a) {
     const int ty = c == 0 ? ty0 : ty1;
     if (ty < 2) continue;
     const BetaComp& g = a.bk.c[c];
-    // lanes the filter leaves open, then (all of them for the tan proposal)
-    // the reference's expressions
-    uint32_t m = 0, open = (1u << P) - 1u;
+    // accepted lanes, and those the filters leave to the reference's expressions
+    uint32_t m = 0, open = 0;
     if (ty == 2) {
-      open = 0;
 #pragma unroll
       for (int l = 0; l < kLanes; ++l) {
         const uint64_t w0 = sw[l][tid], w1 = sw[l][tid + 1], w2 = sw[l][tid + 2];
@@ -134,6 +132,21 @@ __global__ void __launch_bounds__(kMaskThreads) k_chain_masks(ChainArgs a) {
                                    g.f_am1, g.f_band);
           const int f1 = gs_filter(ur_f((uint32_t)(w0 >> 32)), ur_f((uint32_t)(w1 >> 32)) + e,
                                    ur_f((uint32_t)(w2 >> 32)), g.f_px, g.f_inv, g.f_am1, g.f_band);
+          m |= ((f0 == 1 ? 1u : 0u) | (f1 == 1 ? 2u : 0u)) << (2 * l);
+          open |= ((f0 < 0 ? 1u : 0u) | (f1 < 0 ? 2u : 0u)) << (2 * l);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int l = 0; l < kLanes; ++l) {
+        const uint64_t w0 = sw[l][tid], w1 = sw[l][tid + 1];
+        if (DT == SD_F64) {
+          const int f = tan_filter_f64(w0, w1, g.f_am1, g.f_sq);
+          m |= (f == 1 ? 1u : 0u) << l;
+          open |= (f < 0 ? 1u : 0u) << l;
+        } else {
+          const int f0 = tan_filter(ur_f((uint32_t)w0), ur_f((uint32_t)w1), g.f_am1, g.f_sq, kTanDeltaF);
+          const int f1 = tan_filter(ur_f((uint32_t)(w0 >> 32)), ur_f((uint32_t)(w1 >> 32)), g.f_am1, g.f_sq, kTanDeltaF);
           m |= ((f0 == 1 ? 1u : 0u) | (f1 == 1 ? 2u : 0u)) << (2 * l);
           open |= ((f0 < 0 ? 1u : 0u) | (f1 < 0 ? 2u : 0u)) << (2 * l);
         }

@@ -8,6 +8,7 @@
 #include "../../include/gpurand.h"
 
 #include <string>
+#include <vector>
 
 namespace gr {
 
@@ -293,6 +294,17 @@ EngState* engine_state_ptr(gr_engine* e);
 // AVX2 profile only.
 gr_status need_four_lanes(const gr_engine* e, const char* what);
 gr_status set_last_error(gr_status s, const std::string& msg);
+// Several GammaGen objects drawn one after the other, `samples` outputs each
+// (whole packets), row i at out + i * samples elements: what gr_generate gives
+// row by row.  rows: the object that owns the generators keeps their device
+// table there (freed by gamma_rows_free).
+struct GammaRows {
+  TrialRow* dev = nullptr;
+  std::vector<GenState*> state;  // the generators' caches the table points to
+};
+gr_status generate_gamma_rows(gr_engine* e, const std::vector<gr_gen*>& gens, GammaRows& rows, void* out, int dtype,
+                              int64_t samples, cudaStream_t s);
+void gamma_rows_free(GammaRows& rows);
 // Scalar draws on the packet engine (each takes a whole packet and keeps lane
 // 0): stream k of the engine owns samples [s0_k, s0_k + n_k) of `samples`,
 // split as any call splits them, and makes per_sample * n_k draws in stream

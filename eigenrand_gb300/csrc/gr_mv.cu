@@ -625,31 +625,46 @@ __global__ void __launch_bounds__(256)
 
 // =================================================================== Dirichlet
 // rows: K x n row-major (category i's gamma draws in row i); out: K x n
-// col-major.  Tile of 32 samples: coalesced row reads, one column sum per
-// sample, contiguous writes of 32 K-vectors.
-template <typename T>
+// col-major.  Tiles of TS samples: row reads of TS contiguous values, one
+// column sum per sample (in category order), contiguous writes of TS
+// K-vectors.  Bound by HBM.  With 32-sample tiles one warp of eight summed and
+// the writes divided by K twice per value: 64 x 10^6 floats 204 us.
+template <typename T, int TS>
 __global__ void __launch_bounds__(256) k_dirichlet(const T* __restrict__ rows, T* __restrict__ out, int K, int64_t n) {
   extern __shared__ unsigned char dsm_raw[];
-  T* tile = reinterpret_cast<T*>(dsm_raw);  // [K][33]
-  T* tot = tile + (size_t)K * 33;            // [32]
-  const int64_t s0 = (int64_t)blockIdx.x * 32;
-  const int nv = (int)i64min(32, n - s0);
+  T* tile = reinterpret_cast<T*>(dsm_raw);  // [K][TS + 1]
+  T* tot = tile + (size_t)K * (TS + 1);     // [TS]
+  const int64_t s0 = (int64_t)blockIdx.x * TS;
+  const int nv = (int)i64min(TS, n - s0);
   const int tid = threadIdx.x;
-  for (int t = tid; t < K * 32; t += blockDim.x) {
-    const int i = t / 32, c = t % 32;
-    tile[i * 33 + c] = c < nv ? rows[(int64_t)i * n + s0 + c] : T(1);
+  constexpr int VW = 16 / (int)sizeof(T);
+  if (nv == TS && n % VW == 0) {  // rows start on 16 bytes
+#pragma unroll 4
+    for (int t = tid; t < K * (TS / VW); t += blockDim.x) {
+      const int i = t / (TS / VW), c = t % (TS / VW) * VW;
+      const uint4 q = __ldcs(reinterpret_cast<const uint4*>(rows + (int64_t)i * n + s0 + c));
+      const T* v = reinterpret_cast<const T*>(&q);
+#pragma unroll
+      for (int j = 0; j < VW; ++j) tile[i * (TS + 1) + c + j] = v[j];
+    }
+  } else {
+    for (int t = tid; t < K * TS; t += blockDim.x) {
+      const int i = t / TS, c = t % TS;
+      tile[i * (TS + 1) + c] = c < nv ? rows[(int64_t)i * n + s0 + c] : T(1);
+    }
   }
   __syncthreads();
-  if (tid < 32) {
+  if (tid < TS) {
     T s = 0;
-    for (int i = 0; i < K; ++i) s += tile[i * 33 + tid];
+    for (int i = 0; i < K; ++i) s += tile[i * (TS + 1) + tid];
     tot[tid] = s;
   }
   __syncthreads();
   T* o = out + s0 * K;
+  const float rK = 1.0f / (float)K;
   for (int t = tid; t < nv * K; t += blockDim.x) {
-    const int c = t / K, i = t % K;
-    o[t] = tile[i * 33 + c] / tot[c];
+    const int c = (int)(((float)t + 0.5f) * rK);  // t / K: t < 2^17
+    o[t] = tile[(t - c * K) * (TS + 1) + c] / tot[c];
   }
 }
 
@@ -927,25 +942,30 @@ cudaError_t launch_wishart(const void* normals, const void* chis, const void* ch
   return cudaGetLastError();
 }
 
-size_t dirichlet_smem(int K, int dtype) {
-  return ((size_t)K * 33 + 32) * (dtype == GR_F32 ? sizeof(float) : sizeof(double));
+static size_t dirichlet_tile_smem(int K, int dtype, int TS) {
+  return ((size_t)K * (TS + 1) + TS) * (dtype == GR_F32 ? sizeof(float) : sizeof(double));
+}
+size_t dirichlet_smem(int K, int dtype) { return dirichlet_tile_smem(K, dtype, 32); }
+
+template <typename T, int TS>
+static cudaError_t run_dirichlet(const void* rows, void* out, int K, int64_t n, size_t smem, cudaStream_t s) {
+  cudaError_t e = cudaFuncSetAttribute(k_dirichlet<T, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k_dirichlet<T, TS><<<(unsigned)((n + TS - 1) / TS), 256, smem, s>>>((const T*)rows, (T*)out, K, n);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_dirichlet(const void* rows, void* out, int K, int64_t n, int dtype, cudaStream_t s) {
   const size_t smem = dirichlet_smem(K, dtype);
   if (smem > kMvMaxSmem) return cudaErrorInvalidValue;
-  const unsigned grid = (unsigned)((n + 31) / 32);
-  if (dtype == GR_F32) {
-    cudaError_t e = cudaFuncSetAttribute(k_dirichlet<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    k_dirichlet<float><<<grid, 256, smem, s>>>((const float*)rows, (float*)out, K, n);
-  } else {
-    cudaError_t e =
-        cudaFuncSetAttribute(k_dirichlet<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    k_dirichlet<double><<<grid, 256, smem, s>>>((const double*)rows, (double*)out, K, n);
+  // 128-sample tiles while six CTAs fit an SM, 32 for the large dimensions
+  const size_t wide = dirichlet_tile_smem(K, dtype, 128);
+  if (wide <= 36 * 1024) {
+    if (dtype == GR_F32) return run_dirichlet<float, 128>(rows, out, K, n, wide, s);
+    return run_dirichlet<double, 128>(rows, out, K, n, wide, s);
   }
-  return cudaGetLastError();
+  if (dtype == GR_F32) return run_dirichlet<float, 32>(rows, out, K, n, smem, s);
+  return run_dirichlet<double, 32>(rows, out, K, n, smem, s);
 }
 
 cudaError_t launch_multinomial(const Plan& p, const MnArgs& a, const CallSnap* snap, cudaStream_t s) {

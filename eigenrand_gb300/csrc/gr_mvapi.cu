@@ -229,12 +229,14 @@ struct gr_wishart {
   void* chol = nullptr;  // factor in the object's type (aliases L64 for double)
   gr_gen* normal = nullptr;
   std::vector<gr_gen*> chis;
+  GammaRows rows;
   Scratch scratch;
 };
 
 struct gr_dirichlet {
   int dim = 0, dtype = GR_F32;
   std::vector<gr_gen*> gammas;
+  GammaRows rows;
   Scratch scratch;
 };
 
@@ -404,6 +406,7 @@ gr_status gr_wishart_destroy(gr_wishart* g) {
   cudaFree(g->L64);
   gr_gen_destroy(g->normal);
   for (gr_gen* c : g->chis) gr_gen_destroy(c);
+  gamma_rows_free(g->rows);
   delete g;
   return GR_OK;
 }
@@ -469,10 +472,8 @@ gr_status gr_wishart_sample(gr_wishart* g, gr_engine* e, void* dev_out, size_t s
     st = gr_generate(g->normal, e, normals, nnorm, stream);
     if (st != GR_OK) return st;
   }
-  for (int i = 0; i < d; ++i) {
-    st = gr_generate(g->chis[i], e, chis + (size_t)i * samples * es, samples, stream);
-    if (st != GR_OK) return st;
-  }
+  st = generate_gamma_rows(e, g->chis, g->rows, chis, g->dtype, (int64_t)samples, (cudaStream_t)stream);
+  if (st != GR_OK) return st;
   // the tcgen05 products for float WishartGen up to dim 64; test hook
   // GR_WISHART_PRODUCT=mma_sync picks the mma.sync form
   bool umma = wishart_umma_usable(d, g->dtype, g->inverse);
@@ -491,6 +492,7 @@ gr_status gr_wishart_sample(gr_wishart* g, gr_engine* e, void* dev_out, size_t s
 gr_status gr_dirichlet_destroy(gr_dirichlet* g) {
   if (!g) return GR_OK;
   for (gr_gen* x : g->gammas) gr_gen_destroy(x);
+  gamma_rows_free(g->rows);
   delete g;
   return GR_OK;
 }
@@ -530,10 +532,8 @@ gr_status gr_dirichlet_sample(gr_dirichlet* g, gr_engine* e, void* dev_out, size
   gr_status st = g->scratch.need((size_t)g->dim * samples * es);
   if (st != GR_OK) return st;
   char* rows = (char*)g->scratch.p;
-  for (int i = 0; i < g->dim; ++i) {
-    st = gr_generate(g->gammas[i], e, rows + (size_t)i * samples * es, samples, stream);
-    if (st != GR_OK) return st;
-  }
+  st = generate_gamma_rows(e, g->gammas, g->rows, rows, g->dtype, (int64_t)samples, (cudaStream_t)stream);
+  if (st != GR_OK) return st;
   cudaError_t err = launch_dirichlet(rows, dev_out, g->dim, (int64_t)samples, g->dtype, (cudaStream_t)stream);
   if (err != cudaSuccess) return mv_fail(GR_ERR_CUDA, std::string("Dirichlet normalisation: ") + cudaGetErrorString(err));
   return GR_OK;

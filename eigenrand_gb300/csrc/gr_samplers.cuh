@@ -63,6 +63,53 @@ __device__ __forceinline__ int gs_filter_f64(uint64_t bux, uint64_t bvx, uint64_
   return gs_filter(ux, vx, ux2, pxf, inv_a, am1, band);
 }
 
+// Accept test of a tan-proposal trial (GammaGen, alpha > 1, NormalExp.h:588-604)
+// decided by the special-function unit, as gs_filter: with y = tan(pi u),
+// x = sq y + a1 (a1 = alpha - 1, sq = sqrt(2 alpha - 1)), accept when x > 0
+// and ux <= (1 + y^2) exp(a1 log(x / a1) - sq y).
+// delta bounds the absolute errors of sin and cos, here and in the reference's
+// polynomials (sin.approx / cos.approx: 2^-20.5 on [-2 pi, 2 pi]; PTX ISA), so
+// y is off by at most dy = delta (1 + |y|)^2 (|y| <= 64), the exponent with the
+// logarithm of 1 + y^2 by dy (1 + sq |a1 / x - 1|) from y and by
+// 2^-20 (1 + a1 + sq |y| + |a1 log|) from roundings on both sides.  Twice that
+// is the band; where it is wide, or the sign of x open, the caller evaluates
+// the reference's expressions.  Five special-function operations and some
+// twenty others where those take about 150 instructions (double: about 100 of
+// them on the FP64 pipe), and rejected lanes need nothing more.
+__device__ __forceinline__ int tan_filter(float u, float ux, float a1, float sq, float delta) {
+  const float t = 3.14159274f * u;
+  float s, c, rc, ra, rx;
+  asm("sin.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(t));
+  asm("cos.approx.ftz.f32 %0, %1;" : "=f"(c) : "f"(t));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"(c));
+  const float y = s * rc, ay = fabsf(y), dy = delta * (1.0f + ay) * (1.0f + ay);
+  if (!(ay <= 64.0f)) return -1;
+  const float x = fmaf(sq, y, a1), gap = 2.0f * sq * dy + 1e-6f * a1;
+  if (x < -gap) return 0;
+  if (!(x > gap)) return -1;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ra) : "f"(a1));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rx) : "f"(x));
+  const float al = a1 * lg2_approx(x * ra) * 0.693147182f, sy = sq * y;
+  const float tol = 2.0f * (dy * (1.0f + sq * fabsf(sy) * rx) + 0x1p-20f * (1.0f + a1 + fabsf(sy) + fabsf(al)));
+  const float ub = fmaf(y, y, 1.0f) * ex2_approx(1.44269502f * (al - sy));
+  if (!(tol < 0.25f)) return -1;
+  if (ux < ub * (1.0f - tol)) return 1;
+  if (ux > ub * (1.0f + tol)) return 0;
+  return -1;
+}
+constexpr float kTanDeltaF = 0x1p-20f;   // float trials
+constexpr float kTanDeltaD = 0x1p-19f;   // double trials: pi u rounds to float besides
+
+__device__ __forceinline__ int tan_filter_f64(uint64_t bu, uint64_t bux, float a1, float sq) {
+  constexpr uint64_t M = 0xfffffffffffffull;
+  const float u = __uint2float_rn((uint32_t)((bu & M) >> 20)) * 0x1p-32f;
+  const float ux = __uint2float_rn((uint32_t)((bux & M) >> 20)) * 0x1p-32f;
+  // ux within 2^-24: outside that of both ends of the band
+  const int lo = tan_filter(u, ux - 0x1p-23f, a1, sq, kTanDeltaD);
+  const int hi = tan_filter(u, ux + 0x1p-23f, a1, sq, kTanDeltaD);
+  return lo == hi ? lo : -1;
+}
+
 // Candidate of a double GS trial already known to be accepted: xx only
 // (no acceptance bound); ux < px is decided on the integer fraction against
 // tpx = ceil(px * 2^52).
@@ -111,14 +158,20 @@ __device__ __forceinline__ bool rej_trial(const DistParams& d, int64_t t, int j,
     } else if (RK == RK_GAMMA_TAN) {
       const float u = ur_f(word(w0 + j));
       const float ux = ur_f(word(w0 + 8 + j));
-      float ys, yc;
-      sincosf_((float)3.1415926535897932 * u, ys, yc);
-      const float yx = ys / yc;
-      const float xx = d.ff * yx + d.fd;  // sqrt * yx + (alpha - 1)
-      const bool c = 0.0f < xx;
-      const float ub = (yx * yx + 1.0f) * expf_(d.fd * logf_(xx / d.fd) - yx * d.ff);
-      acc = c && (ux <= ub);
-      cbits = f2u(d.fb * xx);
+      const int f = tan_filter(u, ux, d.fd, d.ff, kTanDeltaF);
+      acc = f == 1;
+      if ((CAND && f != 0) || f < 0) {
+        float ys, yc;
+        sincosf_((float)3.1415926535897932 * u, ys, yc);
+        const float yx = ys / yc;
+        const float xx = d.ff * yx + d.fd;  // sqrt * yx + (alpha - 1)
+        if (f < 0) {
+          const bool c = 0.0f < xx;
+          const float ub = (yx * yx + 1.0f) * expf_(d.fd * logf_(xx / d.fd) - yx * d.ff);
+          acc = c && (ux <= ub);
+        }
+        cbits = f2u(d.fb * xx);
+      }
     } else if (RK == RK_BETA_SMALL) {
       const float u1 = ur_f(word(w0 + j));
       const float u2 = ur_f(word(w0 + 8 + j));
@@ -157,16 +210,22 @@ __device__ __forceinline__ bool rej_trial(const DistParams& d, int64_t t, int j,
         acc = ux2 < qx;
       }
     } else if (RK == RK_GAMMA_TAN) {
-      const double u = ur_d(rval(r0));
-      const double ux = ur_d(rval(r0 + 4));
-      double ys, yc;
-      sincos_(3.1415926535897932 * u, ys, yc);
-      const double yx = ys / yc;
-      const double xx = d.df * yx + d.dd;
-      const bool c = 0.0 < xx;
-      const double ub = (yx * yx + 1.0) * exp_(d.dd * log_(xx / d.dd) - yx * d.df);
-      acc = c && (ux <= ub);
-      cbits = d2u(d.db * xx);
+      const int f = tan_filter_f64(rval(r0), rval(r0 + 4), d.fd, d.ff);
+      acc = f == 1;
+      if ((CAND && f != 0) || f < 0) {
+        const double u = ur_d(rval(r0));
+        double ys, yc;
+        sincos_(3.1415926535897932 * u, ys, yc);
+        const double yx = ys / yc;
+        const double xx = d.df * yx + d.dd;
+        if (f < 0) {
+          const double ux = ur_d(rval(r0 + 4));
+          const bool c = 0.0 < xx;
+          const double ub = (yx * yx + 1.0) * exp_(d.dd * log_(xx / d.dd) - yx * d.df);
+          acc = c && (ux <= ub);
+        }
+        cbits = d2u(d.db * xx);
+      }
     } else if (RK == RK_BETA_SMALL) {
       const double u1 = ur_d(rval(r0));
       const double u2 = ur_d(rval(r0 + 4));

@@ -86,3 +86,16 @@ def test_filter_band_covers_the_errors():
         band = 2.0 ** -18 * (1 + 40 / alpha)
         assert np.max(np.abs(q1 / q1x - 1)) < band / 19
         assert np.max(np.abs(q2 / q2x - 1)) < band / 19
+
+
+@pytest.mark.parametrize("tdt", [torch.float32, torch.float64])
+@pytest.mark.parametrize("alpha", [1.0001, 1.05, 1.5, 3.3, 19.5, 200.0, 30000.0])
+def test_tan_filter_decides_as_the_reference(gpulib, oracle, tdt, alpha):
+    """10^6 trials per shape: one accept flag that differs would shift every
+    later value."""
+    er = gpulib
+    u, e = er.Vmt19937_64(5), oracle.Engine(5)
+    npdt = np.float32 if tdt == torch.float32 else np.float64
+    n = 1 << 20 if tdt == torch.float32 else 1 << 19
+    out = er.gamma(n, 1, u, alpha, 1.0, dtype=tdt).reshape(-1).cpu().numpy()
+    assert np.array_equal(bits(out), bits(oracle.generate(e, oracle.Gen(), "GAMMA", n, npdt, alpha, 1.0)))
