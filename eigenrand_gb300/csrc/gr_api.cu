@@ -1783,11 +1783,11 @@ gr_status gr_sample_batched(gr_engine* e, const gr_batch_desc* bd, gr_stream_t s
 gr_status gr_sample(gr_engine* e, const gr_dist_desc* desc, void* dev_out, size_t n, gr_stream_t stream) {
   if (!e || !desc) return fail(GR_ERR_INVALID, "NULL argument");
   cudaStream_t s = (cudaStream_t)stream;
-  // A temporary *Gen: its caches start empty and die with the call.  They
-  // live in engine-owned scratch that is cleared in stream order, so the
-  // call stays asynchronous.
-  if (!e->scratch_gen) GR_CUDA(cudaMalloc(&e->scratch_gen, sizeof(GenState) * (size_t)e->K));
-  GR_CUDA(cudaMemsetAsync(e->scratch_gen, 0, sizeof(GenState) * (size_t)e->K, s));
+  // A temporary *Gen: its caches start empty and die with the call.  The
+  // samplers that carry lanes or packets across trials keep them in
+  // engine-owned scratch that is cleared in stream order, so the call stays
+  // asynchronous; the fixed-draw kinds run without (a NULL state is an empty
+  // one that nothing is left in), one launch less.
   gr_gen tmp;
   tmp.desc = *desc;
   gr_status st = GR_OK;
@@ -1811,8 +1811,6 @@ gr_status gr_sample(gr_engine* e, const gr_dist_desc* desc, void* dev_out, size_
     tmp.dp.bitmask = mask;
     tmp.dp.prob = tmp.table;
     tmp.dp.alias = tmp.table + np;
-    tmp.gst = e->scratch_gen;
-    tmp.gst_K = e->K;
     // pageable source: the table is staged before cudaMemcpyAsync returns
     st = run_call(e, &tmp, tmp.dp, dev_out, n, s);
     cudaFreeAsync(tmp.table, s);
@@ -1822,8 +1820,13 @@ gr_status gr_sample(gr_engine* e, const gr_dist_desc* desc, void* dev_out, size_
   }
   st = make_params(tmp.desc, tmp.dp);
   if (st != GR_OK) return st;
-  tmp.gst = e->scratch_gen;
-  tmp.gst_K = e->K;
+  const Family fam = family_of(tmp.dp);
+  if (fam != Family::Direct && fam != Family::Staged) {
+    if (!e->scratch_gen) GR_CUDA(cudaMalloc(&e->scratch_gen, sizeof(GenState) * (size_t)e->K));
+    GR_CUDA(cudaMemsetAsync(e->scratch_gen, 0, sizeof(GenState) * (size_t)e->K, s));
+    tmp.gst = e->scratch_gen;
+    tmp.gst_K = e->K;
+  }
   st = run_call(e, &tmp, tmp.dp, dev_out, n, s);
   tmp.gst = nullptr;
   return st;
@@ -2008,7 +2011,8 @@ gr_status generate_gamma_rows(gr_engine* e, const std::vector<gr_gen*>& gens, Ga
     }
     if (!same && cap != cudaStreamCaptureStatusNone) ok = false;  // the table's upload cannot be captured
     if (ok && !same) {
-      if (!rows.dev) GR_CUDA(cudaMalloc(&rows.dev, sizeof(TrialRow) * gens.size()));
+      if (!rows.dev)
+        GR_CUDA(scratch_alloc(reinterpret_cast<void**>(&rows.dev), sizeof(TrialRow) * gens.size(), e->device, s));
       // pageable source: staged before the call returns
       GR_CUDA(cudaMemcpyAsync(rows.dev, tab.data(), sizeof(TrialRow) * gens.size(), cudaMemcpyHostToDevice, s));
       rows.state = state;

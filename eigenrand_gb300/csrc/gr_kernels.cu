@@ -530,6 +530,20 @@ __device__ __forceinline__ void st16(void* p, uint32_t a, uint32_t b, uint32_t c
   *reinterpret_cast<uint4*>(p) = make_uint4(a, b, c, d);
 }
 
+// 32 bytes of one packet.  A thread's packet is one 32-byte sector: two 16-byte
+// stores reach L2 as two partial writes of it (8192 x 8192 uniform floats:
+// 79.6 us), the 256-bit store as one.  An output that is only 16-byte aligned
+// (or starts after an odd cached packet) takes the two.
+__device__ __forceinline__ void st32(void* p, const uint64_t a, const uint64_t b, const uint64_t c, const uint64_t d) {
+  if (((uintptr_t)p & 31) == 0) {
+    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
+  } else {
+    reinterpret_cast<ulonglong2*>(p)[0] = make_ulonglong2(a, b);
+    reinterpret_cast<ulonglong2*>(p)[1] = make_ulonglong2(c, d);
+  }
+}
+__device__ __forceinline__ uint64_t two32(uint32_t lo, uint32_t hi) { return (uint64_t)lo | (uint64_t)hi << 32; }
+
 // int32 kinds whose packets are rng.half() words leave raw words in the
 // engine's half cache; DiscreteGen caches its own computed results
 template <int MODE, int KIND>
@@ -553,8 +567,7 @@ __device__ __forceinline__ void emit_packet(const uint64_t (&pk)[kLanes], const 
   if (MODE == M_RAW) {
     if (valid && p.out) {  // p.out == nullptr: discard
       uint64_t* o = reinterpret_cast<uint64_t*>(p.out) + obase + pidx * 4;
-      reinterpret_cast<ulonglong2*>(o)[0] = make_ulonglong2(pk[0], pk[1]);
-      reinterpret_cast<ulonglong2*>(o)[1] = make_ulonglong2(pk[2], pk[3]);
+      st32(o, pk[0], pk[1], pk[2], pk[3]);
     }
   } else if (MODE == M_RAW2) {
     if (valid && p.out)
@@ -600,8 +613,8 @@ __device__ __forceinline__ void emit_packet(const uint64_t (&pk)[kLanes], const 
           v[2 * l + 1] = tf32i<KIND>((uint32_t)(pk[l] >> 32), d, obase + pidx * 8 + 2 * l + 1);
         }
       }
-      reinterpret_cast<float4*>(o)[0] = make_float4(v[0], v[1], v[2], v[3]);
-      reinterpret_cast<float4*>(o)[1] = make_float4(v[4], v[5], v[6], v[7]);
+      st32(o, two32(f2u(v[0]), f2u(v[1])), two32(f2u(v[2]), f2u(v[3])), two32(f2u(v[4]), f2u(v[5])),
+           two32(f2u(v[6]), f2u(v[7])));
     }
   } else if (MODE == M_F64) {
     if (valid) {
@@ -609,8 +622,7 @@ __device__ __forceinline__ void emit_packet(const uint64_t (&pk)[kLanes], const 
       double v[4];
 #pragma unroll
       for (int l = 0; l < kLanes; ++l) v[l] = tf64i<KIND>(pk[l], d, obase + pidx * 4 + l);
-      reinterpret_cast<double2*>(o)[0] = make_double2(v[0], v[1]);
-      reinterpret_cast<double2*>(o)[1] = make_double2(v[2], v[3]);
+      st32(o, d2u(v[0]), d2u(v[1]), d2u(v[2]), d2u(v[3]));
     }
   } else if (MODE == M_W32 || MODE == M_W64) {
     if (valid) {
@@ -627,9 +639,9 @@ __device__ __forceinline__ void emit_packet(const uint64_t (&pk)[kLanes], const 
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[q] = tw32<KIND>(wd[q], d);
         int32_t* o = reinterpret_cast<int32_t*>(p.out) + ob;
-        st16(o, v[0], v[1], v[2], v[3]);
-        if (full) st16(o + 4, v[4], v[5], v[6], v[7]);
-        else if (gs || kHalfKind) {
+        if (full) st32(o, two32(v[0], v[1]), two32(v[2], v[3]), two32(v[4], v[5]), two32(v[6], v[7]));
+        else st16(o, v[0], v[1], v[2], v[3]);
+        if (!full && (gs || kHalfKind)) {
           // leftover half: rng.half() kinds leave raw words in the engine's
           // half() cache; DiscreteGen caches its computed upper 4 results
           uint32_t* cdst = kHalfKind ? st->half_cache : gs->s[0].cache;
@@ -641,13 +653,11 @@ __device__ __forceinline__ void emit_packet(const uint64_t (&pk)[kLanes], const 
 #pragma unroll
         for (int q = 0; q < 4; ++q) v[q] = tw64i<KIND>(wd[q], d, ob + q);
         double* o = reinterpret_cast<double*>(p.out) + ob;
-        reinterpret_cast<double2*>(o)[0] = make_double2(v[0], v[1]);
-        reinterpret_cast<double2*>(o)[1] = make_double2(v[2], v[3]);
+        st32(o, d2u(v[0]), d2u(v[1]), d2u(v[2]), d2u(v[3]));
         if (full) {
 #pragma unroll
           for (int q = 4; q < 8; ++q) v[q] = tw64i<KIND>(wd[q], d, ob + q);
-          reinterpret_cast<double2*>(o)[2] = make_double2(v[4], v[5]);
-          reinterpret_cast<double2*>(o)[3] = make_double2(v[6], v[7]);
+          st32(o + 4, d2u(v[4]), d2u(v[5]), d2u(v[6]), d2u(v[7]));
         } else {
 #pragma unroll
           for (int q = 0; q < 4; ++q) st->half_cache[q] = wd[4 + q];
@@ -691,7 +701,7 @@ __device__ __forceinline__ void emit_packet(const uint64_t (&pk)[kLanes], const 
         reinterpret_cast<float4*>(o + 8 + i0)[0] =
             make_float4(nscale32i<KIND>(cv[0], d, ob + 8 + i0), nscale32i<KIND>(cv[1], d, ob + 9 + i0),
                         nscale32i<KIND>(cv[2], d, ob + 10 + i0), nscale32i<KIND>(cv[3], d, ob + 11 + i0));
-      } else {
+      } else if (gs) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) gs->s[0].cache[i0 + q] = f2u(cv[q]);
       }
@@ -726,7 +736,7 @@ __device__ __forceinline__ void emit_packet(const uint64_t (&pk)[kLanes], const 
       if (ob + 8 <= oend) {
         reinterpret_cast<double2*>(o + 4 + i0)[0] =
             make_double2(nscale64i<KIND>(cv[0], d, ob + 4 + i0), nscale64i<KIND>(cv[1], d, ob + 5 + i0));
-      } else {
+      } else if (gs) {
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           uint64_t b = d2u(cv[q]);
@@ -738,9 +748,14 @@ __device__ __forceinline__ void emit_packet(const uint64_t (&pk)[kLanes], const 
   }
 }
 
+// Kinds whose transform takes a few operations per word.
+template <int MODE, int KIND>
+constexpr bool kLightKind = MODE == M_RAW || MODE == M_RAW0 || MODE == M_RAW2 || KIND == GR_UNIFORM_REAL ||
+                            KIND == GR_UNIFORM_REAL2 || (KIND == GR_BALANCED && MODE != M_W64) || KIND == GR_BERNOULLI ||
+                            KIND == GR_RANDBITS || KIND == GR_UNIFORM_INT;
+
 template <int MODE, int KIND>
 __global__ void __maxnreg__(64) k_direct(Plan p, DistParams d, const CallSnap* snap) {
-  __shared__ uint64_t raw[2][kLanes][kN];
   const int k = blockIdx.x / p.S, s = blockIdx.x % p.S;
   const int tid = threadIdx.x;
   EngState* st = p.eng + k;
@@ -761,8 +776,8 @@ __global__ void __maxnreg__(64) k_direct(Plan p, DistParams d, const CallSnap* s
     cvalid = p.S > 1 ? snap[k].half_valid : st->half_valid;
     cwords = p.S > 1 ? snap[k].half_cache : st->half_cache;
   } else if (kUsesGen) {
-    cvalid = p.S > 1 ? snap[k].gen_valid : gs->s[0].valid;
-    cwords = p.S > 1 ? snap[k].gen_cache : gs->s[0].cache;
+    cvalid = p.S > 1 ? snap[k].gen_valid : (gs ? gs->s[0].valid : 0);
+    cwords = p.S > 1 ? snap[k].gen_cache : (gs ? gs->s[0].cache : nullptr);
   }
   constexpr int CO = ModeInfo<MODE>::kCacheOut;
   const int64_t Q0 = (cvalid && CO) ? min((int64_t)CO, n) : 0;
@@ -789,58 +804,75 @@ __global__ void __maxnreg__(64) k_direct(Plan p, DistParams d, const CallSnap* s
 
   // --- lane windows.  With several segments the last one rewrites st->win,
   // so segment 0 reads the copy the prefix kernel made at call start.
+  const uint64_t* w0;
+  size_t wl = kN;  // stride of the window's lanes
   if (s == 0 && p.S > 1) {
-    for (int i = tid; i < kLanes * kN; i += blockDim.x)
-      (&raw[0][0][0])[i] = p.prefix[((size_t)k * kLanes + i / kN) * kPrefixLen + i % kN];
+    w0 = p.prefix + (size_t)k * kLanes * kPrefixLen;
+    wl = kPrefixLen;
   } else {
-    const uint64_t* w0 = (s == 0) ? &st->win[0][0] : p.segwin + ((size_t)k * (p.S - 1) + (s - 1)) * kLanes * kN;
-    for (int i = tid; i < kLanes * kN; i += blockDim.x) (&raw[0][0][0])[i] = w0[i];
+    w0 = s == 0 ? &st->win[0][0] : p.segwin + ((size_t)k * (p.S - 1) + (s - 1)) * kLanes * kN;
   }
-  __syncthreads();
-
+  // Thread t < 156 holds word t of the last two phases (156 words) of the four
+  // lanes: x[i] and x[i + 156] of the recurrence are its own registers, and
+  // x[i + 1], two phases old, is read from the words every thread puts into
+  // `nbr` as it makes them.  The last thread's x[i + 1] is thread 0's word of
+  // the phase just made: there in every first phase of a pair, made again from
+  // threads 0 and 1's words in the second, so one barrier serves two phases.
+  __shared__ uint64_t nbr[4][kLanes][160];  // [phase mod 4][lane][thread]
+  const int ti = min(tid, kM - 1);
+  uint64_t x[kLanes], c[kLanes], o[kLanes];  // words of phases g - 2, g - 1 and g - 3
+#pragma unroll
+  for (int l = 0; l < kLanes; ++l) {
+    x[l] = o[l] = nbr[2][l][tid] = w0[l * wl + ti];
+    c[l] = nbr[3][l][tid] = w0[l * wl + kM + ti];
+  }
   const int64_t obase = off + Q0;
   const int64_t oend = off + n;
-  int cur = 0;
-  int64_t base = pbeg;
-  for (; base < pend; base += kN) {
-    uint64_t(*old)[kN] = raw[cur];
-    uint64_t(*nw)[kN] = raw[cur ^ 1];
-#pragma unroll 1
+  int slot = 0;  // the phase to make, mod 4
+  for (int64_t base = pbeg; base < pend; base += kN, slot ^= 2) {
+    __syncthreads();
+    const int here = (int)min(pend - base, (int64_t)kN);
+    // the cheap transforms pay for the registers' change of roles: unrolled
+#pragma unroll(kLightKind<MODE, KIND> ? 2 : 1)
     for (int ph = 0; ph < 2; ++ph) {
-      const int i = ph * kM + tid;
-      uint64_t pk[kLanes];
-      const bool act = tid < kM;
-      if (act) {
+      if (ph * kM >= here) break;
+      const int g = slot + ph;
+      uint64_t nb[kLanes], pk[kLanes];
 #pragma unroll
-        for (int l = 0; l < kLanes; ++l) {
-          uint64_t b = (i + 1 < kN) ? old[l][i + 1] : nw[l][0];
-          uint64_t c = (ph == 0) ? old[l][i + kM] : nw[l][i - kM];
-          uint64_t v = twist1(old[l][i], b, c);
-          nw[l][i] = v;
-          pk[l] = temper(v);
-        }
-      } else {
+      for (int l = 0; l < kLanes; ++l) nb[l] = nbr[g ^ 2][l][min(tid + 1, 159)];
+      if (tid == kM - 1) {
 #pragma unroll
-        for (int l = 0; l < kLanes; ++l) pk[l] = 0;
+        for (int l = 0; l < kLanes; ++l)
+          nb[l] = ph == 0 ? nbr[(g + 3) & 3][l][0]
+                          : twist1(nbr[(g + 1) & 3][l][0], nbr[(g + 1) & 3][l][1], nbr[g ^ 2][l][0]);
       }
-      const int64_t pidx = base + i;
-      const bool valid = act && pidx < pend;
-      emit_packet<MODE, KIND>(pk, pidx, valid, p, d, obase, oend, st, gs);
-      __syncthreads();
+#pragma unroll
+      for (int l = 0; l < kLanes; ++l) {
+        const uint64_t v = twist1(x[l], nb[l], c[l]);
+        nbr[g][l][tid] = v;
+        pk[l] = temper(v);
+        o[l] = x[l];
+        x[l] = c[l];
+        c[l] = v;
+      }
+      const int i = ph * kM + tid;
+      emit_packet<MODE, KIND>(pk, base + i, tid < kM && i < here, p, d, obase, oend, st, gs);
     }
-    cur ^= 1;
   }
 
   // --- end-of-call state: new lane windows and cache flags
   if (last) {
     if (Np > 0) {
-      const int64_t nb = (pend - pbeg + kN - 1) / kN;
-      const int rr = (int)(pend - (pbeg + (nb - 1) * kN));  // packets used of the last block, 1..312
-      uint64_t(*lastb)[kN] = raw[cur];
-      uint64_t(*prevb)[kN] = raw[cur ^ 1];
-      for (int t = tid; t < kLanes * kN; t += blockDim.x) {
-        const int l = t / kN, i = t % kN;
-        st->win[l][i] = (i < kN - rr) ? prevb[l][rr + i] : lastb[l][i - (kN - rr)];
+      // the 312 words before packet pend: the end of phase g - 3, phase g - 2
+      // and the first rr of phase g - 1
+      const int rr = (int)((pend - pbeg - 1) % kM) + 1;
+      if (tid < kM) {
+#pragma unroll
+        for (int l = 0; l < kLanes; ++l) {
+          if (tid >= rr) st->win[l][tid - rr] = o[l];
+          st->win[l][kM - rr + tid] = x[l];
+          if (tid < rr) st->win[l][kN - rr + tid] = c[l];
+        }
       }
     }
     if (tid == 0) {
@@ -849,7 +881,7 @@ __global__ void __maxnreg__(64) k_direct(Plan p, DistParams d, const CallSnap* s
       if (MODE == M_N32) left = (r % 16) ? 8 : 0;
       if (MODE == M_N64) left = (r % 8) ? 4 : 0;
       if (kUsesHalf) st->half_valid = left ? 1 : (Q0 ? 0 : st->half_valid);
-      if (kUsesGen) gs->s[0].valid = left ? 1 : 0;
+      if (kUsesGen && gs) gs->s[0].valid = left ? 1 : 0;
       st->consumed += (uint64_t)Np;
     }
   }
@@ -910,7 +942,7 @@ __global__ void __launch_bounds__(kXfThreads) k_xform(Plan p, DistParams d, cons
       if (MODE == M_N32) left = (r % 16) ? 8 : 0;
       if (MODE == M_N64) left = (r % 8) ? 4 : 0;
       if (kUsesHalf) st->half_valid = left ? 1 : (Q0 ? 0 : cvalid);
-      if (kUsesGen) gs->s[0].valid = left ? 1 : 0;
+      if (kUsesGen && gs) gs->s[0].valid = left ? 1 : 0;
     }
     st->consumed += (uint64_t)used;
   }
