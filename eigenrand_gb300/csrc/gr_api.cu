@@ -874,9 +874,15 @@ double poisson_step_halves(float fe) {
 // G(a) e^(a-1) / (pi sqrt(2a - 1) (a - 1)^(a-1)).
 double gamma_yield(int branch, double a) {
   const double e1 = 2.718281828459045;
-  if ((branch >> 8) == 2) return e1 * std::tgamma(a + 1) / (e1 + a);
-  const double b = a - 1;
-  return std::exp(std::lgamma(a) + b - b * std::log(b)) / (3.141592653589793 * std::sqrt(2 * a - 1));
+  double q;
+  if ((branch >> 8) == 2) {
+    q = e1 * std::tgamma(a + 1) / (e1 + a);
+  } else {
+    const double b = a - 1;
+    // the tan proposal's tends to 1 / sqrt(pi)
+    q = a > 1e6 ? 0.5642 : std::exp(std::lgamma(a) + b - b * std::log(b)) / (3.141592653589793 * std::sqrt(2 * a - 1));
+  }
+  return q >= 0.1 ? std::min(q, 1.0) : 0.1;  // shapes outside the sampler's domain: any plan will do
 }
 
 // Fixed units over words in memory.
@@ -942,7 +948,8 @@ double expected_yield(int rk, const DistParams& d, double& slack) {
   if (rk <= 1) return gamma_yield(rk == 0 ? 2 << 8 : 3 << 8, f64 ? d.da : (double)d.fa);
   if (rk == 2) {  // Johnk: G(a + 1) G(b + 1) / G(a + b + 1)
     const double a = f64 ? d.da : (double)d.fa, b = f64 ? d.db : (double)d.fb;
-    return std::tgamma(a + 1) * std::tgamma(b + 1) / std::tgamma(a + b + 1);
+    const double q = std::tgamma(a + 1) * std::tgamma(b + 1) / std::tgamma(a + b + 1);
+    return q >= 0.1 ? std::min(q, 1.0) : 0.1;
   }
   slack = 0.04;
   return reject_yield(rk, d);
@@ -1742,6 +1749,10 @@ gr_status gr_sample_batched(gr_engine* e, const gr_batch_desc* bd, gr_stream_t s
   va.offsets = bd->offsets;
   va.out = bd->out;
   va.status = &e->st[0].status;
+  if (bd->kind == GR_GAMMA) {  // one form only (gr_trials.cu)
+    GR_CUDA(launch_gamma_sets(va, s));
+    return GR_OK;
+  }
   int b = 0;
   while (((int64_t)1 << b) < bd->nsets) ++b;
   int threads = tuned_threads(bd->kind, bd->nsets);
@@ -1755,9 +1766,9 @@ gr_status gr_sample_batched(gr_engine* e, const gr_batch_desc* bd, gr_stream_t s
     GR_CUDA(cudaEventCreate(&e0));
     GR_CUDA(cudaEventCreate(&e1));
     for (int c : cand) {
-      GR_CUDA(launch_vop(bd->kind, c, va, s));  // warm
+      GR_CUDA(launch_vop(c, va, s));  // warm
       GR_CUDA(cudaEventRecord(e0, s));
-      GR_CUDA(launch_vop(bd->kind, c, va, s));
+      GR_CUDA(launch_vop(c, va, s));
       GR_CUDA(cudaEventRecord(e1, s));
       GR_CUDA(cudaEventSynchronize(e1));
       float ms = 0;
@@ -1776,7 +1787,7 @@ gr_status gr_sample_batched(gr_engine* e, const gr_batch_desc* bd, gr_stream_t s
     // call's own semantics simple (identical values)
   }
   if (threads == 0) threads = 160;
-  GR_CUDA(launch_vop(bd->kind, threads, va, s));
+  GR_CUDA(launch_vop(threads, va, s));
   return GR_OK;
 }
 

@@ -269,7 +269,8 @@ struct VopArgs {
   void* out;
   int32_t* status;
 };
-cudaError_t launch_vop(int kind, int threads, const VopArgs& va, cudaStream_t s);
+cudaError_t launch_vop(int threads, const VopArgs& va, cudaStream_t s);  // BinomialVGen sets
+cudaError_t launch_gamma_sets(const VopArgs& va, cudaStream_t s);         // GammaGen<float> sets (gr_trials.cu)
 
 // Outputs per granule: the smallest output count a call (or a stream slice)
 // may have for the kind.  Packets per unit: 2 for the Box-Muller kinds.

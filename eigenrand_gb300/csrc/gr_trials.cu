@@ -36,25 +36,80 @@ namespace {
 
 constexpr int kTrThreads = 320;     // ten warps; 312 of the threads make a block's words
 constexpr int kTrRing = 16 * kN;    // ring words: two blocks of 312 packets of 8
-constexpr int kTrBatch = kN + 1;    // most trials of a batch (one packet each, one straddling)
-constexpr int kTrCand = 8 * (kN + 1) + 8;
 
+// RAW blocks kept untempered: two, each made from the other, or one, made over
+// itself behind one more barrier, where the CTA needs the room.  BATCH: most
+// trials of a batch (a block holds 104 trials of three packets, 156 of two, and
+// at most 313 of one).
+template <int RAW, int BATCH>
 struct TrialSmem {
-  uint64_t raw[2][kLanes][kN];
+  static constexpr int kRaw = RAW, kBatch = BATCH;
+  uint64_t raw[RAW][kLanes][kN];
   alignas(16) uint32_t w[kTrRing];
-  alignas(16) uint32_t cand[kTrCand];  // accepted candidates (double: kTrCand / 2 of them)
-  uint32_t scan[kTrBatch + 7];         // exclusive: (fulls << 16) | lanes appended
-  uint32_t emit[kTrBatch + 7];         // output packet (from the batch's first) of each FIFO packet
-  uint64_t fifo[2][16];                // carried lanes (ping-pong)
+  alignas(16) uint32_t cand[BATCH * 8];  // accepted candidates (double: four per trial)
+  uint32_t scan[BATCH];                  // exclusive: (fulls << 16) | lanes appended
+  uint32_t emit[BATCH + 1];              // output packet (from the batch's first) of each FIFO packet
+  uint64_t fifo[2][16];                  // carried lanes (ping-pong)
   uint32_t warp_tot[kTrThreads / 32];
   int tstar;
-  uint8_t mask[kTrBatch + 7];
+  uint8_t mask[BATCH];
   TrialRow row;
 };
+using EngSmem = TrialSmem<2, kTrThreads>;  // an engine's call
+using SetSmem = TrialSmem<1, 160>;         // a parameter set: beside it lies the next set's window
+
+// Where a stream stands in the ring.
+struct TrialPos {
+  int sp;      // ring index of the next trial's first word
+  int av;      // words made and not used
+  int64_t nb;  // blocks made
+};
+
+// The ten warps that draw; a set's CTA has an eleventh.
+template <class SM>
+__device__ __forceinline__ void tr_sync() {
+  if (SM::kRaw == 2) __syncthreads();
+  else asm volatile("bar.sync 1, %0;" ::"n"(kTrThreads) : "memory");
+}
+
+// The next engine block: two lanes per thread (words 2 h and 2 h + 1 of a packet
+// are neighbours in the ring), word i + 156 from word i made by the same thread,
+// word 311 with the block's word 0 made again.
+template <class SM>
+__device__ __forceinline__ void next_block(SM& sm, TrialPos& ps) {
+  const int from = SM::kRaw == 2 ? (int)(ps.nb & 1) : 0, to = SM::kRaw == 2 ? from ^ 1 : 0;
+  const int tid = threadIdx.x;
+  uint32_t* ring = sm.w + (ps.nb & 1) * (kTrRing / 2);
+  const int h = tid >= kM ? 1 : 0, i = tid - h * kM;
+  uint64_t lo[2], hi[2];
+  if (tid < 2 * kM) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const uint64_t* old = sm.raw[from][2 * h + q];
+      const uint64_t c = old[i + kM];
+      lo[q] = mt_twist(old[i], old[i + 1], c);
+      const uint64_t b = i == kM - 1 ? mt_twist(old[0], old[1], old[kM]) : old[i + kM + 1];
+      hi[q] = mt_twist(c, b, lo[q]);
+    }
+  }
+  if (SM::kRaw == 1) tr_sync<SM>();
+  if (tid < 2 * kM) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      sm.raw[to][2 * h + q][i] = lo[q];
+      sm.raw[to][2 * h + q][i + kM] = hi[q];
+    }
+    *reinterpret_cast<ulonglong2*>(ring + 8 * i + 4 * h) = make_ulonglong2(mt_temper(lo[0]), mt_temper(lo[1]));
+    *reinterpret_cast<ulonglong2*>(ring + 8 * (i + kM) + 4 * h) = make_ulonglong2(mt_temper(hi[0]), mt_temper(hi[1]));
+  }
+  ++ps.nb;
+  ps.av += 8 * kN;
+  tr_sync<SM>();
+}
 
 // A row's candidate at the ring index a of its trial, lane j.
-template <int DT, int RK>
-__device__ __forceinline__ bool trial_eval(const TrialSmem& sm, const DistParams& d, const int rk, const int U, const int a,
+template <int DT, int RK, class SM>
+__device__ __forceinline__ bool trial_eval(const SM& sm, const DistParams& d, const int rk, const int U, const int a,
                                            const int j, uint64_t& c) {
   auto word = [&](int q) -> uint32_t {
     int i = a + q;
@@ -68,8 +123,6 @@ __device__ __forceinline__ bool trial_eval(const TrialSmem& sm, const DistParams
   };
   auto rej = [&](auto k) { return rej_trial<decltype(k)::value, DT>(d, 0, j, word, rval, c); };
   if (RK >= 0) return rej(std::integral_constant<int, RK < 0 ? 0 : RK>{});
-  if (rk == RK_GAMMA_GS) return rej(std::integral_constant<int, RK_GAMMA_GS>{});
-  if (rk == RK_GAMMA_TAN) return rej(std::integral_constant<int, RK_GAMMA_TAN>{});
   // NormalExp.h:527-534 (alpha = 1), :577-587 (integral alpha)
   if (DT == SD_F32) {
     if (rk == kRowExp) {
@@ -95,18 +148,145 @@ __device__ __forceinline__ bool trial_eval(const TrialSmem& sm, const DistParams
   return true;
 }
 
+// Npk output packets of one row to out (CUT: its first `count` values only),
+// from the stream at ps; rcnt lanes carried in sm.fifo[fsl].  False: the block
+// cap came first.
+template <int DT, int RK, bool CUT, class SM, class V>
+__device__ __forceinline__ bool draw_row(SM& sm, const DistParams& d, const int rk, const int U, const float per_packet,
+                                         V* out, const int64_t Npk, int64_t count, TrialPos& ps, int& rcnt, int& fsl,
+                                         const int64_t max_blocks) {
+  constexpr int P = DT == SD_F32 ? 8 : 4;
+  constexpr uint32_t kFull = (1u << P) - 1u;
+  constexpr int kBatch = SM::kBatch;
+  V* cand = reinterpret_cast<V*>(sm.cand);
+  const int tid = threadIdx.x;
+  const int Wt = 8 * U;
+  int64_t left = Npk;
+  while (left > 0) {
+    if (ps.av < Wt) {
+      if (ps.nb >= max_blocks) return false;
+      next_block(sm, ps);
+    }
+    // a batch: the trials whose words exist, and near the end of the row no
+    // more than it should still need
+    const int need = (int)min(left, (int64_t)1 << 20);
+    const float want = (float)need * per_packet;
+    const int B = min(ps.av / Wt, min(kBatch, (int)(CUT ? fminf(want, 1e6f) : want) + 4));
+    // ---- candidates and accept masks
+    for (int e0 = 0; e0 < B * P; e0 += kTrThreads) {
+      const int e = e0 + tid, t = e / P, j = e % P;
+      bool acc = false;
+      uint64_t c = 0;
+      if (e < B * P) {
+        int a = ps.sp + t * Wt;
+        a -= a >= kTrRing ? kTrRing : 0;
+        acc = trial_eval<DT, RK>(sm, d, rk, U, a, j, c);
+      }
+      const uint32_t bal = __ballot_sync(0xffffffffu, acc);
+      if (acc) cand[e] = (V)c;
+      if (j == 0 && e < B * P) sm.mask[t] = (uint8_t)((bal >> (tid & 31)) & kFull);
+    }
+    tr_sync<SM>();
+    // ---- prefix sums over trials: (fulls << 16) |
+    // appended lanes
+    const uint32_t m0 = tid < B ? sm.mask[tid] : 0;
+    const uint32_t v0 = m0 == kFull ? 1u << 16 : (uint32_t)__popc(m0);
+    uint32_t v = v0;
+    if (tid < kBatch) {
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, v, o);
+        if ((tid & 31) >= o) v += x;
+      }
+      if ((tid & 31) == 31) sm.warp_tot[tid >> 5] = v;
+    }
+    if (tid == kTrThreads - 1) sm.tstar = B;
+    tr_sync<SM>();
+    // ---- this thread's trial: its emission, if any
+    if (tid < B) {
+#pragma unroll
+      for (int w = 0; w < kBatch / 32 - 1; ++w) v += w < (tid >> 5) ? sm.warp_tot[w] : 0u;
+      const uint32_t ex = v - v0;
+      const int at = rcnt + (int)(ex & 0xffffu), nf = (int)(ex >> 16);
+      const bool full = m0 == kFull;
+      const bool cross = !full && (at + (int)__popc(m0)) / P > at / P;
+      const int ei = nf + at / P;
+      sm.scan[tid] = ex;
+      if (cross) sm.emit[at / P] = (uint32_t)ei;
+      if ((full || cross) && ei == need - 1) sm.tstar = tid + 1;
+    }
+    tr_sync<SM>();
+    // trials consumed, and the FIFO level and emissions after them
+    const int Bu = sm.tstar;
+    const uint32_t ml = sm.mask[Bu - 1], sl = sm.scan[Bu - 1];
+    const int a_end = rcnt + (int)(sl & 0xffffu) + (ml == kFull ? 0 : __popc(ml));
+    const int nf_end = (int)(sl >> 16) + (ml == kFull ? 1 : 0);
+    const int qe = a_end / P;  // FIFO packets emitted
+    auto put = [&](int at, uint64_t x) {
+      if (RK == RK_BETA_SMALL) x = beta_post<DT == SD_F64>(x, d);
+      if (DT == SD_I32H) {
+        // BinomialGen returns trials - res when p > 1/2 (Discrete.h:1051)
+        const int32_t q = (int32_t)u2f((uint32_t)x);
+        x = (uint32_t)((RK == RK_BINOMIAL && d.ib) ? (int32_t)d.fh - q : q);
+      }
+      if (!CUT || at < count) out[at] = (V)x;
+    };
+    // ---- write outputs
+    for (int e = tid; e < Bu * P; e += kTrThreads) {
+      const int t = e / P, j = e % P;
+      const uint32_t m = sm.mask[t];
+      if (!((m >> j) & 1u)) continue;
+      const uint32_t s = sm.scan[t];
+      const int at = rcnt + (int)(s & 0xffffu);
+      if (m == kFull) {
+        put(((int)(s >> 16) + at / P) * P + j, cand[e]);
+      } else {
+        const int f = at + __popc(m & ((1u << j) - 1u)), q = f / P;
+        if (q < qe) put((int)sm.emit[q] * P + f % P, cand[e]);
+        else sm.fifo[fsl ^ 1][f - qe * P] = cand[e];  // the FIFO keeps the plain draws
+      }
+    }
+    // carried lanes: emitted with the batch's first FIFO packet, or still carried
+    if (tid < rcnt) {
+      if (qe > 0) put((int)sm.emit[0] * P + tid, sm.fifo[fsl][tid]);
+      else sm.fifo[fsl ^ 1][tid] = sm.fifo[fsl][tid];
+    }
+    out += (int64_t)(nf_end + qe) * P;
+    if (CUT) count -= (int64_t)(nf_end + qe) * P;
+    left -= nf_end + qe;
+    rcnt = a_end - qe * P;
+    fsl ^= 1;
+    ps.sp += Bu * Wt;
+    ps.sp -= ps.sp >= kTrRing ? kTrRing : 0;
+    ps.av -= Bu * Wt;
+    tr_sync<SM>();
+  }
+  return true;
+}
+
+// The row's kind picks a copy of the loop of its own: with the kind tested per
+// trial in one loop 64 rows of 10^6 gamma(0.5) floats on 608 engines took 1 660
+// us instead of 1 580, and 2 10^5 parameter sets 12.0 ms instead of 11.2.
+template <int DT, bool CUT, class SM, class V>
+__device__ __forceinline__ bool draw_kind(SM& sm, const TrialRow& row, V* out, const int64_t Npk, const int64_t count,
+                                          TrialPos& ps, int& rcnt, int& fsl, const int64_t max_blocks) {
+  if (row.rk == RK_GAMMA_GS)
+    return draw_row<DT, RK_GAMMA_GS, CUT>(sm, row.d, row.rk, 3, row.per_packet, out, Npk, count, ps, rcnt, fsl, max_blocks);
+  if (row.rk == RK_GAMMA_TAN)
+    return draw_row<DT, RK_GAMMA_TAN, CUT>(sm, row.d, row.rk, 2, row.per_packet, out, Npk, count, ps, rcnt, fsl, max_blocks);
+  return draw_row<DT, -1, CUT>(sm, row.d, row.rk, row.packets, row.per_packet, out, Npk, count, ps, rcnt, fsl, max_blocks);
+}
+
 // RK >= 0: one row (args) of that kind; RK < 0: `rows` rows from memory, row i
 // written at out + i * row_stride elements.
 template <int DT, int RK>
 __global__ void __launch_bounds__(kTrThreads, 4) k_trials(Plan p, TrialRow args, const TrialRow* rows, int nrows,
                                                           int64_t row_stride, int64_t max_blocks) {
   constexpr int P = DT == SD_F32 ? 8 : 4;
-  constexpr uint32_t kFull = (1u << P) - 1u;
   constexpr bool kHalf = DT == SD_I32H;
   using V = typename std::conditional<DT == SD_F64, uint64_t, uint32_t>::type;
   extern __shared__ __align__(16) uint8_t tr_dyn[];
-  TrialSmem& sm = *reinterpret_cast<TrialSmem*>(tr_dyn);
-  V* cand = reinterpret_cast<V*>(sm.cand);
+  EngSmem& sm = *reinterpret_cast<EngSmem*>(tr_dyn);
   const int k = blockIdx.x, tid = threadIdx.x;
   EngState* st = p.eng + k;
   int64_t off, n;
@@ -118,13 +298,9 @@ __global__ void __launch_bounds__(kTrThreads, 4) k_trials(Plan p, TrialRow args,
   for (int i = tid; i < kLanes * kN; i += kTrThreads) (&sm.raw[0][0][0])[i] = (&st->win[0][0])[i];
   // the engine's cached half packet goes before the first block's words
   if (kHalf && tid < 4) sm.w[kTrRing - 4 + tid] = st->half_cache[tid];
-  int sp = c0w ? kTrRing - 4 : 0;  // ring index of the next trial's first word
-  int av = c0w;                    // words there
-  int cur = 0;
-  int64_t nb = 0;  // blocks made
-  bool over = false;
-
-  for (int r = 0; r < (RK < 0 ? nrows : 1) && !over; ++r) {
+  TrialPos ps{c0w ? kTrRing - 4 : 0, c0w, 0};
+  bool ok = true;
+  for (int r = 0; r < (RK < 0 ? nrows : 1) && ok; ++r) {
     __syncthreads();  // the window is there; the last row's carried lanes are out
     if (RK < 0) {
       const uint32_t* src = reinterpret_cast<const uint32_t*>(rows + r);
@@ -132,141 +308,20 @@ __global__ void __launch_bounds__(kTrThreads, 4) k_trials(Plan p, TrialRow args,
       __syncthreads();
     }
     const TrialRow& row = RK < 0 ? sm.row : args;
-    const DistParams& d = row.d;
-    const int U = row.packets, Wt = 8 * U, rk = row.rk;
+    const int rk = row.rk;
     GenSlot* gs = &row.gen[k].s[0];
     V* out = reinterpret_cast<V*>(p.out) + (RK < 0 ? (int64_t)r * row_stride : 0) + off;
-    int rcnt = (RK >= 0 || rk <= RK_GAMMA_TAN) ? gs->rest_cnt : 0;
+    const bool carries = RK >= 0 || rk <= RK_GAMMA_TAN;
+    int rcnt = carries ? gs->rest_cnt : 0, fsl = 0;
     if (tid < 16)
       sm.fifo[0][tid] = DT == SD_F64
                             ? ((uint64_t)gs->rest[2 * (tid & 7)] | ((uint64_t)gs->rest[2 * (tid & 7) + 1] << 32))
                             : (uint64_t)gs->rest[tid];
-    int fsl = 0;
-    int64_t left = Npk;
-    while (left > 0) {
-      if (av < Wt) {
-        if (nb >= max_blocks) {
-          over = true;
-          break;
-        }
-        // the next engine block: two lanes per thread (words 2 h and 2 h + 1 of
-        // a packet are neighbours in the ring), word i + 156 from word i made
-        // by the same thread, word 311 with the block's word 0 made again
-        uint64_t(*old)[kN] = sm.raw[cur];
-        uint64_t(*nw)[kN] = sm.raw[cur ^ 1];
-        uint32_t* ring = sm.w + (nb & 1) * (kTrRing / 2);
-        if (tid < 2 * kM) {
-          const int h = tid >= kM ? 1 : 0, i = tid - h * kM;
-          uint64_t lo[2], hi[2];
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const int l = 2 * h + q;
-            const uint64_t c = old[l][i + kM];
-            lo[q] = mt_twist(old[l][i], old[l][i + 1], c);
-            const uint64_t b = i == kM - 1 ? mt_twist(old[l][0], old[l][1], old[l][kM]) : old[l][i + kM + 1];
-            hi[q] = mt_twist(c, b, lo[q]);
-            nw[l][i] = lo[q];
-            nw[l][i + kM] = hi[q];
-          }
-          *reinterpret_cast<ulonglong2*>(ring + 8 * i + 4 * h) = make_ulonglong2(mt_temper(lo[0]), mt_temper(lo[1]));
-          *reinterpret_cast<ulonglong2*>(ring + 8 * (i + kM) + 4 * h) =
-              make_ulonglong2(mt_temper(hi[0]), mt_temper(hi[1]));
-        }
-        cur ^= 1;
-        ++nb;
-        av += 8 * kN;
-        __syncthreads();
-      }
-      // a batch: the trials whose words exist, and near the end of the row no
-      // more than it should still need
-      const int need = (int)min(left, (int64_t)1 << 20);
-      const int B = min(av / Wt, min(kTrBatch, (int)((float)need * row.per_packet) + 4));
-      // ---- candidates and accept masks
-      for (int e0 = 0; e0 < B * P; e0 += kTrThreads) {
-        const int e = e0 + tid, t = e / P, j = e % P;
-        bool acc = false;
-        uint64_t c = 0;
-        if (e < B * P) {
-          int a = sp + t * Wt;
-          a -= a >= kTrRing ? kTrRing : 0;
-          acc = trial_eval<DT, RK>(sm, d, rk, U, a, j, c);
-        }
-        const uint32_t bal = __ballot_sync(0xffffffffu, acc);
-        if (acc) cand[e] = (V)c;
-        if (j == 0 && e < B * P) sm.mask[t] = (uint8_t)((bal >> (tid & 31)) & kFull);
-      }
-      __syncthreads();
-      // ---- prefix sums over trials: (fulls << 16) | appended lanes
-      const uint32_t m0 = tid < B ? sm.mask[tid] : 0;
-      const uint32_t v0 = m0 == kFull ? 1u << 16 : (uint32_t)__popc(m0);
-      uint32_t v = v0;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t x = __shfl_up_sync(0xffffffffu, v, o);
-        if ((tid & 31) >= o) v += x;
-      }
-      if ((tid & 31) == 31) sm.warp_tot[tid >> 5] = v;
-      if (tid == 0) sm.tstar = B;
-      __syncthreads();
-#pragma unroll
-      for (int w = 0; w < kTrThreads / 32; ++w) v += w < (tid >> 5) ? sm.warp_tot[w] : 0u;
-      // ---- this thread's trial: its emission, if any
-      const uint32_t ex = v - v0;
-      if (tid < B) {
-        const int at = rcnt + (int)(ex & 0xffffu), nf = (int)(ex >> 16);
-        const bool full = m0 == kFull;
-        const bool cross = !full && (at + (int)__popc(m0)) / P > at / P;
-        const int ei = nf + at / P;
-        sm.scan[tid] = ex;
-        if (cross) sm.emit[at / P] = (uint32_t)ei;
-        if ((full || cross) && ei == need - 1) sm.tstar = tid + 1;
-      }
-      __syncthreads();
-      // trials consumed, and the FIFO level and emissions after them
-      const int Bu = sm.tstar;
-      const uint32_t ml = sm.mask[Bu - 1], sl = sm.scan[Bu - 1];
-      const int a_end = rcnt + (int)(sl & 0xffffu) + (ml == kFull ? 0 : __popc(ml));
-      const int nf_end = (int)(sl >> 16) + (ml == kFull ? 1 : 0);
-      const int qe = a_end / P;  // FIFO packets emitted
-      auto put = [&](int at, uint64_t x) {
-        if (RK == RK_BETA_SMALL) x = beta_post<DT == SD_F64>(x, d);
-        if (DT == SD_I32H) {
-          // BinomialGen returns trials - res when p > 1/2 (Discrete.h:1051)
-          const int32_t q = (int32_t)u2f((uint32_t)x);
-          x = (uint32_t)((RK == RK_BINOMIAL && d.ib) ? (int32_t)d.fh - q : q);
-        }
-        out[at] = (V)x;
-      };
-      // ---- write outputs
-      for (int e = tid; e < Bu * P; e += kTrThreads) {
-        const int t = e / P, j = e % P;
-        const uint32_t m = sm.mask[t];
-        if (!((m >> j) & 1u)) continue;
-        const uint32_t s = sm.scan[t];
-        const int at = rcnt + (int)(s & 0xffffu);
-        if (m == kFull) {
-          put(((int)(s >> 16) + at / P) * P + j, cand[e]);
-        } else {
-          const int f = at + __popc(m & ((1u << j) - 1u)), q = f / P;
-          if (q < qe) put((int)sm.emit[q] * P + f % P, cand[e]);
-          else sm.fifo[fsl ^ 1][f - qe * P] = cand[e];  // the FIFO keeps the plain draws
-        }
-      }
-      // carried lanes: emitted with the batch's first FIFO packet, or still carried
-      if (tid < rcnt) {
-        if (qe > 0) put((int)sm.emit[0] * P + tid, sm.fifo[fsl][tid]);
-        else sm.fifo[fsl ^ 1][tid] = sm.fifo[fsl][tid];
-      }
-      out += (int64_t)(nf_end + qe) * P;
-      left -= nf_end + qe;
-      rcnt = a_end - qe * P;
-      fsl ^= 1;
-      sp += Bu * Wt;
-      sp -= sp >= kTrRing ? kTrRing : 0;
-      av -= Bu * Wt;
-      __syncthreads();
-    }
-    if (RK >= 0 || rk <= RK_GAMMA_TAN) {
+    if (RK >= 0)
+      ok = draw_row<DT, RK, false>(sm, row.d, rk, row.packets, row.per_packet, out, Npk, 0, ps, rcnt, fsl, max_blocks);
+    else
+      ok = draw_kind<DT, false>(sm, row, out, Npk, 0, ps, rcnt, fsl, max_blocks);
+    if (carries) {
       if (tid == 0) gs->rest_cnt = rcnt;
       if (DT == SD_F64) {
         if (tid < 8) {
@@ -281,22 +336,97 @@ __global__ void __launch_bounds__(kTrThreads, 4) k_trials(Plan p, TrialRow args,
 
   // ---- engine state: the call ends inside the newest block (a trial is
   // evaluated in the batch after the block that holds its last word)
-  if (tid == 0 && over) atomicOr(&st->status, (int)GR_DEV_REJECT_LIMIT);
-  if (nb > 0) {
-    const int rr = kN - av / 8;  // packets used of it; a half packet counts as used
+  if (tid == 0 && !ok) atomicOr(&st->status, (int)GR_DEV_REJECT_LIMIT);
+  if (ps.nb > 0) {
+    const int cur = (int)(ps.nb & 1);
+    const int rr = kN - ps.av / 8;  // packets used of it; a half packet counts as used
     for (int t = tid; t < kLanes * kN; t += kTrThreads) {
       const int l = t / kN, i = t % kN;
       st->win[l][i] = i < kN - rr ? sm.raw[cur ^ 1][l][rr + i] : sm.raw[cur][l][i - (kN - rr)];
     }
   }
   if (tid == 0) {
-    if (kHalf && nb > 0) {
-      const bool half = (av & 7) == 4;  // ends mid-packet: the upper half stays cached
+    if (kHalf && ps.nb > 0) {
+      const bool half = (ps.av & 7) == 4;  // ends mid-packet: the upper half stays cached
       if (half)
-        for (int q = 0; q < 4; ++q) st->half_cache[q] = sm.w[sp + q];
+        for (int q = 0; q < 4; ++q) st->half_cache[q] = sm.w[ps.sp + q];
       st->half_valid = half ? 1 : 0;
     }
-    st->consumed += (uint64_t)(nb * kN - av / 8);
+    st->consumed += (uint64_t)(ps.nb * kN - ps.av / 8);
+  }
+}
+
+// ---------------------------------------------------------------- parameter sets
+// Batched GammaGen<float> sets: set i from its own Vmt19937_64(seed + 4 i)
+// with a fresh generator, ceil(count / 8) packets of which the first `count`
+// values are kept.  Bound by instruction issue, like the rest of this file.  A
+// CTA takes sets in turn; four threads of an eleventh warp seed the next set's
+// engine (PacketRandomEngine.h:256-265: 311 dependent steps of a 64-bit
+// multiply, 5 us) while the ten others draw from the current one.  2 10^5 sets
+// of up to 4 096 values: 13.4 ms with a CTA per set that seeds first, 11.2 ms
+// here (11.3 with three CTAs per SM and no spilled registers).
+struct VopSmem {
+  SetSmem t;
+  uint64_t seeds[kLanes][kN];
+};
+
+__global__ void __launch_bounds__(kTrThreads + 32, 4) k_gamma_sets(VopArgs va) {
+  extern __shared__ __align__(16) uint8_t tr_dyn[];
+  VopSmem& vs = *reinterpret_cast<VopSmem*>(tr_dyn);
+  SetSmem& sm = vs.t;
+  const int tid = threadIdx.x;
+  for (int64_t set = blockIdx.x; set < va.nsets; set += gridDim.x) {
+    if (set == blockIdx.x) {
+      if (tid >= kTrThreads && tid < kTrThreads + kLanes) {
+        const int l = tid - kTrThreads;
+        uint64_t v = va.seed + 4ull * (uint64_t)set + (uint64_t)l;
+        vs.seeds[l][0] = v;
+        for (int i = 1; i < kN; ++i) vs.seeds[l][i] = v = (v ^ (v >> 62)) * kSeedF + (uint64_t)i;
+      }
+      __syncthreads();
+    }
+    const int64_t count = va.counts[set];
+    if (tid < kTrThreads) {
+      for (int i = tid; i < kLanes * kN; i += kTrThreads) (&sm.raw[0][0][0])[i] = (&vs.seeds[0][0])[i];
+      if (tid == 0) {
+        // GammaGen's branch and constants, NormalExp.h:446-460, 533-604
+        const float alpha = va.a[set];
+        const int cnt = (int)alpha;
+        TrialRow& r = sm.row;
+        r.rk = alpha < 1 ? (int)RK_GAMMA_GS : alpha == 1 ? kRowExp : ((float)cnt == alpha && cnt < 20) ? kRowInt : (int)RK_GAMMA_TAN;
+        r.packets = r.rk == RK_GAMMA_GS ? 3 : r.rk == kRowExp ? 1 : r.rk == kRowInt ? cnt : 2;
+        // trials per output packet: e + a over e G(a + 1) is at most 1.39; the
+        // tan proposal's falls from pi at 1 to 1.77
+        r.per_packet = r.rk == RK_GAMMA_GS ? 1.4f : r.rk == RK_GAMMA_TAN ? 1.77f + 0.35f / (alpha - 0.75f) : 1.0f;
+        r.d.fa = alpha;
+        r.d.fb = va.b[set];
+        r.d.fc = 1 / alpha;
+        r.d.fd = alpha - 1;
+        r.d.fe = (float)(2.7182818284590452 / (alpha + 2.7182818284590452));
+        r.d.ff = sqrtf(2 * alpha - 1);
+        r.d.fh = 0x1p-18f * (1.0f + 40.0f / alpha);
+      }
+    }
+    __syncthreads();
+    if (tid >= kTrThreads) {
+      const int64_t next = set + gridDim.x;
+      if (tid < kTrThreads + kLanes && next < va.nsets) {
+        const int l = tid - kTrThreads;
+        uint64_t v = va.seed + 4ull * (uint64_t)next + (uint64_t)l;
+        vs.seeds[l][0] = v;
+        for (int i = 1; i < kN; ++i) vs.seeds[l][i] = v = (v ^ (v >> 62)) * kSeedF + (uint64_t)i;
+      }
+    } else if (count > 0) {
+      const TrialRow& r = sm.row;
+      TrialPos ps{0, 0, 0};
+      int rcnt = 0, fsl = 0;
+      const int64_t Npk = (count + 7) / 8;
+      const int64_t max_blocks = ((16 * Npk + 4096) * 8 * r.packets) / (kN * 8) + 64;
+      const bool ok = draw_kind<SD_F32, true>(sm, r, reinterpret_cast<uint32_t*>(va.out) + va.offsets[set], Npk, count, ps,
+                                              rcnt, fsl, max_blocks);
+      if (!ok && tid == 0) atomicOr(va.status, (int)GR_DEV_REJECT_LIMIT);
+    }
+    __syncthreads();
   }
 }
 
@@ -307,7 +437,7 @@ cudaError_t run_trials(const Plan& p, const TrialRow& row, const TrialRow* rows,
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  constexpr size_t smem = sizeof(TrialSmem);
+  constexpr size_t smem = sizeof(EngSmem);
   if (!attr[dev]) {
     cudaError_t e = cudaFuncSetAttribute(k_trials<DT, RK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -346,6 +476,23 @@ cudaError_t launch_gamma_rows(const Plan& p, int dtype, const TrialRow* rows, in
                               int64_t max_blocks, cudaStream_t s) {
   if (dtype == GR_F64) return run_trials<SD_F64, -1>(p, TrialRow{}, rows, nrows, row_stride, max_blocks, s);
   return run_trials<SD_F32, -1>(p, TrialRow{}, rows, nrows, row_stride, max_blocks, s);
+}
+
+cudaError_t launch_gamma_sets(const VopArgs& va, cudaStream_t s) {
+  static int grid[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  constexpr size_t smem = sizeof(VopSmem);
+  if (!grid[dev]) {
+    int sms = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gamma_sets, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    grid[dev] = 4 * sms;
+  }
+  k_gamma_sets<<<(unsigned)std::min<int64_t>(va.nsets, grid[dev]), kTrThreads + 32, smem, s>>>(va);
+  return cudaGetLastError();
 }
 
 }  // namespace gr
