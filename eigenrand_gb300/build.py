@@ -25,7 +25,7 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "--fmad=false", "-std=c++17", "-Xcompiler", "-
 SOURCES = ["gr_kernels.cu", "gr_samplers.cu", "gr_vop.cu", "gr_mv.cu", "gr_api.cu", "gr_mvapi.cu", "gr_serve.cu",
            "gr_noalloc.cu", "gr_trunc.cu", "gr_umma.cu", "gr_mncond.cu", "gr_tmvn.cu", "gr_binomv.cu", "gr_chain.cu", "gr_rejw.cu", "gr_trials.cu",
            "gr_poly.cpp"]
-HEADERS = ["gr_dmath.h", "gr_exact.h", "gr_internal.h", "gr_kernels.cuh", "gr_samplers.cuh", "gr_math.cuh", "gr_math_tables.h", "gr_mt.cuh", "gr_mv.cuh", "gr_admit.h", "gr_poly.h"]
+HEADERS = ["gr_dmath.h", "gr_exact.h", "gr_fp64i.h", "gr_internal.h", "gr_kernels.cuh", "gr_samplers.cuh", "gr_math.cuh", "gr_math_tables.h", "gr_mt.cuh", "gr_mv.cuh", "gr_admit.h", "gr_poly.h"]
 
 
 def _nvcc():

@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kMaskThreads) k_chain_masks(ChainArgs a) {
         const uint64_t v = q == 0 ? w0 : (q == 1 ? w1 : w2);
         return ur_f((j & 1) ? (uint32_t)(v >> 32) : (uint32_t)v);
       };
-      auto ud = [&](int q) { return ur_d(q == 0 ? w0 : (q == 1 ? w1 : w2)); };
+      auto ud = [&](int q) { return q == 0 ? w0 : (q == 1 ? w1 : w2); };
       if (c == 0) beta_comp_u<DT, true>(g, ty0, uf, ud, acc);
       else beta_comp_u<DT, true>(g, ty1, uf, ud, acc);
       m |= (acc ? 1u : 0u) << j;
@@ -647,7 +647,7 @@ __device__ __forceinline__ uint64_t chain_value(const ChainArgs& a, const uint64
     return (j & 1) ? (uint32_t)(v >> 32) : (uint32_t)v;
   };
   auto uf = [&](int q) { return ur_f(word(q)); };
-  auto ud = [&](int q) { return ur_d(tw(w, a.p.wstride, x + q, j)); };
+  auto ud = [&](int q) { return tw(w, a.p.wstride, x + q, j); };
   if (DT == SD_F64 && ty == 2)
     return d2u(1.0 * gs_value_f64(tw(w, a.p.wstride, x, j), tw(w, a.p.wstride, x + 1, j), g.tpx, g.d_inv));
   bool acc;
@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(kEmitThreads) k_chain_emit(ChainArgs a, int pa
       reinterpret_cast<float*>(a.p.out)[at] = a.bk.post == 1 ? (a.bk.fpost * q) / (1.0f - q) : q;
     } else {
       const double p1 = u2d(v[0]), p2 = u2d(v[1]);
-      const double q = p1 / (p1 + p2);
+      const double q = div_d(p1, p1 + p2);
       reinterpret_cast<double*>(a.p.out)[at] = a.bk.post == 1 ? (a.bk.dpost * q) / (1.0 - q) : q;
     }
   }

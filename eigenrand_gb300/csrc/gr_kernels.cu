@@ -304,11 +304,6 @@ static_assert(kJumpSpan % 64 == 0 && kJumpPer % 8 == 0, "coefficient bytes stay 
 static_assert((kJumpThreads / 32) * 32 * kJumpOut <= kJumpLoad, "the reduction reuses the prefix buffer");
 
 // ---------------------------------------------------------------- transforms
-__device__ __forceinline__ float ur_f(uint32_t x) { return u2f((x & 0x7fffffu) | (127u << 23)) - 1.0f; }
-__device__ __forceinline__ double ur_d(uint64_t x) {
-  return u2d((x & 0xfffffffffffffull) | (1023ull << 52)) - 1.0;
-}
-
 // Truncated.h inverse-CDF forms, one lane: u is UniformRealGen(phi(lower),
 // phi(upper))'s value.  TruncNormalGen::packetOp (:322-331), lognormal
 // (:593-598), exponential (:477-484), Cauchy (:534-543), extreme value
@@ -338,8 +333,8 @@ __device__ __forceinline__ double trunc64(double u, const DistParams& d) {
   if (KIND == kTruncExponentialKind) return -log_(1.0 - u) * d.dc;
   if (KIND == kTruncCauchyKind) {
     double s, c;
-    sincos_(3.1415926535897932 * (u - 0.5), s, c);
-    return d.dc + d.dd * (s / c);
+    sincos_d<1>(3.1415926535897932 * (u - 0.5), s, c);
+    return d.dc + d.dd * div_d(s, c);
   }
   if (KIND == kTruncExtremeKind) return d.dc - d.dd * log_(-log_(u));
   return d.dd * exp_(log_(-log_(1.0 - u)) * d.dc);
@@ -375,7 +370,7 @@ __device__ __forceinline__ double tf64(uint64_t r, const DistParams& d) {
   if (KIND == GR_UNIFORM_REAL2) return ur_d(r) * d.da + d.db;
   if (KIND == GR_EXPONENTIAL) {
     const double l = log_(one_minus_ur_d(r));
-    return (d.flags & kParamUnitDiv) ? -l : -(l / d.da);
+    return (d.flags & kParamUnitDiv) ? -l : -div_d(l, d.da);
   }
   if (KIND == GR_GAMMA) {
     const double l = -(log_(one_minus_ur_d(r)) / 1.0);
@@ -383,14 +378,14 @@ __device__ __forceinline__ double tf64(uint64_t r, const DistParams& d) {
   }
   if (KIND == GR_CAUCHY) {
     double s, c;
-    sincos_(3.1415926535897932 * (ur_d(r) - 0.5), s, c);
-    return d.da + d.db * (s / c);
+    sincos_pi_centred(r, s, c);
+    return d.da + d.db * div_d(s, c);
   }
   if (KIND == GR_WEIBULL) {
     const double w = exp_(log_(-log_(one_minus_ur_d(r))) * d.da);
     return (d.flags & kParamUnitScale) ? w : w * d.db;
   }
-  if (KIND == GR_EXTREME_VALUE) return d.da - log_(-log_(ur_d(r) + 2.220446049250313e-16 / 8)) * d.db;
+  if (KIND == GR_EXTREME_VALUE) return d.da - log_(-log_(ur_nz_int(r))) * d.db;
   // BernoulliGen<double>: the compare runs on the eight 32-bit words and the
   // blend reads each 64-bit element's sign, the compare of its high word
   if (KIND == GR_BERNOULLI) return ((int32_t)((uint32_t)(r >> 32) & 0x7fffffffu) < d.ia) ? 1.0 : 0.0;
@@ -721,11 +716,9 @@ __device__ __forceinline__ void emit_packet(const uint64_t (&pk)[kLanes], const 
       double sv[2], cv[2];
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
-        const double u2 = ur_d(odd ? pk[2 + q] : other[q]);
-        const double radius = sqrt(-2.0 * log_(one_minus_ur_d(odd ? other[q] : pk[q])));
-        const double theta = (2 * 3.1415926535897932) * u2;
+        const double radius = sqrt_neg2(log_(one_minus_ur_d(odd ? other[q] : pk[q])));
         double sn, cs;
-        sincos_(theta, sn, cs);
+        sincos_2pi_u(odd ? pk[2 + q] : other[q], sn, cs);
         sv[q] = radius * sn;
         cv[q] = radius * cs;
       }
@@ -1339,9 +1332,9 @@ __global__ void __launch_bounds__(256) k_sxform(const uint64_t* w, void* out, in
       double* o = reinterpret_cast<double*>(out) + 2 * u * 4;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const double radius = sqrt(-2.0 * log_(one_minus_ur_d(w1[q])));
+        const double radius = sqrt_neg2(log_(one_minus_ur_d(w1[q])));
         double sn, cs;
-        sincos_((2 * 3.1415926535897932) * ur_d(w1[WPP + q]), sn, cs);
+        sincos_2pi_u(w1[WPP + q], sn, cs);
         o[q] = nscale64<KIND>(radius * sn, d);
         if (2 * u + 1 < npk) o[4 + q] = nscale64<KIND>(radius * cs, d);
       }

@@ -20,6 +20,7 @@
 #include <cstdint>
 
 #include "gr_dmath.h"
+#include "gr_fp64i.h"
 #include "gr_math_tables.h"
 
 namespace gr {
@@ -163,57 +164,11 @@ __device__ __forceinline__ void sincosf_(float x, float& s, float& c) {
   c = u2f(f2u(o2) ^ sign_bit_cos);
 }
 
-// EigenRand psincos, double lanes (MorePacketMath.h:395-491); the float-grade
-// Cephes coefficients are evaluated in double arithmetic, as there.
-__device__ __forceinline__ void sincos_(double x, double& s, double& c) {
-  uint64_t sign_bit_sin = d2u(x) & 0x8000000000000000ull;
-  x = fabs(x);
-  double y = x * 1.27323954473516;
-  int64_t emm2 = (int64_t)floor(y);
-  emm2 = emm2 + 1;
-  emm2 = emm2 & ~(int64_t)1;
-  y = (double)emm2;
-  int64_t emm4 = emm2;
-  uint64_t swap_sign_bit_sin = ((uint64_t)(emm2 & 4)) << 61;
-  emm2 = emm2 & 2;
-  uint64_t poly_mask = (emm2 == 0) ? ~0ull : 0ull;
-  double xmm1 = y * -0.78515625;
-  double xmm2 = y * -2.4187564849853515625e-4;
-  double xmm3 = y * -3.77489497744594108e-8;
-  x = x + xmm1;
-  x = x + xmm2;
-  x = x + xmm3;
-  emm4 = emm4 - 2;
-  emm4 = 4 & ~emm4;
-  uint64_t sign_bit_cos = ((uint64_t)emm4) << 61;
-  sign_bit_sin ^= swap_sign_bit_sin;
-  double z = x * x;
-  double yy = 2.443315711809948E-005;
-  yy = yy * z;
-  yy = yy + -1.388731625493765E-003;
-  yy = yy * z;
-  yy = yy + 4.166664568298827E-002;
-  yy = yy * z;
-  yy = yy * z;
-  double tmp = z * 0.5;
-  yy = yy - tmp;
-  yy = yy + 1.0;
-  double y2 = -1.9515295891E-4;
-  y2 = y2 * z;
-  y2 = y2 + 8.3321608736E-3;
-  y2 = y2 * z;
-  y2 = y2 + -1.6666654611E-1;
-  y2 = y2 * z;
-  y2 = y2 * x;
-  y2 = y2 + x;
-  double ysin2 = u2d(poly_mask & d2u(y2));
-  double ysin1 = u2d(d2u(yy) & ~poly_mask);
-  y2 = y2 - ysin2;
-  yy = yy - ysin1;
-  double o1 = ysin1 + ysin2;
-  double o2 = yy + y2;
-  s = u2d(d2u(o1) ^ sign_bit_sin);
-  c = u2d(d2u(o2) ^ sign_bit_cos);
+// uniforms of the reference from a word: asfloat / asdouble of the fraction in
+// [1, 2), less 1 (exact)
+__device__ __forceinline__ float ur_f(uint32_t x) { return u2f((x & 0x7fffffu) | (127u << 23)) - 1.0f; }
+__device__ __forceinline__ double ur_d(uint64_t x) {
+  return u2d((x & 0xfffffffffffffull) | (1023ull << 52)) - 1.0;
 }
 
 // Inverse error function: M. Giles, "Approximating the erfinv function" (GPU
@@ -279,8 +234,8 @@ __device__ __forceinline__ double erfinv_(double x) {
   const double w = -log_((1.0 - x) * (1.0 + x));
   double p;
   if (w < 6.25) p = horner_d(kErfinvDSmall, w - 3.125);
-  else if (w < 16.0) p = horner_d(kErfinvDMid, __dsqrt_rn(w) - 3.25);
-  else p = horner_d(kErfinvDLarge, __dsqrt_rn(w) - 5.0);
+  else if (w < 16.0) p = horner_d(kErfinvDMid, sqrt_d(w) - 3.25);
+  else p = horner_d(kErfinvDLarge, sqrt_d(w) - 5.0);
   return p * x;
 }
 

@@ -24,11 +24,6 @@ __device__ __forceinline__ uint64_t mt_temper(uint64_t r) {
   return r;
 }
 
-__device__ __forceinline__ float ur_f(uint32_t x) { return u2f((x & 0x7fffffu) | (127u << 23)) - 1.0f; }
-__device__ __forceinline__ double ur_d(uint64_t x) {
-  return u2d((x & 0xfffffffffffffull) | (1023ull << 52)) - 1.0;
-}
-
 // One block (312 packets) of a 4-lane engine, computed by a CTA of >= 156
 // threads: thread t makes new words t and t + 156.  Word t + 156 needs new
 // word t (kept in a register) and, for word 311, new word 0 (recomputed from

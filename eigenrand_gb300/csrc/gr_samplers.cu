@@ -49,18 +49,17 @@ __device__ __forceinline__ void staged_value(const Plan& p, const DistParams& d,
   } else if (DT == SD_F64) {
     const int64_t r0 = u * (int64_t)U * 4 + j;
     if (KIND == GR_GAMMA || KIND == GR_CHI_SQUARED) {
-      double y = ur_d(rword(r0)) + 2.220446049250313e-16 / 8;
-      for (int t = 1; t < U; ++t) y = y * (ur_d(rword(r0 + 4 * t)) + 2.220446049250313e-16 / 8);
+      double y = ur_nz_int(rword(r0));
+      for (int t = 1; t < U; ++t) y = y * ur_nz_int(rword(r0 + 4 * t));
       const double l = log_(y);
       reinterpret_cast<double*>(p.out)[o] = (d.flags & kParamUnitScale) ? -l : -(d.db * l);
     } else if (KIND == GR_STUDENT_T) {
       const double u1 = one_minus_ur_d(rword(r0));
-      const double u2 = ur_d(rword(r0 + 4));
       const double nn = (d.flags & kParamVecA) ? __ldg(static_cast<const double*>(d.vparam) + o) : d.da;
       const double ex = (d.flags & kParamVecA) ? -2.0 / nn : d.dc;
-      const double radius = sqrt(nn * (exp_(log_(u1) * ex) - 1.0));
+      const double radius = sqrt_d(nn * (exp_(log_(u1) * ex) - 1.0));
       double sn, cs;
-      sincos_((2 * 3.1415926535897932) * u2, sn, cs);
+      sincos_2pi_u(rword(r0 + 4), sn, cs);
       reinterpret_cast<double*>(p.out)[o] = radius * sn;
     }
   } else {  // int32 over half packets
@@ -272,16 +271,15 @@ __global__ void __launch_bounds__(256) k_sx_staged(const uint64_t* w, void* out,
   } else {
     const uint64_t* q = w + 4 * k * U + j;
     if (KIND == GR_GAMMA) {
-      double y = ur_d(q[0]) + 2.220446049250313e-16 / 8;
-      for (int t = 1; t < U; ++t) y = y * (ur_d(q[4 * t]) + 2.220446049250313e-16 / 8);
+      double y = ur_nz_int(q[0]);
+      for (int t = 1; t < U; ++t) y = y * ur_nz_int(q[4 * t]);
       const double l = log_(y);
       static_cast<double*>(out)[g] = (d.flags & kParamUnitScale) ? -l : -(d.db * l);
     } else {  // GR_STUDENT_T
       const double u1 = one_minus_ur_d(q[0]);
-      const double u2 = ur_d(q[4]);
-      const double radius = sqrt(d.da * (exp_(log_(u1) * d.dc) - 1.0));
+      const double radius = sqrt_d(d.da * (exp_(log_(u1) * d.dc) - 1.0));
       double sn, cs;
-      sincos_((2 * 3.1415926535897932) * u2, sn, cs);
+      sincos_2pi_u(q[4], sn, cs);
       static_cast<double*>(out)[g] = radius * sn;
     }
   }
@@ -495,8 +493,8 @@ __global__ void __launch_bounds__(32) k_sx_beta(const uint64_t* w, int64_t W, Sx
           for (int t = 1; t < g.ib; ++t) y = y * (ur_f(word(8 * t + lane)) + 1.1920928955078125e-07f / 8);
           v = f2u(-(g.fb * logf_(y)));
         } else {
-          double y = ur_d(rval(lane)) + 2.220446049250313e-16 / 8;
-          for (int t = 1; t < g.ib; ++t) y = y * (ur_d(rval(4 * t + lane)) + 2.220446049250313e-16 / 8);
+          double y = ur_nz_int(rval(lane));
+          for (int t = 1; t < g.ib; ++t) y = y * ur_nz_int(rval(4 * t + lane));
           const double l = log_(y);
           v = d2u((g.flags & kParamUnitScale) ? -l : -(g.db * l));
         }
@@ -913,7 +911,7 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
   auto value = [&](int c, int64_t x, int j) -> uint64_t {
     bool acc;
     auto uf = [&](int q) { return ur_f(word((x + q) * 8 + j)); };
-    auto ud = [&](int q) { return ur_d(rval((x + q) * 4 + j)); };
+    auto ud = [&](int q) { return rval((x + q) * 4 + j); };
     if (c == 0) {
       if (DT == SD_F64 && type0 == 2)
         return d2u(1.0 * gs_value_f64(rval(x * 4 + j), rval((x + 1) * 4 + j), bk.c[0].tpx, bk.c[0].d_inv));
@@ -934,13 +932,12 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
     const BetaComp& g = c == 0 ? bk.c[0] : bk.c[1];
     const bool gsv = c == gc;
     if (DT == SD_F64) {
-      constexpr double e = 2.220446049250313e-16 / 8;
       const uint64_t b0 = rval(x * 4 + j), b1 = rval((x + 1) * 4 + j);
-      double arg = ur_d(b1) + e;
+      double arg = ur_nz_int(b1);
       if (!gsv) {
-        double y = ur_d(b0) + e;
+        double y = ur_nz_int(b0);
         y = y * arg;
-        for (int q = 2; q < g.U; ++q) y = y * (ur_d(rval((x + q) * 4 + j)) + e);
+        for (int q = 2; q < g.U; ++q) y = y * ur_nz_int(rval((x + q) * 4 + j));
         arg = y;
       }
       const double l = log_(arg);
@@ -1005,7 +1002,7 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
               const uint64_t v = q == 0 ? w0 : (q == 1 ? w1 : w2);
               return ur_f((j & 1) ? (uint32_t)(v >> 32) : (uint32_t)v);
             };
-            auto ud = [&](int q) { return ur_d(q == 0 ? w0 : (q == 1 ? w1 : w2)); };
+            auto ud = [&](int q) { return q == 0 ? w0 : (q == 1 ? w1 : w2); };
             if (c == 0) beta_comp_u<DT, true>(bk.c[0], type0, uf, ud, acc);
             else beta_comp_u<DT, true>(bk.c[1], type1, uf, ud, acc);
           }
@@ -1196,8 +1193,8 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
             reinterpret_cast<float*>(p.out)[off + (e0 + i) * P + j] = post ? (bk.fpost * x) / (1.0f - x) : x;
           } else {
             const double p1 = u2d(v[0]), p2 = u2d(v[1]);
-            const double x = p1 / (p1 + p2);
-            reinterpret_cast<double*>(p.out)[off + (e0 + i) * P + j] = post ? (bk.dpost * x) / (1.0 - x) : x;
+            const double x = div_d(p1, p1 + p2);
+            reinterpret_cast<double*>(p.out)[off + (e0 + i) * P + j] = post ? div_d(bk.dpost * x, 1.0 - x) : x;
           }
         }
         // lanes still carried move to the front of each lane buffer

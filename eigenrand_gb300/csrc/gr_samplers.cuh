@@ -194,7 +194,7 @@ __device__ __forceinline__ bool rej_trial(const DistParams& d, int64_t t, int j,
         acc = true;
       } else {
         const double ux = ur_d(rval(r0));
-        const double vx = ur_d(rval(r0 + 4)) + 2.220446049250313e-16 / 8;
+        const double vx = ur_nz_int(rval(r0 + 4));
         const double ux2 = ur_d(rval(r0 + 8));
         const double lv = log_(vx);
         const bool c = ux < d.de;
@@ -213,10 +213,9 @@ __device__ __forceinline__ bool rej_trial(const DistParams& d, int64_t t, int j,
       const int f = tan_filter_f64(rval(r0), rval(r0 + 4), d.fd, d.ff);
       acc = f == 1;
       if ((CAND && f != 0) || f < 0) {
-        const double u = ur_d(rval(r0));
         double ys, yc;
-        sincos_(3.1415926535897932 * u, ys, yc);
-        const double yx = ys / yc;
+        sincos_pi_u(rval(r0), ys, yc);
+        const double yx = div_d(ys, yc);
         const double xx = d.df * yx + d.dd;
         if (f < 0) {
           const double ux = ur_d(rval(r0 + 4));
@@ -232,7 +231,7 @@ __device__ __forceinline__ bool rej_trial(const DistParams& d, int64_t t, int j,
       const double p1 = exp_(log_(u1) * d.dc);
       const double p2 = exp_(log_(u2) * d.dd);
       const double x = p1 + p2;
-      cbits = d2u(p1 / x);
+      cbits = d2u(div_d(p1, x));
       acc = x <= 1.0;
     }
   } else {  // int32 kinds with Packet4f internals over half packets
@@ -286,12 +285,12 @@ __device__ __forceinline__ uint64_t rej_value(const DistParams& d, int64_t t, in
     if (RK == RK_GAMMA_GS) return d2u(d.db * gs_value_f64(rval(r0), rval(r0 + 4), d2u(d.dg), d.dc));
     if (RK == RK_GAMMA_TAN) {
       double ys, yc;
-      sincos_(3.1415926535897932 * ur_d(rval(r0)), ys, yc);
-      return d2u(d.db * (d.df * (ys / yc) + d.dd));
+      sincos_pi_u(rval(r0), ys, yc);
+      return d2u(d.db * (d.df * div_d(ys, yc) + d.dd));
     }
     const double p1 = exp_(log_(ur_d(rval(r0))) * d.dc);
     const double p2 = exp_(log_(ur_d(rval(r0 + 4))) * d.dd);
-    return d2u(p1 / (p1 + p2));
+    return d2u(div_d(p1, p1 + p2));
   }
   float ys, yc;
   sincosf_((float)3.1415926535897932 * ur_f(word(w0 + j)), ys, yc);
@@ -341,8 +340,8 @@ inline BetaComp beta_component(int branch, float af, double ad) {
 }
 
 // Value (closed form) or candidate (rejection trial) of one GammaGen
-// component of sampler type `type` at one lane: Uf(q) / Ud(q) give the
-// lane's uniform in the q-th packet of the draw.  ACC: also decide
+// component of sampler type `type` at one lane: Uf(q) gives the
+// lane's uniform in the q-th packet of the draw, Ud(q) its word.  ACC: also decide
 // acceptance (the rejection types); without it only the candidate is
 // computed, for lanes already known to be accepted (the same expressions,
 // so the same bits).
@@ -377,33 +376,33 @@ __device__ __forceinline__ uint64_t beta_comp_u(const BetaComp g, const int type
     }
     return f2u(1.0f * xx);
   } else {
-    if (type == 0) return d2u(1.0 * (-(log_(1.0 - Ud(0)) / 1.0)));
+    if (type == 0) return d2u(1.0 * (-(log_(one_minus_ur_d(Ud(0))) / 1.0)));
     if (type == 1) {
-      double y = Ud(0) + 2.220446049250313e-16 / 8;
-      for (int t = 1; t < U; ++t) y = y * (Ud(t) + 2.220446049250313e-16 / 8);
+      double y = ur_nz_int(Ud(0));
+      for (int t = 1; t < U; ++t) y = y * ur_nz_int(Ud(t));
       return d2u(-(1.0 * log_(y)));
     }
     if (type == 2) {
-      const double ux = Ud(0), vx = Ud(1) + 2.220446049250313e-16 / 8;
+      const double ux = ur_d(Ud(0)), vx = ur_nz_int(Ud(1));
       const double lv = log_(vx);
       double xx;
       if (ux < g.d_px) {
         xx = exp_(g.d_inv * lv);
-        if (ACC) acc = Ud(2) < exp_(-xx);
+        if (ACC) acc = ur_d(Ud(2)) < exp_(-xx);
       } else {
         xx = 1.0 - lv;
-        if (ACC) acc = Ud(2) < exp_(log_(xx) * g.d_am1);
+        if (ACC) acc = ur_d(Ud(2)) < exp_(log_(xx) * g.d_am1);
       }
       return d2u(1.0 * xx);
     }
     const double a1 = g.d_am1, sq = g.d_sq;
     double ys, yc;
-    sincos_(3.1415926535897932 * Ud(0), ys, yc);
-    const double yx = ys / yc;
+    sincos_pi_u(Ud(0), ys, yc);
+    const double yx = div_d(ys, yc);
     const double xx = sq * yx + a1;
     if (ACC) {
       const double ub = (yx * yx + 1.0) * exp_(a1 * log_(xx / a1) - yx * sq);
-      acc = (0.0 < xx) && (Ud(1) <= ub);
+      acc = (0.0 < xx) && (ur_d(Ud(1)) <= ub);
     }
     return d2u(1.0 * xx);
   }

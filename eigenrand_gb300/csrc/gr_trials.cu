@@ -138,9 +138,8 @@ __device__ __forceinline__ bool trial_eval(const SM& sm, const DistParams& d, co
       const double l = -(log_(one_minus_ur_d(rval(j))) / 1.0);
       c = d2u((d.flags & kParamUnitScale) ? l : d.db * l);
     } else {
-      constexpr double e = 2.220446049250313e-16 / 8;
-      double y = ur_d(rval(j)) + e;
-      for (int t = 1; t < U; ++t) y = y * (ur_d(rval(4 * t + j)) + e);
+      double y = ur_nz_int(rval(j));
+      for (int t = 1; t < U; ++t) y = y * ur_nz_int(rval(4 * t + j));
       const double l = log_(y);
       c = d2u((d.flags & kParamUnitScale) ? -l : -(d.db * l));
     }
