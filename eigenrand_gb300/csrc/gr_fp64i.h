@@ -203,15 +203,15 @@ GRD_HD double scaled52(uint64_t D, uint64_t cm, int cf) {
 //       subtraction of 2 n (DP1 + DP2) gives it;
 //   z / 2 is exact, so (p - z / 2) is one fused operation;
 //   the masked sums at the end are selections (no addend is -0).
-// The first four multiply-and-add steps run on the integer pipes, the other
-// twelve operations (with the two products of a Box-Muller pair) on the FP64
-// pipe.  4096 x 4096 on 608 engines, us, normal / Cauchy: 707 / 1 383 with the
-// reference's operations, the library's square root and quotient; 405 / 768
-// with those two, the angle and the reduction as here; 350 / 636 with two of
-// the four steps in integers, 333 / 511 with four.  Both pipes are then busy
-// for 0.64 of the time.
-// TOP: |x| is below the threshold 2 TOP + 1 in all but unusual calls, which go to
-// sincos_long.
+// The first five steps of both polynomials run on the integer pipes, the other
+// ten operations (with the two products of a Box-Muller pair) on the FP64 pipe.
+// 4096 x 4096 on 608 engines, us, normal / Cauchy: 707 / 1 383 with the
+// reference's operations and the library's square root and quotient; 405 / 768
+// with those two, the angle and the reduction as here; 333 / 511 with four of
+// the five steps, 321 / 521 with five (328 / 575 with four in the kernel as it
+// is now, two words per thread).
+// TOP: |x| is below the threshold 2 TOP + 1, and not tiny, in all but unusual
+// calls, which go to sincos_long.
 GRD_SLOW void sincos_long(double x, double* s, double* c) {
   uint64_t sign_bit_sin = grd_bits(x) & 0x8000000000000000ull;
   x = fabs(x);
@@ -260,9 +260,9 @@ GRD_SLOW void sincos_long(double x, double* s, double* c) {
 template <int TOP>
 GRD_HD void sincos_d(double x, double& s, double& c) {
   const uint64_t ux = grd_bits(x), ax = ux & 0x7fffffffffffffffull;
-  // just below the least |x| with product 3, 5, 9 (the high word decides)
-  constexpr uint32_t kEnd = TOP == 1 ? 0x4002d97cu : TOP == 2 ? 0x400f6a7au : 0x401c463au;
-  if ((uint32_t)(ax >> 32) >= kEnd) {
+  // 2^-63, and just below the least |x| with product 3, 5, 9 (high words)
+  constexpr uint32_t kLow = 0x3c000000u, kEnd = TOP == 1 ? 0x4002d97cu : TOP == 2 ? 0x400f6a7au : 0x401c463au;
+  if ((uint32_t)(ax >> 32) - kLow >= kEnd - kLow) {
     sincos_long(x, &s, &c);
     return;
   }
@@ -279,7 +279,7 @@ GRD_HD void sincos_d(double x, double& s, double& c) {
   const double z = a * a;
   const uint64_t uz = grd_bits(z);
   const uint64_t Z = (uz & 0xfffffffffffffull) | 0x10000000000000ull;
-  const int ez = (int)(uz >> 52) - 1023;  // z = 0: far below every coefficient
+  const int ez = (int)(uz >> 52) - 1023;
   int k;
   uint64_t m = mul53(sc53(0x3ef99eb9c5ac8ebfull), Z, k);                          // 2.443315711809948E-005
   const uint64_t p1 = sub53(sc53(0x3f56c0c33a85cd5full), -10, m, ez + k - 16);     // 1.388731625493765E-003
@@ -289,9 +289,12 @@ GRD_HD void sincos_d(double x, double& s, double& c) {
   const uint64_t p2 = sub53(sc53(0x3fa55554a115bc8full), -5, m, ez + k - 10);  // 4.166664568298827E-002
   m = mul53(q1, Z, k);
   const uint64_t q2 = sub53(sc53(0x3fc5555452709addull), -3, m, ez + k - 7);       // 1.6666654611E-1
-  const double p = grd_double(((uint64_t)(1022 - 5) << 52) + p2), q = grd_double(((uint64_t)(1022 - 3) << 52) + q2);
-  const double yc = fma(-0.5, z, (p * z) * z) + 1.0;
-  const double ys = a - (q * z) * a;
+  m = mul53(p2, Z, k);
+  const double pz = grd_double(((uint64_t)(1022 - 5 + ez + k) << 52) + m);
+  m = mul53(q2, Z, k);
+  const double qz = grd_double(((uint64_t)(1022 - 3 + ez + k) << 52) + m);
+  const double yc = fma(-0.5, z, pz * z) + 1.0;
+  const double ys = a - qz * a;
   const uint64_t bs = grd_bits((n & 1) ? yc : ys), bc = grd_bits((n & 1) ? ys : yc);
   s = grd_double(bs ^ ((ux & 0x8000000000000000ull) ^ ((uint64_t)(n & 2) << 62)));
   c = grd_double(bc ^ ((uint64_t)((n + 1) & 2) << 62));

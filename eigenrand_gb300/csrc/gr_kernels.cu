@@ -23,17 +23,30 @@
 
 namespace gr {
 
+// The twist and the tempering in 32-bit halves: 6 + 12 instructions of the logic
+// pipe and 2 products.  Uniform floats, 8192 x 8192 on 608 engines: 66 us, 73
+// with the 64-bit expressions that the other kernels use (gr_mt.cuh), where
+// these cost 1 to 2 % instead (integral gamma, binomial; the products wait for
+// the pipe that the addressing uses).
 __device__ __forceinline__ uint64_t twist1(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t t = (a & kUpper) | (b & kLower);
-  return (t >> 1) ^ ((0ull - (t & 1ull)) & kMatA) ^ c;
+  const uint32_t ah = (uint32_t)(a >> 32), bl = (uint32_t)b, odd = bl & 1u;
+  const uint32_t tl = ((uint32_t)a & 0x80000000u) | (bl & 0x7fffffffu);
+  const uint32_t lo = __funnelshift_r(tl, ah, 1) ^ (odd * (uint32_t)kMatA) ^ (uint32_t)c;
+  const uint32_t hi = (ah >> 1) ^ (odd * (uint32_t)(kMatA >> 32)) ^ (uint32_t)(c >> 32);
+  return (uint64_t)lo | (uint64_t)hi << 32;
 }
+static_assert(kUpper == ~0ull << 31, "the halves above");
 
 __device__ __forceinline__ uint64_t temper(uint64_t r) {
-  r ^= (r >> 29) & 0x5555555555555555ull;
-  r ^= (r << 17) & 0x71d67fffeda60000ull;
-  r ^= (r << 37) & 0xfff7eee000000000ull;
-  r ^= r >> 43;
-  return r;
+  uint32_t lo = (uint32_t)r, hi = (uint32_t)(r >> 32);
+  lo ^= __funnelshift_r(lo, hi, 29) & 0x55555555u;
+  hi ^= (hi >> 29) & 0x55555555u;
+  const uint32_t l0 = lo;
+  lo ^= (lo << 17) & 0xeda60000u;
+  hi ^= __funnelshift_l(l0, hi, 17) & 0x71d67fffu;
+  hi ^= (lo << 5) & 0xfff7eee0u;
+  lo ^= hi >> 11;
+  return (uint64_t)lo | (uint64_t)hi << 32;
 }
 
 // ---------------------------------------------------------------- seeding
@@ -70,6 +83,10 @@ cudaError_t launch_seed(EngState* st, int K, uint64_t seed, cudaStream_t s) {
 // the same thread made two phases and one phase before, so they stay in
 // registers and only x[i+1], two phases old, comes from the next lane by a
 // shuffle: no shared memory and no barrier between phases.
+__device__ __forceinline__ uint64_t xor64(uint64_t v, int m) {
+  return ((uint64_t)__shfl_xor_sync(0xffffffffu, (uint32_t)(v >> 32), m) << 32) |
+         (uint64_t)__shfl_xor_sync(0xffffffffu, (uint32_t)v, m);
+}
 __device__ __forceinline__ uint64_t shfl64(uint64_t v, int src) {
   return ((uint64_t)__shfl_sync(0xffffffffu, (uint32_t)(v >> 32), src) << 32) |
          (uint64_t)__shfl_sync(0xffffffffu, (uint32_t)v, src);
@@ -525,10 +542,9 @@ __device__ __forceinline__ void st16(void* p, uint32_t a, uint32_t b, uint32_t c
   *reinterpret_cast<uint4*>(p) = make_uint4(a, b, c, d);
 }
 
-// 32 bytes of one packet.  A thread's packet is one 32-byte sector: two 16-byte
-// stores reach L2 as two partial writes of it (8192 x 8192 uniform floats:
-// 79.6 us), the 256-bit store as one.  An output that is only 16-byte aligned
-// (or starts after an odd cached packet) takes the two.
+// 32 bytes of one thread, a sector: two 16-byte stores would reach L2 as two
+// partial writes of it.  An output that is only 16-byte aligned (or starts after
+// an odd cached packet) takes the two.
 __device__ __forceinline__ void st32(void* p, const uint64_t a, const uint64_t b, const uint64_t c, const uint64_t d) {
   if (((uintptr_t)p & 31) == 0) {
     asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
@@ -537,7 +553,6 @@ __device__ __forceinline__ void st32(void* p, const uint64_t a, const uint64_t b
     reinterpret_cast<ulonglong2*>(p)[1] = make_ulonglong2(c, d);
   }
 }
-__device__ __forceinline__ uint64_t two32(uint32_t lo, uint32_t hi) { return (uint64_t)lo | (uint64_t)hi << 32; }
 
 // int32 kinds whose packets are rng.half() words leave raw words in the
 // engine's half cache; DiscreteGen caches its own computed results
@@ -549,206 +564,159 @@ struct CacheUse {
   static constexpr bool gen = (MODE == M_N32) || (MODE == M_N64) || (MODE == M_W32 && KIND == GR_DISCRETE);
 };
 
-// The samples of packet pidx of a call (pk: its four tempered words), output
-// element obase + pidx * OPP on; oend: end of the engine's slice (the half of
-// a packet or unit past it goes to the cache).  Called by whole warps whose
-// lanes hold consecutive packets from an even one on: the Box-Muller kinds
-// exchange words within packet pairs.
-template <int MODE, int KIND>
-__device__ __forceinline__ void emit_packet(const uint64_t (&pk)[kLanes], const int64_t pidx, const bool valid,
-                                            const Plan& p, const DistParams& d, const int64_t obase,
-                                            const int64_t oend, EngState* st, GenState* gs) {
+// The samples of half h of packet pidx of a call (pk: the half's two tempered
+// words), output element obase + pidx * OPP on; oend: end of the engine's slice
+// (the half of a packet or unit past it goes to the cache).  Called by whole
+// warps whose lanes hold consecutive halves from an even packet on: the
+// Box-Muller kinds exchange words within packet pairs.  FULL: the call's last
+// packet is none of these.
+template <int MODE, int KIND, bool FULL = false>
+__device__ __forceinline__ void emit_half(const uint64_t (&pk)[2], const int h, const int64_t pidx, const bool valid,
+                                          const Plan& p, const DistParams& d, const int64_t obase, const int64_t oend,
+                                          EngState* st, GenState* gs) {
   constexpr bool kHalfKind = CacheUse<MODE, KIND>::half_kind;
+  const uint32_t wd[4] = {(uint32_t)pk[0], (uint32_t)(pk[0] >> 32), (uint32_t)pk[1], (uint32_t)(pk[1] >> 32)};
   if (MODE == M_RAW) {
-    if (valid && p.out) {  // p.out == nullptr: discard
-      uint64_t* o = reinterpret_cast<uint64_t*>(p.out) + obase + pidx * 4;
-      st32(o, pk[0], pk[1], pk[2], pk[3]);
-    }
-  } else if (MODE == M_RAW2) {
-    if (valid && p.out)
-      reinterpret_cast<ulonglong2*>(reinterpret_cast<uint64_t*>(p.out) + obase + pidx * 2)[0] =
+    if (valid && p.out)  // p.out == nullptr: discard
+      *reinterpret_cast<ulonglong2*>(reinterpret_cast<uint64_t*>(p.out) + obase + pidx * 4 + 2 * h) =
           make_ulonglong2(pk[0], pk[1]);
-  } else if (MODE == M_F32H) {
-    if (valid) {
-      float* o = reinterpret_cast<float*>(p.out) + obase + pidx * 4;
-      const int64_t ib = obase + pidx * 4;
-      reinterpret_cast<float4*>(o)[0] =
-          make_float4(tf32i<KIND>((uint32_t)pk[0], d, ib), tf32i<KIND>((uint32_t)(pk[0] >> 32), d, ib + 1),
-                      tf32i<KIND>((uint32_t)pk[1], d, ib + 2), tf32i<KIND>((uint32_t)(pk[1] >> 32), d, ib + 3));
-    }
-  } else if (MODE == M_F64H) {
-    if (valid) {
-      double* o = reinterpret_cast<double*>(p.out) + obase + pidx * 2;
-      const int64_t ib = obase + pidx * 2;
-      reinterpret_cast<double2*>(o)[0] = make_double2(tf64i<KIND>(pk[0], d, ib), tf64i<KIND>(pk[1], d, ib + 1));
-    }
+  } else if (MODE == M_RAW2) {
+    if (valid && h == 0 && p.out)
+      *reinterpret_cast<ulonglong2*>(reinterpret_cast<uint64_t*>(p.out) + obase + pidx * 2) = make_ulonglong2(pk[0], pk[1]);
   } else if (MODE == M_RAW0) {
     // a scalar draw takes the engine's whole packet and keeps its first
     // element (StdUniformRealGen::operator(), Dists/Basic.h:533-540)
-    if (valid) reinterpret_cast<uint64_t*>(p.out)[obase / 4 + pidx] = pk[0];
-  } else if (MODE == M_F32) {
-    if (valid) {
-      float* o = reinterpret_cast<float*>(p.out) + obase + pidx * 8;
-      float v[8];
+    if (valid && h == 0) reinterpret_cast<uint64_t*>(p.out)[obase / 4 + pidx] = pk[0];
+  } else if (MODE == M_F32H || MODE == M_F32) {
+    if (valid && (MODE == M_F32 || h == 0)) {
+      const int64_t ib = obase + (MODE == M_F32 ? pidx * 8 + 4 * h : pidx * 4);
+      float v[4];
       if (KIND == kBernoulliVKind) {
         // BernoulliVGen<float>: p = cvttps(a * 2^31), compared signed with
         // the masked word (Basic.h:735-745)
-        const float4* pv = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(d.vparam) + obase + pidx * 8);
-        const float4 q0 = pv[0], q1 = pv[1];
-        const float pa[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+        const float4 a = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(d.vparam) + ib);
+        const float pa[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const uint32_t w = (q & 1) ? (uint32_t)(pk[q >> 1] >> 32) : (uint32_t)pk[q >> 1];
-          v[q] = ((int32_t)(w & 0x7fffffffu) < cvtt_f32(pa[q] * 2147483648.0f)) ? 1.0f : 0.0f;
-        }
+        for (int q = 0; q < 4; ++q)
+          v[q] = ((int32_t)(wd[q] & 0x7fffffffu) < cvtt_f32(pa[q] * 2147483648.0f)) ? 1.0f : 0.0f;
       } else {
 #pragma unroll
-        for (int l = 0; l < kLanes; ++l) {
-          v[2 * l] = tf32i<KIND>((uint32_t)pk[l], d, obase + pidx * 8 + 2 * l);
-          v[2 * l + 1] = tf32i<KIND>((uint32_t)(pk[l] >> 32), d, obase + pidx * 8 + 2 * l + 1);
-        }
+        for (int q = 0; q < 4; ++q) v[q] = tf32i<KIND>(wd[q], d, ib + q);
       }
-      st32(o, two32(f2u(v[0]), f2u(v[1])), two32(f2u(v[2]), f2u(v[3])), two32(f2u(v[4]), f2u(v[5])),
-           two32(f2u(v[6]), f2u(v[7])));
+      *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + ib) = make_float4(v[0], v[1], v[2], v[3]);
     }
-  } else if (MODE == M_F64) {
-    if (valid) {
-      double* o = reinterpret_cast<double*>(p.out) + obase + pidx * 4;
-      double v[4];
-#pragma unroll
-      for (int l = 0; l < kLanes; ++l) v[l] = tf64i<KIND>(pk[l], d, obase + pidx * 4 + l);
-      st32(o, d2u(v[0]), d2u(v[1]), d2u(v[2]), d2u(v[3]));
+  } else if (MODE == M_F64H || MODE == M_F64) {
+    if (valid && (MODE == M_F64 || h == 0)) {
+      const int64_t ib = obase + (MODE == M_F64 ? pidx * 4 + 2 * h : pidx * 2);
+      *reinterpret_cast<double2*>(reinterpret_cast<double*>(p.out) + ib) =
+          make_double2(tf64i<KIND>(pk[0], d, ib), tf64i<KIND>(pk[1], d, ib + 1));
     }
   } else if (MODE == M_W32 || MODE == M_W64) {
     if (valid) {
-      const int64_t ob = obase + pidx * 8;
-      uint32_t wd[8];
-#pragma unroll
-      for (int l = 0; l < kLanes; ++l) {
-        wd[2 * l] = (uint32_t)pk[l];
-        wd[2 * l + 1] = (uint32_t)(pk[l] >> 32);
-      }
-      const bool full = ob + 8 <= oend;
+      const int64_t ob = obase + pidx * 8 + 4 * h;
+      const bool in = FULL || ob + 4 <= oend;
       if (MODE == M_W32) {
-        int32_t v[8];
+        int32_t v[4];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = tw32<KIND>(wd[q], d);
-        int32_t* o = reinterpret_cast<int32_t*>(p.out) + ob;
-        if (full) st32(o, two32(v[0], v[1]), two32(v[2], v[3]), two32(v[4], v[5]), two32(v[6], v[7]));
-        else st16(o, v[0], v[1], v[2], v[3]);
-        if (!full && (gs || kHalfKind)) {
+        for (int q = 0; q < 4; ++q) v[q] = tw32<KIND>(wd[q], d);
+        if (in) {
+          st16(reinterpret_cast<int32_t*>(p.out) + ob, v[0], v[1], v[2], v[3]);
+        } else if (gs || kHalfKind) {
           // leftover half: rng.half() kinds leave raw words in the engine's
           // half() cache; DiscreteGen caches its computed upper 4 results
           uint32_t* cdst = kHalfKind ? st->half_cache : gs->s[0].cache;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) cdst[q] = kHalfKind ? wd[4 + q] : (uint32_t)v[4 + q];
+          for (int q = 0; q < 4; ++q) cdst[q] = kHalfKind ? wd[q] : (uint32_t)v[q];
         }
-      } else {
-        double v[8];
+      } else if (in) {
+        double v[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) v[q] = tw64i<KIND>(wd[q], d, ob + q);
-        double* o = reinterpret_cast<double*>(p.out) + ob;
-        st32(o, d2u(v[0]), d2u(v[1]), d2u(v[2]), d2u(v[3]));
-        if (full) {
+        st32(reinterpret_cast<double*>(p.out) + ob, d2u(v[0]), d2u(v[1]), d2u(v[2]), d2u(v[3]));
+      } else {
 #pragma unroll
-          for (int q = 4; q < 8; ++q) v[q] = tw64i<KIND>(wd[q], d, ob + q);
-          st32(o + 4, d2u(v[4]), d2u(v[5]), d2u(v[6]), d2u(v[7]));
-        } else {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) st->half_cache[q] = wd[4 + q];
-        }
+        for (int q = 0; q < 4; ++q) st->half_cache[q] = wd[q];
       }
     }
-  } else if (MODE == M_N32) {
-    // unit = packets (2j, 2j+1): u1 words in the even thread, u2 in the odd.
-    // Even thread handles lanes i = 0..3 of the unit, odd handles 4..7.
+  } else {
+    // unit = packets (2j, 2j+1): u1 words in the even packet, u2 in the odd.
+    // The even packet's thread makes the pairs of its half's first word, the
+    // odd one's those of the second: they exchange one word.
     const bool odd = (pidx & 1);
-    uint32_t wd[8];
-#pragma unroll
-    for (int l = 0; l < kLanes; ++l) {
-      wd[2 * l] = (uint32_t)pk[l];
-      wd[2 * l + 1] = (uint32_t)(pk[l] >> 32);
-    }
-    uint32_t other[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) other[q] = __shfl_xor_sync(0xffffffffu, odd ? wd[q] : wd[4 + q], 1);
+    const uint64_t other = xor64(odd ? pk[0] : pk[1], 2);
     if (valid) {
       const int64_t unit = pidx >> 1;
-      const int i0 = odd ? 4 : 0;
-      float sv[4], cv[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float u1 = ur_f(odd ? other[q] : wd[q]);
-        const float u2 = ur_f(odd ? wd[4 + q] : other[q]);
-        const float radius = sqrtf((float)-2 * logf_(1.0f - u1));
-        const float theta = (float)(2 * 3.1415926535897932) * u2;
-        float sn, cs;
-        sincosf_(theta, sn, cs);
-        sv[q] = radius * sn;
-        cv[q] = radius * cs;
-      }
-      const int64_t ob = obase + unit * 16;
-      float* o = reinterpret_cast<float*>(p.out) + ob;
-      reinterpret_cast<float4*>(o + i0)[0] =
-          make_float4(nscale32i<KIND>(sv[0], d, ob + i0), nscale32i<KIND>(sv[1], d, ob + i0 + 1),
-                      nscale32i<KIND>(sv[2], d, ob + i0 + 2), nscale32i<KIND>(sv[3], d, ob + i0 + 3));
-      if (ob + 16 <= oend) {
-        reinterpret_cast<float4*>(o + 8 + i0)[0] =
-            make_float4(nscale32i<KIND>(cv[0], d, ob + 8 + i0), nscale32i<KIND>(cv[1], d, ob + 9 + i0),
-                        nscale32i<KIND>(cv[2], d, ob + 10 + i0), nscale32i<KIND>(cv[3], d, ob + 11 + i0));
-      } else if (gs) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) gs->s[0].cache[i0 + q] = f2u(cv[q]);
-      }
-    }
-  } else if (MODE == M_N64) {
-    const bool odd = (pidx & 1);
-    uint64_t other[2];
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      uint64_t sendv = odd ? pk[q] : pk[2 + q];
-      other[q] = ((uint64_t)__shfl_xor_sync(0xffffffffu, (uint32_t)(sendv >> 32), 1) << 32) |
-                 (uint64_t)__shfl_xor_sync(0xffffffffu, (uint32_t)sendv, 1);
-    }
-    if (valid) {
-      const int64_t unit = pidx >> 1;
-      const int i0 = odd ? 2 : 0;
-      double sv[2], cv[2];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const double radius = sqrt_neg2(log_(one_minus_ur_d(odd ? other[q] : pk[q])));
-        double sn, cs;
-        sincos_2pi_u(odd ? pk[2 + q] : other[q], sn, cs);
-        sv[q] = radius * sn;
-        cv[q] = radius * cs;
-      }
-      const int64_t ob = obase + unit * 8;
-      double* o = reinterpret_cast<double*>(p.out) + ob;
-      reinterpret_cast<double2*>(o + i0)[0] =
-          make_double2(nscale64i<KIND>(sv[0], d, ob + i0), nscale64i<KIND>(sv[1], d, ob + i0 + 1));
-      if (ob + 8 <= oend) {
-        reinterpret_cast<double2*>(o + 4 + i0)[0] =
-            make_double2(nscale64i<KIND>(cv[0], d, ob + 4 + i0), nscale64i<KIND>(cv[1], d, ob + 5 + i0));
-      } else if (gs) {
+      const uint64_t w1 = odd ? other : pk[0], w2 = odd ? pk[1] : other;
+      if (MODE == M_N32) {
+        const int i0 = 4 * h + (odd ? 2 : 0);
+        float sv[2], cv[2];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-          uint64_t b = d2u(cv[q]);
-          gs->s[0].cache[2 * (i0 + q)] = (uint32_t)b;
-          gs->s[0].cache[2 * (i0 + q) + 1] = (uint32_t)(b >> 32);
+          const float u1 = ur_f((uint32_t)(w1 >> (32 * q))), u2 = ur_f((uint32_t)(w2 >> (32 * q)));
+          const float radius = sqrtf((float)-2 * logf_(1.0f - u1));
+          const float theta = (float)(2 * 3.1415926535897932) * u2;
+          float sn, cs;
+          sincosf_(theta, sn, cs);
+          sv[q] = radius * sn;
+          cv[q] = radius * cs;
+        }
+        const int64_t ob = obase + unit * 16 + i0;
+        float* o = reinterpret_cast<float*>(p.out) + ob;
+        *reinterpret_cast<float2*>(o) = make_float2(nscale32i<KIND>(sv[0], d, ob), nscale32i<KIND>(sv[1], d, ob + 1));
+        if (ob - i0 + 16 <= oend) {
+          *reinterpret_cast<float2*>(o + 8) =
+              make_float2(nscale32i<KIND>(cv[0], d, ob + 8), nscale32i<KIND>(cv[1], d, ob + 9));
+        } else if (gs) {
+          gs->s[0].cache[i0] = f2u(cv[0]);
+          gs->s[0].cache[i0 + 1] = f2u(cv[1]);
+        }
+      } else {
+        const int i0 = 2 * h + (odd ? 1 : 0);
+        const double radius = sqrt_neg2(log_(one_minus_ur_d(w1)));
+        double sn, cs;
+        sincos_2pi_u(w2, sn, cs);
+        const int64_t ob = obase + unit * 8 + i0;
+        double* o = reinterpret_cast<double*>(p.out) + ob;
+        o[0] = nscale64i<KIND>(radius * sn, d, ob);
+        const double cv = radius * cs;
+        if (ob - i0 + 8 <= oend) {
+          o[4] = nscale64i<KIND>(cv, d, ob + 4);
+        } else if (gs) {
+          const uint64_t b = d2u(cv);
+          gs->s[0].cache[2 * i0] = (uint32_t)b;
+          gs->s[0].cache[2 * i0 + 1] = (uint32_t)(b >> 32);
         }
       }
     }
   }
 }
 
-// Kinds whose transform takes a few operations per word.
+// One CTA per stream or jump segment, two threads per packet of a phase.  The
+// cheap kinds are bound by the logic pipe (uniform floats: 12 of its
+// instructions per sample, 43 of 60 us), float transforms by instruction issue,
+// double ones by the FP64 and logic pipes together (gr_fp64i.h).  608 engines
+// give an SM four CTAs whatever their size: with a thread per packet (160
+// threads) it held 20 warps, here 40, which also store 512 consecutive bytes at
+// a time.  8192 x 8192 on 608 engines, us, before / now: uniform f32 74.9 / 59.5,
+// discrete 143 / 122, weibull f32 309 / 284, exponential f64 746 / 711, lognormal
+// f64 2 168 / 1 876, weibull f64 2 093 / 1 832.
+constexpr int kDirThreads = 320;
+
+// Kinds whose transform takes a few operations per word: their loop is unrolled
+// over two blocks with shared-memory offsets and the registers' roles fixed
+// (0.60 instead of 0.83 warp-instructions per uniform float).
 template <int MODE, int KIND>
 constexpr bool kLightKind = MODE == M_RAW || MODE == M_RAW0 || MODE == M_RAW2 || KIND == GR_UNIFORM_REAL ||
                             KIND == GR_UNIFORM_REAL2 || (KIND == GR_BALANCED && MODE != M_W64) || KIND == GR_BERNOULLI ||
                             KIND == GR_RANDBITS || KIND == GR_UNIFORM_INT;
 
+// Kinds that need more than the 48 registers of four CTAs per SM.
 template <int MODE, int KIND>
-__global__ void __maxnreg__(64) k_direct(Plan p, DistParams d, const CallSnap* snap) {
+constexpr bool kWideKind = MODE == M_F64 && (KIND == kTruncNormalKind || KIND == kTruncLognormalKind);
+
+template <int MODE, int KIND>
+__global__ void __launch_bounds__(kDirThreads, kWideKind<MODE, KIND> ? 2 : 4)
+    k_direct(Plan p, DistParams d, const CallSnap* snap) {
   const int k = blockIdx.x / p.S, s = blockIdx.x % p.S;
   const int tid = threadIdx.x;
   EngState* st = p.eng + k;
@@ -805,67 +773,87 @@ __global__ void __maxnreg__(64) k_direct(Plan p, DistParams d, const CallSnap* s
   } else {
     w0 = s == 0 ? &st->win[0][0] : p.segwin + ((size_t)k * (p.S - 1) + (s - 1)) * kLanes * kN;
   }
-  // Thread t < 156 holds word t of the last two phases (156 words) of the four
-  // lanes: x[i] and x[i + 156] of the recurrence are its own registers, and
-  // x[i + 1], two phases old, is read from the words every thread puts into
-  // `nbr` as it makes them.  The last thread's x[i + 1] is thread 0's word of
-  // the phase just made: there in every first phase of a pair, made again from
-  // threads 0 and 1's words in the second, so one barrier serves two phases.
-  __shared__ uint64_t nbr[4][kLanes][160];  // [phase mod 4][lane][thread]
-  const int ti = min(tid, kM - 1);
-  uint64_t x[kLanes], c[kLanes], o[kLanes];  // words of phases g - 2, g - 1 and g - 3
+  // Threads 2 t and 2 t + 1 (t < 156) hold word t of the last two phases (156
+  // words) of two lanes each, half a packet: x[i] and x[i + 156] of the
+  // recurrence are a thread's own registers, and x[i + 1], two phases old, is
+  // read from the words every thread puts into `nbr` as it makes them.  The
+  // last pair's x[i + 1] is the first pair's word of the phase just made: there
+  // in every first phase of a pair, made again from the first two pairs' words
+  // in the second, so one barrier serves two phases.
+  __shared__ ulonglong2 nbr[4][kDirThreads];  // [phase mod 4][thread]
+  const int h = tid & 1, ti = min(tid >> 1, kM - 1), right = min(tid + 2, kDirThreads - 1);
+  uint64_t x[2], c[2];  // words of phases g - 2 and g - 1
 #pragma unroll
-  for (int l = 0; l < kLanes; ++l) {
-    x[l] = o[l] = nbr[2][l][tid] = w0[l * wl + ti];
-    c[l] = nbr[3][l][tid] = w0[l * wl + kM + ti];
+  for (int l = 0; l < 2; ++l) {
+    x[l] = w0[(2 * h + l) * wl + ti];
+    c[l] = w0[(2 * h + l) * wl + kM + ti];
   }
+  nbr[2][tid] = make_ulonglong2(x[0], x[1]);
+  nbr[3][tid] = make_ulonglong2(c[0], c[1]);
   const int64_t obase = off + Q0;
   const int64_t oend = off + n;
+  // one phase: slot g (mod 4) of nbr, the second of a pair or the first
+  auto phase = [&](const int g, const bool second, uint64_t (&pk)[2]) {
+    ulonglong2 nb = nbr[g ^ 2][right];
+    if (tid >> 1 == kM - 1) {
+      if (!second) {
+        nb = nbr[(g + 3) & 3][h];
+      } else {
+        const ulonglong2 a0 = nbr[(g + 1) & 3][h], a1 = nbr[(g + 1) & 3][2 + h], a2 = nbr[g ^ 2][h];
+        nb = make_ulonglong2(twist1(a0.x, a1.x, a2.x), twist1(a0.y, a1.y, a2.y));
+      }
+    }
+    const uint64_t v0 = twist1(x[0], nb.x, c[0]), v1 = twist1(x[1], nb.y, c[1]);
+    nbr[g][tid] = make_ulonglong2(v0, v1);
+    pk[0] = temper(v0);
+    pk[1] = temper(v1);
+    x[0] = c[0];
+    x[1] = c[1];
+    c[0] = v0;
+    c[1] = v1;
+  };
+  int64_t base = pbeg;
+  if constexpr (kLightKind<MODE, KIND>) {
+    // the cheap transforms: two blocks at a time with every shared-memory
+    // offset and register's role fixed, short of the call's last packet
+    for (; base + 2 * kN < pend; base += 2 * kN) {
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        if ((g & 1) == 0) __syncthreads();
+        uint64_t pk[2];
+        phase(g, g & 1, pk);
+        emit_half<MODE, KIND, true>(pk, h, base + (tid >> 1) + g * kM, tid < 2 * kM, p, d, obase, oend, st, gs);
+      }
+    }
+  }
   int slot = 0;  // the phase to make, mod 4
-  for (int64_t base = pbeg; base < pend; base += kN, slot ^= 2) {
+  for (; base < pend; base += kN, slot ^= 2) {
     __syncthreads();
     const int here = (int)min(pend - base, (int64_t)kN);
-    // the cheap transforms pay for the registers' change of roles: unrolled
-#pragma unroll(kLightKind<MODE, KIND> ? 2 : 1)
+#pragma unroll 1
     for (int ph = 0; ph < 2; ++ph) {
       if (ph * kM >= here) break;
-      const int g = slot + ph;
-      uint64_t nb[kLanes], pk[kLanes];
-#pragma unroll
-      for (int l = 0; l < kLanes; ++l) nb[l] = nbr[g ^ 2][l][min(tid + 1, 159)];
-      if (tid == kM - 1) {
-#pragma unroll
-        for (int l = 0; l < kLanes; ++l)
-          nb[l] = ph == 0 ? nbr[(g + 3) & 3][l][0]
-                          : twist1(nbr[(g + 1) & 3][l][0], nbr[(g + 1) & 3][l][1], nbr[g ^ 2][l][0]);
-      }
-#pragma unroll
-      for (int l = 0; l < kLanes; ++l) {
-        const uint64_t v = twist1(x[l], nb[l], c[l]);
-        nbr[g][l][tid] = v;
-        pk[l] = temper(v);
-        o[l] = x[l];
-        x[l] = c[l];
-        c[l] = v;
-      }
-      const int i = ph * kM + tid;
-      emit_packet<MODE, KIND>(pk, base + i, tid < kM && i < here, p, d, obase, oend, st, gs);
+      uint64_t pk[2];
+      phase(slot + ph, ph, pk);
+      const int i = ph * kM + (tid >> 1);
+      emit_half<MODE, KIND>(pk, h, base + i, tid < 2 * kM && i < here, p, d, obase, oend, st, gs);
     }
   }
 
   // --- end-of-call state: new lane windows and cache flags
   if (last) {
-    if (Np > 0) {
+    if (Np > 0 && tid < 2 * kM) {
       // the 312 words before packet pend: the end of phase g - 3, phase g - 2
-      // and the first rr of phase g - 1
+      // and the first rr of phase g - 1, each thread's own
       const int rr = (int)((pend - pbeg - 1) % kM) + 1;
-      if (tid < kM) {
+      const int g1 = (int)((pend - pbeg - 1) / kM) & 3;  // phase g - 1
+      const ulonglong2 o3 = nbr[(g1 + 2) & 3][tid];
 #pragma unroll
-        for (int l = 0; l < kLanes; ++l) {
-          if (tid >= rr) st->win[l][tid - rr] = o[l];
-          st->win[l][kM - rr + tid] = x[l];
-          if (tid < rr) st->win[l][kN - rr + tid] = c[l];
-        }
+      for (int l = 0; l < 2; ++l) {
+        uint64_t* win = st->win[2 * h + l];
+        if (ti >= rr) win[ti - rr] = l ? o3.y : o3.x;
+        win[kM - rr + ti] = x[l];
+        if (ti < rr) win[kN - rr + ti] = c[l];
       }
     }
     if (tid == 0) {
@@ -881,7 +869,7 @@ __global__ void __maxnreg__(64) k_direct(Plan p, DistParams d, const CallSnap* s
 }
 
 // The same transforms over words that k_words_* left in memory: one thread per
-// packet, grid (packets, engines).  Packets [wbase, wbase + wcount) of every
+// half packet, grid (packets, engines).  Packets [wbase, wbase + wcount) of every
 // engine's call are in memory; block 0 of an engine leaves the engine state.
 constexpr int kXfThreads = 256;
 template <int MODE, int KIND>
@@ -905,13 +893,15 @@ __global__ void __launch_bounds__(kXfThreads) k_xform(Plan p, DistParams d, cons
   const int64_t Np = (MODE == M_N32 || MODE == M_N64) ? 2 * ((r + 2 * OPP - 1) / (2 * OPP)) : (r + OPP - 1) / OPP;
   const int64_t obase = off + Q0, oend = off + n;
   const int64_t pend = min(p.wbase + p.wcount, Np);
-  const int64_t pidx = p.wbase + (int64_t)blockIdx.x * kXfThreads + tid;
+  const int64_t pidx = p.wbase + (int64_t)blockIdx.x * (kXfThreads / 2) + (tid >> 1);
+  const int h = tid & 1;
   const uint64_t* w = p.words + (size_t)k * kLanes * p.wstride;
   const bool valid = pidx < pend;
-  uint64_t pk[kLanes];
+  uint64_t pk[2];
 #pragma unroll
-  for (int l = 0; l < kLanes; ++l) pk[l] = valid ? temper(w[(size_t)l * p.wstride + kN + (pidx - p.wbase)]) : 0;
-  emit_packet<MODE, KIND>(pk, pidx, valid, p, d, obase, oend, st, gs);
+  for (int l = 0; l < 2; ++l)
+    pk[l] = valid ? temper(w[(size_t)(2 * h + l) * p.wstride + kN + (pidx - p.wbase)]) : 0;
+  emit_half<MODE, KIND>(pk, h, pidx, valid, p, d, obase, oend, st, gs);
   if (blockIdx.x != 0) return;
   if (p.wbase == 0 && tid < Q0) {  // outputs served from the cache
     const int i = tid;
@@ -944,10 +934,10 @@ __global__ void __launch_bounds__(kXfThreads) k_xform(Plan p, DistParams d, cons
 template <int MODE, int KIND>
 static cudaError_t run_direct(const Plan& p, const DistParams& d, const CallSnap* snap, cudaStream_t s) {
   if (p.words) {
-    const dim3 grid((unsigned)((p.wcount + kXfThreads - 1) / kXfThreads), (unsigned)p.K);
+    const dim3 grid((unsigned)((p.wcount + kXfThreads / 2 - 1) / (kXfThreads / 2)), (unsigned)p.K);
     k_xform<MODE, KIND><<<grid, kXfThreads, 0, s>>>(p, d, snap);
   } else {
-    k_direct<MODE, KIND><<<p.K * p.S, 160, 0, s>>>(p, d, snap);
+    k_direct<MODE, KIND><<<p.K * p.S, kDirThreads, 0, s>>>(p, d, snap);
   }
   return cudaGetLastError();
 }
