@@ -80,9 +80,9 @@ constexpr uint32_t kItemFirst = 1, kItemLast = 2;       // first / last item of 
 // byte offset 128 (the K-adjacent core matrix), stride byte offset 1024 (the
 // next 8-row group), version 1; the start address (>> 4) is added in.
 constexpr uint64_t kDescConst = ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46);
-// the same with another stride byte offset (8-row group pitch)
-__host__ __device__ constexpr uint64_t kDescConstW(uint32_t sbo) {
-  return ((uint64_t)(128 >> 4) << 16) | ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46);
+// the same with other pitches of the core matrices, along K and along rows
+__host__ __device__ constexpr uint64_t kDescConstW(uint32_t lbo, uint32_t sbo) {
+  return ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46);
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -709,6 +709,10 @@ __device__ __forceinline__ void commit1(uint64_t* bar) {
 }
 
 constexpr int kWishUThreads = 128;
+// Pitch of the K-adjacent core matrices (8 rows of 16 bytes).  In step 3 the
+// lanes of a warp write one row's consecutive k: at a pitch of 128 bytes eight
+// of them meet in a bank, at 144 none.
+constexpr uint32_t kWishCore = 144;
 
 // Wait for an MMA commit by polling mbarrier.test_wait (non-blocking) from
 // lane 0 of each warp; bounded like mbar_wait.
@@ -748,24 +752,36 @@ __device__ __forceinline__ bool wish_wait(uint64_t* bar, uint32_t parity, volati
 
 }  // namespace
 
+// DP: the dimension rounded up to 16, 32 or 64; FULL: d == DP, every offset a
+// constant.  Bound by instruction issue, then by the tensor pipe: the second
+// product makes 128 x 128 values of which the draws' diagonal blocks are kept.
+// 10^5 draws with their normals and chi-squared draws, us, dim 16 / 32 / 64: 256 /
+// 770 / 3 994 with run-time offsets (2 400 instructions per warp and tile at dim
+// 32), bank conflicts and two stages (three CTAs per SM at dim 32); 239 / 637 /
+// 3 461 without the conflicts and with one stage (four CTAs); 202 / 526 / 2 471 as
+// here.
+template <int DP, bool FULL>
 __global__ void __launch_bounds__(kWishUThreads)
     k_wishart_umma(const float* __restrict__ normals, const float* __restrict__ chis, const float* __restrict__ chol,
-                   float* __restrict__ out, int d, int dp, int64_t samples, int32_t* status) {
+                   float* __restrict__ out, int dim, int64_t samples, int32_t* status) {
+  constexpr int dp = DP;
+  const int d = FULL ? DP : dim;
   extern __shared__ __align__(1024) unsigned char wu_dyn[];
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)wu_dyn + 1023) & ~(uintptr_t)1023);
   float* Bhi = reinterpret_cast<float*>(base);  // L: dp rows x dp k
-  float* Blo = Bhi + dp * dp;
-  float* Xhi = Blo + dp * dp;  // A^T of the tile (128 rows x dp k), then S (stacked T)
-  float* Xlo = Xhi + 128 * dp;
-  float* stage0 = Xlo + 128 * dp;  // the tile's normals (G draws, contiguous in HBM), double buffered
+  constexpr uint32_t SBO = (uint32_t)(dp / 4) * kWishCore;  // bytes between 8-row groups
+  float* Blo = Bhi + dp * SBO / 32;
+  float* Xhi = Blo + dp * SBO / 32;  // A^T of the tile (128 rows x dp k), then S (stacked T)
+  float* Xlo = Xhi + 128 * SBO / 32;
+  float* stage = Xlo + 128 * SBO / 32;  // the tile's normals (G draws, contiguous in HBM)
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_abort;
   const int tid = threadIdx.x, warp = tid >> 5;
-  const int G = 128 / dp;
-  const uint32_t SBO = (uint32_t)dp * 32;  // bytes between 8-row groups: dp/4 core matrices of 128 bytes
+  constexpr int G = 128 / dp;
   auto koff = [&](int row, int k) -> uint32_t {
-    return ((uint32_t)(row >> 3) * SBO + (uint32_t)(k >> 2) * 128u + (uint32_t)(row & 7) * 16u + (uint32_t)(k & 3) * 4u) >> 2;
+    return ((uint32_t)(row >> 3) * SBO + (uint32_t)(k >> 2) * kWishCore + (uint32_t)(row & 7) * 16u +
+            (uint32_t)(k & 3) * 4u) >> 2;
   };
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
@@ -797,58 +813,64 @@ __global__ void __launch_bounds__(kWishUThreads)
   const int64_t nper = (int64_t)d * (d - 1) / 2;
   const int64_t ntiles = (samples + G - 1) / G;
   const uint32_t idesc1 = umma_idesc_tf32(128, dp), idesc2 = umma_idesc_tf32(128, 128);
-  const uint64_t dsc = kDescConstW(SBO);
+  const uint64_t dsc = kDescConstW(kWishCore, SBO);
   const uint64_t bh = dsc | (uint64_t)(smem_u32(Bhi) >> 4), bl = dsc | (uint64_t)(smem_u32(Blo) >> 4);
   const uint64_t xh = dsc | (uint64_t)(smem_u32(Xhi) >> 4), xl = dsc | (uint64_t)(smem_u32(Xlo) >> 4);
-  const int stage_len = (G * (int)nper + 3) & ~3;
-  float* stages[2] = {stage0, stage0 + stage_len};
-  // a tile's normals into a stage buffer with cp.async (4-byte copies: the
-  // tile's start need not be 16-byte aligned); lands while the previous tile
-  // is processed
-  auto prefetch = [&](int64_t t, float* dst) {
+  // a tile's normals into the stage with cp.async, from step 2 of the tile
+  // before on (its step 1 was the stage's last reader): 16-byte copies where
+  // every tile starts on a 16-byte boundary, 4-byte ones elsewhere
+  const bool wide = ((G * nper) & 3) == 0 && ((uintptr_t)normals & 15) == 0;
+  auto prefetch = [&](int64_t t) {
     if (t < ntiles) {
       const int64_t j0 = t * G, nd = (samples - j0 < G ? samples - j0 : G);
-      const int cnt = (int)(nd * nper);
+      const int cnt = (int)(nd * nper), n16 = wide ? cnt / 4 : 0;
       const float* src = normals + j0 * nper;
-      for (int q = tid; q < cnt; q += kWishUThreads)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst + q)), "l"(src + q) : "memory");
+      for (int q = tid; q < n16; q += kWishUThreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(stage + 4 * q)), "l"(src + 4 * q)
+                     : "memory");
+      for (int q = 4 * n16 + tid; q < cnt; q += kWishUThreads)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(stage + q)), "l"(src + q) : "memory");
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  prefetch(blockIdx.x, stages[0]);
-  int sb = 0;
+  auto chi_of = [&](int64_t t) {  // the diagonal's chi-squared draw of lane (g, i)
+    const int64_t j = t * G + g;
+    return (j < samples && i < d) ? chis[(int64_t)i * samples + j] : 0.0f;
+  };
+  prefetch(blockIdx.x);
+  float chi = chi_of(blockIdx.x);
   uint32_t phase = 0;
   for (int64_t tile = blockIdx.x; tile < ntiles && !s_abort; tile += gridDim.x) {
     const int64_t j = tile * G + g;
     const bool jok = j < samples;
-    const float diag = (jok && i < d) ? sqrtf(chis[(int64_t)i * samples + j]) : 0.0f;
-    // ---- 1. this tile's normals (prefetched), the next tile's on their way,
-    // then row (g, i) of the stacked A^T = column i of A_g, tf32 parts, into
-    // shared memory
+    const float diag = sqrtf(chi);
+    // ---- 1. row (g, i) of the stacked A^T = column i of A_g, tf32 parts, into
+    // shared memory, from this tile's normals (prefetched)
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    prefetch(tile + gridDim.x, stages[sb ^ 1]);
-    const float* stage = stages[sb];
-    sb ^= 1;
-    const int nb = g * (int)nper + i * (d - 1) - i * (i - 1) / 2;  // its normals start here in the stage
+    // its normals start at nb in the stage, k = i + 1 first
+    const int nb = g * (int)nper + i * (d - 1) - i * (i - 1) / 2;
+    const float* col = stage + nb - i - 1;
+    const int kend = jok && i < d ? d : 0;
+    const float dg = kend ? diag : 0.0f;
+    float* xh_row = Xhi + koff(tid, 0);
+    float* xl_row = Xlo + koff(tid, 0);
+#pragma unroll
     for (int k0 = 0; k0 < dp; k0 += 4) {
       float4 h, l;
       float v[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int k = k0 + q;
-        v[q] = 0.0f;
-        if (jok && i < d && k < d) {
-          if (k > i) v[q] = stage[nb + (k - i - 1)];
-          else if (k == i) v[q] = diag;
-        }
+        v[q] = k == i ? dg : 0.0f;
+        if (k > i && k < kend) v[q] = col[k];
       }
       split_tf32(v[0], h.x, l.x);
       split_tf32(v[1], h.y, l.y);
       split_tf32(v[2], h.z, l.z);
       split_tf32(v[3], h.w, l.w);
-      *reinterpret_cast<float4*>(Xhi + koff(tid, k0)) = h;
-      *reinterpret_cast<float4*>(Xlo + koff(tid, k0)) = l;
+      *reinterpret_cast<float4*>(xh_row + k0 / 4 * (kWishCore / 4)) = h;
+      *reinterpret_cast<float4*>(xl_row + k0 / 4 * (kWishCore / 4)) = l;
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -857,17 +879,22 @@ __global__ void __launch_bounds__(kWishUThreads)
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;");
       for (int ks = 0; ks < dp / 8; ++ks) {
-        const uint64_t o = 16u * (uint64_t)ks;
+        const uint64_t o = (uint64_t)(kWishCore / 8) * (uint64_t)ks;
         mma_tf32_ss(tmem, xl + o, bh + o, idesc1, ks > 0 ? 1u : 0u);
         mma_tf32_ss(tmem, xh + o, bl + o, idesc1, 1u);
         mma_tf32_ss(tmem, xh + o, bh + o, idesc1, 1u);
       }
       commit1(&bar);
     }
+    prefetch(tile + gridDim.x);
+    chi = chi_of(tile + gridDim.x);
     if (!wish_wait(&bar, phase, &s_abort, status)) break;
     phase ^= 1u;
     asm volatile("tcgen05.fence::after_thread_sync;");
     // ---- 3. S[(g, r)][i] = T_g[r][i], split, over A^T (consumed)
+    float* sh = Xhi + koff(g * dp, i);
+    float* sl = Xlo + koff(g * dp, i);
+#pragma unroll
     for (int c0 = 0; c0 < dp; c0 += 16) {
       uint32_t r[16];
       asm volatile(
@@ -880,9 +907,9 @@ __global__ void __launch_bounds__(kWishUThreads)
       for (int q = 0; q < 16; ++q) {
         float hf, lf;
         split_tf32(__uint_as_float(r[q]), hf, lf);
-        const uint32_t o = koff(g * dp + c0 + q, i);
-        Xhi[o] = hf;
-        Xlo[o] = lf;
+        const uint32_t o = koff(c0 + q, 0);
+        sh[o] = hf;
+        sl[o] = lf;
       }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -892,7 +919,7 @@ __global__ void __launch_bounds__(kWishUThreads)
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;");
       for (int ks = 0; ks < dp / 8; ++ks) {
-        const uint64_t o = 16u * (uint64_t)ks;
+        const uint64_t o = (uint64_t)(kWishCore / 8) * (uint64_t)ks;
         mma_tf32_ss(tmem, xl + o, xh + o, idesc2, ks > 0 ? 1u : 0u);
         mma_tf32_ss(tmem, xh + o, xl + o, idesc2, 1u);
         mma_tf32_ss(tmem, xh + o, xh + o, idesc2, 1u);
@@ -906,8 +933,11 @@ __global__ void __launch_bounds__(kWishUThreads)
     {
       const int r = i;
       const int c0 = dp >= 32 ? (32 * warp / dp) * dp : 32 * warp;  // the warp's first column (warp-uniform)
-      const int width = dp >= 32 ? dp : 32;
-      float* o = out + j * (int64_t)d * d;
+      constexpr int width = dp >= 32 ? dp : 32;
+      float* o = out + j * (int64_t)d * d + r;
+      const int first = dp >= 32 ? 0 : (g & 1) * dp;  // the lane's first column of those read
+      const bool store = jok && r < d;
+#pragma unroll
       for (int cc = 0; cc < width; cc += 16) {
         uint32_t v[16];
         asm volatile(
@@ -916,11 +946,13 @@ __global__ void __launch_bounds__(kWishUThreads)
               "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
             : "r"(tmem + lane_addr + (uint32_t)(c0 + cc)));
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (store && (dp >= 32 || first == cc)) {
+          const int s0 = dp >= 32 ? cc : 0;  // column within the draw's block
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          const int sc = c0 + cc + q - g * dp;  // column within the draw's block
-          if (jok && r < d && sc >= 0 && sc < d) o[(int64_t)sc * d + r] = __uint_as_float(v[q]);
+          for (int q = 0; q < 16; ++q)
+            if (FULL || s0 + q < d) o[(s0 + q) * d] = __uint_as_float(v[q]);
         }
+        __syncwarp();
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -944,28 +976,28 @@ bool wishart_umma_usable(int d, int dtype, int inverse) {
   return dtype == GR_F32 && !inverse && d >= 1 && d <= kWishUmmaMaxDim;
 }
 
-cudaError_t launch_wishart_umma(const float* normals, const float* chis, const float* chol, float* out, int d,
-                                int64_t samples, int32_t* status, cudaStream_t s) {
-  if (d < 1 || d > kWishUmmaMaxDim || samples <= 0) return samples == 0 ? cudaSuccess : cudaErrorInvalidValue;
-  int dp = 16;
-  while (dp < d) dp <<= 1;
-  const int G = 128 / dp;
+template <int DP, bool FULL>
+static cudaError_t run_wishart_umma(const float* normals, const float* chis, const float* chol, float* out, int d,
+                                    int64_t samples, int32_t* status, cudaStream_t s) {
+  constexpr int dp = DP, G = 128 / dp;
+  const auto kernel = k_wishart_umma<DP, FULL>;
   // 128 tensor-memory columns per CTA: four CTAs per SM; shared memory is
   // sized so that no more than four are resident (a fifth would wait in
   // tcgen05.alloc), fewer where a CTA needs more
   const size_t stage_len = ((size_t)G * d * (d - 1) / 2 + 3) & ~(size_t)3;
-  size_t smem = 1024 + (size_t)(2 * dp * dp + 2 * 128 * dp + 2 * stage_len) * sizeof(float);
+  const size_t sbo = (size_t)(dp / 4) * kWishCore;  // bytes of eight rows
+  size_t smem = 1024 + 2 * (size_t)(dp + 128) / 8 * sbo + stage_len * sizeof(float);
   if (smem < 52 * 1024) smem = 52 * 1024;
   int dev = 0, sms = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (smem + 4096 > (size_t)optin) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(k_wishart_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   // all of the SM's unified L1 / shared memory as shared memory, so that
   // several CTAs fit
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_wishart_umma, cudaFuncAttributePreferredSharedMemoryCarveout,
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                              (int)cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
   // resident CTAs per SM from the SM's shared memory (the occupancy API
@@ -975,7 +1007,7 @@ cudaError_t launch_wishart_umma(const float* normals, const float* chis, const f
   cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
   cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
   cudaFuncAttributes fa;
-  e = cudaFuncGetAttributes(&fa, k_wishart_umma);
+  e = cudaFuncGetAttributes(&fa, kernel);
   if (e != cudaSuccess) return e;
   const size_t per_cta = smem + fa.sharedSizeBytes + (size_t)reserved;
   int per = (int)((size_t)sm_smem / per_cta);
@@ -984,8 +1016,22 @@ cudaError_t launch_wishart_umma(const float* normals, const float* chis, const f
   const int64_t tiles = (samples + G - 1) / G;
   const int64_t cap = (int64_t)sms * per;
   const int64_t grid = tiles < cap ? tiles : cap;
-  k_wishart_umma<<<(unsigned)grid, kWishUThreads, smem, s>>>(normals, chis, chol, out, d, dp, samples, status);
+  kernel<<<(unsigned)grid, kWishUThreads, smem, s>>>(normals, chis, chol, out, d, samples, status);
   return cudaGetLastError();
+}
+
+cudaError_t launch_wishart_umma(const float* normals, const float* chis, const float* chol, float* out, int d,
+                                int64_t samples, int32_t* status, cudaStream_t s) {
+  if (d < 1 || d > kWishUmmaMaxDim || samples <= 0) return samples == 0 ? cudaSuccess : cudaErrorInvalidValue;
+#define GR_WU(DP)                                                                                                \
+  if (d <= DP)                                                                                                   \
+    return d == DP ? run_wishart_umma<DP, true>(normals, chis, chol, out, d, samples, status, s)                 \
+                   : run_wishart_umma<DP, false>(normals, chis, chol, out, d, samples, status, s);
+  GR_WU(16)
+  GR_WU(32)
+  GR_WU(64)
+#undef GR_WU
+  return cudaErrorInvalidValue;
 }
 
 int umma_padded_dim(int d) { return (d + 15) / 16 * 16; }
