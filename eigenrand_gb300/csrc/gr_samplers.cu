@@ -793,6 +793,16 @@ constexpr int kBetaRing = 1024;  // positions whose accept masks are kept (a pow
 // lanes and FIFO lanes, so a chase that fell behind catches up.
 // TY0 / TY1: the components' sampler types when known at compile time (the
 // kernel then carries only their code), else -1.
+// ONE: exactly one component is a rejection sampler.  The trial-by-trial chase
+// (125 ns a trial, one warp) then bounds the kernel, so the workers also resolve,
+// for every position and number of carried lanes, the visit that would start
+// there (how many trials, full or carried lanes after it): the chase is one
+// look-up per output, and the workers list the accepted lanes of the visits it
+// took.  GS masks: one thread per 64-bit word, its uniforms converted once for
+// the three trials they are in.  What bounds it now is instruction issue.
+// Beta(0.5, 2), 4096 x 4096 on 608 engines, us, float / double: 1 176 / 2 200 with
+// the trial-by-trial chase, 980 / 2 014 with look-ups, 806 / 1 873 with the masks
+// by word.
 // ===========================================================================
 namespace {
 
@@ -812,8 +822,16 @@ struct BcStep {
   int nrec, nf, fs[2], A[2], f[2];
 };
 
-template <int DT>
+template <int DT, bool ONE>
 __host__ __device__ constexpr size_t bc_smem_bytes() {
+  if (ONE)
+    return (size_t)3 * kLanes * kN * 8 +                                                 // raw windows
+           (size_t)2 * kBcRec * 8 +                                                      // outputs of a step
+           ((size_t)bc_lb<DT>() + (size_t)(kBcFull + kBcRec) * beta_lanes<DT>()) *       // lane buffer, full-
+               (DT == SD_F64 ? 8 : 4) +                                                  //   trial and positional values
+           (size_t)kBetaRing * beta_lanes<DT>() +                                        // visits per position
+           (size_t)kBcRec * 2 + (size_t)kBcFull * 2 + (size_t)bc_lb<DT>() * 2 +          // sources, full trials, tasks
+           (size_t)kBetaRing;                                                            // masks per position
   return (size_t)3 * kLanes * kN * 8 +                                                   // raw windows
          ((size_t)2 * bc_lb<DT>() + (size_t)(kBcFull + kBcRec) * beta_lanes<DT>()) *     // lane buffers, full-
              (DT == SD_F64 ? 8 : 4) +                                                    //   trial and positional values
@@ -825,7 +843,8 @@ __host__ __device__ constexpr size_t bc_smem_bytes() {
 
 }  // namespace
 
-template <int DT, int TY0, int TY1>  // DT: SD_F32 or SD_F64
+// DT: SD_F32 or SD_F64
+template <int DT, int TY0, int TY1, bool ONE>
 __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks) {
   constexpr int NT = kBcThreads;
   constexpr int kBcWork = NT - 32;
@@ -835,13 +854,16 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
   using V = typename std::conditional<DT == SD_F64, uint64_t, uint32_t>::type;
   extern __shared__ __align__(16) uint64_t bc_dyn[];
   uint64_t(*raw)[kLanes][kN] = reinterpret_cast<uint64_t(*)[kLanes][kN]>(bc_dyn);
-  V* lanebuf = reinterpret_cast<V*>(bc_dyn + 3 * kLanes * kN);          // [2][LB]
-  V* fullval = lanebuf + 2 * LB;                                         // [kBcFull][P]
+  // ONE: [1][LB] lanes, single-buffered sources and tasks, xrec and visits
+  uint64_t* xrec = bc_dyn + 3 * kLanes * kN;                             // [2][kBcRec]
+  V* lanebuf = reinterpret_cast<V*>(xrec + (ONE ? 2 * kBcRec : 0));      // [2][LB]
+  V* fullval = lanebuf + (ONE ? 1 : 2) * LB;                             // [kBcFull][P]
   V* posval = fullval + kBcFull * P;                                     // [kBcRec][P]
-  int16_t* rec = reinterpret_cast<int16_t*>(posval + kBcRec * P);        // [2][kBcRec][2]
-  int16_t* fpos = rec + 2 * kBcRec * 2;                                  // [2][kBcFull]
-  uint16_t* ptask = reinterpret_cast<uint16_t*>(fpos + 2 * kBcFull);     // [2][2][LB]
-  uint8_t* pmask = reinterpret_cast<uint8_t*>(ptask + 2 * 2 * LB);       // [2][kBetaRing]
+  uint8_t* visits = reinterpret_cast<uint8_t*>(posval + kBcRec * P);     // [kBetaRing][P]
+  int16_t* rec = reinterpret_cast<int16_t*>(visits + (ONE ? kBetaRing * P : 0));  // [2][kBcRec][2]
+  int16_t* fpos = rec + (ONE ? kBcRec : 2 * kBcRec * 2);                 // [2][kBcFull]
+  uint16_t* ptask = reinterpret_cast<uint16_t*>(fpos + (ONE ? 1 : 2) * kBcFull);  // [2][2][LB]
+  uint8_t* pmask = reinterpret_cast<uint8_t*>(ptask + (ONE ? 1 : 2 * 2) * LB);    // [2][kBetaRing]
   __shared__ BcStep s_step[2];
   __shared__ int s_done, s_err, s_fc[2];
   __shared__ int64_t s_end;
@@ -863,13 +885,15 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
   // component whose positional values are computed with them
   const int bc = type0 >= 2 ? 0 : (type1 >= 2 ? 1 : -1);
   const int ob = bc == 0 ? 1 : (bc == 1 ? 0 : 1);
+  const int rc = ONE ? bc : 0;  // ONE: the rejection component; its buffers are the only ones
+  const int Ur = rc == 0 ? U0 : U1, Uc = rc == 0 ? U1 : U0;
   load_window(raw[2], &st->win[0][0], kN);  // block -1; block b lives in window b mod 3
   // carried lanes of the two GammaGens (generator slots 1 and 2)
   if (tid < 2 * 8) {
     const int c = tid / 8, j = tid % 8;
     const GenSlot& g = gs->s[1 + c];
-    if (j < g.rest_cnt)
-      lanebuf[c * LB + j] = (V)(DT == SD_F64 ? ((uint64_t)g.rest[2 * j] | ((uint64_t)g.rest[2 * j + 1] << 32))
+    if (j < g.rest_cnt && (!ONE || c == rc))
+      lanebuf[(ONE ? 0 : c) * LB + j] = (V)(DT == SD_F64 ? ((uint64_t)g.rest[2 * j] | ((uint64_t)g.rest[2 * j + 1] << 32))
                                              : (uint64_t)g.rest[j]);
   }
   if (tid == 0) {
@@ -887,8 +911,8 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
     wb1 = (int)((B + 2) % 3);
     wb2 = (int)((B + 1) % 3);
   };
-  auto tword = [&](int64_t rel, int l) -> uint64_t {
-    int dd = (int)(rel - ring_new);
+  // word l of the packet at dd, relative to the newest block's first
+  auto tword = [&](int dd, int l) -> uint64_t {
     int w = wb0;
     if (dd < 0) {
       dd += kN;
@@ -901,24 +925,23 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
     if ((unsigned)dd >= (unsigned)kN) dd = 0;  // outside the ring: never read past the buffers
     return mt_temper(raw[w][l][dd]);
   };
-  auto word = [&](int64_t w) -> uint32_t {
-    const uint64_t v = tword(w >> 3, (int)((w & 7) >> 1));
-    return (w & 1) ? (uint32_t)(v >> 32) : (uint32_t)v;
+  auto word = [&](int dd, int j) -> uint32_t {
+    const uint64_t v = tword(dd, j >> 1);
+    return (j & 1) ? (uint32_t)(v >> 32) : (uint32_t)v;
   };
-  auto rval = [&](int64_t r) -> uint64_t { return tword(r >> 2, (int)(r & 3)); };
   // value of an accepted trial lane or a closed-form draw; double GS lanes
   // use the branch threshold in integer form
-  auto value = [&](int c, int64_t x, int j) -> uint64_t {
+  auto value = [&](int c, int x, int j) -> uint64_t {
     bool acc;
-    auto uf = [&](int q) { return ur_f(word((x + q) * 8 + j)); };
-    auto ud = [&](int q) { return rval((x + q) * 4 + j); };
+    auto uf = [&](int q) { return ur_f(word(x + q, j)); };
+    auto ud = [&](int q) { return tword(x + q, j); };
     if (c == 0) {
       if (DT == SD_F64 && type0 == 2)
-        return d2u(1.0 * gs_value_f64(rval(x * 4 + j), rval((x + 1) * 4 + j), bk.c[0].tpx, bk.c[0].d_inv));
+        return d2u(1.0 * gs_value_f64(tword(x, j), tword(x + 1, j), bk.c[0].tpx, bk.c[0].d_inv));
       return beta_comp_u<DT, false>(bk.c[0], type0, uf, ud, acc);
     }
     if (DT == SD_F64 && type1 == 2)
-      return d2u(1.0 * gs_value_f64(rval(x * 4 + j), rval((x + 1) * 4 + j), bk.c[1].tpx, bk.c[1].d_inv));
+      return d2u(1.0 * gs_value_f64(tword(x, j), tword(x + 1, j), bk.c[1].tpx, bk.c[1].d_inv));
     return beta_comp_u<DT, false>(bk.c[1], type1, uf, ud, acc);
   };
   // The GS + integral-alpha pairs: the value of either component is one log
@@ -927,17 +950,17 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
   // lane of a warp shares the log whichever component it computes.
   constexpr bool kFused = (TY0 == 2 && TY1 == 1) || (TY0 == 1 && TY1 == 2);
   constexpr int gc = TY0 == 2 ? 0 : 1;  // the GS component of a fused pair
-  auto value_task = [&](int c, int64_t x, int j) -> uint64_t {
+  auto value_task = [&](int c, int x, int j) -> uint64_t {
     if (!kFused) return value(c, x, j);
     const BetaComp& g = c == 0 ? bk.c[0] : bk.c[1];
     const bool gsv = c == gc;
     if (DT == SD_F64) {
-      const uint64_t b0 = rval(x * 4 + j), b1 = rval((x + 1) * 4 + j);
+      const uint64_t b0 = tword(x, j), b1 = tword(x + 1, j);
       double arg = ur_nz_int(b1);
       if (!gsv) {
         double y = ur_nz_int(b0);
         y = y * arg;
-        for (int q = 2; q < g.U; ++q) y = y * ur_nz_int(rval((x + q) * 4 + j));
+        for (int q = 2; q < g.U; ++q) y = y * ur_nz_int(tword(x + q, j));
         arg = y;
       }
       const double l = log_(arg);
@@ -945,12 +968,12 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
       return d2u(1.0 * (((b0 & 0xfffffffffffffull) < g.tpx) ? exp_(g.d_inv * l) : 1.0 - l));
     } else {
       constexpr float e = 1.1920928955078125e-07f / 8;
-      const float u0 = ur_f(word(x * 8 + j)), u1 = ur_f(word((x + 1) * 8 + j));
+      const float u0 = ur_f(word(x, j)), u1 = ur_f(word(x + 1, j));
       float arg = u1 + e;
       if (!gsv) {
         float y = u0 + e;
         y = y * arg;
-        for (int q = 2; q < g.U; ++q) y = y * (ur_f(word((x + q) * 8 + j)) + e);
+        for (int q = 2; q < g.U; ++q) y = y * (ur_f(word(x + q, j)) + e);
         arg = y;
       }
       const float l = logf_(arg);
@@ -965,20 +988,85 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
   // lane) walks a run of consecutive positions and slides a window of the
   // lane's three tempered words along it (one word fetched per position);
   // a ballot per step gives the masks of the warp's 32 / P runs.
-  auto masks = [&](int64_t from, int64_t to, int t, int T) {
-    if (nrej == 0 || to <= from) return;
+  auto masks = [&](int64_t first, int64_t last, int t, int T) {
+    if (nrej == 0 || last <= first) return;
+    const int from = (int)(first - ring_new), to = (int)(last - ring_new), rm = (int)(ring_new & (kBetaRing - 1));
+    if (ONE && (TY0 == 2 || TY1 == 2 || (rc == 0 ? type0 : type1) == 2)) {
+      // GS trials: a thread per 64-bit word (two float lanes), whose uniforms
+      // it converts once for the three trials they are in
+      const BetaComp& g = bk.c[TY0 == 2 ? 0 : TY1 == 2 ? 1 : rc];
+      const int runs = (T >> 5) * 8;
+      const int L = (to - from + runs - 1) / runs;
+      const int wl = t & 3, x0 = from + ((t >> 5) * 8 + (t & 31) / 4) * L;
+      const uint64_t* next = x0 < 0 ? &raw[wb1][wl][x0 + kN] : &raw[wb0][wl][min(x0, kN - 1)];
+      int turn = x0 < 0 ? -x0 : kN;  // packets until the newest block begins
+      uint64_t w0 = 0, w1 = 0, w2 = 0;
+      float a0 = 0, a1 = 0, a2 = 0, b0 = 0, b1 = 0, b2 = 0;
+      for (int i = -2; i < L; ++i) {
+        const int x = x0 + i;
+        w0 = w1;
+        w1 = w2;
+        a0 = a1;
+        a1 = a2;
+        b0 = b1;
+        b1 = b2;
+        if (x < to) {
+          w2 = mt_temper(*next);
+          ++next;
+          if (--turn == 0) next = raw[wb0][wl];
+          if (DT == SD_F32) {
+            a2 = ur_f((uint32_t)w2);
+            b2 = ur_f((uint32_t)(w2 >> 32));
+          } else {
+            a2 = __uint2float_rn((uint32_t)((w2 & 0xfffffffffffffull) >> 20)) * 0x1p-32f;
+          }
+        }
+        if (i < 0) continue;
+        int fa = 0, fb = 0;
+        if (x < to) {
+          if (DT == SD_F32) {
+            constexpr float e = 1.1920928955078125e-07f / 8;
+            fa = gs_filter(a0, a1 + e, a2, g.f_px, g.f_inv, g.f_am1, g.f_band);
+            fb = gs_filter(b0, b1 + e, b2, g.f_px, g.f_inv, g.f_am1, g.f_band);
+          } else {
+            // gs_filter_f64's range tests
+            fa = fabsf(a0 - g.f_px) <= 0x1p-21f || a1 < 0x1.001p-12f
+                     ? -1 : gs_filter(a0, a1, a2, g.f_px, g.f_inv, g.f_am1, g.f_band);
+          }
+          auto exact = [&](int hi) -> int {
+            auto uf = [&](int q) { return hi ? (q == 0 ? b0 : (q == 1 ? b1 : b2)) : (q == 0 ? a0 : (q == 1 ? a1 : a2)); };
+            auto ud = [&](int q) { return q == 0 ? w0 : (q == 1 ? w1 : w2); };
+            bool acc;
+            beta_comp_u<DT, true>(g, 2, uf, ud, acc);
+            return acc ? 1 : 0;
+          };
+          if (fa < 0) fa = exact(0);
+          if (fb < 0) fb = exact(1);
+        }
+        __syncwarp();
+        const uint32_t ba = __ballot_sync(FULL, fa == 1) >> (t & 28) & 15u;
+        uint32_t m = ba;
+        if (DT == SD_F32) {
+          const uint32_t bb = __ballot_sync(FULL, fb == 1) >> (t & 28) & 15u;
+          const uint32_t ea = (ba | ba << 2) & 0x33u, eb = (bb | bb << 2) & 0x33u;
+          m = ((ea | ea << 1) & 0x55u) | ((eb | eb << 1) & 0x55u) << 1;
+        }
+        if (x < to && wl == 0) pmask[(rm + x) & (kBetaRing - 1)] = (uint8_t)m;
+      }
+      return;
+    }
     constexpr int G = 32 / P;
     const int runs = (T >> 5) * G;
-    const int L = ((int)(to - from) + runs - 1) / runs;
+    const int L = (to - from + runs - 1) / runs;
     const int r = (t >> 5) * G + (t & 31) / P, j = t & (P - 1);
     const int lw = DT == SD_F64 ? j : (j >> 1);  // the lane's 64-bit word
-    const int64_t x0 = from + (int64_t)r * L;
+    const int x0 = from + r * L;
     for (int ci = 0; ci < nrej; ++ci) {
       const int c = nrej == 2 ? ci : rej0;
       const int ty = c == 0 ? type0 : type1;
       uint64_t w0 = 0, w1 = tword(x0, lw), w2 = tword(x0 + 1, lw);
       for (int i = 0; i < L; ++i) {
-        const int64_t x = x0 + i;
+        const int x = x0 + i;
         const bool valid = x < to;
         w0 = w1;
         w1 = w2;
@@ -1009,16 +1097,50 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
         }
         const uint32_t bal = __ballot_sync(FULL, acc);
         if (valid && j == 0)
-          pmask[c * kBetaRing + (int)(x & (kBetaRing - 1))] =
+          pmask[(ONE ? 0 : c) * kBetaRing + ((rm + x) & (kBetaRing - 1))] =
               (uint8_t)((bal >> (threadIdx.x & 31 & ~(P - 1))) & ((1u << P) - 1));
       }
+    }
+  };
+  // ONE: the visits that start at positions [from, to): byte f of a position's
+  // entry is the visit with f carried lanes, 16 trials + 8 (ends with a full
+  // trial) + lanes carried after it; 0: more than 15 trials.  After n trials
+  // with S accepted lanes the visits with f >= P - S are over.
+  using E = typename std::conditional<P == 8, uint64_t, uint32_t>::type;
+  auto build = [&](int64_t from, int64_t to, int t, int T) {
+    constexpr E kOnes = (E)0x0101010101010101ull, kPat = (E)0x0706050403020100ull;
+    for (int64_t x = from + t; x < to; x += T) {
+      E w = 0, over = 0;
+      int S = 0;
+      for (int n = 1; n < 16; ++n) {
+        const int m = __popc(pmask[(int)((x + (int64_t)(n - 1) * Ur) & (kBetaRing - 1))]);
+        if (m == P) {
+          w |= ((kPat + (E)S * kOnes) | (E)(16 * n + 8) * kOnes) & ~over;
+          over = ~(E)0;
+        } else {
+          S += m;
+          const E now = (S >= P ? ~(E)0 : S > 0 ? ~(E)0 << (8 * (P - S)) : (E)0) & ~over;
+          const E after = S >= P ? kPat + (E)(S - P) * kOnes : S > 0 ? kPat << (8 * (P - S)) : (E)0;
+          w |= (after | (E)(16 * n) * kOnes) & now;
+          over |= now;
+        }
+        if (over == ~(E)0) break;
+      }
+      reinterpret_cast<E*>(visits)[(int)(x & (kBetaRing - 1))] = w;
     }
   };
   // block 0 and its masks (all threads)
   mt_block(raw[2], raw[0], [&](int, const uint64_t*) {});
   set_ring(0);
-  masks(0, kN - umax + 1, tid, NT);
+  // (ONE: a short call's, no more than it should need)
+  int64_t M = kN - umax + 1;  // positions with masks
+  if (ONE) M = min(M, 16 * Ur + 32 + (Uc + 3 * Ur) * min(Npk, (int64_t)kN));
+  masks(0, M, tid, NT);
   __syncthreads();
+  if (ONE) {
+    build(0, M - 16 * Ur, tid, NT);
+    __syncthreads();
+  }
 
   // chase state (warp 0, the same in every lane)
   int64_t cx = 0, cE = 0;
@@ -1031,7 +1153,6 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
   bool done = false;
   for (int64_t t = 0;; ++t) {
     const bool gen = !done && t + 1 < max_blocks;
-    const int64_t M = (t + 1) * kN - umax + 1;  // positions with masks
     if (warp == 0) {
       if (!done) {
         // ---- chase step t into buffer t mod 2
@@ -1045,7 +1166,46 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
         int nrec = 0, nf = 0, A[2] = {cf[0], cf[1]};
         const bool lag = cx < (t - 1) * kN;
         const int Mr = (int)(M - base), bm = (int)(base & (kBetaRing - 1));
-        if (!lag) {
+        if (ONE && !lag) {
+          // one look-up per output; every trial of a visit that starts below
+          // Mr - 16 Ur has its mask
+          const int pkr = (int)(pk_lim - base), left = (int)min(Npk - cE, (int64_t)kBcRec);
+          int xr = 0, f = cf[rc], At = f;
+          while (nrec < left) {
+            const int xt = rc == 0 ? xr : xr + Uc;
+            if (xt >= Mr - 16 * Ur || At + 2 * P > LB || nf >= kBcFull) break;
+            const uint32_t v = visits[((bm + xt) & (kBetaRing - 1)) * P + f];
+            int nt = v >> 4, full = (v >> 3) & 1, f2 = v & 7;
+            if (nt == 0) {  // a long visit: trial by trial
+              int acc = 0, cn = 0, y = xt;
+              bool end = false;
+              for (; y < Mr && nt < 127 && !end; y += Ur) {
+                cn = __popc(pmask[(bm + y) & (kBetaRing - 1)]);
+                ++nt;
+                if (cn == P) full = 1;
+                else acc += cn;
+                end = full || f + acc >= P;
+              }
+              if (!end) break;
+              f2 = full ? f + acc : f + acc - P;
+            }
+            const int xe = xr + Uc + nt * Ur;
+            if (xe > pkr) break;
+            if (lane == 0)
+              xrec[q * kBcRec + nrec] = (uint64_t)(uint32_t)(xt | At << 16) |
+                                        (uint64_t)(uint32_t)(nf | (nt | full << 7) << 8 | f << 16) << 32;
+            At += full ? f2 - f : f2 + P - f;
+            nf += full;
+            f = f2;
+            xr = xe;
+            ++nrec;
+          }
+          A[rc] = At;
+          cf[rc] = f;
+          cx = base + xr;
+          cE += nrec;
+        }
+        if (!ONE && !lag) {
           while (cE < Npk && nrec < kBcRec) {
             const int64_t xs = cx;
             const int cf0 = cf[0], cf1 = cf[1], A0 = A[0], A1 = A[1], nfs = nf;
@@ -1143,6 +1303,22 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
         const int16_t* rq = rec + q * kBcRec * 2;
         uint16_t* tq = ptask + q * 2 * LB;
         set_ring(t);
+        const int rbase = (int)(base - ring_new);
+        if (ONE) {
+          // the outputs' sources and the accepted partial lanes, in order
+          const int bm = (int)(base & (kBetaRing - 1)), fs = rc == 0 ? fs0 : fs1;
+          for (int i = tt; i < nrec; i += kBcWork) {
+            const uint64_t v = xrec[q * kBcRec + i];
+            const int x = (int)(v & 0xffff), Ai = (int)(v >> 16) & 0xffff, hi = (int)(v >> 32);
+            const int nt = (hi >> 8) & 0x7f, full = (hi >> 15) & 1;
+            int at = Ai - fs;
+            for (int y = x; y < x + (nt - full) * Ur; y += Ur)
+              for (uint32_t m = pmask[(bm + y) & (kBetaRing - 1)]; m; m &= m - 1) ptask[at++] = (uint16_t)((y << 3) | (__ffs(m) - 1));
+            if (full) fpos[hi & 0xff] = (int16_t)(x + (nt - 1) * Ur);
+            rec[i] = (int16_t)(full ? kBcFullTag + (hi & 0xff) : -(1 + Ai - (hi >> 16)));
+          }
+          asm volatile("bar.sync 1, %0;" ::"r"(kBcWork) : "memory");
+        }
         // one task list, one lane per thread: full trials of the buffered
         // component, the accepted partial-trial lanes, positional values of
         // the other component
@@ -1155,23 +1331,28 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
             const int i = u / P;
             j = u % P;
             c = bc;
-            rel = fpos[q * kBcFull + i];
+            rel = fpos[(ONE ? 0 : q * kBcFull) + i];
             dst = fullval + i * P + j;
           } else if (u < t1) {
             c = u < t0 + tp0 ? 0 : 1;
             const int qq = c == 0 ? u - t0 : u - t0 - tp0;
-            const int tk = tq[c * LB + qq];
+            const int tk = ONE ? ptask[qq] : tq[c * LB + qq];
             j = tk & 7;
             rel = tk >> 3;
-            dst = lanebuf + c * LB + (c == 0 ? fs0 : fs1) + qq;
+            dst = lanebuf + (ONE ? 0 : c * LB) + (c == 0 ? fs0 : fs1) + qq;
           } else {
             const int i = (u - t1) / P;
             j = (u - t1) % P;
             c = ob;
-            rel = rq[i * 2 + ob];
+            if (ONE) {
+              const uint64_t v = xrec[q * kBcRec + i];
+              rel = (int)(v & 0xffff) + (rc == 0 ? ((int)(v >> 40) & 0x7f) * Ur : -Uc);
+            } else {
+              rel = rq[i * 2 + ob];
+            }
             dst = (rel >= 0 && rel < kBcFullTag) ? posval + i * P + j : nullptr;
           }
-          if (dst) *dst = (V)value_task(c, base + rel, j);
+          if (dst) *dst = (V)value_task(c, rbase + rel, j);
         }
         asm volatile("bar.sync 1, %0;" ::"r"(kBcWork) : "memory");
         // output packets
@@ -1181,11 +1362,15 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
           uint64_t v[2];
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
-            const int src = rq[i * 2 + c];
-            if (src < 0) v[c] = (uint64_t)lanebuf[c * LB + (-src - 1) + j];
+            if (ONE && c == ob) {
+              v[c] = (uint64_t)posval[i * P + j];
+              continue;
+            }
+            const int src = ONE ? rec[i] : rq[i * 2 + c];
+            if (src < 0) v[c] = (uint64_t)lanebuf[(ONE ? 0 : c * LB) + (-src - 1) + j];
             else if (src >= kBcFullTag) v[c] = (uint64_t)fullval[(src - kBcFullTag) * P + j];
             else if (c == ob) v[c] = (uint64_t)posval[i * P + j];
-            else v[c] = value(c, base + src, j);  // both components closed form
+            else v[c] = value(c, rbase + src, j);  // both components closed form
           }
           if (DT == SD_F32) {
             const float p1 = u2f((uint32_t)v[0]), p2 = u2f((uint32_t)v[1]);
@@ -1201,9 +1386,10 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
         V carry = 0;
         const int cc = tt / 8, cj = tt % 8;
         const bool mover = tt < 16 && cj < S.f[cc];
-        if (mover) carry = lanebuf[cc * LB + S.A[cc] - S.f[cc] + cj];
+        V* lb = lanebuf + (ONE ? 0 : cc * LB);
+        if (mover) carry = lb[S.A[cc] - S.f[cc] + cj];
         asm volatile("bar.sync 1, %0;" ::"r"(kBcWork) : "memory");
-        if (mover) lanebuf[cc * LB + cj] = carry;
+        if (mover) lb[cj] = carry;
       }
       if (gen) {
         // ---- block t + 1 and its masks.  Word i < 156 of the new block needs
@@ -1224,10 +1410,16 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
         }
         asm volatile("bar.sync 1, %0;" ::"r"(kBcWork) : "memory");
         set_ring(t + 1);
-        masks(M, M + kN, tt, kBcWork);
+        const int64_t M1 = (t + 2) * kN - umax + 1;
+        masks(M, M1, tt, kBcWork);
+        if (ONE) {
+          asm volatile("bar.sync 1, %0;" ::"r"(kBcWork) : "memory");
+          build(M - 16 * Ur, M1 - 16 * Ur, tt, kBcWork);
+        }
       }
     }
     __syncthreads();
+    if (gen) M = (t + 2) * kN - umax + 1;
     if (done || s_err) break;
     done = s_done != 0;
     if (gen) B = t + 1;
@@ -1267,7 +1459,7 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
   if (tid < 2 * 8) {
     const int c = tid / 8, j = tid % 8;
     GenSlot& g = gs->s[1 + c];
-    const uint64_t v = j < s_fc[c] ? (uint64_t)lanebuf[c * LB + j] : 0;
+    const uint64_t v = j < s_fc[c] && (!ONE || c == rc) ? (uint64_t)lanebuf[(ONE ? 0 : c) * LB + j] : 0;
     if (DT == SD_F64) {
       g.rest[2 * j] = (uint32_t)v;
       g.rest[2 * j + 1] = (uint32_t)(v >> 32);
@@ -1295,22 +1487,23 @@ static cudaError_t run_beta(const Plan& p, const DistParams& d, int64_t max_bloc
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  constexpr size_t smem = bc_smem_bytes<DT>();
+  constexpr size_t smem = bc_smem_bytes<DT, false>(), smem1 = bc_smem_bytes<DT, true>();
   if (!attr[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(k_beta<DT, -1, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_beta<DT, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_beta<DT, 1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_beta<DT, -1, -1, false>, kAttr, (int)smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_beta<DT, -1, -1, true>, kAttr, (int)smem1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_beta<DT, 2, 1, true>, kAttr, (int)smem1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_beta<DT, 1, 2, true>, kAttr, (int)smem1);
     if (e != cudaSuccess) return e;
     attr[dev] = true;
   }
   // the GS + integral-alpha pairs (beta(a < 1, integer b) and the mirror)
   // have kernels of their own
   const int t0 = bk.c[0].type, t1 = bk.c[1].type;
-  if (t0 == 2 && t1 == 1) k_beta<DT, 2, 1><<<p.K, kBcThreads, smem, s>>>(p, bk, max_blocks);
-  else if (t0 == 1 && t1 == 2) k_beta<DT, 1, 2><<<p.K, kBcThreads, smem, s>>>(p, bk, max_blocks);
-  else k_beta<DT, -1, -1><<<p.K, kBcThreads, smem, s>>>(p, bk, max_blocks);
+  if (t0 == 2 && t1 == 1) k_beta<DT, 2, 1, true><<<p.K, kBcThreads, smem1, s>>>(p, bk, max_blocks);
+  else if (t0 == 1 && t1 == 2) k_beta<DT, 1, 2, true><<<p.K, kBcThreads, smem1, s>>>(p, bk, max_blocks);
+  else if ((t0 >= 2) != (t1 >= 2)) k_beta<DT, -1, -1, true><<<p.K, kBcThreads, smem1, s>>>(p, bk, max_blocks);
+  else k_beta<DT, -1, -1, false><<<p.K, kBcThreads, smem, s>>>(p, bk, max_blocks);
   return cudaGetLastError();
 }
 
