@@ -117,11 +117,14 @@ cudaError_t preload_raw_stream_kernels();
 // packet aligned.  Returns cudaErrorNotSupported for other kinds.
 cudaError_t launch_direct(const Plan& p, const DistParams& d, const CallSnap* snap, cudaStream_t s);
 
-// Multi-packet fixed units (gr_samplers.cu): U packets (or half packets) per
+// Multi-packet fixed units: U packets (or half packets) per
 // unit of P outputs.  With words in memory (p.words): units [u0, u0 + cnt) of
-// every engine; without, the whole call, one CTA per engine.
+// every engine (gr_samplers.cu); without, the whole call, one CTA per engine
+// (launch_units, gr_trials.cu).
 cudaError_t launch_staged(const Plan& p, const DistParams& d, const CallSnap* snap, int U, int64_t u0, int64_t cnt,
                           cudaStream_t s);
+
+cudaError_t launch_units(const Plan& p, const DistParams& d, int U, cudaStream_t s);
 
 // Rejection samplers resolved with CompressMask semantics (gr_trials.cu); one
 // CTA per stream.  rk: 0 gamma alpha<1 (GS), 1 gamma tan proposal,

@@ -1,12 +1,12 @@
-// Samplers whose draws per output span several packets.
+// Samplers whose draws per output span several packets, over words in memory
+// (k_staged_words; on many engines k_units of gr_trials.cu) or drawn with a
+// scalar engine (k_sx_*), and the samplers that walk their stream: Poisson,
+// Beta, UniformInt, NegativeBinomial.
 //
-// k_staged: a unit of P outputs consumes a fixed run of U packets (or U half
-// packets for the int32 kinds), e.g. GammaGen with integer alpha < 20
-// multiplies alpha uniforms per output (EigenRand/Dists/NormalExp.h:577-587),
-// BinomialGen with trials < 25 compares `trials` uniforms
-// (Discrete.h:1000-1009).  The CTA keeps the tempered packets of the last two
-// blocks in shared memory; a unit is evaluated as soon as its last packet
-// exists.  Fixed consumption means jump-ahead segments still apply.
+// A unit of P outputs of the fixed-unit kinds consumes a run of U packets (or U
+// half packets for the int32 kinds): GammaGen with integer alpha < 20 multiplies
+// alpha uniforms per output (EigenRand/Dists/NormalExp.h:577-587), BinomialGen
+// with trials < 25 compares `trials` uniforms (Discrete.h:1000-1009).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -23,162 +23,6 @@
 #include "gr_samplers.cuh"
 
 namespace gr {
-
-// Lane j of unit u (the call's words: word / rword) to output element o.
-template <int KIND, int DT, class WF, class RF>
-__device__ __forceinline__ void staged_value(const Plan& p, const DistParams& d, int U, int64_t u, int j, int64_t o,
-                                             WF&& word, RF&& rword) {
-  const int64_t wpu = (DT == SD_I32H) ? 4 * (int64_t)U : 8 * (int64_t)U;  // u32 words per unit
-  if (DT == SD_F32) {
-    const int64_t w0 = u * wpu + j;  // full kinds: c0w == 0
-    if (KIND == GR_GAMMA || KIND == GR_CHI_SQUARED) {
-      float y = ur_f(word(w0)) + 1.1920928955078125e-07f / 8;
-      for (int t = 1; t < U; ++t) y = y * (ur_f(word(w0 + 8 * t)) + 1.1920928955078125e-07f / 8);
-      reinterpret_cast<float*>(p.out)[o] = -(d.fb * logf_(y));
-    } else if (KIND == GR_STUDENT_T) {
-      const float u1 = 1.0f - ur_f(word(w0));
-      const float u2 = ur_f(word(w0 + 8));
-      // StudentTVGen (NormalExp.h:327-342): n of the element, -2 / n per lane
-      const float nn = (d.flags & kParamVecA) ? __ldg(static_cast<const float*>(d.vparam) + o) : d.fa;
-      const float ex = (d.flags & kParamVecA) ? -2.0f / nn : d.fc;
-      const float radius = sqrtf(nn * (expf_(logf_(u1) * ex) - 1.0f));
-      float sn, cs;
-      sincosf_((float)(2 * 3.1415926535897932) * u2, sn, cs);
-      reinterpret_cast<float*>(p.out)[o] = radius * sn;
-    }
-  } else if (DT == SD_F64) {
-    const int64_t r0 = u * (int64_t)U * 4 + j;
-    if (KIND == GR_GAMMA || KIND == GR_CHI_SQUARED) {
-      double y = ur_nz_int(rword(r0));
-      for (int t = 1; t < U; ++t) y = y * ur_nz_int(rword(r0 + 4 * t));
-      const double l = log_(y);
-      reinterpret_cast<double*>(p.out)[o] = (d.flags & kParamUnitScale) ? -l : -(d.db * l);
-    } else if (KIND == GR_STUDENT_T) {
-      const double u1 = one_minus_ur_d(rword(r0));
-      const double nn = (d.flags & kParamVecA) ? __ldg(static_cast<const double*>(d.vparam) + o) : d.da;
-      const double ex = (d.flags & kParamVecA) ? -2.0 / nn : d.dc;
-      const double radius = sqrt_d(nn * (exp_(log_(u1) * ex) - 1.0));
-      double sn, cs;
-      sincos_2pi_u(rword(r0 + 4), sn, cs);
-      reinterpret_cast<double*>(p.out)[o] = radius * sn;
-    }
-  } else {  // int32 over half packets
-    const int64_t w0 = u * wpu + j;
-    if (KIND == GR_BINOMIAL) {
-      int32_t res = d.ia;  // trials
-      for (int t = 0; t < U; ++t) res += (d.fa <= ur_f(word(w0 + 4 * t))) ? -1 : 0;
-      reinterpret_cast<int32_t*>(p.out)[o] = res;
-    }
-  }
-}
-
-template <int KIND, int DT>
-__global__ void __launch_bounds__(160)
-    k_staged(Plan p, DistParams d, int U) {
-  __shared__ uint64_t raw[2][kLanes][kN];
-  __shared__ uint64_t tp[2][kN][kLanes];
-  const int k = blockIdx.x;
-  const int tid = threadIdx.x;
-  EngState* st = p.eng + k;
-  constexpr int P = DT == SD_F32 ? 8 : 4;
-
-  const int64_t g0 = (int64_t)k * p.gran_per_k + min((int64_t)k, p.gran_rem);
-  const int64_t ng = p.gran_per_k + ((int64_t)k < p.gran_rem ? 1 : 0);
-  const int64_t off = g0 * p.gran, n = ng * p.gran;
-  if (n == 0) return;
-
-  // half-packet kinds start with the engine's cached half, if any
-  int c0w = 0;
-  uint32_t cw[4] = {0, 0, 0, 0};
-  if (DT == SD_I32H) {
-    if (st->half_valid) {
-      c0w = 4;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) cw[q] = st->half_cache[q];
-    }
-  }
-  const int64_t wpu = (DT == SD_I32H) ? 4 * (int64_t)U : 8 * (int64_t)U;  // u32 words per unit
-  const int64_t u_end = n / P;
-  // last packet holding a word of unit u_end-1
-  const int64_t w_last = u_end * wpu - 1 - c0w;
-  const int64_t p_last = w_last < 0 ? -1 : w_last / 8;
-  const int64_t np_seg = p_last + 1;
-  load_window(raw[0], &st->win[0][0], kN);
-  __syncthreads();
-
-  int64_t ring_new = 0;  // newest ring block's first packet (ring_packet)
-  int ring_slot = 0;
-  auto word = [&](int64_t wq) -> uint32_t {  // cache-inclusive u32 word
-    if (wq < c0w) return cw[wq];
-    const int64_t w = wq - c0w;
-    const uint64_t v = ring_packet(tp, w >> 3, ring_new, ring_slot)[(w & 7) >> 1];
-    return (w & 1) ? (uint32_t)(v >> 32) : (uint32_t)v;
-  };
-  auto rword = [&](int64_t r) -> uint64_t {  // u64 lane value r of the packet stream (full kinds)
-    return ring_packet(tp, r >> 2, ring_new, ring_slot)[r & 3];
-  };
-
-  int64_t u_next = 0;
-  int cur = 0;
-  int64_t nb = 0;
-  for (int64_t base = 0; base < np_seg || (np_seg <= 0 && base == 0); base += kN, ++nb) {
-    if (np_seg > 0) {
-      uint64_t(*old)[kN] = raw[cur];
-      uint64_t(*nw)[kN] = raw[cur ^ 1];
-      const int slot = (int)(nb & 1);
-      mt_block(old, nw, [&](int i, const uint64_t* pk) {
-#pragma unroll
-        for (int l = 0; l < kLanes; ++l) tp[slot][i][l] = pk[l];
-      });
-      cur ^= 1; ring_new = nb * kN; ring_slot = slot;
-    }
-    // units whose last packet is now available
-    const int64_t avail = base + kN;  // packets [.., avail) exist
-    int64_t u_ready = u_end;
-    {
-      // largest u with ((u+1)*wpu - 1 - c0w)/8 < avail
-      const int64_t lim = avail * 8 + c0w;  // words (cache-inclusive) available
-      const int64_t by_words = lim / wpu;
-      if (by_words < u_ready) u_ready = by_words;
-    }
-    const int64_t cnt = (u_ready - u_next) * P;
-    for (int64_t e = tid; e < cnt; e += blockDim.x) {
-      const int64_t u = u_next + e / P;
-      const int j = (int)(e % P);
-      const int64_t o = off + u * P + j;
-      staged_value<KIND, DT>(p, d, U, u, j, o, word, rword);
-    }
-    u_next = u_ready;
-    __syncthreads();
-    if (u_next >= u_end) break;
-  }
-
-  // the loop stops right after the block holding p_last: ceil(np_seg/312)
-  // blocks were generated and raw[cur] is the last of them
-  if (np_seg > 0) {
-    const int64_t nblk = (np_seg + kN - 1) / kN;
-    const int rr2 = (int)(np_seg - (nblk - 1) * kN);  // in [1, 312]
-    store_window(st, raw[cur], raw[cur ^ 1], rr2);
-  }
-  if (tid == 0) {
-    if (DT == SD_I32H) {
-      // the last unit ends mid-packet: its upper half stays cached
-      const bool half_left = (w_last >= 0) && ((w_last & 7) == 3);
-      if (half_left) {
-        const int64_t rel = p_last;
-        const int slot = (int)((rel / kN) & 1);
-        st->half_cache[0] = (uint32_t)tp[slot][rel % kN][2];
-        st->half_cache[1] = (uint32_t)(tp[slot][rel % kN][2] >> 32);
-        st->half_cache[2] = (uint32_t)tp[slot][rel % kN][3];
-        st->half_cache[3] = (uint32_t)(tp[slot][rel % kN][3] >> 32);
-        st->half_valid = 1;
-      } else {
-        st->half_valid = 0;
-      }
-    }
-    st->consumed += (uint64_t)(p_last + 1);
-  }
-}
 
 // Units [u0, u0 + cnt) of every engine over words in memory, one thread per
 // output lane; block 0 of an engine leaves its state.
@@ -231,7 +75,7 @@ __global__ void __launch_bounds__(256) k_staged_words(Plan p, DistParams d, cons
 // reads U uniform packets from pre-drawn 64-bit words, float packets as
 // rawbits_34 of three draws (c.lo, c.hi, b.lo, top bytes, b.hi, a.lo, a.hi,
 // top bytes; a the first draw), double packets as four draws in order; the
-// same per-lane arithmetic as k_staged.  One thread per output lane.
+// same per-lane arithmetic as staged_value.  One thread per output lane.
 template <int KIND, int DT>
 __global__ void __launch_bounds__(256) k_sx_staged(const uint64_t* w, void* out, int64_t npk, DistParams d, int U) {
   constexpr int P = DT == SD_F32 ? 8 : 4;
@@ -308,7 +152,7 @@ static cudaError_t run_staged(const Plan& p, const DistParams& d, const CallSnap
     k_staged_words<KIND, DT>
         <<<dim3((unsigned)((cnt * P + 255) / 256), (unsigned)p.K), 256, 0, s>>>(p, d, snap, U, u0, cnt);
   } else {
-    k_staged<KIND, DT><<<p.K, 160, 0, s>>>(p, d, U);
+    return launch_units(p, d, U, s);
   }
   return cudaGetLastError();
 }

@@ -408,4 +408,54 @@ __device__ __forceinline__ uint64_t beta_comp_u(const BetaComp g, const int type
   }
 }
 
+// Lane j of unit u (the call's words: word / rword) to output element o.
+template <int KIND, int DT, class WF, class RF>
+__device__ __forceinline__ void staged_value(const Plan& p, const DistParams& d, int U, int64_t u, int j, int64_t o,
+                                             WF&& word, RF&& rword) {
+  const int64_t wpu = (DT == SD_I32H) ? 4 * (int64_t)U : 8 * (int64_t)U;  // u32 words per unit
+  if (DT == SD_F32) {
+    const int64_t w0 = u * wpu + j;  // full kinds: c0w == 0
+    if (KIND == GR_GAMMA || KIND == GR_CHI_SQUARED) {
+      float y = ur_f(word(w0)) + 1.1920928955078125e-07f / 8;
+      for (int t = 1; t < U; ++t) y = y * (ur_f(word(w0 + 8 * t)) + 1.1920928955078125e-07f / 8);
+      reinterpret_cast<float*>(p.out)[o] = -(d.fb * logf_(y));
+    } else if (KIND == GR_STUDENT_T) {
+      const float u1 = 1.0f - ur_f(word(w0));
+      const float u2 = ur_f(word(w0 + 8));
+      // StudentTVGen (NormalExp.h:327-342): n of the element, -2 / n per lane
+      const float nn = (d.flags & kParamVecA) ? __ldg(static_cast<const float*>(d.vparam) + o) : d.fa;
+      const float ex = (d.flags & kParamVecA) ? -2.0f / nn : d.fc;
+      const float radius = sqrtf(nn * (expf_(logf_(u1) * ex) - 1.0f));
+      float sn, cs;
+      sincosf_((float)(2 * 3.1415926535897932) * u2, sn, cs);
+      reinterpret_cast<float*>(p.out)[o] = radius * sn;
+    }
+  } else if (DT == SD_F64) {
+    const int64_t r0 = u * (int64_t)U * 4 + j;
+    if (KIND == GR_GAMMA || KIND == GR_CHI_SQUARED) {
+      double y = ur_nz_int(rword(r0));
+      for (int t = 1; t < U; ++t) y = y * ur_nz_int(rword(r0 + 4 * t));
+      const double l = log_(y);
+      reinterpret_cast<double*>(p.out)[o] = (d.flags & kParamUnitScale) ? -l : -(d.db * l);
+    } else if (KIND == GR_STUDENT_T) {
+      const double u1 = one_minus_ur_d(rword(r0));
+      const double nn = (d.flags & kParamVecA) ? __ldg(static_cast<const double*>(d.vparam) + o) : d.da;
+      const double ex = (d.flags & kParamVecA) ? -2.0 / nn : d.dc;
+      const double radius = sqrt_d(nn * (exp_(log_(u1) * ex) - 1.0));
+      double sn, cs;
+      sincos_2pi_u(rword(r0 + 4), sn, cs);
+      reinterpret_cast<double*>(p.out)[o] = radius * sn;
+    }
+  } else {  // int32 over half packets
+    const int64_t w0 = u * wpu + j;
+    if (KIND == GR_BINOMIAL) {
+      int32_t res = d.ia;  // trials
+      // p <= F 2^-23 with the fraction's integer F (p 2^23 is exact)
+      const int least = d.fa <= 1.0f ? (int)ceilf(d.fa * 8388608.0f) : 1 << 23;
+      for (int t = 0; t < U; ++t) res += (int)(word(w0 + 4 * t) & 0x7fffffu) >= least ? -1 : 0;
+      reinterpret_cast<int32_t*>(p.out)[o] = res;
+    }
+  }
+}
+
 }  // namespace gr

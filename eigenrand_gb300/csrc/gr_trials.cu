@@ -263,6 +263,30 @@ __device__ __forceinline__ bool draw_row(SM& sm, const DistParams& d, const int 
   return true;
 }
 
+// The engine's state after a call that ends inside the newest block (a trial or
+// unit is evaluated in the batch after the block that holds its last word).
+template <bool HALF>
+__device__ __forceinline__ void leave_engine(const EngSmem& sm, EngState* st, const TrialPos& ps) {
+  const int tid = threadIdx.x;
+  if (ps.nb > 0) {
+    const int cur = (int)(ps.nb & 1);
+    const int rr = kN - ps.av / 8;  // packets used of it; a half packet counts as used
+    for (int t = tid; t < kLanes * kN; t += kTrThreads) {
+      const int l = t / kN, i = t % kN;
+      st->win[l][i] = i < kN - rr ? sm.raw[cur ^ 1][l][rr + i] : sm.raw[cur][l][i - (kN - rr)];
+    }
+  }
+  if (tid == 0) {
+    if (HALF && ps.nb > 0) {
+      const bool half = (ps.av & 7) == 4;  // ends mid-packet: the upper half stays cached
+      if (half)
+        for (int q = 0; q < 4; ++q) st->half_cache[q] = sm.w[ps.sp + q];
+      st->half_valid = half ? 1 : 0;
+    }
+    st->consumed += (uint64_t)(ps.nb * kN - ps.av / 8);
+  }
+}
+
 // The row's kind picks a copy of the loop of its own: with the kind tested per
 // trial in one loop 64 rows of 10^6 gamma(0.5) floats on 608 engines took 1 660
 // us instead of 1 580, and 2 10^5 parameter sets 12.0 ms instead of 11.2.
@@ -333,26 +357,81 @@ __global__ void __launch_bounds__(kTrThreads, 4) k_trials(Plan p, TrialRow args,
     }
   }
 
-  // ---- engine state: the call ends inside the newest block (a trial is
-  // evaluated in the batch after the block that holds its last word)
   if (tid == 0 && !ok) atomicOr(&st->status, (int)GR_DEV_REJECT_LIMIT);
-  if (ps.nb > 0) {
-    const int cur = (int)(ps.nb & 1);
-    const int rr = kN - ps.av / 8;  // packets used of it; a half packet counts as used
-    for (int t = tid; t < kLanes * kN; t += kTrThreads) {
-      const int l = t / kN, i = t % kN;
-      st->win[l][i] = i < kN - rr ? sm.raw[cur ^ 1][l][rr + i] : sm.raw[cur][l][i - (kN - rr)];
+  leave_engine<kHalf>(sm, st, ps);
+}
+
+// ---------------------------------------------------------------- fixed units
+// Kinds whose unit of P outputs takes U packets (half packets for the int32
+// kind): the units whose words exist, a thread per output.  Bound by instruction
+// issue.  4096 x 4096 on 608 engines, us, with packets of 64-bit words found by
+// 64-bit position / here: gamma(5) f32 213 / 154, f64 526 / 471, binomial(20) 842 /
+// 474.
+template <int KIND, int DT>
+__global__ void __launch_bounds__(kTrThreads, 4) k_units(Plan p, DistParams d, int U) {
+  constexpr int P = DT == SD_F32 ? 8 : 4;
+  constexpr bool kHalf = DT == SD_I32H;
+  extern __shared__ __align__(16) uint8_t tr_dyn[];
+  EngSmem& sm = *reinterpret_cast<EngSmem*>(tr_dyn);
+  const int k = blockIdx.x, tid = threadIdx.x;
+  EngState* st = p.eng + k;
+  const int64_t g0 = (int64_t)k * p.gran_per_k + min((int64_t)k, p.gran_rem);
+  const int64_t ng = p.gran_per_k + ((int64_t)k < p.gran_rem ? 1 : 0);
+  const int64_t off = g0 * p.gran, n = ng * p.gran;
+  if (n == 0) return;
+  const int Wt = (kHalf ? 4 : 8) * U;
+  const int c0w = (kHalf && st->half_valid) ? 4 : 0;
+  for (int i = tid; i < kLanes * kN; i += kTrThreads) (&sm.raw[0][0][0])[i] = (&st->win[0][0])[i];
+  if (kHalf && tid < 4) sm.w[kTrRing - 4 + tid] = st->half_cache[tid];
+  __syncthreads();
+  TrialPos ps{c0w ? kTrRing - 4 : 0, c0w, 0};
+  int64_t left = n / P, o = off;
+  while (left > 0) {
+    while (ps.av < Wt) next_block(sm, ps);
+    const int B = (int)min((int64_t)(ps.av / Wt), left);
+    for (int e = tid; e < B * P; e += kTrThreads) {
+      const int t = e / P, j = e % P;
+      int a = ps.sp + t * Wt;
+      a -= a >= kTrRing ? kTrRing : 0;
+      auto word = [&](int64_t q) -> uint32_t {
+        int i = a + (int)q;
+        i -= i >= kTrRing ? kTrRing : 0;
+        return sm.w[i];
+      };
+      auto rword = [&](int64_t r) -> uint64_t {
+        int i = a + 2 * (int)r;
+        i -= i >= kTrRing ? kTrRing : 0;
+        return *reinterpret_cast<const uint64_t*>(&sm.w[i]);
+      };
+      staged_value<KIND, DT>(p, d, U, 0, j, o + e, word, rword);
     }
+    o += (int64_t)B * P;
+    left -= B;
+    ps.sp += B * Wt;
+    ps.sp -= ps.sp >= kTrRing ? kTrRing : 0;
+    ps.av -= B * Wt;
+    __syncthreads();
   }
-  if (tid == 0) {
-    if (kHalf && ps.nb > 0) {
-      const bool half = (ps.av & 7) == 4;  // ends mid-packet: the upper half stays cached
-      if (half)
-        for (int q = 0; q < 4; ++q) st->half_cache[q] = sm.w[ps.sp + q];
-      st->half_valid = half ? 1 : 0;
-    }
-    st->consumed += (uint64_t)(ps.nb * kN - ps.av / 8);
+  leave_engine<kHalf>(sm, st, ps);
+  // a call served from the cached half packet alone leaves none
+  if (kHalf && tid == 0 && ps.nb == 0 && c0w) st->half_valid = ps.av ? 1 : 0;
+}
+
+template <int KIND, int DT>
+cudaError_t run_units(const Plan& p, const DistParams& d, int U, cudaStream_t s) {
+  static bool attr[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (U < 1 || U > kTrRing / 2 / 8) return cudaErrorNotSupported;
+  if (!attr[dev]) {
+    cudaError_t e =
+        cudaFuncSetAttribute(k_units<KIND, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EngSmem));
+    if (e != cudaSuccess) return e;
+    attr[dev] = true;
   }
+  k_units<KIND, DT><<<p.K, kTrThreads, sizeof(EngSmem), s>>>(p, d, U);
+  return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------- parameter sets
@@ -468,6 +547,20 @@ cudaError_t launch_reject(const Plan& p, const DistParams& d, int rk, float per_
 #undef GR_RJ
   if (rk == RK_POISSON && dt == SD_I32H) return run_trials<SD_I32H, RK_POISSON>(p, row, nullptr, 1, 0, max_blocks, s);
   if (rk == RK_BINOMIAL && dt == SD_I32H) return run_trials<SD_I32H, RK_BINOMIAL>(p, row, nullptr, 1, 0, max_blocks, s);
+  return cudaErrorNotSupported;
+}
+
+cudaError_t launch_units(const Plan& p, const DistParams& d, int U, cudaStream_t s) {
+  const bool f32 = d.dtype == GR_F32, f64 = d.dtype == GR_F64;
+  if (d.kind == GR_GAMMA || d.kind == GR_CHI_SQUARED) {
+    if (f32) return run_units<GR_GAMMA, SD_F32>(p, d, U, s);
+    if (f64) return run_units<GR_GAMMA, SD_F64>(p, d, U, s);
+  }
+  if (d.kind == GR_STUDENT_T) {
+    if (f32) return run_units<GR_STUDENT_T, SD_F32>(p, d, U, s);
+    if (f64) return run_units<GR_STUDENT_T, SD_F64>(p, d, U, s);
+  }
+  if (d.kind == GR_BINOMIAL && d.dtype == GR_I32) return run_units<GR_BINOMIAL, SD_I32H>(p, d, U, s);
   return cudaErrorNotSupported;
 }
 
