@@ -52,9 +52,16 @@ def version():
     return _L.gr_version().decode()
 
 
+# A small call is bound by its host path, so that path stays short (32 x 32
+# floats, us a call: 20.9 with a Stream object, an empty and a transposed tensor,
+# a descriptor filled field by field and c_void_p objects; 7.4 as here).
+_CUDA = torch.device("cuda")
+
+
 def _stream_ptr(stream=None):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    if stream is not None:
+        return stream.cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 class Vmt19937_64:
@@ -140,11 +147,12 @@ class P8_mt19937_64(_ScalarEngine):
 def _empty(rows, cols, dtype, out):
     if out is not None:
         return out
-    return torch.empty((cols, rows), dtype=dtype, device="cuda").t()
+    # column-major, as Eigen's default
+    return torch.empty_strided((rows, cols), (1, rows if rows > 1 else 1), dtype=dtype, device=_CUDA)
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def raw_u64(urng, n, out=None, stream=None):
@@ -160,12 +168,7 @@ _DT = {torch.float32: F32, torch.float64: F64, torch.int32: I32}
 
 
 def _desc(kind, dtype, a=0.0, b=0.0, trials=0, weights=None):
-    d = _lib.DistDesc()
-    d.kind = KINDS[kind]
-    d.dtype = _DT[dtype]
-    d.a = float(a)
-    d.b = float(b)
-    d.trials = int(trials)
+    d = _lib.DistDesc(KINDS[kind], _DT[dtype], float(a), float(b), int(trials))
     keep = None
     if weights is not None:
         keep = (ctypes.c_double * len(weights))(*[float(w) for w in weights])
