@@ -239,20 +239,25 @@ cudaError_t launch_words(const EngState* st, const GenState* gen, int K, const W
 
 // ---------------------------------------------------------------- jump
 // segwin[k][s1][l][j] = XOR over the polynomial's set coefficients i of
-// prefix word i + j.  One CTA per (engine, segment s >= 1, lane, quarter of the
-// terms); its warps split the quarter, lane q of a warp covers output words
+// prefix word i + j.  One CTA per (engine, segment s >= 1, lane, part of the
+// terms); its warps split the part, lane q of a warp covers output words
 // [11 q, 11 q + 11) (an odd stride: the 8-byte shared-memory reads are free of
 // bank conflicts).  A thread slides a register window over the prefix words;
 // four coefficients at a time, the same for the whole warp, pick one of 16
 // unrolled cases, in which three-input XORs take 1.25 operations per 32-bit
-// word on average where one conditional XOR per term takes 2.  Quarters meet
+// word on average where one conditional XOR per term takes 2.  Parts meet
 // by atomic XOR (segwin zeroed beforehand).  Bound by issue.
 constexpr int kJumpThreads = 256;
-constexpr int kJumpParts = 8;
-constexpr int kJumpPer = 19968 / (kJumpParts * (kJumpThreads / 32));  // 312 terms per warp
 constexpr int kJumpOut = 11;
-constexpr int kJumpSpan = kJumpPer * (kJumpThreads / 32);             // terms per CTA
-constexpr int kJumpLoad = kJumpSpan + 32 * kJumpOut + 8;              // prefix words a CTA reads
+// PARTS CTAs per segment and lane
+template <int PARTS>
+struct JumpDims {
+  static constexpr int kPer = 19968 / (PARTS * (kJumpThreads / 32));  // terms per warp
+  static constexpr int kSpan = kPer * (kJumpThreads / 32);            // terms per CTA
+  static constexpr int kLoad = kSpan + 32 * kJumpOut + 8;             // prefix words a CTA reads
+  static constexpr int kRed = (kJumpThreads / 32) * 32 * kJumpOut;    // the warps' sums, in the same memory
+  static_assert(PARTS * kSpan == 19968 && kSpan % 64 == 0 && kPer % 8 == 0, "coefficient bytes stay within one word");
+};
 
 // acc[j] ^= the words of terms 0 / 1 (at w[j], w[j + 1]) whose coefficient
 // bits are set; c is the same in every thread of the warp
@@ -269,9 +274,12 @@ __device__ __forceinline__ void xor_terms2(uint64_t (&acc)[kJumpOut], const uint
   }
 }
 
+template <int PARTS>
 __global__ void __launch_bounds__(kJumpThreads, 4)
     k_jump(const uint64_t* prefix, const uint64_t* polys, int S, unsigned long long* segwin) {
-  __shared__ uint64_t px[kJumpLoad];
+  using D = JumpDims<PARTS>;
+  constexpr int kJumpParts = PARTS, kJumpPer = D::kPer, kJumpSpan = D::kSpan, kJumpLoad = D::kLoad;
+  __shared__ uint64_t px[kJumpLoad > D::kRed ? kJumpLoad : D::kRed];
   __shared__ uint64_t cf[kJumpSpan / 64];
   const int nseg = S - 1;
   const int part = blockIdx.x % kJumpParts;
@@ -317,8 +325,7 @@ __global__ void __launch_bounds__(kJumpThreads, 4)
     atomicXor(dst + j, (unsigned long long)v);
   }
 }
-static_assert(kJumpSpan % 64 == 0 && kJumpPer % 8 == 0, "coefficient bytes stay within one word");
-static_assert((kJumpThreads / 32) * 32 * kJumpOut <= kJumpLoad, "the reduction reuses the prefix buffer");
+constexpr int kJumpFew = 39, kJumpMany = 8, kJumpFewMax = 160;
 
 // ---------------------------------------------------------------- transforms
 // Truncated.h inverse-CDF forms, one lane: u is UniformRealGen(phi(lower),
@@ -954,14 +961,20 @@ cudaError_t launch_jump(const uint64_t* prefix, const uint64_t* polys, int K, in
   const int ctas = K * (S - 1) * kLanes;
   cudaError_t e = cudaMemsetAsync(segwin, 0, (size_t)ctas * kN * sizeof(uint64_t), s);
   if (e != cudaSuccess) return e;
-  k_jump<<<ctas * kJumpParts, kJumpThreads, 0, s>>>(prefix, polys, S, reinterpret_cast<unsigned long long*>(segwin));
+  // One engine, us: 4 segments 22.2 with 8 parts each, 14.3 with 39; 8: 26.4 and
+  // 21.6; 13: 34.6 and 29.5.  The gap closes (a part reads 350 words beside its
+  // own), and 1 300 CTAs of eight parts fill the GPU anyway.
+  unsigned long long* dst = reinterpret_cast<unsigned long long*>(segwin);
+  if (ctas <= kJumpFewMax) k_jump<kJumpFew><<<ctas * kJumpFew, kJumpThreads, 0, s>>>(prefix, polys, S, dst);
+  else k_jump<kJumpMany><<<ctas * kJumpMany, kJumpThreads, 0, s>>>(prefix, polys, S, dst);
   return cudaGetLastError();
 }
 
 cudaError_t preload_raw_stream_kernels() {
   cudaFuncAttributes a;
   cudaError_t e = cudaFuncGetAttributes(&a, k_prefix);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_jump);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_jump<kJumpFew>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_jump<kJumpMany>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_direct<M_RAW, kRawKind>);
   return e;
 }
