@@ -639,19 +639,19 @@ gr_status prepare_segments(gr_engine* e, Plan& p, int S, int64_t J, int delta, c
 constexpr int64_t kWordsCap = (int64_t)1 << 22;  // packets of all engines (128 MB: about one L2)
 
 // Segments for n packets per engine.  In a row a lane makes 156 words in about
-// 36 ns; a segment more costs the jump kernel about 1.9 us of the whole GPU per
+// 25 ns; a segment more costs the jump kernel about 1.9 us of the whole GPU per
 // engine, and the prefix (8 us), the jump kernel's shortest run (7) and their
 // launches about 20 us once.
 void plan_words(int K, int64_t n, int& S, int64_t& J) {
   S = 1;
   J = n + (n & 1);
-  double best = (double)n * 0.23;  // ns
+  double best = (double)n * 0.16;  // ns
   for (int m = 14; m <= 24; ++m) {
     const int64_t j = (int64_t)1 << m;
     const int64_t segs = (n + j - 1) / j;
     if (segs < 2) break;
     if (segs > 128 || segs * K > 1024) continue;
-    const double cost = (double)j * 0.23 + (double)(segs - 1) * K * 1900.0 + 20500.0;
+    const double cost = (double)j * 0.16 + (double)(segs - 1) * K * 1900.0 + 20500.0;
     if (cost < best) {
       best = cost;
       S = (int)segs;

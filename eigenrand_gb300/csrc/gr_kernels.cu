@@ -97,7 +97,8 @@ __device__ __forceinline__ uint64_t shfl64(uint64_t v, int src) {
 // thread, of which the first 40 (36) are its own and the rest a halo that
 // repeats the next warp's work.  The halo loses one word every two phases (its
 // last word misses its neighbour), so the warps exchange words only every 48
-// phases.  Bound by issue: 24 instructions per warp and phase.  Measured
+// phases.  Bound by the logic pipe, at one warp per scheduler two cycles an
+// instruction: some 24 of them per warp and phase.  Measured
 // against the one-barrier-per-phase form (156 threads, three shared-memory
 // reads per word): 20 280 words in 4.5 us against 17 us.
 // win: the CTA's 312-word window in shared memory (loaded, all threads past
@@ -118,8 +119,24 @@ __device__ __forceinline__ void lane_words_wide(uint64_t* win, int64_t n, Put&& 
       // words past the window (the last warp's halo) are made here
       c[j] = i < kM ? win[kM + i] : twist1(win[i - kM], win[i - kM + 1], win[i]);
     }
-    const int phases = (int)min((int64_t)48, (n - base + kM - 1) / kM);
-    for (int ph = 0; ph < phases; ++ph) {
+    int ph = 0;
+    if (n - base >= 48 * kM) {
+      // the words' roles alternate: two phases per trip, without moves (131 072
+      // words 31 us with them, 21 without; the shuffles a trip ahead: no change)
+      for (; ph < 48; ph += 2) {
+        const uint64_t n0 = shfl64(a[0], src);
+        const uint64_t n1 = shfl64(c[0], src);
+        a[0] = twist1(a[0], a[1], c[0]);
+        a[1] = twist1(a[1], n0, c[1]);
+        if (own) put(base + i0, a[0], a[1]);
+        c[0] = twist1(c[0], c[1], a[0]);
+        c[1] = twist1(c[1], n1, a[1]);
+        if (own) put(base + kM + i0, c[0], c[1]);
+        base += 2 * kM;
+      }
+    }
+    const int phases = ph ? 48 : (int)min((int64_t)48, (n - base + kM - 1) / kM);
+    for (; ph < phases; ++ph) {
       const uint64_t nb = shfl64(a[0], src);
       const uint64_t v0 = twist1(a[0], a[1], c[0]), v1 = twist1(a[1], nb, c[1]);
       const int64_t i = base + i0;
