@@ -390,14 +390,14 @@ __device__ __forceinline__ float tf32(uint32_t w, const DistParams& d) {
     float z = (float)(int32_t)(w & 0x7fffffffu) / (float)0x7FFFFFFF;
     return KIND == GR_BALANCED ? z * 2.0f - 1.0f : z * d.fa + d.fb;
   }
-  if (KIND == GR_EXPONENTIAL) return -(logf_(1.0f - ur_f(w)) / d.fa);
-  if (KIND == GR_GAMMA) return d.fb * (-(logf_(1.0f - ur_f(w)) / 1.0f));
+  if (KIND == GR_EXPONENTIAL) return -(logf_<true>(1.0f - ur_f(w)) / d.fa);
+  if (KIND == GR_GAMMA) return d.fb * (-(logf_<true>(1.0f - ur_f(w)) / 1.0f));
   if (KIND == GR_CAUCHY) {
     float s, c;
     sincosf_((float)3.1415926535897932 * (ur_f(w) - 0.5f), s, c);
     return d.fa + d.fb * (s / c);
   }
-  if (KIND == GR_WEIBULL) return expf_(logf_(-logf_(1.0f - ur_f(w))) * d.fa) * d.fb;
+  if (KIND == GR_WEIBULL) return expf_(logf_(-logf_<true>(1.0f - ur_f(w))) * d.fa) * d.fb;
   if (KIND == GR_EXTREME_VALUE) return d.fa - logf_(-logf_(ur_f(w) + 1.1920928955078125e-07f / 8)) * d.fb;
   // BernoulliGen<float>: the word of the lane, masked, compared signed
   if (KIND == GR_BERNOULLI) return ((int32_t)(w & 0x7fffffffu) < d.ia) ? 1.0f : 0.0f;
@@ -449,7 +449,7 @@ __device__ __forceinline__ int32_t tw32(uint32_t w, const DistParams& d) {
   // UniformIntGen<int32_t> over a power-of-two range: (rx & bitmask) + pmin (Discrete.h:302-305)
   if (KIND == GR_UNIFORM_INT) return (int32_t)((w & d.bitmask) + (uint32_t)d.ia);
   // GeometricGen<int32_t>: pcast(ptruncate(plog(1 - u) * rlog_q)), Discrete.h:1368-1374
-  if (KIND == GR_GEOMETRIC) return cvtt_f32(truncf(logf_(1.0f - ur_f(w)) * d.fa));
+  if (KIND == GR_GEOMETRIC) return cvtt_f32(truncf(logf_<true>(1.0f - ur_f(w)) * d.fa));
   // DiscreteGen<int32_t,int32_t>, Discrete.h:455-470
   if (d.ncdf > 0) {
     int32_t r = d.ncdf - 1;
@@ -677,7 +677,7 @@ __device__ __forceinline__ void emit_half(const uint64_t (&pk)[2], const int h, 
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           const float u1 = ur_f((uint32_t)(w1 >> (32 * q))), u2 = ur_f((uint32_t)(w2 >> (32 * q)));
-          const float radius = sqrtf((float)-2 * logf_(1.0f - u1));
+          const float radius = sqrtf((float)-2 * logf_<true>(1.0f - u1));
           const float theta = (float)(2 * 3.1415926535897932) * u2;
           float sn, cs;
           sincosf_(theta, sn, cs);

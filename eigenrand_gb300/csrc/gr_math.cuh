@@ -30,27 +30,23 @@ __device__ __forceinline__ float u2f(uint32_t u) { return __uint_as_float(u); }
 __device__ __forceinline__ uint64_t d2u(double f) { return (uint64_t)__double_as_longlong(f); }
 __device__ __forceinline__ double u2d(uint64_t u) { return __longlong_as_double((long long)u); }
 
+// NORMAL: x is known to be a positive normal number.  The exponent e and the
+// bits of m come from the distance to sqrt(1/2)'s bits.
+template <bool NORMAL = false>
 __device__ __forceinline__ float logf_(float x) {
   uint32_t ux = f2u(x);
   int e = 0;
-  if (ux - 0x00800000u >= 0x7f000000u) {  // not a positive normal number
+  if (!NORMAL && ux - 0x00800000u >= 0x7f000000u) {  // not a positive normal number
     if (x != x) return x;
     if (x < 0.0f) return u2f(0x7fc00000u);
     if (x == 0.0f) return -__int_as_float(0x7f800000);
     if (ux == 0x7f800000u) return x;
-    x = x * 8388608.0f;
-    ux = f2u(x);
+    ux = f2u(x * 8388608.0f);
     e = -23;
   }
-  e += (int)((ux >> 23) & 0xff) - 126;
-  float m = u2f((ux & 0x007fffffu) | 0x3f000000u);
-  float f;
-  if (m < 0.70710678118654752f) {
-    e -= 1;
-    f = (m + m) - 1.0f;
-  } else {
-    f = m - 1.0f;
-  }
+  const int k = (int)(ux - 0x3f3504f3u) >> 23;  // 0x3f3504f3: sqrt(1/2)
+  e += k;
+  const float f = u2f(ux - ((uint32_t)k << 23)) - 1.0f;
   float z = f * f;
   float p = 7.149753720e-02f;
   p = fmaf(p, f, -1.157120094e-01f);
@@ -112,30 +108,21 @@ __device__ __forceinline__ int32_t cvtt_f32(float x) {
 __device__ __forceinline__ double log_(double x) { return grd_log(x); }
 __device__ __forceinline__ double exp_(double x) { return grd_exp(x); }
 
-// EigenRand psincos, float lanes (MorePacketMath.h:297-393).
+// EigenRand psincos, float lanes (MorePacketMath.h:297-393), for |x| <= 2 pi.
+// Rounds as the reference's sequence does: y DP1 and y DP2 are exact (y an even
+// integer up to 8, 8 and 11 bits), x - y DP1 - y DP2 is exact (multiples of
+// 2^-24 below 1), so one fused operation with DP1 + DP2 gives it; z / 2 is exact;
+// and the masked sums at the end are selections (no addend is -0).  With the
+// logarithm's exponent from one subtraction, 4096 x 4096 on 608 engines, us:
+// normal 51 -> 45, exponential 48 -> 41, Weibull 75 -> 63, gamma(1) 42 -> 35.
 __device__ __forceinline__ void sincosf_(float x, float& s, float& c) {
-  uint32_t sign_bit_sin = f2u(x) & 0x80000000u;
+  const uint32_t sign = f2u(x) & 0x80000000u;
   x = fabsf(x);
-  float y = x * (float)1.27323954473516;
-  int32_t emm2 = __float2int_rz(y);
-  emm2 = emm2 + 1;
-  emm2 = emm2 & ~1;
-  y = (float)emm2;
-  int32_t emm4 = emm2;
-  uint32_t swap_sign_bit_sin = ((uint32_t)(emm2 & 4)) << 29;
-  emm2 = emm2 & 2;
-  uint32_t poly_mask = (emm2 == 0) ? 0xffffffffu : 0u;
-  float xmm1 = y * (float)-0.78515625;
-  float xmm2 = y * (float)-2.4187564849853515625e-4;
-  float xmm3 = y * (float)-3.77489497744594108e-8;
-  x = x + xmm1;
-  x = x + xmm2;
-  x = x + xmm3;
-  emm4 = emm4 - 2;
-  emm4 = 4 & ~emm4;
-  uint32_t sign_bit_cos = ((uint32_t)emm4) << 29;
-  sign_bit_sin ^= swap_sign_bit_sin;
-  float z = x * x;
+  const uint32_t j = ((uint32_t)__float2int_rz(x * (float)1.27323954473516) + 1u) & ~1u;
+  const float y = (float)(int32_t)j;
+  x = fmaf(y, -0.785398125648498535f, x);
+  x = x + y * (float)-3.77489497744594108e-8;
+  const float z = x * x;
   float yy = (float)2.443315711809948E-005;
   yy = yy * z;
   yy = yy + (float)-1.388731625493765E-003;
@@ -143,8 +130,7 @@ __device__ __forceinline__ void sincosf_(float x, float& s, float& c) {
   yy = yy + (float)4.166664568298827E-002;
   yy = yy * z;
   yy = yy * z;
-  float tmp = z * 0.5f;
-  yy = yy - tmp;
+  yy = fmaf(-0.5f, z, yy);
   yy = yy + 1.0f;
   float y2 = (float)-1.9515295891E-4;
   y2 = y2 * z;
@@ -154,14 +140,10 @@ __device__ __forceinline__ void sincosf_(float x, float& s, float& c) {
   y2 = y2 * z;
   y2 = y2 * x;
   y2 = y2 + x;
-  float ysin2 = u2f(poly_mask & f2u(y2));
-  float ysin1 = u2f(f2u(yy) & ~poly_mask);
-  y2 = y2 - ysin2;
-  yy = yy - ysin1;
-  float o1 = ysin1 + ysin2;
-  float o2 = yy + y2;
-  s = u2f(f2u(o1) ^ sign_bit_sin);
-  c = u2f(f2u(o2) ^ sign_bit_cos);
+  const bool swap = (j & 2u) != 0;
+  // the sine is negative in octants 4 to 7, the cosine in 2 to 5
+  s = u2f(f2u(swap ? yy : y2) ^ (sign ^ ((j & 4u) << 29)));
+  c = u2f(f2u(swap ? y2 : yy) ^ (((j + 2u) & 4u) << 29));
 }
 
 // uniforms of the reference from a word: asfloat / asdouble of the fraction in
