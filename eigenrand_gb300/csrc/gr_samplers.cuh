@@ -76,7 +76,8 @@ __device__ __forceinline__ int gs_filter_f64(uint64_t bux, uint64_t bvx, uint64_
 // the reference's expressions.  Five special-function operations and some
 // twenty others where those take about 150 instructions (double: about 100 of
 // them on the FP64 pipe), and rejected lanes need nothing more.
-__device__ __forceinline__ int tan_filter(float u, float ux, float a1, float sq, float delta) {
+// eps: absolute error of ux.
+__device__ __forceinline__ int tan_filter(float u, float ux, float a1, float sq, float delta, float eps = 0.0f) {
   const float t = 3.14159274f * u;
   float s, c, rc, ra, rx;
   asm("sin.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(t));
@@ -93,8 +94,8 @@ __device__ __forceinline__ int tan_filter(float u, float ux, float a1, float sq,
   const float tol = 2.0f * (dy * (1.0f + sq * fabsf(sy) * rx) + 0x1p-20f * (1.0f + a1 + fabsf(sy) + fabsf(al)));
   const float ub = fmaf(y, y, 1.0f) * ex2_approx(1.44269502f * (al - sy));
   if (!(tol < 0.25f)) return -1;
-  if (ux < ub * (1.0f - tol)) return 1;
-  if (ux > ub * (1.0f + tol)) return 0;
+  if (ux + eps < ub * (1.0f - tol)) return 1;
+  if (ux - eps > ub * (1.0f + tol)) return 0;
   return -1;
 }
 constexpr float kTanDeltaF = 0x1p-20f;   // float trials
@@ -104,10 +105,8 @@ __device__ __forceinline__ int tan_filter_f64(uint64_t bu, uint64_t bux, float a
   constexpr uint64_t M = 0xfffffffffffffull;
   const float u = __uint2float_rn((uint32_t)((bu & M) >> 20)) * 0x1p-32f;
   const float ux = __uint2float_rn((uint32_t)((bux & M) >> 20)) * 0x1p-32f;
-  // ux within 2^-24: outside that of both ends of the band
-  const int lo = tan_filter(u, ux - 0x1p-23f, a1, sq, kTanDeltaD);
-  const int hi = tan_filter(u, ux + 0x1p-23f, a1, sq, kTanDeltaD);
-  return lo == hi ? lo : -1;
+  // ux is within 2^-24
+  return tan_filter(u, ux, a1, sq, kTanDeltaD, 0x1p-23f);
 }
 
 // Candidate of a double GS trial already known to be accepted: xx only
