@@ -77,20 +77,20 @@ def kernel_of(name, compat=False):
     compat: the single-engine kernels)."""
     base, tag = name.split("/")
     if compat:
+        words = "k_words_wide in jump-ahead segments + "
         if base == "beta":
-            return f"k_beta<{'float' if tag == 'f32' else 'double'}, GS, integral> (one CTA, visit table)"
+            return words + "k_chain_masks/visits/table/compose/walk/scan/emit/finish"
         if base == "poisson4":
-            return "k_poisson (one CTA)"
+            return words + "k_pois_steps + k_chain_table/compose/walk/scan + k_pois_emit/finish"
         if base in ("gamma0.5", "poisson100"):
-            return "k_rs_count/scan/write/gather/finish (segmented rejection)"
-        return "k_prefix + k_jump + " + ("k_staged" if base in ("gamma5", "binomial20") else "k_direct") + \
-            " (jump-ahead segments)"
+            return words + "k_rw_masks/scan/emit/finish"
+        return words + ("k_staged_words" if base in ("gamma5", "binomial20") else "k_xform")
     if base == "beta":
         return f"k_beta<{'float' if tag == 'f32' else 'double'}, GS, integral>"
     if base in ("gamma0.5", "poisson100"):
-        return "k_reject"
+        return "k_trials"
     if base in ("gamma5", "binomial20"):
-        return "k_staged"
+        return "k_units"
     if base == "poisson4":
         return "k_poisson"
     return "k_direct"
