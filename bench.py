@@ -101,12 +101,11 @@ def kernel_of(name, compat=False):
 # launch; the capture command is in the named profiles/ summary), and what
 # binds the kernel when it is not HBM
 MEASURED = {
-    "uniformReal/f32": {"dram_bytes_per_sample": 3.276, "profile": "profiles/k_direct_uniform_f32_8192sq.md"},
-    "beta/f64": {"dram_bytes_per_sample": 5.19, "fp64_pipe_active": 0.270, "issue_active": 0.633,
-                 "note": "issue-bound on the integer double log / exp of the masks and values (the walk "
-                         "runs on its own warp): issue active 63%, ALU 52%, FP64 pipe 27% (not HBM)",
-                 "profile": "profiles/k_beta_f64_2048sq.md"},
-}
+    "uniformReal/f32": {"dram_bytes_per_sample": 3.287, "profile": "profiles/k_direct_uniform_f32_8192sq.md"},
+    "beta/f64": {"dram_bytes_per_sample": 5.158, "fp64_pipe_active": 0.197, "issue_active": 0.603,
+                 "note": "issue-bound on the masks and the integer double log / exp of the values (the walk "
+                         "looks whole visits up): issue active 60%, ALU 55%, FP64 pipe 20% (not HBM)",
+                 "profile": "profiles/k_beta_f64_2048sq.md"}
 
 
 def roofline_entry(name, pd, hbm_peak, peaks, measured=True):

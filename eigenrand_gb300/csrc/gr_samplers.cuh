@@ -256,7 +256,7 @@ __device__ __forceinline__ bool rej_trial(const DistParams& d, int64_t t, int j,
       cbits = f2u(fres);
     }
   }
-        return acc;
+  return acc;
 }
 
 // The candidate of a trial's lane that is known to be accepted: rej_trial's
