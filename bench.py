@@ -105,7 +105,8 @@ MEASURED = {
     "beta/f64": {"dram_bytes_per_sample": 5.158, "fp64_pipe_active": 0.197, "issue_active": 0.603,
                  "note": "issue-bound on the masks and the integer double log / exp of the values (the walk "
                          "looks whole visits up): issue active 60%, ALU 55%, FP64 pipe 20% (not HBM)",
-                 "profile": "profiles/k_beta_f64_2048sq.md"}
+                 "profile": "profiles/k_beta_f64_2048sq.md"},
+}
 
 
 def roofline_entry(name, pd, hbm_peak, peaks, measured=True):
