@@ -864,7 +864,10 @@ __global__ void __launch_bounds__(kDirThreads, kWideKind<MODE, KIND> ? 2 : 4)
     }
   }
 
-  // --- end-of-call state: new lane windows and cache flags
+  // --- end-of-call state: new lane windows and cache flags.  A call that the
+  // cache serves whole has met no barrier yet: every thread has read the flag
+  // before it changes.
+  if (CO > 0 && Np == 0) __syncthreads();
   if (last) {
     if (Np > 0 && tid < 2 * kM) {
       // the 312 words before packet pend: the end of phase g - 3, phase g - 2
