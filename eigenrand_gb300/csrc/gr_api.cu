@@ -62,10 +62,15 @@ JumpCache& jump_cache() {
   return c;
 }
 
-gr_status get_jump_polys(int dev, int64_t J, int delta, int need, const uint64_t** out) {
+// make = false: *out is null if they have not been made yet.
+gr_status get_jump_polys(int dev, int64_t J, int delta, int need, const uint64_t** out, bool make = true) {
   JumpCache& jc = jump_cache();
   std::lock_guard<std::mutex> lk(jc.mu);
   auto& ent = jc.tab[std::make_tuple(dev, J, delta)];
+  if (ent.count < need && !make) {
+    *out = nullptr;
+    return GR_OK;
+  }
   if (ent.count < need) {
     // every entry is made at full size (127 = the most segments a call uses)
     // so a buffer that running kernels may read is never replaced
@@ -101,9 +106,35 @@ ScratchPools& scratch_pools() {
   static ScratchPools p;
   return p;
 }
+// The device's pool, made when it is first asked for (null: it cannot be).
+cudaMemPool_t scratch_pool(ScratchPools& sp, int dev) {
+  auto& e = sp.tab[dev];
+  if (!e.first) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t made = nullptr;
+    if (cudaMemPoolCreate(&made, &props) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    uint64_t keep = kScratchKeep;
+    if (cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+      cudaGetLastError();
+      cudaMemPoolDestroy(made);
+      return nullptr;
+    }
+    e.first = made;
+  }
+  return e.first;
+}
+// An engine was made (the pool comes with it, so that a captured call finds it)
+// or destroyed.
 void scratch_engine(int dev, int delta) {
   ScratchPools& sp = scratch_pools();
   std::lock_guard<std::mutex> lk(sp.mu);
+  if (delta > 0) scratch_pool(sp, dev);
   auto& e = sp.tab[dev];
   e.second += delta;
   if (e.second <= 0 && e.first) cudaMemPoolTrimTo(e.first, 0);
@@ -113,26 +144,9 @@ cudaError_t scratch_alloc(void** p, size_t bytes, int dev, cudaStream_t s) {
   {
     ScratchPools& sp = scratch_pools();
     std::lock_guard<std::mutex> lk(sp.mu);
-    auto& e = sp.tab[dev];
-    if (!e.first) {
-      cudaMemPoolProps props{};
-      props.allocType = cudaMemAllocationTypePinned;
-      props.location.type = cudaMemLocationTypeDevice;
-      props.location.id = dev;
-      cudaMemPool_t made = nullptr;
-      cudaError_t err = cudaMemPoolCreate(&made, &props);
-      if (err != cudaSuccess) return err;
-      uint64_t keep = kScratchKeep;
-      err = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
-      if (err != cudaSuccess) {
-        cudaMemPoolDestroy(made);
-        return err;
-      }
-      e.first = made;
-    }
-    pool = e.first;
+    pool = scratch_pool(sp, dev);
   }
-  return cudaMallocFromPoolAsync(p, bytes, pool, s);
+  return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaErrorMemoryAllocation;
 }
 
 }  // namespace
@@ -147,7 +161,7 @@ struct gr_engine {
   uint64_t* prefix = nullptr;
   uint64_t* segwin = nullptr;
   size_t segwin_words = 0;
-  CallSnap* snap = nullptr;
+  CallSnap* snap = nullptr;         // in st's allocation, behind the states
   GenState* scratch_gen = nullptr;  // caches of temporary generators (gr_sample)
   uint64_t* tailw = nullptr;        // draws of a call's partial last packet
 };
@@ -208,11 +222,12 @@ gr_status gr_engine_create(gr_engine** out, uint64_t seed, int32_t lanes, int32_
   e->lanes = lanes;
   e->seed = seed;
   cudaGetDevice(&e->device);
-  cudaError_t err = cudaMalloc(&e->st, sizeof(EngState) * (size_t)streams);
+  cudaError_t err = cudaMalloc(&e->st, (sizeof(EngState) + sizeof(CallSnap)) * (size_t)streams);
   if (err != cudaSuccess) {
     delete e;
     return cuda_fail(err, "cudaMalloc(engine state)");
   }
+  e->snap = reinterpret_cast<CallSnap*>(e->st + streams);
   err = launch_seed(e->st, e->K, seed, nullptr);
   if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
   if (err != cudaSuccess) {
@@ -230,7 +245,6 @@ gr_status gr_engine_destroy(gr_engine* e) {
   cudaFree(e->st);
   cudaFree(e->prefix);
   cudaFree(e->segwin);
-  cudaFree(e->snap);
   cudaFree(e->scratch_gen);
   cudaFree(e->tailw);
   scratch_engine(e->device, -1);
@@ -601,14 +615,14 @@ Family family_of(const DistParams& dp) {
   return Family::Unsupported;
 }
 
-// Room for the prefix and for the windows of an S-segment call.
+// Room for the prefix and for the windows of an S-segment call of prepare_segments.
 gr_status reserve_windows(gr_engine* e, int S) {
   if (!e->prefix) GR_CUDA(cudaMalloc(&e->prefix, sizeof(uint64_t) * (size_t)kPrefixLen * kLanes * (size_t)e->K));
-  if (!e->snap) GR_CUDA(cudaMalloc(&e->snap, sizeof(CallSnap) * (size_t)e->K));
   const size_t need = (size_t)e->K * (S - 1) * kLanes * kN;
   if (e->segwin_words < need) {
     cudaFree(e->segwin);
     e->segwin = nullptr;
+    e->segwin_words = 0;
     GR_CUDA(cudaMalloc(&e->segwin, sizeof(uint64_t) * need));
     e->segwin_words = need;
   }
@@ -660,26 +674,40 @@ void plan_words(int K, int64_t n, int& S, int64_t& J) {
   }
 }
 
+// The polynomials of a call in S segments of J packets, or null: none to be had
+// (no memory, or a stream capture, which may not make them), and the words are
+// made in one segment.
+const uint64_t* words_polys(int dev, int S, int64_t J, cudaStream_t stream) {
+  const uint64_t* polys = nullptr;
+  if (get_jump_polys(dev, J, 0, S - 1, &polys, false) == GR_OK && polys) return polys;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(stream, &cap);
+  if (cap == cudaStreamCaptureStatusNone && get_jump_polys(dev, J, 0, S - 1, &polys) == GR_OK) return polys;
+  cudaGetLastError();
+  return nullptr;
+}
+
 // Makes n packets of raw words per engine in new scratch (freed by the caller
 // in stream order) and fills the plan's words fields; the engine's state is
-// left as it is.  first: also snapshot the caches.  *got = false: no scratch
-// memory, nothing was launched, and the caller takes the path that needs none.
+// left as it is.  first: also snapshot the caches.  The prefix and the windows of
+// the segments lie behind the words: a captured call then needs nothing that a
+// later, longer call replaces.  *got = false: no scratch memory, nothing was
+// launched, and the caller takes the path that needs none.
 gr_status make_words(gr_engine* e, Plan& p, int64_t n, bool first, void** buf, bool* got, cudaStream_t stream) {
   n += n & 1;
   const int64_t stride = kN + n;
   *got = false;
-  if (!e->snap) GR_CUDA(cudaMalloc(&e->snap, sizeof(CallSnap) * (size_t)e->K));
   WordsArgs a{};
   plan_words(e->K, n, a.S, a.J);
-  if (a.S > 1) {
-    gr_status st = reserve_windows(e, a.S);
-    if (st != GR_OK) return st;
-    const uint64_t* polys = nullptr;
-    st = get_jump_polys(e->device, a.J, 0, a.S - 1, &polys);
-    if (st != GR_OK) return st;
-    p.segwin = polys;  // until the launch below
+  const uint64_t* polys = a.S > 1 ? words_polys(e->device, a.S, a.J, stream) : nullptr;
+  if (!polys) {
+    a.S = 1;
+    a.J = n;
   }
-  const cudaError_t err = scratch_alloc(buf, sizeof(uint64_t) * (size_t)e->K * kLanes * (size_t)stride, e->device, stream);
+  const size_t lanes = (size_t)e->K * kLanes;
+  const size_t words = lanes * (size_t)stride, prefix = a.S > 1 ? lanes * kPrefixLen : 0;
+  const size_t wins = lanes * kN * (size_t)(a.S - 1);
+  const cudaError_t err = scratch_alloc(buf, sizeof(uint64_t) * (words + prefix + wins), e->device, stream);
   if (err == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     return GR_OK;
@@ -691,13 +719,13 @@ gr_status make_words(gr_engine* e, Plan& p, int64_t n, bool first, void** buf, b
   a.snap = first ? e->snap : nullptr;
   cudaError_t le = cudaSuccess;
   if (a.S > 1) {
-    le = launch_prefix(e->st, p.gen, e->K, e->prefix, first ? e->snap : nullptr, stream);
-    if (le == cudaSuccess) le = launch_jump(e->prefix, p.segwin, e->K, a.S, e->segwin, stream);
-    a.segwin = e->segwin;
+    uint64_t* segwin = a.words + words + prefix;
+    le = launch_prefix(e->st, p.gen, e->K, a.words + words, first ? e->snap : nullptr, stream);
+    if (le == cudaSuccess) le = launch_jump(a.words + words, polys, e->K, a.S, segwin, stream);
+    a.segwin = segwin;
     a.snap = nullptr;
   }
   if (le == cudaSuccess) le = launch_words(e->st, p.gen, e->K, a, stream);
-  p.segwin = nullptr;
   if (le != cudaSuccess) {
     cudaFreeAsync(*buf, stream);
     return cuda_fail(le, "raw word kernels");
