@@ -139,14 +139,21 @@ void scratch_engine(int dev, int delta) {
   e.second += delta;
   if (e.second <= 0 && e.first) cudaMemPoolTrimTo(e.first, 0);
 }
-cudaError_t scratch_alloc(void** p, size_t bytes, int dev, cudaStream_t s) {
+// A call's scratch: one allocation, taken before its first launch, so that a call
+// that has started cannot run out.  Null: none to be had, and the call takes the
+// path that needs none.  Test hook: GR_SCRATCH_FAIL, if set, makes it null.
+char* scratch_alloc(size_t bytes, int dev, cudaStream_t s) {
+  if (std::getenv("GR_SCRATCH_FAIL")) return nullptr;
   cudaMemPool_t pool = nullptr;
   {
     ScratchPools& sp = scratch_pools();
     std::lock_guard<std::mutex> lk(sp.mu);
     pool = scratch_pool(sp, dev);
   }
-  return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaErrorMemoryAllocation;
+  void* p = nullptr;
+  if (pool && cudaMallocFromPoolAsync(&p, bytes, pool, s) == cudaSuccess) return static_cast<char*>(p);
+  cudaGetLastError();
+  return nullptr;
 }
 
 }  // namespace
@@ -163,6 +170,7 @@ struct gr_engine {
   size_t segwin_words = 0;
   CallSnap* snap = nullptr;         // in st's allocation, behind the states
   GenState* scratch_gen = nullptr;  // caches of temporary generators (gr_sample)
+  size_t scratch_cap = SIZE_MAX;    // most bytes of scratch a call takes
   uint64_t* tailw = nullptr;        // draws of a call's partial last packet
 };
 
@@ -649,8 +657,28 @@ gr_status prepare_segments(gr_engine* e, Plan& p, int S, int64_t J, int delta, c
 // Calls on few engines: the raw words of every engine are made in memory
 // first (launch_words, S jump-ahead segments per engine when that is shorter
 // than making them in a row), and the transforms then read them on the whole
-// GPU.  A scratch buffer holds at most kWordsCap packets per engine set.
-constexpr int64_t kWordsCap = (int64_t)1 << 22;  // packets of all engines (128 MB: about one L2)
+// GPU.  The words are made a chunk at a time, all chunks in the same buffer.
+constexpr int64_t kWordsCap = (int64_t)1 << 22;  // packets of all engines in a chunk (128 MB: about one L2)
+
+constexpr size_t al256(size_t x) { return (x + 255) / 256 * 256; }
+
+// What chunks of c leave for the last one.
+constexpr int64_t last_chunk(int64_t total, int64_t c) { return total - (total - 1) / c * c; }
+
+// The largest chunk, at most `chunk` and (where that is more) at least `least`, for which the call's
+// scratch is no more than the engine's limit (0: there is none); *bytes: that
+// scratch.  need(c): bytes for chunks of c.
+template <class Need>
+int64_t fit_chunk(const gr_engine* e, int64_t chunk, int64_t least, Need&& need, size_t* bytes) {
+  least = std::min(least, chunk);
+  for (;; chunk = std::max(chunk / 2, least)) {
+    *bytes = need(chunk);
+    if (*bytes <= e->scratch_cap) return chunk;
+    if (chunk <= least) break;
+  }
+  *bytes = 0;
+  return 0;
+}
 
 // Segments for n packets per engine.  In a row a lane makes 156 words in about
 // 25 ns; a segment more costs the jump kernel about 1.9 us of the whole GPU per
@@ -687,16 +715,24 @@ const uint64_t* words_polys(int dev, int S, int64_t J, cudaStream_t stream) {
   return nullptr;
 }
 
-// Makes n packets of raw words per engine in new scratch (freed by the caller
-// in stream order) and fills the plan's words fields; the engine's state is
-// left as it is.  first: also snapshot the caches.  The prefix and the windows of
-// the segments lie behind the words: a captured call then needs nothing that a
-// later, longer call replaces.  *got = false: no scratch memory, nothing was
-// launched, and the caller takes the path that needs none.
-gr_status make_words(gr_engine* e, Plan& p, int64_t n, bool first, void** buf, bool* got, cudaStream_t stream) {
+// Bytes of n packets of raw words per engine, with the prefix and the windows of
+// their segments.
+size_t words_bytes(int K, int64_t n) {
+  n += n & 1;
+  int S;
+  int64_t J;
+  plan_words(K, n, S, J);
+  const size_t words = kN + (size_t)n + (S > 1 ? kPrefixLen + (size_t)(S - 1) * kN : 0);
+  return al256(sizeof(uint64_t) * kLanes * (size_t)K * words);
+}
+
+// Makes n packets of raw words per engine in buf (words_bytes) and fills the plan's
+// words fields; the engine's state is left as it is.  first: also snapshot the
+// caches.  The prefix and the windows of the segments lie behind the words: a
+// captured call then needs nothing that a later, longer call replaces.
+gr_status make_words(gr_engine* e, Plan& p, int64_t n, bool first, char* buf, cudaStream_t stream) {
   n += n & 1;
   const int64_t stride = kN + n;
-  *got = false;
   WordsArgs a{};
   plan_words(e->K, n, a.S, a.J);
   const uint64_t* polys = a.S > 1 ? words_polys(e->device, a.S, a.J, stream) : nullptr;
@@ -704,36 +740,24 @@ gr_status make_words(gr_engine* e, Plan& p, int64_t n, bool first, void** buf, b
     a.S = 1;
     a.J = n;
   }
-  const size_t lanes = (size_t)e->K * kLanes;
-  const size_t words = lanes * (size_t)stride, prefix = a.S > 1 ? lanes * kPrefixLen : 0;
-  const size_t wins = lanes * kN * (size_t)(a.S - 1);
-  const cudaError_t err = scratch_alloc(buf, sizeof(uint64_t) * (words + prefix + wins), e->device, stream);
-  if (err == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    return GR_OK;
-  }
-  if (err != cudaSuccess) return cuda_fail(err, "scratch memory");
-  a.words = static_cast<uint64_t*>(*buf);
+  a.words = reinterpret_cast<uint64_t*>(buf);
   a.stride = stride;
   a.n = n;
   a.snap = first ? e->snap : nullptr;
-  cudaError_t le = cudaSuccess;
+  cudaError_t err = cudaSuccess;
   if (a.S > 1) {
-    uint64_t* segwin = a.words + words + prefix;
-    le = launch_prefix(e->st, p.gen, e->K, a.words + words, first ? e->snap : nullptr, stream);
-    if (le == cudaSuccess) le = launch_jump(a.words + words, polys, e->K, a.S, segwin, stream);
+    const size_t lanes = (size_t)e->K * kLanes;
+    uint64_t *prefix = a.words + lanes * (size_t)stride, *segwin = prefix + lanes * kPrefixLen;
+    err = launch_prefix(e->st, p.gen, e->K, prefix, a.snap, stream);
+    if (err == cudaSuccess) err = launch_jump(prefix, polys, e->K, a.S, segwin, stream);
     a.segwin = segwin;
     a.snap = nullptr;
   }
-  if (le == cudaSuccess) le = launch_words(e->st, p.gen, e->K, a, stream);
-  if (le != cudaSuccess) {
-    cudaFreeAsync(*buf, stream);
-    return cuda_fail(le, "raw word kernels");
-  }
+  if (err == cudaSuccess) err = launch_words(e->st, p.gen, e->K, a, stream);
+  if (err != cudaSuccess) return cuda_fail(err, "raw word kernels");
   p.words = a.words;
   p.wstride = stride;
   p.wcount = n;
-  *got = true;
   return GR_OK;
 }
 
@@ -758,25 +782,27 @@ int64_t words_from(const DistParams& dp) {
 gr_status run_fixed(gr_engine* e, Plan p, const DistParams& dp, int64_t packets, int ppu, cudaStream_t stream,
                     const char* what) {
   if (e->K < 128 && packets > words_from(dp) && p.out) {
-    const int64_t chunk = std::max<int64_t>(kWordsCap / e->K & ~(int64_t)1, 2);
-    bool done = true;
-    for (int64_t at = 0; at < packets; at += chunk) {
-      void* buf = nullptr;
-      bool got = false;
-      gr_status st = make_words(e, p, std::min(chunk, packets - at), at == 0, &buf, &got, stream);
-      if (st != GR_OK) return st;
-      if (!got && at == 0) {
-        done = false;
-        break;
+    size_t bytes = 0;
+    const int64_t most = std::min(kWordsCap / e->K, packets + 1) & ~(int64_t)1;
+    const int64_t chunk = fit_chunk(
+        e, most, 1024,
+        [&](int64_t c) {
+          c &= ~(int64_t)1;
+          return std::max(words_bytes(e->K, c), words_bytes(e->K, last_chunk(packets, c)));
+        },
+        &bytes) & ~(int64_t)1;
+    if (char* buf = chunk ? scratch_alloc(bytes, e->device, stream) : nullptr) {
+      gr_status st = GR_OK;
+      for (int64_t at = 0; st == GR_OK && at < packets; at += chunk) {
+        st = make_words(e, p, std::min(chunk, packets - at), at == 0, buf, stream);
+        if (st != GR_OK) break;
+        p.wbase = at;
+        const cudaError_t err = launch_direct(p, dp, e->snap, stream);
+        if (err != cudaSuccess) st = cuda_fail(err, what);
       }
-      if (!got) return fail(GR_ERR_CUDA, "out of memory for the call's scratch");
-      p.wbase = at;
-      const cudaError_t err = launch_direct(p, dp, e->snap, stream);
       cudaFreeAsync(buf, stream);
-      if (err != cudaSuccess) return cuda_fail(err, what);
+      return st;
     }
-    if (done) return GR_OK;
-    p.words = nullptr;
   }
   int S;
   int64_t J;
@@ -918,6 +944,21 @@ constexpr int64_t kStagedMin = 624;               // packets per engine
 constexpr int kStagedMaxK = 128;                  // engines
 constexpr int64_t kStagedCap = (int64_t)1 << 22;  // packets of words at a time, all engines
 
+// Scratch of a chain's chunks, of which each makes `again` of its packets once
+// more: the words and the layout of the first and of the last chunk.
+template <class Next, class Layout>
+size_t chunks_bytes(int K, int64_t left, int64_t chunk, int64_t again, Next&& next, Layout&& layout) {
+  size_t most = 0;
+  for (int64_t before = 0; left > 0;) {
+    const int64_t n = next(chunk, left);
+    left -= n - again;
+    if (n == before) continue;
+    most = std::max(most, layout(n).bytes + words_bytes(K, n));
+    before = n;
+  }
+  return most;
+}
+
 // PoissonGen's walk through words in memory (gr_chain.cu), then the one-CTA
 // walk for whatever the planned packets did not hold.
 constexpr int64_t kPoisMin = 512;               // output packets per engine
@@ -929,42 +970,38 @@ gr_status run_poisson_call(gr_engine* e, const Plan& p0, const DistParams& wd, i
   const double hl = poisson_step_halves(wd.fe);
   int64_t left = (int64_t)std::ceil(((double)npk + 4.0 * std::sqrt((double)npk)) * hl * 0.5 * 1.03 * scale) + 64;
   Plan p = p0;
-  int64_t* done = nullptr;
-  cudaError_t err = scratch_alloc(reinterpret_cast<void**>(&done), sizeof(int64_t) * (size_t)e->K, e->device, stream);
-  if (err != cudaSuccess) return cuda_fail(err, "scratch memory");
-  err = cudaMemsetAsync(done, 0, sizeof(int64_t) * (size_t)e->K, stream);
-  gr_status st = err == cudaSuccess ? GR_OK : cuda_fail(err, "Poisson chain");
-  const int64_t chunk = std::max<int64_t>(kPoisCap / e->K & ~(int64_t)1, 512);
-  while (st == GR_OK && left > 0) {
-    // what a chunk leaves over (less than one step's packets) is made again
-    const int64_t n = std::min(chunk, left + 32 + (left & 1));
-    left -= n - 32;
-    const ChainLayout L = poisson_layout(e->K, n, n > 4096 ? 1024 : 0);
-    void *words = nullptr, *scratch = nullptr;
-    bool got = false;
-    err = scratch_alloc(&scratch, L.bytes, e->device, stream);
-    if (err != cudaSuccess) {
-      cudaGetLastError();
-      break;
-    }
-    st = make_words(e, p, n, true, &words, &got, stream);
-    if (st == GR_OK && got) {
-      err = launch_poisson_words(p, wd, e->snap, L, static_cast<char*>(scratch), done, stream);
+  // what a chunk leaves over (less than one step's packets) is made again
+  auto next = [](int64_t c, int64_t l) { return std::min(c, l + 32 + (l & 1)); };
+  auto layout = [&](int64_t n) { return poisson_layout(e->K, n, n > 4096 ? 1024 : 0); };
+  const size_t counts = al256(sizeof(int64_t) * (size_t)e->K);
+  size_t bytes = 0;
+  const int64_t chunk = fit_chunk(
+      e, next(std::max<int64_t>(kPoisCap / e->K, 512) & ~(int64_t)1, left), 512,
+      [&](int64_t c) { return counts + chunks_bytes(e->K, left, c & ~(int64_t)1, 32, next, layout); }, &bytes) & ~(int64_t)1;
+  char* buf = chunk ? scratch_alloc(bytes, e->device, stream) : nullptr;
+  gr_status st = GR_OK;
+  if (buf) {
+    int64_t* done = reinterpret_cast<int64_t*>(buf);
+    cudaError_t err = cudaMemsetAsync(done, 0, sizeof(int64_t) * (size_t)e->K, stream);
+    if (err != cudaSuccess) st = cuda_fail(err, "Poisson chain");
+    while (st == GR_OK && left > 0) {
+      const int64_t n = next(chunk, left);
+      left -= n - 32;
+      const ChainLayout L = layout(n);
+      st = make_words(e, p, n, true, buf + counts + L.bytes, stream);
+      if (st != GR_OK) break;
+      err = launch_poisson_words(p, wd, e->snap, L, buf + counts, done, stream);
       if (err != cudaSuccess) st = cuda_fail(err, "Poisson chain kernels");
-      cudaFreeAsync(words, stream);
     }
-    cudaFreeAsync(scratch, stream);
-    p.words = nullptr;
-    if (!got) break;
-  }
-  if (st == GR_OK) {
     p.words = nullptr;
     p.done = done;
+  }
+  if (st == GR_OK) {
     p.S = 1;
-    err = launch_walk(p, wd, max_blocks, stream);
+    const cudaError_t err = launch_walk(p, wd, max_blocks, stream);
     if (err != cudaSuccess) st = cuda_fail(err, "walk sampling kernel");
   }
-  cudaFreeAsync(done, stream);
+  if (buf) cudaFreeAsync(buf, stream);
   return st;
 }
 
@@ -1000,40 +1037,40 @@ gr_status run_reject_call(gr_engine* e, const Plan& p0, const DistParams& dp, in
   int64_t left = (int64_t)std::ceil(((double)npk + 8.0 * std::sqrt((double)npk)) / q * (1.0 + slack) * scale) + 16;
   const int64_t U = rk == 0 ? 3 : (rk >= 3 ? 1 : 2);  // packets per trial
   Plan p = p0;
-  int64_t* done = nullptr;
-  cudaError_t err = scratch_alloc(reinterpret_cast<void**>(&done), sizeof(int64_t) * (size_t)e->K, e->device, stream);
-  if (err != cudaSuccess) return cuda_fail(err, "scratch memory");
-  err = cudaMemsetAsync(done, 0, sizeof(int64_t) * (size_t)e->K, stream);
-  gr_status st = err == cudaSuccess ? GR_OK : cuda_fail(err, "rejection sampler");
-  const int64_t chunk = std::max<int64_t>(kRejectCap / e->K / U, 64);
-  while (st == GR_OK && left > 0) {
-    const int64_t T = std::min(chunk, left);
-    left -= T;
-    const RwLayout L = reject_words_layout(e->K, T);
-    void *words = nullptr, *scratch = nullptr;
-    bool got = false;
-    err = scratch_alloc(&scratch, L.bytes, e->device, stream);
-    if (err != cudaSuccess) {
-      cudaGetLastError();
-      break;
-    }
-    st = make_words(e, p, T * U, true, &words, &got, stream);
-    if (st == GR_OK && got) {
-      err = launch_reject_words(p, dp, rk, e->snap, L, static_cast<char*>(scratch), done, stream);
+  const size_t counts = al256(sizeof(int64_t) * (size_t)e->K);
+  size_t bytes = 0;
+  const int64_t chunk = fit_chunk(
+      e, std::min(std::max<int64_t>(kRejectCap / e->K / U, 64), left), 64,
+      [&](int64_t c) {
+        const int64_t l = last_chunk(left, c);
+        return counts + std::max(reject_words_layout(e->K, c).bytes + words_bytes(e->K, c * U),
+                                 reject_words_layout(e->K, l).bytes + words_bytes(e->K, l * U));
+      },
+      &bytes);
+  char* buf = chunk ? scratch_alloc(bytes, e->device, stream) : nullptr;
+  gr_status st = GR_OK;
+  if (buf) {
+    int64_t* done = reinterpret_cast<int64_t*>(buf);
+    cudaError_t err = cudaMemsetAsync(done, 0, sizeof(int64_t) * (size_t)e->K, stream);
+    if (err != cudaSuccess) st = cuda_fail(err, "rejection sampler");
+    while (st == GR_OK && left > 0) {
+      const int64_t T = std::min(chunk, left);
+      left -= T;
+      const RwLayout L = reject_words_layout(e->K, T);
+      st = make_words(e, p, T * U, true, buf + counts + L.bytes, stream);
+      if (st != GR_OK) break;
+      err = launch_reject_words(p, dp, rk, e->snap, L, buf + counts, done, stream);
       if (err != cudaSuccess) st = cuda_fail(err, "rejection sampling kernels");
-      cudaFreeAsync(words, stream);
     }
-    cudaFreeAsync(scratch, stream);
     p.words = nullptr;
-    if (!got) break;
+    p.done = done;
   }
   if (st == GR_OK) {
-    p.done = done;
     p.S = 1;
-    err = launch_reject(p, dp, rk, (float)(1.0 / q), max_blocks, stream);
+    const cudaError_t err = launch_reject(p, dp, rk, (float)(1.0 / q), max_blocks, stream);
     if (err != cudaSuccess) st = cuda_fail(err, "rejection sampling kernel");
   }
-  cudaFreeAsync(done, stream);
+  if (buf) cudaFreeAsync(buf, stream);
   return st;
 }
 
@@ -1055,45 +1092,41 @@ gr_status run_chain_call(gr_engine* e, const Plan& p0, const DistParams& wd, int
   int64_t left = (int64_t)std::ceil(per * ((double)npk + (closed ? 0.0 : 8.0 * std::sqrt((double)npk))) * scale) + 64;
   const bool both = (br[0] >> 8) >= 2 && (br[1] >> 8) >= 2;
   Plan p = p0;
-  int64_t* done = nullptr;
-  cudaError_t err = scratch_alloc(reinterpret_cast<void**>(&done), sizeof(int64_t) * (size_t)e->K, e->device, stream);
-  if (err != cudaSuccess) return cuda_fail(err, "scratch memory");
-  err = cudaMemsetAsync(done, 0, sizeof(int64_t) * (size_t)e->K, stream);
-  gr_status st = err == cudaSuccess ? GR_OK : cuda_fail(err, "beta chain");
-  const int64_t chunk = std::max<int64_t>(kChainCap / e->K, 1024);
-  while (st == GR_OK && left > 0) {
-    // what a chunk leaves over (less than one output's packets) is made again
-    const int64_t n = std::min(chunk, left + 64);
-    left -= n - 64;
+  // what a chunk leaves over (less than one output's packets) is made again
+  auto next = [](int64_t c, int64_t l) { return std::min(c, l + 64); };
+  auto layout = [&](int64_t n) {
     const bool seg = n > 8192 && (both ? e->K < 64 : (e->K < 256 || n > 65536));
-    const ChainLayout L = chain_layout(wd, e->K, n, seg ? 1024 : 0);
-    void *words = nullptr, *scratch = nullptr;
-    bool got = false;
-    if (L.bytes) {
-      err = scratch_alloc(&scratch, L.bytes, e->device, stream);
-      if (err != cudaSuccess) {
-        cudaGetLastError();
-        break;
-      }
-    }
-    st = make_words(e, p, n, false, &words, &got, stream);
-    if (st == GR_OK && got) {
-      err = launch_chain(p, wd, L, static_cast<char*>(scratch), done, stream);
+    return chain_layout(wd, e->K, n, seg ? 1024 : 0);
+  };
+  const size_t counts = al256(sizeof(int64_t) * (size_t)e->K);
+  size_t bytes = 0;
+  const int64_t chunk = fit_chunk(
+      e, next(std::max<int64_t>(kChainCap / e->K, 1024), left), 1024,
+      [&](int64_t c) { return counts + chunks_bytes(e->K, left, c, 64, next, layout); }, &bytes);
+  char* buf = chunk ? scratch_alloc(bytes, e->device, stream) : nullptr;
+  gr_status st = GR_OK;
+  if (buf) {
+    int64_t* done = reinterpret_cast<int64_t*>(buf);
+    cudaError_t err = cudaMemsetAsync(done, 0, sizeof(int64_t) * (size_t)e->K, stream);
+    if (err != cudaSuccess) st = cuda_fail(err, "beta chain");
+    while (st == GR_OK && left > 0) {
+      const int64_t n = next(chunk, left);
+      left -= n - 64;
+      const ChainLayout L = layout(n);
+      st = make_words(e, p, n, false, buf + counts + L.bytes, stream);
+      if (st != GR_OK) break;
+      err = launch_chain(p, wd, L, buf + counts, done, stream);
       if (err != cudaSuccess) st = cuda_fail(err, "beta chain kernels");
-      cudaFreeAsync(words, stream);
     }
-    if (scratch) cudaFreeAsync(scratch, stream);
-    p.words = nullptr;
-    if (!got) break;
-  }
-  if (st == GR_OK) {
     p.words = nullptr;
     p.done = done;
+  }
+  if (st == GR_OK) {
     p.S = 1;
-    err = launch_walk(p, wd, max_blocks, stream);
+    const cudaError_t err = launch_walk(p, wd, max_blocks, stream);
     if (err != cudaSuccess) st = cuda_fail(err, "walk sampling kernel");
   }
-  cudaFreeAsync(done, stream);
+  if (buf) cudaFreeAsync(buf, stream);
   return st;
 }
 
@@ -1279,26 +1312,27 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
   // threshold is a few blocks' worth of packets
   const int64_t per_u = half ? (U + 1) / 2 : U;
   if (e->K <= kStagedMaxK && units * per_u > kStagedMin) {
-    const int64_t chunk = std::max<int64_t>(kStagedCap / e->K / per_u, 1);
-    bool started = false;
-    for (int64_t u0 = 0; u0 < units; u0 += chunk) {
-      const int64_t cnt = std::min(chunk, units - u0);
-      void* buf = nullptr;
-      bool got = false;
-      gr_status st = make_words(e, p, half ? (cnt * U + 1) / 2 : cnt * U, true, &buf, &got, stream);
-      if (st != GR_OK) return st;
-      if (!got) {
-        if (started) return fail(GR_ERR_CUDA, "out of memory for the call's scratch");
-        break;
+    auto packets = [&](int64_t cnt) { return half ? (cnt * U + 1) / 2 : cnt * U; };
+    size_t bytes = 0;
+    const int64_t chunk = fit_chunk(
+        e, std::min(std::max<int64_t>(kStagedCap / e->K / per_u, 1), units), 1,
+        [&](int64_t c) {
+          return std::max(words_bytes(e->K, packets(c)), words_bytes(e->K, packets(last_chunk(units, c))));
+        },
+        &bytes);
+    if (char* buf = chunk ? scratch_alloc(bytes, e->device, stream) : nullptr) {
+      gr_status st = GR_OK;
+      for (int64_t u0 = 0; st == GR_OK && u0 < units; u0 += chunk) {
+        const int64_t cnt = std::min(chunk, units - u0);
+        st = make_words(e, p, packets(cnt), true, buf, stream);
+        if (st != GR_OK) break;
+        const cudaError_t err = launch_staged(p, dp, e->snap, U, u0, cnt, stream);
+        if (err != cudaSuccess) st = cuda_fail(err, "staged sampling kernel");
       }
-      started = true;
-      const cudaError_t err = launch_staged(p, dp, e->snap, U, u0, cnt, stream);
       cudaFreeAsync(buf, stream);
-      if (err != cudaSuccess) return cuda_fail(err, "staged sampling kernel");
+      return st;
     }
-    if (started) return GR_OK;
   }
-  p.words = nullptr;
   const cudaError_t err = launch_staged(p, dp, nullptr, U, 0, units, stream);
   if (err != cudaSuccess) return cuda_fail(err, "staged sampling kernel");
   return GR_OK;
@@ -2050,8 +2084,13 @@ gr_status generate_gamma_rows(gr_engine* e, const std::vector<gr_gen*>& gens, Ga
     }
     if (!same && cap != cudaStreamCaptureStatusNone) ok = false;  // the table's upload cannot be captured
     if (ok && !same) {
-      if (!rows.dev)
-        GR_CUDA(scratch_alloc(reinterpret_cast<void**>(&rows.dev), sizeof(TrialRow) * gens.size(), e->device, s));
+      if (!rows.dev && cudaMalloc(&rows.dev, sizeof(TrialRow) * gens.size()) != cudaSuccess) {
+        cudaGetLastError();
+        rows.dev = nullptr;
+        ok = false;
+      }
+    }
+    if (ok && !same) {
       // pageable source: staged before the call returns
       GR_CUDA(cudaMemcpyAsync(rows.dev, tab.data(), sizeof(TrialRow) * gens.size(), cudaMemcpyHostToDevice, s));
       rows.state = state;
