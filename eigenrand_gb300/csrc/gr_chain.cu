@@ -53,8 +53,11 @@ __host__ __device__ constexpr int entry_states() {
   return entry_offsets<R0, R1>() * (R0 ? P : 1) * (R1 ? P : 1);
 }
 
+// An output "adds" to a component's carried lanes unless its draw was one fully
+// accepted trial.  adds[c]: the segment's last such output plus 1; prev[c]: the
+// last segment before it that has one, plus 1 (0: none).
 struct ChainSeg {
-  int32_t nrec, bad;
+  int32_t nrec, bad, adds[2], prev[2];
 };
 
 struct ChainArgs {
@@ -69,6 +72,7 @@ struct ChainArgs {
   ChainSeg* seg;
   int64_t* ebase;
   uint32_t* rec;   // per output packet: x | lanes carried << 24 (component 0), << 27 (component 1)
+  uint16_t* prev;  // [rejection components][K * Sg][L.rcap] the segment's last output before it that adds, plus 1
   int64_t* done;
   int32_t M;       // positions with masks
 };
@@ -207,8 +211,11 @@ __global__ void __launch_bounds__(kVisThreads) k_chain_visits(ChainArgs a) {
 // ---------------------------------------------------------------- the chain
 // One output packet from state (x, f0, f1); v0 / v1: the components' visit
 // entries.  False: a draw the masks do not finish.
+// adds0, adds1: whether the draws add to the carried lanes (one trial that leaves
+// as many was fully accepted: entry == lanes carried).
 template <int P, bool R0, bool R1, class V0, class V1>
-__device__ __forceinline__ bool chain_step(int& x, int& f0, int& f1, int U0, int U1, V0&& v0, V1&& v1) {
+__device__ __forceinline__ bool chain_step(int& x, int& f0, int& f1, int U0, int U1, V0&& v0, V1&& v1, bool& adds0,
+                                           bool& adds1) {
   int y = x + U0, g0 = f0;
   if (R0) {
     const uint32_t e = v0(x, f0);
@@ -216,12 +223,14 @@ __device__ __forceinline__ bool chain_step(int& x, int& f0, int& f1, int U0, int
     if (t == kNoVisit<P>) return false;
     y = x + (t + 1) * U0;
     g0 = P == 1 ? 0 : (int)(e & 7u);
+    adds0 = e != (uint32_t)f0;
   }
   if (R1) {
     const uint32_t e = v1(y, f1);
     const int t = visit_trials<P>(e);
     if (t == kNoVisit<P>) return false;
     y += (t + 1) * U1;
+    adds1 = e != (uint32_t)f1;
     f1 = (int)(e & 7u);
   } else {
     y += U1;
@@ -327,8 +336,8 @@ __global__ void __launch_bounds__(32 * table_warps<P, R0, R1>()) k_chain_table(C
     for (int i = lane; i < na; i += 32) {
       const uint32_t v = st[i];
       int sx = (int)(v & 0xffffu), c0 = (int)((v >> 16) & 255), c1 = (int)(v >> 24);
-      bool ok = v != 0xffffffffu;
-      while (ok && sx < be) ok = chain_step<P, R0, R1>(sx, c0, c1, U0, U1, v0, v1);
+      bool ok = v != 0xffffffffu, adds0, adds1;
+      while (ok && sx < be) ok = chain_step<P, R0, R1>(sx, c0, c1, U0, U1, v0, v1, adds0, adds1);
       const int code = ok ? state_code<P, R0, R1>(sx - be, c0, c1) : kEsc;
       st[i] = code == kEsc ? 0xffffffffu : ((uint32_t)sx | (uint32_t)c0 << 16 | (uint32_t)c1 << 24);
       if (code != kEsc) claim[code] = (uint16_t)i;
@@ -453,7 +462,7 @@ __global__ void __launch_bounds__(32) k_chain_walk(ChainArgs a) {
   } else {
     const int code = a.entry[sg];
     if (code == kEsc) {
-      if (lane == 0) a.seg[sg] = ChainSeg{0, 1};
+      if (lane == 0) a.seg[sg] = ChainSeg{0, 1, {0, 0}, {0, 0}};
       return;
     }
     state_of<P, R0, R1>(code, o, f0, f1);
@@ -472,7 +481,10 @@ __global__ void __launch_bounds__(32) k_chain_walk(ChainArgs a) {
   };
   uint32_t* rec = a.rec + (size_t)sg * a.L.rcap;
   const int want = (int)min(limit_of(a, k), (int64_t)a.L.rcap);
-  int x = lo + o, nrec = 0, bad = 0;
+  // [0]: the first rejection component's, [1]: the second's
+  uint16_t* prev0 = a.prev + (size_t)sg * a.L.rcap;
+  uint16_t* prev1 = prev0 + (NR == 2 ? (size_t)a.p.K * Sg * a.L.rcap : 0);
+  int x = lo + o, nrec = 0, bad = 0, last0 = 0, last1 = 0;
   int tile = x / kTile;
   fetch(tile, 0);
   for (int b = 0;; b ^= 1) {
@@ -488,12 +500,20 @@ __global__ void __launch_bounds__(32) k_chain_walk(ChainArgs a) {
       while (x < stop && nrec < want) {
         const uint32_t r = (uint32_t)x | (uint32_t)f0 << 24 | (uint32_t)f1 << 27;
         int y = x;
-        if (!chain_step<P, R0, R1>(y, f0, f1, U0, U1, v0, v1) || (R0 && !R1 && P > 1 && y > (int)a.L.n)) {
+        bool adds0 = false, adds1 = false;
+        if (!chain_step<P, R0, R1>(y, f0, f1, U0, U1, v0, v1, adds0, adds1) || (R0 && !R1 && P > 1 && y > (int)a.L.n)) {
           bad = 1;
           break;
         }
         x = y;
-        rec[nrec++] = r;
+        rec[nrec] = r;
+        if (P > 1) {
+          if (R0) prev0[nrec] = (uint16_t)last0;
+          if (R1) prev1[nrec] = (uint16_t)last1;
+        }
+        ++nrec;
+        if (adds0) last0 = nrec;
+        if (adds1) last1 = nrec;
       }
       s_x = (bad || nrec >= want || x >= hi) ? -1 : x;
     }
@@ -504,20 +524,22 @@ __global__ void __launch_bounds__(32) k_chain_walk(ChainArgs a) {
     ++tile;
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  if (lane == 0) a.seg[sg] = ChainSeg{nrec, bad};
+  if (lane == 0) a.seg[sg] = ChainSeg{nrec, bad, {last0, last1}, {0, 0}};
 }
 
 // ---------------------------------------------------------------- scan
 __global__ void __launch_bounds__(1024) k_chain_scan(ChainArgs a) {
   __shared__ int64_t s_tot[32];
+  __shared__ int s_top[2][32];
   __shared__ int64_t s_carry;
-  __shared__ int s_bad;
+  __shared__ int s_bad, s_last[2];
   const int k = blockIdx.x, tid = threadIdx.x, Sg = a.L.Sg;
   ChainSeg* seg = a.seg + (size_t)k * Sg;
   int64_t* eb = a.ebase + (size_t)k * (Sg + 1);
   if (tid == 0) {
     s_carry = 0;
     s_bad = INT32_MAX;
+    s_last[0] = s_last[1] = 0;
   }
   __syncthreads();
   for (int s = tid; s < Sg; s += blockDim.x)
@@ -528,25 +550,60 @@ __global__ void __launch_bounds__(1024) k_chain_scan(ChainArgs a) {
     const int s = b + tid;
     const int64_t v = (s < Sg && s <= lastgood) ? seg[s].nrec : 0;
     int64_t x = v;
+    int top[2];  // the last segment up to this one with an output that adds, plus 1
+#pragma unroll
+    for (int c = 0; c < 2; ++c) top[c] = (s < Sg && seg[s].adds[c]) ? s + 1 : 0;
     for (int o = 1; o < 32; o <<= 1) {
       const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if ((tid & 31) >= o) x += y;
+      const int t0 = __shfl_up_sync(0xffffffffu, top[0], o), t1 = __shfl_up_sync(0xffffffffu, top[1], o);
+      if ((tid & 31) >= o) {
+        x += y;
+        top[0] = max(top[0], t0);
+        top[1] = max(top[1], t1);
+      }
     }
-    if ((tid & 31) == 31) s_tot[tid >> 5] = x;
+    if ((tid & 31) == 31) {
+      s_tot[tid >> 5] = x;
+      s_top[0][tid >> 5] = top[0];
+      s_top[1][tid >> 5] = top[1];
+    }
     __syncthreads();
     if (tid < 32) {
-      int64_t t = tid < (int)(blockDim.x >> 5) ? s_tot[tid] : 0;
+      const bool have = tid < (int)(blockDim.x >> 5);
+      int64_t t = have ? s_tot[tid] : 0;
+      int p0 = have ? s_top[0][tid] : 0, p1 = have ? s_top[1][tid] : 0;
       for (int o = 1; o < 32; o <<= 1) {
         const int64_t y = __shfl_up_sync(0xffffffffu, t, o);
-        if (tid >= o) t += y;
+        const int t0 = __shfl_up_sync(0xffffffffu, p0, o), t1 = __shfl_up_sync(0xffffffffu, p1, o);
+        if (tid >= o) {
+          t += y;
+          p0 = max(p0, t0);
+          p1 = max(p1, t1);
+        }
       }
       s_tot[tid] = t;
+      s_top[0][tid] = p0;
+      s_top[1][tid] = p1;
     }
     __syncthreads();
     const int64_t incl = s_carry + x + ((tid >> 5) ? s_tot[(tid >> 5) - 1] : 0);
-    if (s < Sg) eb[s] = incl - v;
+    int before[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int up = __shfl_up_sync(0xffffffffu, top[c], 1);
+      before[c] = max(max(s_last[c], (tid >> 5) ? s_top[c][(tid >> 5) - 1] : 0), (tid & 31) ? up : 0);
+    }
+    if (s < Sg) {
+      eb[s] = incl - v;
+      seg[s].prev[0] = before[0];
+      seg[s].prev[1] = before[1];
+    }
     __syncthreads();
-    if (tid == (int)blockDim.x - 1) s_carry = incl;
+    if (tid == (int)blockDim.x - 1) {
+      s_carry = incl;
+      s_last[0] = max(before[0], top[0]);
+      s_last[1] = max(before[1], top[1]);
+    }
     __syncthreads();
   }
   if (tid == 0) eb[Sg] = s_carry;
@@ -604,23 +661,28 @@ __device__ __forceinline__ int draw_start(const ChainArgs& a, int k, int c, bool
 
 // The lane `dist` places before the end of component c's FIFO as it is before
 // output i of segment s: position and lane of its trial (kEntInit: a lane
-// carried into the call).
+// carried into the call).  From one output that adds lanes to the one before it:
+// output by output, the last lanes of a shape whose trials nearly all are fully
+// accepted took milliseconds.
 template <int DT>
 __device__ __forceinline__ void carried_lane(const ChainArgs& a, int k, int c, bool R0, bool R1, int s, int64_t i, int dist,
                                              uint32_t& pos, int& lane) {
   const Visits v = visits_of<DT>(a, k, c, R0, R1);
+  const ChainSeg* seg = a.seg + (size_t)k * a.L.Sg;
+  const uint16_t* prev = a.prev + (c == 1 && R0 ? (size_t)a.p.K * a.L.Sg * a.L.rcap : 0) + (size_t)k * a.L.Sg * a.L.rcap;
+  int q = i < seg[s].nrec ? prev[(size_t)s * a.L.rcap + i] : seg[s].adds[c];
   for (;;) {
-    while (i == 0 && s > 0) {
-      --s;
-      i = a.seg[(size_t)k * a.L.Sg + s].nrec;
+    if (q == 0) {
+      s = seg[s].prev[c] - 1;
+      if (s < 0) {
+        pos = kEntInit;
+        lane = max(a.p.gen[k].s[1 + c].rest_cnt - dist, 0);
+        return;
+      }
+      q = seg[s].adds[c];
     }
-    if (i == 0) {
-      pos = kEntInit;
-      lane = max(a.p.gen[k].s[1 + c].rest_cnt - dist, 0);
-      return;
-    }
-    --i;
-    const uint32_t r = __ldg(a.rec + ((size_t)k * a.L.Sg + s) * a.L.rcap + i);
+    const size_t at = (size_t)s * a.L.rcap + q - 1;
+    const uint32_t r = __ldg(a.rec + (size_t)k * a.L.Sg * a.L.rcap + at);
     const int x = draw_start<DT>(a, k, c, R0, R1, r), f = (int)((r >> (c ? 27 : 24)) & 7u);
     int last, pushed;
     v.scan(x, f, -1, last, pushed, pos, lane);
@@ -629,6 +691,7 @@ __device__ __forceinline__ void carried_lane(const ChainArgs& a, int k, int c, b
       return;
     }
     dist -= pushed;
+    q = prev[at];
   }
 }
 
@@ -1011,6 +1074,7 @@ ChainLayout layout_of(int K, int64_t n, int64_t M, int32_t J, int P, int NR, int
   L.o_seg = take(segs * sizeof(ChainSeg));
   L.o_ebase = take((segs + K) * 8);
   L.o_rec = take(segs * L.rcap * 4);
+  L.o_prev = take(P > 1 ? segs * L.rcap * 2 * NR : 0);
   L.bytes = o;
   return L;
 }
@@ -1075,9 +1139,11 @@ cudaError_t launch_chain(const Plan& p, const DistParams& d, const ChainLayout& 
   a.ebase = reinterpret_cast<int64_t*>(scratch + L.o_ebase);
   a.vis = reinterpret_cast<uint8_t*>(scratch + L.o_vis);
   a.rec = reinterpret_cast<uint32_t*>(scratch + L.o_rec);
+  a.prev = reinterpret_cast<uint16_t*>(scratch + L.o_prev);
   a.done = done;
   a.M = (int32_t)(L.n - std::max({a.bk.c[0].U, a.bk.c[1].U, 3}) + 1);
   if (a.M <= 0) return cudaSuccess;
+  if (L.ns == 0 && L.mstride && L.rcap > 0xfffe) return cudaErrorInvalidValue;  // 16-bit places (gr_api.cu splits long calls)
   return d.dtype == GR_F64 ? run_chain_types<SD_F64>(a, s) : run_chain_types<SD_F32>(a, s);
 }
 

@@ -176,7 +176,7 @@ struct ChainLayout {
   int32_t rcap;        // output packets per segment
   int32_t groups, gsz; // segment groups of the composition, segments per group
   int64_t mstride;     // positions of a mask array
-  size_t o_mask, o_vis, o_tab, o_gtab, o_entry, o_seg, o_ebase, o_rec, bytes;
+  size_t o_mask, o_vis, o_tab, o_gtab, o_entry, o_seg, o_ebase, o_rec, o_prev, bytes;
 };
 ChainLayout chain_layout(const DistParams& d, int K, int64_t n, int32_t J);
 cudaError_t launch_chain(const Plan& p, const DistParams& d, const ChainLayout& L, char* scratch, int64_t* done,

@@ -199,10 +199,51 @@ __global__ void __launch_bounds__(1024) k_rw_scan(RwArgs a) {
 
 // The FIFO lane `dist` places before the end of the FIFO as it is after trial
 // t: its trial and lane (trial -1: one of the lanes carried into the call).
+//
+// fifo_far: the trials of t's tile are walked backwards, eight at a time where all
+// are fully accepted; a lane of an earlier tile is found by its place in the FIFO,
+// which the counts before each tile bracket.  Trial by trial all the way, shapes
+// whose trials nearly all are fully accepted took up to 220 ms for 2^24 values
+// (beta(1e-4, 1e-4) double; 1.7 ms so), gamma(1e-6) float 20 ms (0.38).
+template <int P>
+__device__ __noinline__ int2 fifo_far(const uint8_t* mk, const int64_t* st, int carried, int t, int dist) {
+  constexpr uint64_t kAllFull = P == 8 ? ~0ull : 0x0f0f0f0f0f0f0f0full;
+  for (;;) {
+    const int tile = t >= 0 ? t / kTileTrials : 0, first = tile * kTileTrials;
+    while (t >= first) {
+      if ((t & 7) == 7 && __ldg(reinterpret_cast<const uint64_t*>(mk + t - 7)) == kAllFull) {
+        t -= 8;
+        continue;
+      }
+      uint32_t m = __ldg(mk + t);
+      const int cn = __popc(m);
+      if (cn != P) {
+        if (dist <= cn) {
+          for (int r = cn - dist; r > 0; --r) m &= m - 1;
+          return make_int2(t, __ffs(m) - 1);
+        }
+        dist -= cn;
+      }
+      --t;
+    }
+    const int64_t q = st[2 * tile + 1] - dist;  // its place in the FIFO
+    if (q < carried) return make_int2(-1, max((int)q, 0));
+    int lo = 0, hi = tile;  // lanes before tile lo <= q < lanes before tile hi
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) / 2;
+      if (st[2 * mid + 1] <= q) lo = mid;
+      else hi = mid;
+    }
+    t = hi * kTileTrials - 1;
+    dist = (int)(st[2 * hi + 1] - q);
+  }
+}
 template <int P>
 __device__ __forceinline__ void fifo_lane(const RwArgs& a, int k, int64_t& t, int64_t dist, int& j) {
   const uint8_t* mk = a.mask + (size_t)k * a.L.mstride;
-  for (; t >= 0; --t) {
+  // ordinary shapes find it a few trials back, in the same tile
+  const int64_t stop = max(t - 16, (t & ~(int64_t)(kTileTrials - 1)) - 1);
+  for (; t > stop; --t) {
     uint32_t m = __ldg(mk + t);
     const int cn = __popc(m);
     if (cn == P) continue;
@@ -213,7 +254,9 @@ __device__ __forceinline__ void fifo_lane(const RwArgs& a, int k, int64_t& t, in
     }
     dist -= cn;
   }
-  j = max(a.p.gen[k].s[0].rest_cnt - (int)dist, 0);
+  const int2 f = fifo_far<P>(mk, a.start + (size_t)k * a.L.tiles * 2, a.p.gen[k].s[0].rest_cnt, (int)t, (int)dist);
+  t = f.x;
+  j = f.y;
 }
 
 template <int RK, int DT>
