@@ -1258,8 +1258,8 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
     if (e->K <= kRejectMaxK && npk >= kRejectMin)
       return run_reject_call(e, p, dp, rk, npk, max_blocks, stream);
     double slack = 0;
-    // the integer samplers accept about half of their candidates
-    const float per_packet = rk <= 2 ? (float)(1.0 / expected_yield(rk, dp, slack)) : 2.0f;
+    // the integer samplers accept somewhat less than half of their candidates
+    const float per_packet = rk <= 2 ? (float)(1.0 / expected_yield(rk, dp, slack)) : 2.4f;
     cudaError_t err = launch_reject(p, dp, rk, per_packet, max_blocks, stream);
     if (err != cudaSuccess) return cuda_fail(err, "rejection sampling kernel");
     return GR_OK;

@@ -905,42 +905,50 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
     const int r = (t >> 5) * G + (t & 31) / P, j = t & (P - 1);
     const int lw = DT == SD_F64 ? j : (j >> 1);  // the lane's 64-bit word
     const int x0 = from + r * L;
+    // the filters decide most positions; a thread then evaluates those they leave
+    // open one after the other (L is 16 at most), or every position in which one of
+    // the warp's lanes is open would cost all of them the reference's expressions
     for (int ci = 0; ci < nrej; ++ci) {
       const int c = nrej == 2 ? ci : rej0;
       const int ty = c == 0 ? type0 : type1;
+      const BetaComp& g = c == 0 ? bk.c[0] : bk.c[1];
+      const int sh = (j & 1) * 32;
+      uint32_t accepted = 0, open = 0;
       uint64_t w0 = 0, w1 = tword(x0, lw), w2 = tword(x0 + 1, lw);
       for (int i = 0; i < L; ++i) {
-        const int x = x0 + i;
-        const bool valid = x < to;
         w0 = w1;
         w1 = w2;
-        w2 = tword(x + 2, lw);
-        bool acc = false;
-        if (valid) {
-          int f = -1;
-          if (DT == SD_F32 && ty == 2) {  // special-function pre-test of a GS trial
-            const BetaComp& g = c == 0 ? bk.c[0] : bk.c[1];
-            const int sh = (j & 1) * 32;
-            f = gs_filter(ur_f((uint32_t)(w0 >> sh)), ur_f((uint32_t)(w1 >> sh)) + 1.1920928955078125e-07f / 8,
-                          ur_f((uint32_t)(w2 >> sh)), g.f_px, g.f_inv, g.f_am1, g.f_band);
-          }
-          if (DT == SD_F64 && ty == 2)
-            f = c == 0 ? gs_filter_f64(w0, w1, w2, bk.c[0].f_px, bk.c[0].f_inv, bk.c[0].f_am1, bk.c[0].f_band)
-                       : gs_filter_f64(w0, w1, w2, bk.c[1].f_px, bk.c[1].f_inv, bk.c[1].f_am1, bk.c[1].f_band);
-          if (f >= 0) {
-            acc = f == 1;
-          } else {
-            auto uf = [&](int q) {
-              const uint64_t v = q == 0 ? w0 : (q == 1 ? w1 : w2);
-              return ur_f((j & 1) ? (uint32_t)(v >> 32) : (uint32_t)v);
-            };
-            auto ud = [&](int q) { return q == 0 ? w0 : (q == 1 ? w1 : w2); };
-            if (c == 0) beta_comp_u<DT, true>(bk.c[0], type0, uf, ud, acc);
-            else beta_comp_u<DT, true>(bk.c[1], type1, uf, ud, acc);
-          }
+        w2 = tword(x0 + i + 2, lw);
+        if (x0 + i >= to) continue;
+        int f;
+        if (DT == SD_F64)
+          f = ty == 2 ? gs_filter_f64(w0, w1, w2, g.f_px, g.f_inv, g.f_am1, g.f_band)
+                      : tan_filter_f64(w0, w1, g.f_am1, g.f_sq);
+        else
+          f = ty == 2 ? gs_filter(ur_f((uint32_t)(w0 >> sh)), ur_f((uint32_t)(w1 >> sh)) + 1.1920928955078125e-07f / 8,
+                                  ur_f((uint32_t)(w2 >> sh)), g.f_px, g.f_inv, g.f_am1, g.f_band)
+                      : tan_filter(ur_f((uint32_t)(w0 >> sh)), ur_f((uint32_t)(w1 >> sh)), g.f_am1, g.f_sq, kTanDeltaF);
+        accepted |= (f == 1 ? 1u : 0u) << i;
+        open |= (f < 0 ? 1u : 0u) << i;
+      }
+      while (__any_sync(FULL, open != 0)) {
+        if (open) {
+          const int i = __ffs(open) - 1;
+          open &= open - 1;
+          const uint64_t v0 = tword(x0 + i, lw), v1 = tword(x0 + i + 1, lw), v2 = tword(x0 + i + 2, lw);
+          auto uf = [&](int q) { return ur_f((uint32_t)((q == 0 ? v0 : (q == 1 ? v1 : v2)) >> sh)); };
+          auto ud = [&](int q) { return q == 0 ? v0 : (q == 1 ? v1 : v2); };
+          bool acc = false;
+          if (c == 0) beta_comp_u<DT, true>(bk.c[0], type0, uf, ud, acc);
+          else beta_comp_u<DT, true>(bk.c[1], type1, uf, ud, acc);
+          accepted |= (acc ? 1u : 0u) << i;
         }
-        const uint32_t bal = __ballot_sync(FULL, acc);
-        if (valid && j == 0)
+        __syncwarp();
+      }
+      for (int i = 0; i < L; ++i) {
+        const int x = x0 + i;
+        const uint32_t bal = __ballot_sync(FULL, (accepted >> i) & 1u);
+        if (x < to && j == 0)
           pmask[(ONE ? 0 : c) * kBetaRing + ((rm + x) & (kBetaRing - 1))] =
               (uint8_t)((bal >> (threadIdx.x & 31 & ~(P - 1))) & ((1u << P) - 1));
       }
@@ -1013,7 +1021,8 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
         if (ONE && !lag) {
           // one look-up per output; every trial of a visit that starts below
           // Mr - 16 Ur has its mask
-          const int pkr = (int)(pk_lim - base), left = (int)min(Npk - cE, (int64_t)kBcRec);
+          const int64_t rest = Npk - cE;
+          const int pkr = (int)(pk_lim - base), left = (int)min(rest, (int64_t)kBcRec);
           int xr = 0, f = cf[rc], At = f;
           while (nrec < left) {
             const int xt = rc == 0 ? xr : xr + Uc;
@@ -1043,6 +1052,35 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
             f = f2;
             xr = xe;
             ++nrec;
+          }
+          // the call's last outputs go trial by trial to the end of the masks: left for
+          // the next step they cost a block, and the way back from it (96 packets of
+          // beta(0.5, 2) on 64 engines, us, float / double: 42 / 49, 29 / 34 so)
+          if (rest - nrec <= 16) {
+#pragma unroll 1
+            while (nrec < left && At + 2 * P <= LB && nf < kBcFull) {
+              const int xt = rc == 0 ? xr : xr + Uc;
+              int nt = 0, acc = 0, full = 0;
+              bool end = false;
+#pragma unroll 1
+              for (int y = xt; y < Mr && nt < 127 && !end; y += Ur) {
+                const int cn = __popc(pmask[(bm + y) & (kBetaRing - 1)]);
+                ++nt;
+                if (cn == P) full = 1;
+                else acc += cn;
+                end = full || f + acc >= P;
+              }
+              const int xe = xr + Uc + nt * Ur;
+              if (!end || xe > pkr) break;
+              if (lane == 0)
+                xrec[q * kBcRec + nrec] = (uint64_t)(uint32_t)(xt | At << 16) |
+                                          (uint64_t)(uint32_t)(nf | (nt | full << 7) << 8 | f << 16) << 32;
+              At += acc;
+              nf += full;
+              f += full ? acc : acc - P;
+              xr = xe;
+              ++nrec;
+            }
           }
           A[rc] = At;
           cf[rc] = f;
