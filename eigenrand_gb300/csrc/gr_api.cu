@@ -13,7 +13,6 @@
 #include <cstring>
 #include <limits>
 #include <map>
-#include <random>
 #include <mutex>
 #include <string>
 #include <tuple>
@@ -814,73 +813,6 @@ gr_status run_fixed(gr_engine* e, Plan p, const DistParams& dp, int64_t packets,
   return GR_OK;
 }
 
-// Fraction of accepted candidate lanes of a rejection family (the expected
-// output packets per trial), estimated once per parameter set on the host by
-// evaluating the acceptance test on 4096 pseudo-random lanes.  Used only to
-// plan how many trials the segments of a long call cover; the result does not
-// depend on it.
-double reject_yield(int rk, const DistParams& d) {
-  static std::mutex mu;
-  static std::map<std::vector<double>, double> cache;
-  const std::vector<double> key = {(double)rk, (double)d.dtype, d.fa, d.fb, d.fc, d.fd, d.fe, d.ff, d.fg, d.fh,
-                                   d.da, d.db, (double)d.ia, (double)d.ib, (double)d.ic};
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = cache.find(key);
-    if (it != cache.end()) return it->second;
-  }
-  std::mt19937_64 rng(0x5eed);
-  auto u = [&]() { return (double)(rng() >> 11) * (1.0 / 9007199254740992.0); };
-  const double pi = 3.14159265358979323846, e1 = 2.7182818284590452;
-  const double alpha = d.dtype == GR_F64 ? d.da : (double)d.fa;
-  const int N = 4096;
-  int acc = 0;
-  for (int i = 0; i < N; ++i) {
-    bool ok = false;
-    if (rk == 0) {  // GammaGen alpha < 1
-      const double ux = u(), vx = u() + 1e-12, ux2 = u();
-      const double lv = std::log(vx);
-      double xx, qx;
-      if (ux < e1 / (alpha + e1)) {
-        xx = std::exp(lv / alpha);
-        qx = std::exp(-xx);
-      } else {
-        xx = 1.0 - lv;
-        qx = std::exp(std::log(xx) * (alpha - 1));
-      }
-      ok = ux2 < qx;
-    } else if (rk == 1) {  // GammaGen tan proposal
-      const double yx = std::tan(pi * u()), ux = u();
-      const double sq = std::sqrt(2 * alpha - 1), xx = sq * yx + (alpha - 1);
-      ok = xx > 0 && ux <= (yx * yx + 1) * std::exp((alpha - 1) * std::log(xx / (alpha - 1)) - yx * sq);
-    } else if (rk == 2) {  // BetaGen a, b < 1
-      const double a = d.dtype == GR_F64 ? d.da : d.fa, b = d.dtype == GR_F64 ? d.db : d.fb;
-      ok = std::pow(u(), 1 / a) + std::pow(u(), 1 / b) <= 1.0;
-    } else if (rk == 3) {  // PoissonGen mean >= 12
-      const double yx = std::tan(pi * u()), u2 = u();
-      const double fres = std::trunc(d.fa * yx + d.fb);
-      ok = fres >= 0 && u2 <= 0.9 * (yx * yx + 1) * std::exp(fres * d.fc - std::lgamma(fres + 1) - d.fd);
-    } else {  // BinomialGen tan proposal
-      const double yx = std::tan(pi * u()), u2 = u();
-      const double fres = std::trunc(d.fa * yx + d.fb);
-      if (fres >= 0 && fres <= d.fh) {
-        const double tt = d.fg - std::lgamma(fres + 1) - std::lgamma(d.fh + 1 - fres) + fres * d.fc + (d.fh - fres) * d.fd;
-        ok = u2 <= 1.2 * d.fa * (1 + yx * yx) * std::exp(tt);
-      }
-    }
-    acc += ok ? 1 : 0;
-  }
-  const double q = std::max((double)acc / N, 1.0 / N);
-  std::lock_guard<std::mutex> lk(mu);
-  cache[key] = q;
-  return q;
-}
-
-// Expected half packets one PoissonGen packetOp consumes (the longest of
-// its four lanes' multiplicative loops, threshold fe = exp(-mean) in float),
-// estimated once per threshold on the host from 4096 simulated packets.  Used
-// only to plan how many segments a long call covers; the result does not
-// depend on it.
 // The engine blocks a rejection or walk kernel may generate in one call
 // (its iteration cap).  GR_MAX_BLOCKS (tests) lowers the cap so that a call
 // runs into it: the kernel stops, records GR_DEV_REJECT_LIMIT in the engine's
@@ -892,35 +824,22 @@ int64_t block_cap(int64_t planned) {
   return c > 0 ? std::min<int64_t>(planned, (int64_t)c) : planned;
 }
 
+// The expected counts below size plans; results do not depend on them.  All are
+// closed forms: found by simulation on the host, once per parameter set, they cost a
+// call with new parameters up to a millisecond.
+
+// Expected half packets one PoissonGen packetOp consumes: 1 more than the
+// largest of its four lanes' Poisson counts (fe = exp(-mean)).
 double poisson_step_halves(float fe) {
-  static std::mutex mu;
-  static std::map<float, double> cache;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = cache.find(fe);
-    if (it != cache.end()) return it->second;
+  const double mean = -std::log((double)fe);
+  double p = fe, F = p, e = 1.0;
+  for (int k = 0; k < 63; ++k) {
+    const double f = std::min(F, 1.0);
+    e += 1.0 - f * f * f * f;
+    p *= mean / (k + 1);
+    F += p;
   }
-  std::mt19937_64 rng(0x5eed);
-  auto u = [&]() { return (float)((double)(rng() >> 40) * (1.0 / 16777216.0)); };
-  const int N = 4096;
-  double tot = 0;
-  for (int i = 0; i < N; ++i) {
-    int L = 0;
-    for (int j = 0; j < 4; ++j) {
-      float v = 1.0f;
-      int it = 0;
-      do {
-        v *= u();
-        ++it;
-      } while (fe < v && it < 64);
-      L = std::max(L, it);
-    }
-    tot += L;
-  }
-  const double m = tot / N;
-  std::lock_guard<std::mutex> lk(mu);
-  cache[fe] = m;
-  return m;
+  return e >= 1.0 ? std::min(e, 64.0) : 64.0;  // a mean outside the sampler's domain: any plan will do
 }
 
 // Probability that a lane of a GammaGen rejection trial is accepted: GS
@@ -1011,13 +930,22 @@ double expected_yield(int rk, const DistParams& d, double& slack) {
   slack = 0;
   const bool f64 = d.dtype == GR_F64;
   if (rk <= 1) return gamma_yield(rk == 0 ? 2 << 8 : 3 << 8, f64 ? d.da : (double)d.fa);
+  double q;
   if (rk == 2) {  // Johnk: G(a + 1) G(b + 1) / G(a + b + 1)
     const double a = f64 ? d.da : (double)d.fa, b = f64 ? d.db : (double)d.fb;
-    const double q = std::tgamma(a + 1) * std::tgamma(b + 1) / std::tgamma(a + b + 1);
-    return q >= 0.1 ? std::min(q, 1.0) : 0.1;
+    q = std::tgamma(a + 1) * std::tgamma(b + 1) / std::tgamma(a + b + 1);
+  } else {
+    // the proposal has the density 1 / (pi s (1 + y^2)), so the chance of each count is
+    // c / (pi s) times its bound without the factor 1 + y^2.  Poisson: c = 0.9, s =
+    // sqrt(2 mean), the bound is the count's probability over that of the mean;
+    // binomial: c / s = 1.2, the bound the count's probability.  Proposals in (-1, 0) count
+    // as 0 too, at a bound that is cut there.
+    slack = 0.04;
+    const double pi = 3.141592653589793, m = d.fb;
+    if (rk == 3) q = m > 1e6 ? 0.5078 : 0.9 / (pi * d.fa) * std::exp(m - m * std::log(m) + std::lgamma(m + 1));
+    else q = 1.2 / pi * (1.0 + 0.8 * std::exp((double)d.fh * d.fd));
   }
-  slack = 0.04;
-  return reject_yield(rk, d);
+  return q >= 0.1 ? std::min(q, 1.0) : 0.1;
 }
 
 // Rejection samplers through words in memory (gr_rejw.cu), then the
@@ -1258,8 +1186,8 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
     if (e->K <= kRejectMaxK && npk >= kRejectMin)
       return run_reject_call(e, p, dp, rk, npk, max_blocks, stream);
     double slack = 0;
-    // the integer samplers accept somewhat less than half of their candidates
-    const float per_packet = rk <= 2 ? (float)(1.0 / expected_yield(rk, dp, slack)) : 2.4f;
+    // (the integer samplers' with a margin: their batches are short)
+    const float per_packet = (float)((rk <= 2 ? 1.0 : 1.2) / expected_yield(rk, dp, slack));
     cudaError_t err = launch_reject(p, dp, rk, per_packet, max_blocks, stream);
     if (err != cudaSuccess) return cuda_fail(err, "rejection sampling kernel");
     return GR_OK;
@@ -2327,7 +2255,8 @@ gr_status sengine_reject(gr_sengine* se, const DistParams& dp, int rk, void* out
   const int64_t wpt = (rk == 0 ? 3 : 2) * (dt == GR_F32 ? 3 : 4);
   const int64_t need = (int64_t)(n / (size_t)P);
   const int64_t mcap = kTruncChunkMax - 1;
-  const double q = reject_yield(rk, dp);
+  double slack;
+  const double q = expected_yield(rk, dp, slack);
   char* buf = nullptr;
   int64_t have_m = 0;
   auto layout = [&](int64_t m, size_t off[8]) {

@@ -1,0 +1,53 @@
+"""Calls whose parameters no call had before: the plans' expected counts are closed
+forms, so such a call takes the host no longer than another (a simulation per
+parameter set took up to a millisecond), and the plans they size give the same
+values, against the oracle, where the expectation is least exact: binomial at
+means near 1, Poisson at 12 and at a large mean."""
+import time
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA GPU", allow_module_level=True)
+
+
+@pytest.mark.parametrize("kind,lo,hi,t", [("POISSON", 1.0, 11.0, 0), ("POISSON", 13.0, 200.0, 0), ("BINOMIAL", 0.1, 0.9, 100)])
+def test_host_time(gpulib, kind, lo, hi, t):
+    er = gpulib
+    u = er.Vmt19937_64(4)
+    out = torch.empty(4 * 2000, 1, dtype=torch.int32, device="cuda")
+
+    def per_call(params):
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        for a in params:
+            er._sample(kind, 4 * 2000, 1, u, torch.int32, float(a), 0.0, t, out=out)
+        torch.cuda.synchronize()
+        return (time.perf_counter() - t0) / len(params)
+
+    fresh = np.linspace(lo, hi, 150)
+    per_call(fresh[:5])
+    new = per_call(fresh[5:])
+    again = per_call(fresh[5:])
+    assert new < 2 * again + 20e-6
+
+
+@pytest.mark.parametrize("kind,a,t", [("BINOMIAL", 0.04, 25), ("BINOMIAL", 0.01, 100), ("BINOMIAL", 0.0025, 1000),
+                                      ("BINOMIAL", 0.96, 30), ("POISSON", 12.0, 0), ("POISSON", 2e5, 0), ("POISSON", 0.01, 0)])
+@pytest.mark.parametrize("streams,calls", [(1, (70000, 4000, 9)), (400, (96, 200, 3))])
+def test_values(gpulib, oracle, kind, a, t, streams, calls):
+    er = gpulib
+    u = er.Vmt19937_64(19, streams=streams)
+    g = er._Gen(torch.int32, a, 0.0, trials=t, kind=kind)
+    which = sorted({0, streams - 1})
+    es = {k: (oracle.Engine(19 + 4 * k), oracle.Gen()) for k in which}
+    for pk in calls:
+        n = 4 * pk
+        out = g.generate(n * streams, 1, u).reshape(-1).cpu().numpy()
+        for k in which:
+            assert np.array_equal(out[k * n:(k + 1) * n], oracle.generate(*es[k], kind, n, np.int32, a, 0.0, t))
+    u.sync()
