@@ -760,27 +760,87 @@ gr_status make_words(gr_engine* e, Plan& p, int64_t n, bool first, char* buf, cu
   return GR_OK;
 }
 
-// Packets per engine above which a fixed-draw call on few engines goes through
-// words in memory.  One CTA per engine spends 0.9 us (bit conversions), 3 us
-// (float log, sincos) or 25 us (their double forms) per 312 packets; the
-// second launch and the scratch take about 6 us.  One engine, 2 048 packets:
-// float uniform 11.8 us fused and 13.6 us through memory, float normal 21.4
-// and 14.7, double normal (4 096 packets) 152 and 21; 131 072 values: 43 and
-// 17, 118 and 18, 1146 and 28.
-int64_t words_from(const DistParams& dp) {
+// Which calls go through words in memory.  One CTA per engine costs a fixed 4 to
+// 15 us and then a time per packet that does not depend on the engine count K (up
+// to one CTA per SM); the way through memory costs 11 us (fixed draws) to 90 us
+// (beta) and then little per packet on one engine, but in proportion to K.  So
+// each kind has a size from which the second is faster, which grows with K, and
+// an engine count from which it never is.  Sizes where both take the same time,
+// measured with each path forced, on 1 / 32 / 64 / 128 engines (-: none):
+//   packets    uniform f32 4 860 / 9 766 / - / -, f64 3 636 / 4 824 / 8 529 / -; normal f32
+//              1 707 / 2 119 / 2 733 / 6 179, exponential f32 1 726 / 2 146 / 3 413 /
+//              8 192; normal f64 455 / 512 / 518 / 812, exponential f64 901 / 843 / 1 050 /
+//              1 676
+//   units      gamma(2) f32 563 / 779 / 1 102 / 3 543, gamma(5) f32 384 / 400 / 582 / 1 581, f64
+//              219 / 201 / 256 / 512, gamma(19) f32 145 / 164 / 172 / 269, f64 53 / 53 / 61 / 64;
+//              Student t f64 164 / 161 / 194 / 202; binomial of 1 trial 2 338 / 3 134 /
+//              4 548 / -, of 20 320 / 327 / 445 / 1 053
+//   outputs    gamma(0.5) f32 977 / 1 094 / 1 276 / 2 325, f64 592 / 672 / 729 / 933; gamma(2.5)
+//   (packets)  f32 688 / 750 / 890 / 1 435, f64 422 / 476 / 531 / 815; beta(0.4, 0.7) f32 1 276 /
+//              1 494 / 2 048 / 5 015, f64 770 / 922 / 1 210 / 4 096; Poisson(100) 982 / 1 174 /
+//              1 507 / 2 805; binomial(100, 0.3) 542 / 630 / 771 / 1 229
+//              Poisson(0.5) 3 315 / 3 342 / 3 375 / 3 415, (4) 658 / 775 / 796 / 839, (11.9) 113 /
+//              128 / 148 / 177
+//              beta(0.5, 2) f32 572 / 725 / 904 / 1 177, f64 453 / 454 / 512 / 710; beta(0.05, 19)
+//              103 / 116 / 128 / 274; beta(3, 2.5) 140 / 160 / 166 / 192; beta(2.5, 1.5) f32 41 / 47 /
+//              47 / 66, f64 46 / 56 / 65 / 74; beta(1, 3) 58 / 71 / 75 / 76
+constexpr int64_t kNever = INT64_MAX;
+
+// base (1 + K^2 / k2) up to `most` engines, rounded down.
+int64_t grown(double base, int K, double k2, int most) {
+  return K > most ? kNever : (int64_t)(base * (1.0 + (double)K * K / k2));
+}
+
+// Packets per engine above which a fixed-draw call does.
+int64_t words_from(const DistParams& dp, int K) {
   const int k = dp.kind >= kVecBase ? dp.kind - kVecBase : dp.kind;
+  const bool f64 = dp.dtype == GR_F64;
+  const bool balanced = k == GR_BALANCED || k == GR_BALANCED2;
   const bool light = k == kRawKind || k == kRawLane0Kind || k == GR_UNIFORM_REAL || k == GR_UNIFORM_REAL2 ||
-                     k == GR_BALANCED || k == GR_BALANCED2 || k == GR_BERNOULLI || k == kBernoulliVKind ||
-                     k == GR_RANDBITS || k == GR_UNIFORM_INT;
-  if (light) return 2560;
-  return dp.dtype == GR_F64 ? 156 : 624;
+                     (balanced && !f64) || k == GR_BERNOULLI || k == kBernoulliVKind || k == GR_RANDBITS ||
+                     k == GR_UNIFORM_INT;
+  if (light) return K > 64 ? kNever : f64 ? 3600 + 64 * K : 5000 + 180 * K;
+  if (K > 127) return kNever;
+  return f64 && !balanced ? 450 + 5 * K / 2 : 1500 + 16 * K;
+}
+
+// Units per engine above which a call of fixed units of U packets (half packets for the
+// int32 kind) does.
+int64_t units_from(const DistParams& dp, int U, int K) {
+  if (dp.dtype == GR_I32) return grown(6900.0 / (U + 1.5), K, 8000, 96);
+  if (dp.dtype == GR_F32) return grown(4200.0 / (U + 6), K, 8000, 128);
+  return grown(dp.kind == GR_STUDENT_T ? 165.0 : 1100.0 / U, K, 20000, 128);
+}
+
+// Output packets per engine above which a call of a CompressMask rejection sampler does.
+int64_t reject_from(int rk, bool f64, int K) {
+  if (rk == 2) return grown(f64 ? 780 : 1300, K, 4000, 128);
+  if (f64) return grown(rk == 0 ? 600 : 430, K, 30000, 256);
+  return grown(rk == 0 || rk == 3 ? 1000 : rk == 1 ? 700 : 560, K, 12000, 192);
+}
+
+// ... of Poisson's walk; halves: half packets per step.
+int64_t poisson_from(double halves, int K) {
+  return (int64_t)(std::min(3400.0, 36000.0 / (halves * halves)) * (1.0 + K / 512.0));
+}
+
+// Packets per engine (expected draws) above which a call of beta's general branch does;
+// t0, t1: the components' sampler types.
+int64_t chain_from(int t0, int t1, bool f64, int K) {
+  const bool r0 = t0 >= 2, r1 = t1 >= 2;
+  if (!r0 && !r1) return grown(300, K, 50000, 256);
+  if (r0 && r1) return grown(470, K, 50000, 256);
+  if ((r0 ? t0 : t1) == 3) return grown(f64 ? 1150 : 1000, K, 40000, 256);
+  // GS: with an integral shape the one-CTA kernel is a special one
+  if ((r0 ? t1 : t0) == 0) return grown(2100, K, 15000, 192);
+  return grown(f64 ? 2800 : 3200, K, 15000, 192);
 }
 
 // A fixed-draw kind (launch_direct) over `packets` packets per engine at
 // most, whole units of ppu packets.
 gr_status run_fixed(gr_engine* e, Plan p, const DistParams& dp, int64_t packets, int ppu, cudaStream_t stream,
                     const char* what) {
-  if (e->K < 128 && packets > words_from(dp) && p.out) {
+  if (packets > words_from(dp, e->K) && p.out) {
     size_t bytes = 0;
     const int64_t most = std::min(kWordsCap / e->K, packets + 1) & ~(int64_t)1;
     const int64_t chunk = fit_chunk(
@@ -859,8 +919,6 @@ double gamma_yield(int branch, double a) {
 }
 
 // Fixed units over words in memory.
-constexpr int64_t kStagedMin = 624;               // packets per engine
-constexpr int kStagedMaxK = 128;                  // engines
 constexpr int64_t kStagedCap = (int64_t)1 << 22;  // packets of words at a time, all engines
 
 // Scratch of a chain's chunks, of which each makes `again` of its packets once
@@ -880,7 +938,6 @@ size_t chunks_bytes(int K, int64_t left, int64_t chunk, int64_t again, Next&& ne
 
 // PoissonGen's walk through words in memory (gr_chain.cu), then the one-CTA
 // walk for whatever the planned packets did not hold.
-constexpr int64_t kPoisMin = 512;               // output packets per engine
 constexpr int64_t kPoisCap = (int64_t)1 << 22;  // packets of words at a time, all engines
 gr_status run_poisson_call(gr_engine* e, const Plan& p0, const DistParams& wd, int64_t npk, int64_t max_blocks,
                            cudaStream_t stream) {
@@ -951,8 +1008,6 @@ double expected_yield(int rk, const DistParams& d, double& slack) {
 // Rejection samplers through words in memory (gr_rejw.cu), then the
 // one-CTA-per-engine kernel for whatever the planned trials did not make
 // (usually nothing).
-constexpr int64_t kRejectMin = 512;              // output packets per engine
-constexpr int kRejectMaxK = 256;                 // engines
 constexpr int64_t kRejectCap = (int64_t)1 << 23;  // packets of words at a time, all engines
 gr_status run_reject_call(gr_engine* e, const Plan& p0, const DistParams& dp, int rk, int64_t npk, int64_t max_blocks,
                           cudaStream_t stream) {
@@ -1005,15 +1060,19 @@ gr_status run_reject_call(gr_engine* e, const Plan& p0, const DistParams& dp, in
 // BetaGen's general branch through words in memory (gr_chain.cu), then the
 // one-CTA-per-engine walk for whatever the planned packets did not hold
 // (usually nothing).  The expected packets per output only size the plan.
-constexpr int64_t kChainMin = 192;              // output packets per engine
-constexpr int kChainMaxK = 256;                 // engines
-constexpr int64_t kChainCap = (int64_t)1 << 23;  // packets of words at a time, all engines
-gr_status run_chain_call(gr_engine* e, const Plan& p0, const DistParams& wd, int64_t npk, int64_t max_blocks,
-                         cudaStream_t stream) {
+// Expected packets per output packet.
+double chain_packets(const DistParams& wd) {
   const int br[2] = {wd.ia, wd.ib};
   const double al[2] = {wd.da, wd.db};
   double per = 0;
   for (int c = 0; c < 2; ++c) per += (br[c] & 255) / ((br[c] >> 8) >= 2 ? gamma_yield(br[c], al[c]) : 1.0);
+  return per;
+}
+constexpr int64_t kChainCap = (int64_t)1 << 23;  // packets of words at a time, all engines
+gr_status run_chain_call(gr_engine* e, const Plan& p0, const DistParams& wd, int64_t npk, int64_t max_blocks,
+                         cudaStream_t stream) {
+  const int br[2] = {wd.ia, wd.ib};
+  const double per = chain_packets(wd);
   const char* sc = std::getenv("GR_WALK_PLAN_SCALE");  // tests: see run_packets
   const double scale = sc ? std::max(0.0, std::atof(sc)) : 1.0;
   const bool closed = (br[0] >> 8) < 2 && (br[1] >> 8) < 2;
@@ -1183,7 +1242,7 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
     const int64_t wt = rk == 0 ? 24 : (rk >= 3 ? 8 : 16);  // words per trial
     const int64_t npk = nk_max / P;
     const int64_t max_blocks = block_cap(((16 * npk + 4096) * wt) / (kN * 8) + 64);
-    if (e->K <= kRejectMaxK && npk >= kRejectMin)
+    if (npk > reject_from(rk, dp.dtype == GR_F64, e->K))
       return run_reject_call(e, p, dp, rk, npk, max_blocks, stream);
     double slack = 0;
     // (the integer samplers' with a margin: their batches are short)
@@ -1212,7 +1271,8 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
       wd.ia = dp.kind == GR_BINOMIAL ? dp.ia : 0;
       wd.ic = dp.kind == GR_BINOMIAL ? dp.ib : 0;
       max_blocks = block_cap((npk * 64) / (2 * kN) + 64);
-      if (e->K <= kChainMaxK && npk >= kPoisMin) return run_poisson_call(e, p, wd, npk, max_blocks, stream);
+      if (e->K <= 256 && npk > 100 && npk > poisson_from(poisson_step_halves(wd.fe), e->K))
+        return run_poisson_call(e, p, wd, npk, max_blocks, stream);
     } else {
       const bool f32 = dp.dtype == GR_F32;
       wd.ia = gamma_branch(dp.da, f32);
@@ -1220,7 +1280,8 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
       wd.fa = (float)dp.da;
       wd.fb = (float)dp.db;
       max_blocks = (npk * 64) / kN + 64;
-      if (npk >= kChainMin && e->K <= kChainMaxK) return run_chain_call(e, p, wd, npk, block_cap(max_blocks), stream);
+      if (e->K <= 256 && (double)npk * chain_packets(wd) > (double)chain_from(wd.ia >> 8, wd.ib >> 8, !f32, e->K))
+        return run_chain_call(e, p, wd, npk, block_cap(max_blocks), stream);
     }
     max_blocks = block_cap(max_blocks);
     cudaError_t err = launch_walk(p, wd, max_blocks, stream);
@@ -1236,10 +1297,8 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
   if (dp.kind == GR_STUDENT_T) U = 2;
   if (dp.kind == GR_BINOMIAL) U = dp.ia;
   const int64_t units = nk_max / P;
-  // few engines: words in memory.  A unit is U words and one value, so the
-  // threshold is a few blocks' worth of packets
   const int64_t per_u = half ? (U + 1) / 2 : U;
-  if (e->K <= kStagedMaxK && units * per_u > kStagedMin) {
+  if (units > units_from(dp, (int)U, e->K)) {
     auto packets = [&](int64_t cnt) { return half ? (cnt * U + 1) / 2 : cnt * U; };
     size_t bytes = 0;
     const int64_t chunk = fit_chunk(
