@@ -40,6 +40,7 @@ EXPORTS = [
     "gr_truncmvn_create", "gr_truncmvn_sample", "gr_truncmvn_destroy",
     "gr_server_create", "gr_server_set_mvnormal", "gr_server_submit", "gr_server_progress", "gr_server_read",
     "gr_server_release", "gr_server_cancel", "gr_server_cancel_client", "gr_server_fail_allocs", "gr_server_pending",
+    "gr_server_memory",
     "gr_server_now", "gr_server_destroy",
 ]
 
@@ -173,6 +174,7 @@ def load(path=None):
         "gr_server_cancel_client": (i32, [vp, i32]),
         "gr_server_fail_allocs": (i32, [vp, i32]),
         "gr_server_pending": (i32, [vp, ctypes.POINTER(sz), ctypes.POINTER(sz), ctypes.POINTER(sz)]),
+        "gr_server_memory": (i32, [vp, ctypes.POINTER(sz)]),
         "gr_server_now": (ctypes.c_double, []),
         "gr_server_destroy": (i32, [vp]),
         "gr_last_error": (ctypes.c_char_p, []),

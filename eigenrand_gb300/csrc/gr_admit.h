@@ -3,11 +3,16 @@
 // Requests queue in arrival order.  One pass of admit() starts, in that
 // order, every request whose client has nothing running or queued ahead of
 // it (a client's engine is sequential, so its requests run one at a time and
-// in order), whose output fits in what is left of the device-memory budget,
-// while stream slots are free.  A request that does not fit is skipped
+// in order), whose output and scratch fit in what is left of the device-memory
+// budget, while stream slots are free.  A request that does not fit is skipped
 // (later, smaller requests of other clients go ahead) until it has waited
 // longer than starve_s; from then on nothing behind it is admitted until it
 // fits.  Memory is held from admission until the caller releases the result.
+// A request may ask for scratch besides, which it holds until its work is done.
+// It waits for it only while other requests run, whose end gives scratch back:
+// with none running it starts with what the held results leave (admit() says how
+// much), so a caller that keeps results never waits for memory that only its own
+// release would free.
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -21,6 +26,7 @@ struct AdmitReq {
   int client;
   size_t bytes;
   double arrival;  // seconds
+  size_t scratch = 0;
 };
 
 class Admission {
@@ -45,16 +51,20 @@ class Admission {
         ++it;
         continue;
       }
-      if (used_ + r.bytes > budget_) {
+      size_t scratch = r.scratch;
+      if (running_ == 0 && used_ + r.bytes <= budget_) scratch = scratch < budget_ - used_ - r.bytes ? scratch : budget_ - used_ - r.bytes;
+      if (used_ + r.bytes + scratch > budget_) {
         blocked[r.client] = 1;
         if (now - r.arrival > starve_s_) break;  // hold everything behind it back
         ++it;
         continue;
       }
-      used_ += r.bytes;
+      used_ += r.bytes + scratch;
       busy_[r.client] = 1;
+      ++running_;
       --free_slots_;
       out.push_back(r);
+      out.back().scratch = scratch;
       it = queue_.erase(it);
     }
     return out;
@@ -73,6 +83,7 @@ class Admission {
   // the request's GPU work is done: its slot and its client are free again
   void finish(int client) {
     busy_[client] = 0;
+    --running_;
     ++free_slots_;
   }
   // the request's memory is given back
@@ -88,6 +99,7 @@ class Admission {
   std::vector<char> busy_;
   size_t budget_;
   size_t used_ = 0;
+  int running_ = 0;
   int free_slots_;
   double starve_s_;
 };

@@ -140,11 +140,11 @@ void scratch_engine(int dev, int delta) {
 }
 // A call's scratch: one allocation, taken before its first launch, so that a call
 // that has started cannot run out.  Null: none to be had, and the call takes the
-// path that needs none.  Test hook: GR_SCRATCH_FAIL, if set, makes it null.
-char* scratch_alloc(size_t bytes, int dev, cudaStream_t s) {
+// path that needs none.  pool: taken from there rather than from the library's.
+// Test hook: GR_SCRATCH_FAIL, if set, makes it null.
+char* scratch_alloc(size_t bytes, int dev, cudaMemPool_t pool, cudaStream_t s) {
   if (std::getenv("GR_SCRATCH_FAIL")) return nullptr;
-  cudaMemPool_t pool = nullptr;
-  {
+  if (!pool) {
     ScratchPools& sp = scratch_pools();
     std::lock_guard<std::mutex> lk(sp.mu);
     pool = scratch_pool(sp, dev);
@@ -169,7 +169,10 @@ struct gr_engine {
   size_t segwin_words = 0;
   CallSnap* snap = nullptr;         // in st's allocation, behind the states
   GenState* scratch_gen = nullptr;  // caches of temporary generators (gr_sample)
-  size_t scratch_cap = SIZE_MAX;    // most bytes of scratch a call takes
+  // most bytes of scratch a call takes, and the pool it takes them from (null: the
+  // library's); set by the serving loop
+  size_t scratch_cap = SIZE_MAX;
+  cudaMemPool_t scratch_pool = nullptr;
   uint64_t* tailw = nullptr;        // draws of a call's partial last packet
 };
 
@@ -661,6 +664,10 @@ constexpr int64_t kWordsCap = (int64_t)1 << 22;  // packets of all engines in a 
 
 constexpr size_t al256(size_t x) { return (x + 255) / 256 * 256; }
 
+// A call whose scratch is limited to less than this many packets or trials at a time
+// takes the path that needs none: several launches a chunk would cost more.
+constexpr int64_t kLeastChunk = 4096;
+
 // What chunks of c leave for the last one.
 constexpr int64_t last_chunk(int64_t total, int64_t c) { return total - (total - 1) / c * c; }
 
@@ -837,20 +844,22 @@ int64_t chain_from(int t0, int t1, bool f64, int K) {
 }
 
 // A fixed-draw kind (launch_direct) over `packets` packets per engine at
-// most, whole units of ppu packets.
+// most, whole units of ppu packets.  want (here and below), if given: only the
+// bytes of scratch the call would take.
 gr_status run_fixed(gr_engine* e, Plan p, const DistParams& dp, int64_t packets, int ppu, cudaStream_t stream,
-                    const char* what) {
+                    const char* what, size_t* want = nullptr) {
   if (packets > words_from(dp, e->K) && p.out) {
     size_t bytes = 0;
     const int64_t most = std::min(kWordsCap / e->K, packets + 1) & ~(int64_t)1;
     const int64_t chunk = fit_chunk(
-        e, most, 1024,
+        e, most, words_from(dp, e->K) + 1,
         [&](int64_t c) {
           c &= ~(int64_t)1;
           return std::max(words_bytes(e->K, c), words_bytes(e->K, last_chunk(packets, c)));
         },
         &bytes) & ~(int64_t)1;
-    if (char* buf = chunk ? scratch_alloc(bytes, e->device, stream) : nullptr) {
+    if (want) *want = chunk ? bytes : 0;
+    if (char* buf = chunk && !want ? scratch_alloc(bytes, e->device, e->scratch_pool, stream) : nullptr) {
       gr_status st = GR_OK;
       for (int64_t at = 0; st == GR_OK && at < packets; at += chunk) {
         st = make_words(e, p, std::min(chunk, packets - at), at == 0, buf, stream);
@@ -863,6 +872,7 @@ gr_status run_fixed(gr_engine* e, Plan p, const DistParams& dp, int64_t packets,
       return st;
     }
   }
+  if (want) return GR_OK;
   int S;
   int64_t J;
   plan_segments(e, packets, ppu, S, J);
@@ -940,7 +950,7 @@ size_t chunks_bytes(int K, int64_t left, int64_t chunk, int64_t again, Next&& ne
 // walk for whatever the planned packets did not hold.
 constexpr int64_t kPoisCap = (int64_t)1 << 22;  // packets of words at a time, all engines
 gr_status run_poisson_call(gr_engine* e, const Plan& p0, const DistParams& wd, int64_t npk, int64_t max_blocks,
-                           cudaStream_t stream) {
+                           cudaStream_t stream, size_t* want = nullptr) {
   const char* sc = std::getenv("GR_WALK_PLAN_SCALE");  // tests: see run_chain_call
   const double scale = sc ? std::max(0.0, std::atof(sc)) : 1.0;
   const double hl = poisson_step_halves(wd.fe);
@@ -952,9 +962,13 @@ gr_status run_poisson_call(gr_engine* e, const Plan& p0, const DistParams& wd, i
   const size_t counts = al256(sizeof(int64_t) * (size_t)e->K);
   size_t bytes = 0;
   const int64_t chunk = fit_chunk(
-      e, next(std::max<int64_t>(kPoisCap / e->K, 512) & ~(int64_t)1, left), 512,
+      e, next(std::max<int64_t>(kPoisCap / e->K, 512) & ~(int64_t)1, left), kLeastChunk,
       [&](int64_t c) { return counts + chunks_bytes(e->K, left, c & ~(int64_t)1, 32, next, layout); }, &bytes) & ~(int64_t)1;
-  char* buf = chunk ? scratch_alloc(bytes, e->device, stream) : nullptr;
+  if (want) {
+    *want = chunk ? bytes : 0;
+    return GR_OK;
+  }
+  char* buf = chunk ? scratch_alloc(bytes, e->device, e->scratch_pool, stream) : nullptr;
   gr_status st = GR_OK;
   if (buf) {
     int64_t* done = reinterpret_cast<int64_t*>(buf);
@@ -1010,7 +1024,7 @@ double expected_yield(int rk, const DistParams& d, double& slack) {
 // (usually nothing).
 constexpr int64_t kRejectCap = (int64_t)1 << 23;  // packets of words at a time, all engines
 gr_status run_reject_call(gr_engine* e, const Plan& p0, const DistParams& dp, int rk, int64_t npk, int64_t max_blocks,
-                          cudaStream_t stream) {
+                          cudaStream_t stream, size_t* want = nullptr) {
   double slack = 0;
   const double q = expected_yield(rk, dp, slack);
   // GR_REJECT_PLAN_SCALE (tests) scales the planned trials; below 1 the
@@ -1023,14 +1037,18 @@ gr_status run_reject_call(gr_engine* e, const Plan& p0, const DistParams& dp, in
   const size_t counts = al256(sizeof(int64_t) * (size_t)e->K);
   size_t bytes = 0;
   const int64_t chunk = fit_chunk(
-      e, std::min(std::max<int64_t>(kRejectCap / e->K / U, 64), left), 64,
+      e, std::min(std::max<int64_t>(kRejectCap / e->K / U, 64), left), kLeastChunk,
       [&](int64_t c) {
         const int64_t l = last_chunk(left, c);
         return counts + std::max(reject_words_layout(e->K, c).bytes + words_bytes(e->K, c * U),
                                  reject_words_layout(e->K, l).bytes + words_bytes(e->K, l * U));
       },
       &bytes);
-  char* buf = chunk ? scratch_alloc(bytes, e->device, stream) : nullptr;
+  if (want) {
+    *want = chunk ? bytes : 0;
+    return GR_OK;
+  }
+  char* buf = chunk ? scratch_alloc(bytes, e->device, e->scratch_pool, stream) : nullptr;
   gr_status st = GR_OK;
   if (buf) {
     int64_t* done = reinterpret_cast<int64_t*>(buf);
@@ -1070,7 +1088,7 @@ double chain_packets(const DistParams& wd) {
 }
 constexpr int64_t kChainCap = (int64_t)1 << 23;  // packets of words at a time, all engines
 gr_status run_chain_call(gr_engine* e, const Plan& p0, const DistParams& wd, int64_t npk, int64_t max_blocks,
-                         cudaStream_t stream) {
+                         cudaStream_t stream, size_t* want = nullptr) {
   const int br[2] = {wd.ia, wd.ib};
   const double per = chain_packets(wd);
   const char* sc = std::getenv("GR_WALK_PLAN_SCALE");  // tests: see run_packets
@@ -1088,9 +1106,13 @@ gr_status run_chain_call(gr_engine* e, const Plan& p0, const DistParams& wd, int
   const size_t counts = al256(sizeof(int64_t) * (size_t)e->K);
   size_t bytes = 0;
   const int64_t chunk = fit_chunk(
-      e, next(std::max<int64_t>(kChainCap / e->K, 1024), left), 1024,
+      e, next(std::max<int64_t>(kChainCap / e->K, 1024), left), kLeastChunk,
       [&](int64_t c) { return counts + chunks_bytes(e->K, left, c, 64, next, layout); }, &bytes);
-  char* buf = chunk ? scratch_alloc(bytes, e->device, stream) : nullptr;
+  if (want) {
+    *want = chunk ? bytes : 0;
+    return GR_OK;
+  }
+  char* buf = chunk ? scratch_alloc(bytes, e->device, e->scratch_pool, stream) : nullptr;
   gr_status st = GR_OK;
   if (buf) {
     int64_t* done = reinterpret_cast<int64_t*>(buf);
@@ -1117,7 +1139,8 @@ gr_status run_chain_call(gr_engine* e, const Plan& p0, const DistParams& wd, int
   return st;
 }
 
-gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, size_t n, cudaStream_t stream);
+gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, size_t n, cudaStream_t stream,
+                      size_t* want = nullptr);
 
 // The n % P elements after the last whole packet of a call: the scalar
 // operator(), one engine packet each, drawn from the last stream (whose slice
@@ -1197,7 +1220,9 @@ gr_status run_call(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, siz
   return run_tail(e, dp, static_cast<char*>(out) + whole * es, r, stream);
 }
 
-gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, size_t n, cudaStream_t stream) {
+gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, size_t n, cudaStream_t stream,
+                      size_t* want) {
+  if (want) *want = 0;
   const int gran = kind_granule(dp.kind, dp.dtype);
   if (n % (size_t)gran) {
     return fail(GR_ERR_INVALID, "size must be a multiple of " + std::to_string(gran) +
@@ -1209,6 +1234,7 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
   if (fam == Family::Unsupported) return fail(GR_ERR_UNSUPPORTED, "this parameter set is not implemented yet");
   if (dp.kind == GR_BINOMIAL && dp.ia <= 0) {
     // BinomialGen with 0 trials draws nothing and returns 0 (Discrete.h:1000-1009)
+    if (want) return GR_OK;
     GR_CUDA(cudaMemsetAsync(out, 0, n * sizeof(int32_t), stream));
     return GR_OK;
   }
@@ -1232,18 +1258,19 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
     const int ppu = kind_packets_per_unit(dp.kind, dp.dtype);
     int64_t packets_max = (nk_max + opp - 1) / opp;
     if (ppu == 2) packets_max += packets_max & 1;
-    return run_fixed(e, p, dp, packets_max, ppu, stream, "sampling kernel");
+    return run_fixed(e, p, dp, packets_max, ppu, stream, "sampling kernel", want);
   }
 
   if (fam == Family::Reject) {
-    if (!p.gen) return fail(GR_ERR_INVALID, "rejection samplers need a generator state");
+    if (!p.gen && !want) return fail(GR_ERR_INVALID, "rejection samplers need a generator state");
     const int P = (dp.dtype == GR_F32) ? 8 : 4;
     const int rk = reject_code(dp);
     const int64_t wt = rk == 0 ? 24 : (rk >= 3 ? 8 : 16);  // words per trial
     const int64_t npk = nk_max / P;
     const int64_t max_blocks = block_cap(((16 * npk + 4096) * wt) / (kN * 8) + 64);
     if (npk > reject_from(rk, dp.dtype == GR_F64, e->K))
-      return run_reject_call(e, p, dp, rk, npk, max_blocks, stream);
+      return run_reject_call(e, p, dp, rk, npk, max_blocks, stream, want);
+    if (want) return GR_OK;
     double slack = 0;
     // (the integer samplers' with a margin: their batches are short)
     const float per_packet = (float)((rk <= 2 ? 1.0 : 1.2) / expected_yield(rk, dp, slack));
@@ -1272,7 +1299,7 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
       wd.ic = dp.kind == GR_BINOMIAL ? dp.ib : 0;
       max_blocks = block_cap((npk * 64) / (2 * kN) + 64);
       if (e->K <= 256 && npk > 100 && npk > poisson_from(poisson_step_halves(wd.fe), e->K))
-        return run_poisson_call(e, p, wd, npk, max_blocks, stream);
+        return run_poisson_call(e, p, wd, npk, max_blocks, stream, want);
     } else {
       const bool f32 = dp.dtype == GR_F32;
       wd.ia = gamma_branch(dp.da, f32);
@@ -1281,8 +1308,9 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
       wd.fb = (float)dp.db;
       max_blocks = (npk * 64) / kN + 64;
       if (e->K <= 256 && (double)npk * chain_packets(wd) > (double)chain_from(wd.ia >> 8, wd.ib >> 8, !f32, e->K))
-        return run_chain_call(e, p, wd, npk, block_cap(max_blocks), stream);
+        return run_chain_call(e, p, wd, npk, block_cap(max_blocks), stream, want);
     }
+    if (want) return GR_OK;
     max_blocks = block_cap(max_blocks);
     cudaError_t err = launch_walk(p, wd, max_blocks, stream);
     if (err != cudaSuccess) return cuda_fail(err, "walk sampling kernel");
@@ -1302,12 +1330,13 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
     auto packets = [&](int64_t cnt) { return half ? (cnt * U + 1) / 2 : cnt * U; };
     size_t bytes = 0;
     const int64_t chunk = fit_chunk(
-        e, std::min(std::max<int64_t>(kStagedCap / e->K / per_u, 1), units), 1,
+        e, std::min(std::max<int64_t>(kStagedCap / e->K / per_u, 1), units), units_from(dp, (int)U, e->K) + 1,
         [&](int64_t c) {
           return std::max(words_bytes(e->K, packets(c)), words_bytes(e->K, packets(last_chunk(units, c))));
         },
         &bytes);
-    if (char* buf = chunk ? scratch_alloc(bytes, e->device, stream) : nullptr) {
+    if (want) *want = chunk ? bytes : 0;
+    if (char* buf = chunk && !want ? scratch_alloc(bytes, e->device, e->scratch_pool, stream) : nullptr) {
       gr_status st = GR_OK;
       for (int64_t u0 = 0; st == GR_OK && u0 < units; u0 += chunk) {
         const int64_t cnt = std::min(chunk, units - u0);
@@ -1320,6 +1349,7 @@ gr_status run_packets(gr_engine* e, gr_gen* g, const DistParams& dp, void* out, 
       return st;
     }
   }
+  if (want) return GR_OK;
   const cudaError_t err = launch_staged(p, dp, nullptr, U, 0, units, stream);
   if (err != cudaSuccess) return cuda_fail(err, "staged sampling kernel");
   return GR_OK;
@@ -2114,14 +2144,33 @@ void gamma_rows_free(GammaRows& rows) {
 // ---- engine scratch reservation (serving loop) -------------------------------
 namespace gr {
 
-// Allocates the scratch a segmented call may need (prefix, call snapshot,
-// windows for up to max_segments segments, the temporary-generator caches), so
-// that later calls on this engine allocate nothing.
+// Allocates what an engine owns and makes only when a call needs it: the prefix and the
+// windows of a call that runs in segments without words in memory (engine_scratch: no
+// memory for them), the caches of temporary generators.
 gr_status engine_reserve(gr_engine* e, int max_segments) {
   gr_status st = reserve_windows(e, std::max(max_segments, 2));
   if (st != GR_OK) return st;
   if (!e->scratch_gen) GR_CUDA(cudaMalloc(&e->scratch_gen, sizeof(GenState) * (size_t)e->K));
   return GR_OK;
+}
+
+// Bytes of scratch that gr_sample of n values takes where it may have all it asks for.
+size_t sample_scratch(gr_engine* e, const gr_dist_desc& desc, size_t n) {
+  DistParams dp;
+  if (make_params(desc, dp) != GR_OK) return 0;  // the call will say so
+  const size_t cap = e->scratch_cap;
+  e->scratch_cap = SIZE_MAX;
+  size_t want = 0;
+  n -= n % (size_t)kind_granule(dp.kind, dp.dtype);
+  const gr_status st = run_packets(e, nullptr, dp, e->st, n, nullptr, &want);
+  e->scratch_cap = cap;
+  return st == GR_OK ? want : 0;
+}
+
+// The engine's calls take their scratch from `pool`, `cap` bytes at most.
+void engine_scratch(gr_engine* e, cudaMemPool_t pool, size_t cap) {
+  e->scratch_pool = pool;
+  e->scratch_cap = cap;
 }
 
 }  // namespace gr

@@ -144,8 +144,12 @@ gr_status build_discrete_table(const std::vector<double>& w, std::vector<int32_t
 // Host side (gr_api.cu): plans and launches k_multinomial on an engine, with
 // the same slice / jump-segment split as the fixed-consumption samplers.
 gr_status run_multinomial(gr_engine* e, GenState* gst, const MnArgs& a, int64_t samples, cudaStream_t s);
-// Host side (gr_api.cu): pre-allocates an engine's segmented-call scratch.
+// Host side (gr_api.cu): allocates what the engine owns and a call may need; the
+// scratch of a gr_sample call; where an engine's calls take it from, and how much
+// at most (a call that may have less takes it in smaller chunks, or does without).
 gr_status engine_reserve(gr_engine* e, int max_segments);
+size_t sample_scratch(gr_engine* e, const gr_dist_desc& desc, size_t n);
+void engine_scratch(gr_engine* e, cudaMemPool_t pool, size_t cap);
 // Host side (gr_mvapi.cu): a second MvNormalGen with the same mean and factor
 // (no refactorisation) and its own StdNormalGen.
 gr_status mvnormal_clone(const gr_mvnormal* src, gr_mvnormal** out);

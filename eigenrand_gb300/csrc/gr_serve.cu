@@ -3,8 +3,9 @@
 // Host-side scheduler only: requests are admitted by gr::Admission (arrival
 // order, one request per client at a time, device-memory budget, stream
 // slots), launched on a free slot's stream through the library's own C ABI,
-// and harvested by polling one event per slot.  Outputs come from a
-// stream-ordered memory pool reserved for the server.
+// and harvested by polling one event per slot.  Outputs and the scratch of the
+// calls come from a stream-ordered memory pool reserved for the server, and both
+// count against the budget.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -41,7 +42,9 @@ struct ServeReq {
   uint64_t gen = 0;   // scalars generated (count rounded up)
   uint64_t units = 0; // value passed to the sampling call (samples for MvNormal)
   size_t bytes = 0;
-  size_t charged = 0;  // bytes held in the admission budget (from admission to release)
+  size_t scratch = 0;  // bytes of scratch its call asks for; from admission: may take
+  size_t charged = 0;  // bytes held in the admission budget (from admission: the scratch until the
+                       // call has run, the output until the release)
   void* dev_out = nullptr;
   int slot = -1;
   int state = kQueued;
@@ -114,7 +117,7 @@ gr_status gr_server_create(gr_server** out, int32_t nclients, const uint64_t* se
     st = gr_engine_create(&e, seeds[c], 4, 1);
     if (st == GR_OK) {
       s->eng.push_back(e);
-      st = engine_reserve(e, 128);  // segmented calls then allocate nothing
+      st = engine_reserve(e, 128);  // a call's scratch is then all it allocates
     }
   }
   int dev = 0;
@@ -197,15 +200,25 @@ gr_status gr_server_submit(gr_server* s, const gr_request* r, uint64_t* ticket) 
     q.gen = (r->count + P - 1) / P * P;
     q.units = q.gen;
     q.bytes = q.gen * elem_bytes(r->dtype);
-    // data-dependent samplers also take transient scratch (the FIFO lane
-    // buffer and packet positions of a segmented call): budget 1.5x more
+    // the result of a data-dependent sampler keeps 1.5x more (the room that its
+    // scratch once had: which requests fit a budget stays as it was)
     const int k = r->kind;
     if (k == GR_GAMMA || k == GR_BETA || k == GR_POISSON || k == GR_BINOMIAL || k == GR_CHI_SQUARED ||
         k == GR_STUDENT_T)
       q.bytes += q.bytes + q.bytes / 2;
   }
+  // the call's scratch, all that it asks for or what the budget leaves for it
+  if (q.bytes <= s->adm->budget()) {
+    gr_dist_desc d{};
+    d.kind = r->kind == GR_SERVE_MVNORMAL ? (int32_t)GR_NORMAL_STD : r->kind;
+    d.dtype = r->kind == GR_SERVE_MVNORMAL ? (int32_t)GR_F32 : r->dtype;
+    d.a = r->a;
+    d.b = r->b;
+    d.trials = r->trials;
+    q.scratch = std::min(sample_scratch(s->eng[r->client], d, q.gen), s->adm->budget() - q.bytes);
+  }
   q.ticket = s->next_ticket++;
-  if (!s->adm->submit(AdmitReq{q.ticket, r->client, q.bytes, q.r.arrival}))
+  if (!s->adm->submit(AdmitReq{q.ticket, r->client, q.bytes, q.r.arrival, q.scratch}))
     return sfail(GR_ERR_NOMEM, "request larger than the server's memory budget");
   *ticket = q.ticket;
   s->reqs.emplace(q.ticket, q);
@@ -223,6 +236,8 @@ gr_status gr_server_progress(gr_server* s, gr_completion* done, size_t cap, size
     ServeReq& q = s->reqs[t];
     q.completed = gr_server_now();
     q.state = kDone;
+    s->adm->release(q.scratch);
+    q.charged -= q.scratch;
     if (e != cudaSuccess) q.status = sfail(GR_ERR_CUDA, std::string("request: ") + cudaGetErrorString(e));
     if (q.cancelled) {  // its work is done: the result goes straight back
       q.status = GR_ERR_CANCELLED;
@@ -248,7 +263,8 @@ gr_status gr_server_progress(gr_server* s, gr_completion* done, size_t cap, size
     cudaStream_t st = s->streams[slot];
     q.slot = slot;
     q.admitted = now;
-    q.charged = q.bytes;
+    q.scratch = a.scratch;
+    q.charged = q.bytes + q.scratch;
     gr_status rs = GR_OK;
     if (s->fail_allocs > 0) {
       --s->fail_allocs;
@@ -262,6 +278,7 @@ gr_status gr_server_progress(gr_server* s, gr_completion* done, size_t cap, size
     if (rs == GR_OK) {
       s->held += q.bytes;
       gr_engine* e = s->eng[q.r.client];
+      engine_scratch(e, s->pool, q.scratch);
       if (q.r.kind == GR_SERVE_MVNORMAL) {
         rs = gr_mvnormal_sample(s->mv[q.r.client], e, q.dev_out, q.units, st);
       } else {
@@ -279,6 +296,8 @@ gr_status gr_server_progress(gr_server* s, gr_completion* done, size_t cap, size
       q.status = rs;
       q.state = kDone;
       q.completed = gr_server_now();
+      s->adm->release(q.scratch);
+      q.charged -= q.scratch;
       s->free_slots.push_back(slot);
       s->adm->finish(q.r.client);
       s->done.push_back(q.ticket);
@@ -383,6 +402,14 @@ gr_status gr_server_cancel_client(gr_server* s, int32_t client) {
 gr_status gr_server_fail_allocs(gr_server* s, int32_t n) {
   if (!s || n < 0) return sfail(GR_ERR_INVALID, "bad argument");
   s->fail_allocs = n;
+  return GR_OK;
+}
+
+gr_status gr_server_memory(const gr_server* s, size_t* most) {
+  if (!s || !most) return sfail(GR_ERR_INVALID, "NULL argument");
+  uint64_t high = 0;
+  SV_CUDA(cudaMemPoolGetAttribute(s->pool, cudaMemPoolAttrUsedMemHigh, &high));
+  *most = (size_t)high;
   return GR_OK;
 }
 

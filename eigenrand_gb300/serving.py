@@ -105,3 +105,9 @@ class Server:
         q, r, b = ctypes.c_size_t(), ctypes.c_size_t(), ctypes.c_size_t()
         _lib.check(_L.gr_server_pending(self._h, ctypes.byref(q), ctypes.byref(r), ctypes.byref(b)))
         return q.value, r.value, b.value
+
+    def memory(self):
+        """The most device memory that results and scratch have had at a time, bytes."""
+        m = ctypes.c_size_t()
+        _lib.check(_L.gr_server_memory(self._h, ctypes.byref(m)))
+        return m.value

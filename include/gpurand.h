@@ -344,7 +344,9 @@ gr_status gr_truncmvn_destroy(gr_truncmvn* g);
  * this is the request loop the sampling path is deployed behind.  Each client
  * owns a device-resident Vmt19937_64 (streams = 1) seeded by the caller.
  * Requests of mixed kinds and sizes queue in arrival order and are admitted
- * while stream slots are free and their output fits the device-memory budget;
+ * while stream slots are free and their output and the scratch of their call fit
+ * the device-memory budget (with nothing else running, a call gets what is left for
+ * its scratch and runs in smaller steps);
  * admitted requests run concurrently on the GPU and complete out of order.  A
  * client's requests run one at a time, in submission order, so every result
  * equals that client's plain call sequence run alone: gr_sample (a fresh
@@ -401,6 +403,8 @@ gr_status gr_server_cancel_client(gr_server* s, int32_t client);
  * runs for them and the client's engine is not advanced) */
 gr_status gr_server_fail_allocs(gr_server* s, int32_t n);
 gr_status gr_server_pending(const gr_server* s, size_t* queued, size_t* running, size_t* bytes_held);
+/* the most device memory that results and scratch have had at a time, bytes */
+gr_status gr_server_memory(const gr_server* s, size_t* most);
 double gr_server_now(void);
 gr_status gr_server_destroy(gr_server* s);
 
