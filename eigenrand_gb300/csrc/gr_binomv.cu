@@ -49,10 +49,10 @@ __device__ __forceinline__ bool bv_trial(const BvLane& L, uint32_t w1, uint32_t 
   const float ys = sn / cs;
   fres = truncf(L.sqrt_v * ys + L.mean);
   const float p1 = ((float)1.2 * L.sqrt_v) * (1.0f + ys * ys);
-  float t = (L.g1 - lgamma_approxf_(fres + 1.0f)) - lgamma_approxf_((L.ptrials + 1.0f) - fres);
+  float t = (L.g1 - lgamma_approxf_<true>(fres + 1.0f)) - lgamma_approxf_<true>((L.ptrials + 1.0f) - fres);
   t = t + fres * L.lsp;
   t = t + (L.ptrials - fres) * L.lsq;
-  const float p2 = expf_(t);
+  const float p2 = expf_<true>(t);
   const float u2 = bv_ur(w2);
   return (0.0f <= fres) && (fres <= L.ptrials) && (u2 <= p1 * p2);
 }
@@ -179,10 +179,10 @@ __device__ __forceinline__ int64_t bv_chain(Src& src, const BinomVArgs& a, int64
     }
     const float spg = pvg < 1.0f - pvg ? pvg : 1.0f - pvg;  // pmin(p, 1 - p)
     const float meang = (float)trg * spg;
-    const float g1g = lgamma_approxf_((float)trg + 1.0f);
+    const float g1g = lgamma_approxf_<true>((float)trg + 1.0f);
     const float svg = sqrtf((2.0f * meang) * (1.0f - spg));
     const float lspg = logf_(spg), lsqg = logf_(1.0f - spg);
-    const float neg = expf_(-meang);
+    const float neg = expf_<true>(-meang);
     const int kend = npk - e0 < 8 ? (int)(npk - e0) : 8;
     for (int kk = 0; kk < kend; ++kk) {
       src.mark();
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(32) k_int_words(const uint64_t* w, int64_t nwo
           if (src.abort) break;
           const float yx = ys / yc;
           const float xx = d.fc * yx + d.fd;
-          const float ub = (yx * yx + 1.0f) * expf_(d.fd * logf_(xx / d.fd) - yx * d.fc);
+          const float ub = (yx * yx + 1.0f) * expf_<true>(d.fd * logf_(xx / d.fd) - yx * d.fc);
           uint32_t rb;
           if (compress(f2u(d.fb * xx), (0.0f < xx) && (ux <= ub), rb)) {
             mean = u2f(rb);
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(32) k_int_words(const uint64_t* w, int64_t nwo
         }
       }
       if (!src.abort) {
-        const float pne = expf_(-mean);
+        const float pne = expf_<true>(-mean);
         if (mask4(12.0f < mean) == 0) {
           float val = 1.0f;
           for (;;) {
@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(32) k_int_words(const uint64_t* w, int64_t nwo
             r += c ? 1 : 0;
           }
         } else {
-          const float sq = sqrtf(2.0f * mean), lm = logf_(mean), g1 = mean * lm - lgamma_approxf_(mean + 1.0f);
+          const float sq = sqrtf(2.0f * mean), lm = logf_(mean), g1 = mean * lm - lgamma_approxf_<true>(mean + 1.0f);
           for (;;) {
             float s2, c2;
             sincosf_(fpi * bv_ur(src.next()), s2, c2);
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(32) k_int_words(const uint64_t* w, int64_t nwo
             const float p1 = (yx * yx + 1.0f) * 0.9f;
             const float u2 = bv_ur(src.next());
             if (src.abort) break;
-            const float p2 = expf_((fres * lm - lgamma_approxf_(fres + 1.0f)) - g1);
+            const float p2 = expf_<true>((fres * lm - lgamma_approxf_<true>(fres + 1.0f)) - g1);
             uint32_t rb;
             if (compress(f2u(fres), (0.0f <= fres) && (u2 <= p1 * p2), rb)) {
               r = cvtt_f32(u2f(rb));
@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(32) k_int_words(const uint64_t* w, int64_t nwo
           const float yx = sn / cs2;
           fres = truncf(d.fa * yx + d.fb);  // sqrt(2 mean) * yx + mean
           const float p1 = (yx * yx + 1.0f) * 0.9f;
-          const float p2 = expf_((fres * d.fc - lgamma_approxf_(fres + 1.0f)) - d.fd);
+          const float p2 = expf_<true>((fres * d.fc - lgamma_approxf_<true>(fres + 1.0f)) - d.fd);
           acc = (0.0f <= fres) && (bv_ur(w2) <= p1 * p2);
         }
         uint32_t rb;

@@ -32,21 +32,48 @@ __device__ __forceinline__ double u2d(uint64_t u) { return __longlong_as_double(
 
 // NORMAL: x is known to be a positive normal number.  The exponent e and the
 // bits of m come from the distance to sqrt(1/2)'s bits.
-template <bool NORMAL = false>
+// SERIAL (also expf_): the special cases tested one by one and the exponent found
+// by comparing, rather than behind one test and from one subtraction.  The same
+// values; a kernel of one warp per engine is bound by the latency of its chain,
+// which can be shorter so, where those bound by issue gain up to 8 % from fewer
+// operations.  2^22 values on 608 engines, us: negative binomial of 5 trials 2 989
+// with the serial exponential, 3 120 without; per-element binomial 2 252 with both
+// (the logarithm that of its lgamma), 2 316 with the exponential alone.
+template <bool NORMAL = false, bool SERIAL = false>
 __device__ __forceinline__ float logf_(float x) {
   uint32_t ux = f2u(x);
   int e = 0;
-  if (!NORMAL && ux - 0x00800000u >= 0x7f000000u) {  // not a positive normal number
+  float f;
+  if (SERIAL) {
     if (x != x) return x;
     if (x < 0.0f) return u2f(0x7fc00000u);
     if (x == 0.0f) return -__int_as_float(0x7f800000);
     if (ux == 0x7f800000u) return x;
-    ux = f2u(x * 8388608.0f);
-    e = -23;
+    if (ux < 0x00800000u) {
+      ux = f2u(x * 8388608.0f);
+      e = -23;
+    }
+    e += (int)((ux >> 23) & 0xff) - 126;
+    const float m = u2f((ux & 0x007fffffu) | 0x3f000000u);
+    if (m < 0.70710678118654752f) {
+      e -= 1;
+      f = (m + m) - 1.0f;
+    } else {
+      f = m - 1.0f;
+    }
+  } else {
+    if (!NORMAL && ux - 0x00800000u >= 0x7f000000u) {  // not a positive normal number
+      if (x != x) return x;
+      if (x < 0.0f) return u2f(0x7fc00000u);
+      if (x == 0.0f) return -__int_as_float(0x7f800000);
+      if (ux == 0x7f800000u) return x;
+      ux = f2u(x * 8388608.0f);
+      e = -23;
+    }
+    const int k = (int)(ux - 0x3f3504f3u) >> 23;  // 0x3f3504f3: sqrt(1/2)
+    e += k;
+    f = u2f(ux - ((uint32_t)k << 23)) - 1.0f;
   }
-  const int k = (int)(ux - 0x3f3504f3u) >> 23;  // 0x3f3504f3: sqrt(1/2)
-  e += k;
-  const float f = u2f(ux - ((uint32_t)k << 23)) - 1.0f;
   float z = f * f;
   float p = 7.149753720e-02f;
   p = fmaf(p, f, -1.157120094e-01f);
@@ -66,8 +93,9 @@ __device__ __forceinline__ float logf_(float x) {
   return r;
 }
 
+template <bool SERIAL = false>
 __device__ __forceinline__ float expf_(float x) {
-  const bool wide = !(fabsf(x) <= 87.0f);  // beyond, 2^n leaves the normal range (or x is NaN)
+  const bool wide = SERIAL || !(fabsf(x) <= 87.0f);  // beyond, 2^n leaves the normal range (or x is NaN)
   if (wide) {
     if (x != x) return x;
     if (x > 88.72283935546875f) return __int_as_float(0x7f800000);
@@ -221,13 +249,14 @@ __device__ __forceinline__ double erfinv_(double x) {
   return p * x;
 }
 
+template <bool SERIAL = false>
 __device__ __forceinline__ float lgamma_approxf_(float x) {
   float x_3 = x + 3.0f;
-  float ret = (x_3 + -0.5f) * logf_(x_3);
+  float ret = (x_3 + -0.5f) * logf_<false, SERIAL>(x_3);
   ret = ret - x_3;
   ret = ret + (float)0.9189385332046727;
   ret = ret + (float)(1 / 12.) / x_3;
-  ret = ret - logf_(((x_3 - 1.0f) * (x_3 - 2.0f)) * x);
+  ret = ret - logf_<false, SERIAL>(((x_3 - 1.0f) * (x_3 - 2.0f)) * x);
   return ret;
 }
 

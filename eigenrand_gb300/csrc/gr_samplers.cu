@@ -1678,7 +1678,7 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_negbin(Plan p, DistParams d, 
         if (abort) break;
         const float yx = ys / yc;
         const float xx = gsq * yx + a1;
-        const float ub = (yx * yx + 1.0f) * expf_(a1 * logf_(xx / a1) - yx * gsq);
+        const float ub = (yx * yx + 1.0f) * expf_<true>(a1 * logf_(xx / a1) - yx * gsq);
         uint32_t r;
         if (compress(f2u(beta * xx), (0.0f < xx) && (ux <= ub), r)) {
           mean = u2f(r);
@@ -1687,7 +1687,7 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_negbin(Plan p, DistParams d, 
       }
     }
     if (abort) break;
-    const float pne = expf_(-mean);
+    const float pne = expf_<true>(-mean);
     if (mask4(12.0f < mean) == 0) {
       float val = 1.0f;
       int32_t res = 0;
@@ -1710,7 +1710,7 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_negbin(Plan p, DistParams d, 
         const float p1 = (yx * yx + 1.0f) * 0.9f;
         const float u2 = ur_f(next());
         if (abort) break;
-        const float p2 = expf_((fres * lm - lgamma_approxf_(fres + 1.0f)) - g1);
+        const float p2 = expf_<true>((fres * lm - lgamma_approxf_(fres + 1.0f)) - g1);
         uint32_t r;
         if (compress(f2u(fres), (0.0f <= fres) && (u2 <= p1 * p2), r)) {
           if (lane < 4) out[e * 4 + lane] = cvtt_f32(u2f(r));
