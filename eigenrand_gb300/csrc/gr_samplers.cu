@@ -984,12 +984,14 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
   // block 0 and its masks (all threads)
   mt_block(raw[2], raw[0], [&](int, const uint64_t*) {});
   set_ring(0);
-  // (ONE: a short call's, no more than it should need)
+  // (ONE: a short call's, no more than it should need; up to 16 outputs go without
+  // look-ups)
+  const bool looks = ONE && Npk > 16;
   int64_t M = kN - umax + 1;  // positions with masks
-  if (ONE) M = min(M, 16 * Ur + 32 + (Uc + 3 * Ur) * min(Npk, (int64_t)kN));
+  if (ONE) M = min(M, (looks ? 16 * Ur : 0) + 32 + (Uc + 3 * Ur) * min(Npk, (int64_t)kN));
   masks(0, M, tid, NT);
   __syncthreads();
-  if (ONE) {
+  if (looks) {
     build(0, M - 16 * Ur, tid, NT);
     __syncthreads();
   }
@@ -1024,7 +1026,7 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
           const int64_t rest = Npk - cE;
           const int pkr = (int)(pk_lim - base), left = (int)min(rest, (int64_t)kBcRec);
           int xr = 0, f = cf[rc], At = f;
-          while (nrec < left) {
+          while (looks && nrec < left) {
             const int xt = rc == 0 ? xr : xr + Uc;
             if (xt >= Mr - 16 * Ur || At + 2 * P > LB || nf >= kBcFull) break;
             const uint32_t v = visits[((bm + xt) & (kBetaRing - 1)) * P + f];
@@ -1294,7 +1296,7 @@ __global__ void __maxnreg__(80) k_beta(Plan p, BetaConsts bk, int64_t max_blocks
         set_ring(t + 1);
         const int64_t M1 = (t + 2) * kN - umax + 1;
         masks(M, M1, tt, kBcWork);
-        if (ONE) {
+        if (looks) {
           asm volatile("bar.sync 1, %0;" ::"r"(kBcWork) : "memory");
           build(M - 16 * Ur, M1 - 16 * Ur, tt, kBcWork);
         }
