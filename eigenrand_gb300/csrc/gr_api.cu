@@ -806,9 +806,13 @@ int64_t words_from(const DistParams& dp, int K) {
   const bool light = k == kRawKind || k == kRawLane0Kind || k == GR_UNIFORM_REAL || k == GR_UNIFORM_REAL2 ||
                      (balanced && !f64) || k == GR_BERNOULLI || k == kBernoulliVKind || k == GR_RANDBITS ||
                      k == GR_UNIFORM_INT;
-  if (light) return K > 64 ? kNever : f64 ? 3600 + 64 * K : 5000 + 180 * K;
+  // per-element calls are bound by the host up to twice the size (their arrays are
+  // looked at first), and more launches cost it more: normal(mean, stdev) of 2 048
+  // packets from Python 32.6 us in one launch, 35.0 through memory
+  const int per_element = dp.kind >= kVecBase ? 2 : 1;
+  if (light) return K > 64 ? kNever : per_element * (f64 ? 3600 + 64 * K : 5000 + 180 * K);
   if (K > 127) return kNever;
-  return f64 && !balanced ? 450 + 5 * K / 2 : 1500 + 16 * K;
+  return per_element * (f64 && !balanced ? 450 + 5 * K / 2 : 1500 + 16 * K);
 }
 
 // Units per engine above which a call of fixed units of U packets (half packets for the
