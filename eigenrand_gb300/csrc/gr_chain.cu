@@ -528,6 +528,8 @@ __global__ void __launch_bounds__(32) k_chain_walk(ChainArgs a) {
 }
 
 // ---------------------------------------------------------------- scan
+// A0, A1: the components whose outputs add to carried lanes.
+template <bool A0, bool A1>
 __global__ void __launch_bounds__(1024) k_chain_scan(ChainArgs a) {
   __shared__ int64_t s_tot[32];
   __shared__ int s_top[2][32];
@@ -552,10 +554,10 @@ __global__ void __launch_bounds__(1024) k_chain_scan(ChainArgs a) {
     int64_t x = v;
     int top[2];  // the last segment up to this one with an output that adds, plus 1
 #pragma unroll
-    for (int c = 0; c < 2; ++c) top[c] = (s < Sg && seg[s].adds[c]) ? s + 1 : 0;
+    for (int c = 0; c < 2; ++c) top[c] = ((c ? A1 : A0) && s < Sg && seg[s].adds[c]) ? s + 1 : 0;
     for (int o = 1; o < 32; o <<= 1) {
       const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
-      const int t0 = __shfl_up_sync(0xffffffffu, top[0], o), t1 = __shfl_up_sync(0xffffffffu, top[1], o);
+      const int t0 = A0 ? __shfl_up_sync(0xffffffffu, top[0], o) : 0, t1 = A1 ? __shfl_up_sync(0xffffffffu, top[1], o) : 0;
       if ((tid & 31) >= o) {
         x += y;
         top[0] = max(top[0], t0);
@@ -574,7 +576,7 @@ __global__ void __launch_bounds__(1024) k_chain_scan(ChainArgs a) {
       int p0 = have ? s_top[0][tid] : 0, p1 = have ? s_top[1][tid] : 0;
       for (int o = 1; o < 32; o <<= 1) {
         const int64_t y = __shfl_up_sync(0xffffffffu, t, o);
-        const int t0 = __shfl_up_sync(0xffffffffu, p0, o), t1 = __shfl_up_sync(0xffffffffu, p1, o);
+        const int t0 = A0 ? __shfl_up_sync(0xffffffffu, p0, o) : 0, t1 = A1 ? __shfl_up_sync(0xffffffffu, p1, o) : 0;
         if (tid >= o) {
           t += y;
           p0 = max(p0, t0);
@@ -590,13 +592,17 @@ __global__ void __launch_bounds__(1024) k_chain_scan(ChainArgs a) {
     int before[2];
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
+      if (!(c ? A1 : A0)) {
+        before[c] = 0;
+        continue;
+      }
       const int up = __shfl_up_sync(0xffffffffu, top[c], 1);
       before[c] = max(max(s_last[c], (tid >> 5) ? s_top[c][(tid >> 5) - 1] : 0), (tid & 31) ? up : 0);
     }
     if (s < Sg) {
       eb[s] = incl - v;
-      seg[s].prev[0] = before[0];
-      seg[s].prev[1] = before[1];
+      if (A0) seg[s].prev[0] = before[0];
+      if (A1) seg[s].prev[1] = before[1];
     }
     __syncthreads();
     if (tid == (int)blockDim.x - 1) {
@@ -661,17 +667,18 @@ __device__ __forceinline__ int draw_start(const ChainArgs& a, int k, int c, bool
 
 // The lane `dist` places before the end of component c's FIFO as it is before
 // output i of segment s: position and lane of its trial (kEntInit: a lane
-// carried into the call).  From one output that adds lanes to the one before it:
-// output by output, the last lanes of a shape whose trials nearly all are fully
-// accepted took milliseconds.
+// carried into the call).  A few outputs back one by one, where ordinary shapes find
+// it, then from one output that adds lanes to the one before it: output by output all
+// the way, the last lanes of a shape whose trials nearly all are fully accepted took
+// milliseconds.
 template <int DT>
 __device__ __forceinline__ void carried_lane(const ChainArgs& a, int k, int c, bool R0, bool R1, int s, int64_t i, int dist,
                                              uint32_t& pos, int& lane) {
   const Visits v = visits_of<DT>(a, k, c, R0, R1);
   const ChainSeg* seg = a.seg + (size_t)k * a.L.Sg;
   const uint16_t* prev = a.prev + (c == 1 && R0 ? (size_t)a.p.K * a.L.Sg * a.L.rcap : 0) + (size_t)k * a.L.Sg * a.L.rcap;
-  int q = i < seg[s].nrec ? prev[(size_t)s * a.L.rcap + i] : seg[s].adds[c];
-  for (;;) {
+  int q = (int)i;  // the output looked at next, plus 1
+  for (int back = 0;; ++back) {
     if (q == 0) {
       s = seg[s].prev[c] - 1;
       if (s < 0) {
@@ -691,7 +698,7 @@ __device__ __forceinline__ void carried_lane(const ChainArgs& a, int k, int c, b
       return;
     }
     dist -= pushed;
-    q = prev[at];
+    q = back < 4 ? q - 1 : prev[at];
   }
 }
 
@@ -1006,7 +1013,7 @@ cudaError_t run_core(const ChainArgs& a, cudaStream_t s) {
     k_chain_compose<P, R0, R1><<<dim3(a.L.groups, K), 512, csm, s>>>(a, 0);
   }
   k_chain_walk<P, R0, R1><<<(unsigned)(K * Sg), 32, (size_t)2 * NR * (kTile + kPad) * P, s>>>(a);
-  k_chain_scan<<<K, Sg > 256 ? 1024 : 256, 0, s>>>(a);
+  k_chain_scan<R0 && (P > 1), R1><<<K, Sg > 256 ? 1024 : 256, 0, s>>>(a);
   return cudaGetLastError();
 }
 
