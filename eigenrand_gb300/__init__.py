@@ -53,8 +53,8 @@ def version():
 
 
 # A small call is bound by its host path, so that path stays short (32 x 32
-# floats, us a call: 20.9 with a Stream object, an empty and a transposed tensor,
-# a descriptor filled field by field and c_void_p objects; 7.4 as here).
+# floats, us a call: 20.0 with a Stream object, an empty and a transposed tensor,
+# a descriptor filled field by field and c_void_p objects; 9.6 as here).
 _CUDA = torch.device("cuda")
 
 

@@ -955,7 +955,7 @@ size_t chunks_bytes(int K, int64_t left, int64_t chunk, int64_t again, Next&& ne
 constexpr int64_t kPoisCap = (int64_t)1 << 22;  // packets of words at a time, all engines
 gr_status run_poisson_call(gr_engine* e, const Plan& p0, const DistParams& wd, int64_t npk, int64_t max_blocks,
                            cudaStream_t stream, size_t* want = nullptr) {
-  const char* sc = std::getenv("GR_WALK_PLAN_SCALE");  // tests: see run_chain_call
+  const char* sc = std::getenv("GR_WALK_PLAN_SCALE");  // tests: as in run_chain_call
   const double scale = sc ? std::max(0.0, std::atof(sc)) : 1.0;
   const double hl = poisson_step_halves(wd.fe);
   int64_t left = (int64_t)std::ceil(((double)npk + 4.0 * std::sqrt((double)npk)) * hl * 0.5 * 1.03 * scale) + 64;
@@ -1095,7 +1095,9 @@ gr_status run_chain_call(gr_engine* e, const Plan& p0, const DistParams& wd, int
                          cudaStream_t stream, size_t* want = nullptr) {
   const int br[2] = {wd.ia, wd.ib};
   const double per = chain_packets(wd);
-  const char* sc = std::getenv("GR_WALK_PLAN_SCALE");  // tests: see run_packets
+  // GR_WALK_PLAN_SCALE (tests) scales the planned packets; below 1 the one-CTA kernel
+  // makes the rest, which must give the same result
+  const char* sc = std::getenv("GR_WALK_PLAN_SCALE");
   const double scale = sc ? std::max(0.0, std::atof(sc)) : 1.0;
   const bool closed = (br[0] >> 8) < 2 && (br[1] >> 8) < 2;
   int64_t left = (int64_t)std::ceil(per * ((double)npk + (closed ? 0.0 : 8.0 * std::sqrt((double)npk))) * scale) + 64;

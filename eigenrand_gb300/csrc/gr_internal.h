@@ -8,7 +8,6 @@ namespace gr {
 constexpr int kN = 312;      // MT19937-64 state words
 constexpr int kM = 156;      // MT19937-64 shift
 constexpr int kLanes = 4;    // Vmt19937_64 lanes under AVX2 (Pmt19937_64<Packet8i>)
-constexpr int kPrefix = 20280;  // 65 blocks: >= 19937 + 312 words for a jump
 
 constexpr uint64_t kMatA = 0xb5026f5aa96619e9ull;
 constexpr uint64_t kSeedF = 6364136223846793005ull;

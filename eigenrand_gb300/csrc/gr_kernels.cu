@@ -260,10 +260,10 @@ cudaError_t launch_words(const EngState* st, const GenState* gen, int K, const W
 // terms); its warps split the part, lane q of a warp covers output words
 // [11 q, 11 q + 11) (an odd stride: the 8-byte shared-memory reads are free of
 // bank conflicts).  A thread slides a register window over the prefix words;
-// four coefficients at a time, the same for the whole warp, pick one of 16
-// unrolled cases, in which three-input XORs take 1.25 operations per 32-bit
-// word on average where one conditional XOR per term takes 2.  Parts meet
-// by atomic XOR (segwin zeroed beforehand).  Bound by issue.
+// two coefficients at a time, the same for the whole warp, pick one of four
+// unrolled cases: none, either word, or both in three-input XORs, 0.75 operations
+// per 32-bit word for the two terms on average.  Parts meet by atomic XOR (segwin
+// zeroed beforehand).  Bound by issue.
 constexpr int kJumpThreads = 256;
 constexpr int kJumpOut = 11;
 // PARTS CTAs per segment and lane
@@ -558,7 +558,6 @@ template <int MODE>
 struct ModeInfo {
   static constexpr int OPP = (MODE == M_RAW || MODE == M_RAW0) ? 4 : MODE == M_F32 ? 8 : MODE == M_F64 ? 4 : MODE == M_N32 ? 8 : MODE == M_N64 ? 4
                            : MODE == M_RAW2 ? 2 : MODE == M_F32H ? 4 : MODE == M_F64H ? 2 : 8;
-  static constexpr bool kHalfCache = MODE == M_W64;  // randbits handled separately below
   static constexpr int kCacheOut = MODE == M_N32 ? 8 : MODE == M_N64 ? 4 : (MODE == M_W32 || MODE == M_W64) ? 4 : 0;
 };
 
@@ -721,9 +720,10 @@ __device__ __forceinline__ void emit_half(const uint64_t (&pk)[2], const int h, 
 // double ones by the FP64 and logic pipes together (gr_fp64i.h).  608 engines
 // give an SM four CTAs whatever their size: with a thread per packet (160
 // threads) it held 20 warps, here 40, which also store 512 consecutive bytes at
-// a time.  8192 x 8192 on 608 engines, us, before / now: uniform f32 74.9 / 59.5,
-// discrete 143 / 122, weibull f32 309 / 284, exponential f64 746 / 711, lognormal
-// f64 2 168 / 1 876, weibull f64 2 093 / 1 832.
+// a time.  8192 x 8192 on 608 engines, us, a thread per packet / two, with the other
+// code as it was then: uniform f32 74.9 / 59.5, discrete 143 / 122, weibull f32 309 /
+// 284, exponential f64 746 / 711, lognormal f64 2 168 / 1 876, weibull f64 2 093 /
+// 1 832 (now 57.4, 124, 236, 700, 1 902, 1 809).
 constexpr int kDirThreads = 320;
 
 // Kinds whose transform takes a few operations per word: their loop is unrolled

@@ -260,14 +260,4 @@ __device__ __forceinline__ float lgamma_approxf_(float x) {
   return ret;
 }
 
-__device__ __forceinline__ double lgamma_approx_(double x) {
-  double x_3 = x + 3.0;
-  double ret = (x_3 + -0.5) * log_(x_3);
-  ret = ret - x_3;
-  ret = ret + 0.9189385332046727;
-  ret = ret + (1 / 12.) / x_3;
-  ret = ret - log_(((x_3 - 1.0) * (x_3 - 2.0)) * x);
-  return ret;
-}
-
 }  // namespace gr

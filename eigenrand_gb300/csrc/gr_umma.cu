@@ -694,15 +694,6 @@ __device__ __forceinline__ void mma_tf32_ss(uint32_t dtmem, uint64_t a, uint64_t
       "l"(a), "l"(b), "r"(idesc), "r"(acc));
 }
 
-__device__ __forceinline__ void mma_tf32_ts1(uint32_t dtmem, uint32_t atmem, uint64_t b, uint32_t idesc,
-                                             uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(dtmem),
-      "r"(atmem), "l"(b), "r"(idesc), "r"(acc));
-}
-
 __device__ __forceinline__ void commit1(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
