@@ -29,10 +29,11 @@ def test_host_time(gpulib, kind, lo, hi, t):
         torch.cuda.synchronize()
         return (time.perf_counter() - t0) / len(params)
 
-    fresh = np.linspace(lo, hi, 150)
-    per_call(fresh[:5])
-    new = per_call(fresh[5:])
-    again = per_call(fresh[5:])
+    # the least of several sets: a pause of the host machine counts for one only
+    sets = [np.linspace(lo, hi, 60) + 1e-4 * i for i in range(5)]
+    per_call(sets[0])
+    new = min(per_call(x) for x in sets[1:])
+    again = min(per_call(x) for x in sets[1:])
     assert new < 2 * again + 20e-6
 
 
